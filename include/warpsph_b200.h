@@ -660,6 +660,20 @@ int sph_dfsph_density_solve(const SphParams* p, const SphJacobiConfig* cfg, int6
                             float* p_out, float* accel_out, float* history, int32_t* iterations,
                             int32_t* status, void* stream);
 
+/* Either solve (mode 0: divergence-free, 1: density) with the pair gradients
+ * m_j gradW(x_ij, H_j) computed once and kept for every iteration: the arguments and results
+ * of sph_dfsph_div_solve / sph_dfsph_density_solve, a caller-owned 256-byte aligned buffer of
+ * sph_dfsph_gradient_bytes(n, entries, dim) bytes, and `entries`, the length of `list` that
+ * the rows lie in (max offs + cnt).  Four words per entry in 3D, two in 2D, one in 1D. */
+int64_t sph_dfsph_gradient_bytes(int64_t n, int64_t entries, int32_t dim);
+int sph_dfsph_solve_cached(int32_t mode, const SphParams* p, const SphJacobiConfig* cfg, int64_t n, int64_t entries,
+                           const float* x, const float* H, const float* m, const float* rho,
+                           const float* v, const float* dvdt, const float* p_init, const float* dt,
+                           const int32_t* offs, const int32_t* cnt, const int32_t* list,
+                           void* workspace, int64_t workspace_bytes, void* gradients, int64_t gradient_bytes,
+                           float* p_out, float* accel_out, float* history, int32_t* iterations,
+                           int32_t* status, void* stream);
+
 /* ---------------------------------------------------------------- weakly compressible (delta-SPH) */
 /* EOS (modules/eos/weaklyCompressible.py:4-44), density diffusion terms
  * (enumTypes.py:53-58, DensityDiffusionScheme) and pressure terms (enumTypes.py:60-66). */

@@ -229,3 +229,28 @@ def test_nonfinite_inputs_report_status(cuda):
                                              G["dvdt"], G["p_prev"], 2e-3, adj)
     assert int(st.item()) & 0x2, f"status {int(st.item()):#x}"
     assert int(it.item()) < 32
+
+
+# rows and sizes on both sides of the cached solve's splits: 8 lanes holding 48 entries (up to
+# 4,736 particles), 4 lanes holding 40 (up to 18,944), a loop over particles above
+CACHED = [(1, 37, 1.0), (1, 5000, 6.0), (2, 24, 1.0), (2, 69, 1.4), (2, 97, 1.0), (2, 138, 1.0), (3, 9, 1.0), (3, 15, 1.2), (3, 27, 1.0)]
+
+
+@pytest.mark.parametrize("dim,n_side,h_scale", CACHED)
+@pytest.mark.parametrize("mode", [ops.DIVERGENCE_FREE, ops.DENSITY])
+def test_cached_gradients_match_uncached_solve(cuda, dim, n_side, h_scale, mode):
+    """The solve over cached pair gradients against the one that forms them in every iteration
+    (the same sums in another order: the bound of the oracle comparison at 8 iterations)."""
+    cfg, p, P, G, adj, nb = incompressible_case(dim, n_side, 90 + dim, cuda, h_spread=0.1, h_scale=h_scale)
+    c = jcfg(2, 8, 0.0)
+    args = (G["positions"], G["supports"], G["masses"], G["rho"], G["velocities"], G["dvdt"], G["p_prev"], 2e-3, adj)
+    pr, acc, hist, it, st = ops.jacobi_solve(p, mode, c, *args)
+    keep, ops._gradient_buffer = ops._gradient_buffer, lambda *a: None
+    try:
+        pr0, acc0, hist0, it0, st0 = ops.jacobi_solve(p, mode, c, *args)
+    finally:
+        ops._gradient_buffer = keep
+    assert int(it.item()) == int(it0.item()) == 8 and int(st.item()) == int(st0.item())
+    assert_close(hist.cpu().numpy()[:, :3], hist0.cpu().numpy()[:, :3], 1e-4, 1e-4, "history")
+    assert_close(pr.cpu().numpy(), pr0.cpu().numpy(), 1e-4, 1e-4, "pressure")
+    assert_close(acc.cpu().numpy(), acc0.cpu().numpy(), 1e-4, 1e-4, "pressure acceleration")

@@ -172,10 +172,12 @@ _PROTOS = {
     "sph_mlp_grad_tc": [_P, _I64, _P, _P, _P, _P, _P, _P],
     "sph_mlp_adam": [_P, _P, _P, _P, _I64, C.c_float, C.c_float, C.c_float, C.c_float, _I64, _P],
     "sph_dfsph_div_solve": [_P, _P, _I64] + [_P] * 12 + [_I64] + [_P] * 6,
+    "sph_dfsph_gradient_bytes": [_I64, _I64, _I32],
+    "sph_dfsph_solve_cached": [_I32, _P, _P, _I64, _I64] + [_P] * 12 + [_I64, _P, _I64] + [_P] * 6,
     "sph_dfsph_density_solve": [_P, _P, _I64] + [_P] * 12 + [_I64] + [_P] * 6,
 }
 _RESTYPE = {"sph_version": C.c_char_p, "sph_last_error_string": C.c_char_p, "sph_launch_count": C.c_int64, "sph_launch_count_conditional": C.c_int64,
-            "sph_dfsph_workspace_size": C.c_int64,
+            "sph_dfsph_workspace_size": C.c_int64, "sph_dfsph_gradient_bytes": C.c_int64,
             "sph_mlp_param_count": C.c_int64, "sph_ensemble_neighbors_workspace_size": C.c_int64,
             "sph_ensemble_step_workspace_size": C.c_int64}
 

@@ -109,6 +109,39 @@ __device__ __forceinline__ float shift_partial(int i, int lane, const DevParams&
     return s;
 }
 
+// ---------------------------------------------------------------- cached pair gradients
+// A solve evaluates the same pair gradients m_j gradW(x_ij, H_j) twice per iteration.  The
+// prep pass, which forms them anyway, stores them by row entry and the iterations stream them
+// back: in 3D with the neighbour's index in the fourth word, one 16-byte load per entry.
+// They are read once per phase, so they bypass L1, which is left to the gathers.
+template <int D> constexpr int pair_grad_floats() { return D == 3 ? 4 : D; }
+template <int D> __device__ __forceinline__ void put_pair_grad(float* __restrict__ grads, int k, int j, float mj, const Vec<D>& g) {
+    if constexpr (D == 3)
+        reinterpret_cast<float4*>(grads)[k] = make_float4(mj * g.v[0], mj * g.v[1], mj * g.v[2], __int_as_float(j));
+    else if constexpr (D == 2)
+        reinterpret_cast<float2*>(grads)[k] = make_float2(mj * g.v[0], mj * g.v[1]);
+    else
+        grads[k] = mj * g.v[0];
+}
+template <int D> __device__ __forceinline__ void get_pair_grad(const float* __restrict__ grads, const int32_t* __restrict__ list, int k,
+                                                               int& j, Vec<D>& g) {
+    if constexpr (D == 3) {
+        float4 t;
+        asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+            : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "l"(reinterpret_cast<const float4*>(grads) + k));
+        g.v[0] = t.x; g.v[1] = t.y; g.v[2] = t.z;
+        j = __float_as_int(t.w);
+    } else {
+        j = __ldg(list + k);
+        if constexpr (D == 2) {
+            asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];"
+                : "=f"(g.v[0]), "=f"(g.v[1]) : "l"(reinterpret_cast<const float2*>(grads) + k));
+        } else {
+            g.v[0] = __ldg(grads + k);
+        }
+    }
+}
+
 // ---------------------------------------------------------------- prep: divergence, alpha, source, diagonal
 // mode -1: standalone (div_out and/or alpha_out); 0: divergence-free solve; 1: density solve.
 template <int KF, int D, int G>
@@ -118,7 +151,8 @@ k_dfsph_prep(int n, DevParams P, int mode, float rho0, const float* __restrict__
              const float* __restrict__ dvdt, const float* __restrict__ dtp, const int32_t* __restrict__ offs,
              const int32_t* __restrict__ cnt, const int32_t* __restrict__ list, float* __restrict__ div_out,
              float* __restrict__ alpha_out, const float* __restrict__ p_init, int init_mode, float* __restrict__ src,
-             float* __restrict__ diag, float* __restrict__ p0) {
+             float* __restrict__ diag, float* __restrict__ p0, float* __restrict__ grads = nullptr,
+             float2* __restrict__ pq = nullptr) {
     Grp<G> g(n);
     const bool want_div = div_out || src, want_alpha = alpha_out || diag;
     const float dt = dtp ? *dtp : 0.f;
@@ -144,6 +178,7 @@ k_dfsph_prep(int n, DevParams P, int mode, float rho0, const float* __restrict__
             float W;
             Vec<D> gS, gG;
             kernelWG<KF, D>(xij, r, Hj, W, gS);
+            if (grads) put_pair_grad<D>(grads, k, j, mj, gS);
             if (Hj == Hi) gG = gS; else kernelWG<KF, D>(xij, r, Hi, W, gG);
             if (want_div) {
                 Vec<D> vj = load_vec<D>(v, j);
@@ -187,6 +222,7 @@ k_dfsph_prep(int n, DevParams P, int mode, float rho0, const float* __restrict__
         diag[i] = a > -1e-6f ? -1e-6f : a;
         p0[i] = init_mode ? p_init[i] : 0.f;
     }
+    if (pq) pq[i] = make_float2(p0[i], 1.f / (rho[i] * rho[i]));
 }
 
 // ---------------------------------------------------------------- standalone accel / shift passes
@@ -278,6 +314,7 @@ k_jacobi(JacobiArgs a) {
     const float dtf = a.mode == 0 ? dt : dt * dt;
     JacobiCtl* c = a.ctl;
     float mu = 0.f;
+    unsigned int arrived = 0;
     int it = 0;
     bool converged = false;
 
@@ -310,7 +347,7 @@ k_jacobi(JacobiArgs a) {
             }
         }
         if (converged || it >= a.max_it) break;
-        if (!grid_barrier(&c->bar, a.barrier_ns)) { jacobi_gave_up(a, it); return; }
+        if (!grid_barrier(&c->bar, arrived, a.barrier_ns)) { jacobi_gave_up(a, it); return; }
 
         // ------------------------------------------------ phase B: shift, residual, update
         double psum = 0.0, esum = 0.0;
@@ -354,7 +391,7 @@ k_jacobi(JacobiArgs a) {
             atomicMin(&c->mm[sl][0], lo);
             atomicMax(&c->mm[sl][1], hi);
         }
-        if (!grid_barrier(&c->bar, a.barrier_ns)) { jacobi_gave_up(a, it); return; }
+        if (!grid_barrier(&c->bar, arrived, a.barrier_ns)) { jacobi_gave_up(a, it); return; }
 
         // ------------------------------------------------ decide (identical in every block)
         const int sl = it % 3;
@@ -386,6 +423,222 @@ k_jacobi(JacobiArgs a) {
     }
 }
 
+// The same solve over cached pair gradients g_ij = m_j gradW(x_ij, H_j):
+//   phase A   a_i = -sum_j (p_i / rho_i^2 + p_j / rho_j^2) g_ij
+//   phase B   s_i = -sum_j (1 / rho_j) (a_j - a_i) . g_ij
+// An entry is one streamed load and one gather of the neighbour's (p, 1 / rho^2) or (a, 1 / rho),
+// packed in one word pair or quad, instead of five gathers, a minimum image and a kernel
+// gradient with its divisions.  U entries per lane are loaded together.  The gathered arrays
+// are rewritten by other blocks between the phases: they are read with plain loads, which the
+// acquire of the grid barrier makes current, and so may hit L1.
+//
+// Large solves are bound by the stream of gradients from HBM (16 bytes per entry and phase in
+// 3D): 1,000,000 particles with 40 neighbours take 134 us per phase, 5.0 TB/s of stream, where
+// k_jacobi took 353 us; 4 lanes per particle with 5 entries in flight beat 8 x 4 (149 us) and
+// 16 x 3 (168 us).  Small solves are bound by the latency of a phase and its barrier.  With
+// HOLD a group keeps one particle for the whole solve, its first G * U entries in registers, so
+// a phase is one gather, one reduction and one barrier; more entries are loaded each time.
+// 9,216 particles: 3.7 us per phase and barrier against 4.5 us streaming and 10.8 us in k_jacobi;
+// 4,096 particles in 3D: 160 us a solve of 33 phases with 8 lanes against 182 us with 4 and 197 us
+// streaming.  The blocks' partial sums go to one slot each, which every block adds up after
+// the barrier: four atomics per block on one line cost 144 blocks 1 us per iteration more.
+struct JacobiGradArgs {
+    int n, mode, min_it, max_it;
+    float omega, tol;
+    const float *rho, *src, *diag, *dtp, *grads;
+    const int32_t *offs, *cnt, *list;
+    float2* pq;        // (un-gauged pressure of the last update, 1 / rho^2)
+    float4* a4;        // (pressure acceleration, 1 / rho)
+    struct JacobiSums* sums;   // per block
+    float* p_out;
+    float* acc;
+    float* hist;
+    int32_t* iters_out;
+    int32_t* status_out;
+    JacobiCtl* ctl;
+    unsigned long long barrier_ns;
+};
+template <int D> __device__ __forceinline__ Vec<D> vec_of(const float4& t) {
+    Vec<D> r;
+    r.v[0] = t.x;
+    if constexpr (D > 1) r.v[1] = t.y;
+    if constexpr (D > 2) r.v[2] = t.z;
+    return r;
+}
+
+// Partial sums of one block: sum p, sum of the error term, min p and max p (ordered encoding).
+struct JacobiSums { double p, e; unsigned int lo, hi; };
+// Sums over the block, in a fixed order, returned to every thread.
+template <int BLOCK> __device__ __forceinline__ JacobiSums block_sums(JacobiSums t, JacobiSums* sh) {
+    t.p = warp_sum(t.p); t.e = warp_sum(t.e);
+    t.lo = warp_min_u(t.lo); t.hi = warp_max_u(t.hi);
+    __syncthreads();                              // earlier readers of sh are done
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+    __syncthreads();
+    t = sh[0];
+    #pragma unroll
+    for (int w = 1; w < BLOCK / 32; ++w) { t.p += sh[w].p; t.e += sh[w].e; t.lo = min(t.lo, sh[w].lo); t.hi = max(t.hi, sh[w].hi); }
+    return t;
+}
+
+template <int D, int G, int U, int BLOCK, int MINB, bool HOLD>
+__global__ void __launch_bounds__(BLOCK, MINB)
+k_jacobi_grad(JacobiGradArgs a) {
+    constexpr int PPB = BLOCK / G;
+    __shared__ JacobiSums sh[BLOCK / 32];
+    const int lane = threadIdx.x & (G - 1);
+    const int n = a.n;
+    const int rounds = (n + (int)gridDim.x * PPB - 1) / ((int)gridDim.x * PPB);
+    const float dt = *a.dtp;
+    const float dtf = a.mode == 0 ? dt : dt * dt;
+    JacobiCtl* c = a.ctl;
+    float mu = 0.f;
+    unsigned int arrived = 0;
+    int it = 0;
+    bool converged = false, gave_up = false;
+
+    // U entries of the row of particle i from entry q on (past the row's end: no gradient)
+    int j[U];
+    Vec<D> g[U];
+    auto load_entries = [&](int i, int q, int e) {
+        #pragma unroll
+        for (int u = 0; u < U; ++u) {
+            j[u] = i; g[u] = vzero<D>();
+            if (q + u * G < e) get_pair_grad<D>(a.grads, a.list, q + u * G, j[u], g[u]);
+        }
+    };
+    // HOLD: one particle per group for the whole solve, its first G * U entries in registers
+    int hb = 0, he = 0;
+    if (HOLD) {
+        const int i = (int)blockIdx.x * PPB + (int)threadIdx.x / G;
+        if (i < n) { hb = a.offs[i]; he = hb + a.cnt[i]; }
+        load_entries(i < n ? i : 0, hb + lane, he);
+    }
+
+    for (;;) {
+        // ------------------------------------------------ phase A: pressure acceleration
+        for (int rd = 0; rd < rounds; ++rd) {
+            const int i = (rd * (int)gridDim.x + (int)blockIdx.x) * PPB + (int)threadIdx.x / G;
+            const bool valid = i < n;
+            Vec<D> s = vzero<D>();
+            if (valid) {
+                const float2 ti = a.pq[i];
+                const float qi = (ti.x - mu) * ti.y;
+                const int b = HOLD ? hb : a.offs[i], e = HOLD ? he : b + a.cnt[i];
+                bool reload = false;
+                for (int q = b + lane; q < e; q += G * U) {
+                    if (!HOLD || q != b + lane) { load_entries(i, q, e); reload = HOLD; }
+                    float2 t[U];
+                    #pragma unroll
+                    for (int u = 0; u < U; ++u) t[u] = a.pq[j[u]];
+                    #pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const float w = qi + (t[u].x - mu) * t[u].y;
+                        #pragma unroll
+                        for (int d = 0; d < D; ++d) s.v[d] += w * g[u].v[d];
+                    }
+                }
+                if (HOLD && reload) load_entries(i, b + lane, e);
+            }
+            #pragma unroll
+            for (int d = 0; d < D; ++d) s.v[d] = gsum<G>(s.v[d]);
+            if (valid && lane == 0)
+                a.a4[i] = make_float4(-s.v[0], D > 1 ? -s.v[D > 1 ? 1 : 0] : 0.f, D > 2 ? -s.v[D > 2 ? 2 : 0] : 0.f, 1.f / a.rho[i]);
+        }
+        if (converged || it >= a.max_it) break;
+        if (!grid_barrier(&c->bar, arrived, a.barrier_ns)) { gave_up = true; break; }
+
+        // ------------------------------------------------ phase B: shift, residual, update
+        double psum = 0.0, esum = 0.0;
+        unsigned int pmin = 0xffffffffu, pmax = 0u;
+        for (int rd = 0; rd < rounds; ++rd) {
+            const int i = (rd * (int)gridDim.x + (int)blockIdx.x) * PPB + (int)threadIdx.x / G;
+            const bool valid = i < n;
+            float s = 0.f;
+            if (valid) {
+                const Vec<D> ai = vec_of<D>(a.a4[i]);
+                const int b = HOLD ? hb : a.offs[i], e = HOLD ? he : b + a.cnt[i];
+                bool reload = false;
+                for (int q = b + lane; q < e; q += G * U) {
+                    if (!HOLD || q != b + lane) { load_entries(i, q, e); reload = HOLD; }
+                    float4 t[U];
+                    #pragma unroll
+                    for (int u = 0; u < U; ++u) t[u] = a.a4[j[u]];
+                    #pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const Vec<D> aj = vec_of<D>(t[u]);
+                        float w = 0.f;
+                        #pragma unroll
+                        for (int d = 0; d < D; ++d) w += (aj.v[d] - ai.v[d]) * g[u].v[d];
+                        s += t[u].w * w;
+                    }
+                }
+                if (HOLD && reload) load_entries(i, b + lane, e);
+            }
+            s = gsum<G>(s);
+            if (valid && lane == 0) {
+                const float r = a.src[i] - dtf * (-s);
+                float pb = (a.pq[i].x - mu) + a.omega * r / a.diag[i];
+                float e;
+                if (a.mode == 1) {
+                    pb = pb < 0.f ? 0.f : pb;                       // incompressible.py:108
+                    e = -r < -a.tol ? -a.tol : -r;                  // :111
+                } else {
+                    e = fabsf(r);                                   // divergenceFree.py:112
+                }
+                a.pq[i].x = pb;
+                psum += (double)pb;
+                esum += (double)e;
+                const unsigned int o = f2o(pb);
+                pmin = min(pmin, o);
+                pmax = max(pmax, o);
+            }
+        }
+        JacobiSums t = block_sums<BLOCK>(JacobiSums{psum, esum, pmin, pmax}, sh);
+        if (threadIdx.x == 0) a.sums[blockIdx.x] = t;
+        if (!grid_barrier(&c->bar, arrived, a.barrier_ns)) { gave_up = true; break; }
+
+        // ------------------------------------------------ decide (identical in every block: each sums
+        // every block's partial sums in the same order)
+        t = JacobiSums{0.0, 0.0, 0xffffffffu, 0u};
+        for (int q = threadIdx.x; q < (int)gridDim.x; q += BLOCK) {
+            const JacobiSums o = a.sums[q];
+            t.p += o.p; t.e += o.e; t.lo = min(t.lo, o.lo); t.hi = max(t.hi, o.hi);
+        }
+        t = block_sums<BLOCK>(t, sh);
+        const double ps = t.p, es = t.e;
+        const float lo = o2f(t.lo), hi = o2f(t.hi);
+        const double mean = ps / (double)n;
+        const double err = es / (double)n;
+        mu = a.mode == 0 ? (float)mean : 0.f;                       // divergenceFree.py:104
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            a.hist[it * 4 + 0] = (float)err;
+            a.hist[it * 4 + 1] = lo - mu;
+            a.hist[it * 4 + 2] = hi - mu;
+            a.hist[it * 4 + 3] = (float)(mean - (double)mu);
+        }
+        const bool finite = isfinite(err);
+        if (!finite) { if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(&c->bar.status, SPH_STATUS_NONFINITE); }
+        converged = (it >= a.min_it && err < (double)a.tol) || !finite;
+        ++it;
+    }
+    // the results of this block's particles, which its own lead lanes wrote: the last phase A
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int i = (rd * (int)gridDim.x + (int)blockIdx.x) * PPB + (int)threadIdx.x / G;
+        if (i >= n || lane != 0) continue;
+        store_vec<D>(a.acc, i, vec_of<D>(a.a4[i]));
+        a.p_out[i] = a.pq[i].x - mu;
+    }
+    if (threadIdx.x == 0) {
+        int st = gave_up ? SPH_STATUS_TIMEOUT : *(volatile int*)&c->bar.status;
+        if (blockIdx.x == 0) {
+            if (!gave_up && !converged && a.max_it > 0) st |= SPH_STATUS_NOT_CONVERGED;
+            *a.iters_out = it;
+        }
+        if (st) atomicOr(a.status_out, st);
+    }
+}
+
 // ---------------------------------------------------------------- host side
 constexpr size_t kCtlBytes = 256;
 static_assert(sizeof(JacobiCtl) <= kCtlBytes, "control block");
@@ -394,8 +647,17 @@ static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
 static int64_t dfsph_ws_bytes(int64_t n) { return (int64_t)(kCtlBytes + 3 * align256((size_t)n * sizeof(float))); }
 
-template <int KF, int D>
-static int launch_jacobi(JacobiArgs& a, cudaStream_t s) {
+// SMs of the current device (a B200's 148 where the query fails: the launch then reports why).
+static int device_sms() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    return sms;
+}
+
+// One cooperative launch of a persistent solve kernel over n particles (KERN names the kernel, so
+// that each instantiation keeps its own occupancy).
+template <auto KERN, int BLOCK, int PPB, typename Args>
+static int launch_persistent(Args& a, cudaStream_t s) {
     static std::mutex mu;
     static int cached_dev = -1, blocks_per_sm = 0, num_sms = 0;
     int dev = 0;
@@ -409,25 +671,33 @@ static int launch_jacobi(JacobiArgs& a, cudaStream_t s) {
             if (e != cudaSuccess || !coop) return set_error(SPH_ERR_UNSUPPORTED, "jacobi: device %d has no cooperative launch", dev);
             e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
             if (e != cudaSuccess) return set_error(SPH_ERR_CUDA, "jacobi: SM count: %s", cudaGetErrorString(e));
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_jacobi<KF, D>, JAC_BLOCK, 0);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, KERN, BLOCK, 0);
             if (e != cudaSuccess || blocks_per_sm < 1) return set_error(SPH_ERR_CUDA, "jacobi: occupancy query failed");
             cached_dev = dev;
         }
     }
-    const int64_t need = (a.n + JAC_PPB - 1) / JAC_PPB;
+    const int64_t need = (a.n + PPB - 1) / PPB;
     const int grid = (int)std::min<int64_t>(need, (int64_t)blocks_per_sm * num_sms);
     void* args[] = {&a};
     count_launch();
-    e = cudaLaunchCooperativeKernel((const void*)k_jacobi<KF, D>, dim3(grid), dim3(JAC_BLOCK), args, 0, s);
+    e = cudaLaunchCooperativeKernel((const void*)KERN, dim3(grid), dim3(BLOCK), args, 0, s);
     if (e != cudaSuccess) return set_error(SPH_ERR_CUDA, "jacobi: cooperative launch: %s", cudaGetErrorString(e));
     return SPH_OK;
+}
+
+// Bytes per row entry and in all of the buffer of cached pair gradients: the particles' (p, 1 / rho^2)
+// and (a, 1 / rho), then one gradient per entry.
+constexpr size_t kSumsBytes = 2048 * sizeof(JacobiSums);     // of at most 2048 co-resident blocks
+static int64_t dfsph_grad_bytes(int64_t n, int64_t entries, int dim) {
+    return (int64_t)(kSumsBytes + align256((size_t)n * sizeof(float2)) + align256((size_t)n * sizeof(float4)) +
+                     align256((size_t)entries * (dim == 3 ? 4 : dim) * sizeof(float)));
 }
 
 static int dfsph_solve(int mode, const SphParams* p, const SphJacobiConfig* cfg, int64_t n, const float* x, const float* H,
                        const float* m, const float* rho, const float* v, const float* dvdt, const float* p_init,
                        const float* dt, const int32_t* offs, const int32_t* cnt, const int32_t* list, void* ws,
                        int64_t ws_bytes, float* p_out, float* accel_out, float* history, int32_t* iterations, int32_t* status,
-                       void* stream) {
+                       void* stream, int64_t entries = 0, void* gradients = nullptr, int64_t gradient_bytes = 0) {
     PAIR_PRELUDE();
     WSPH_CHECK_PTR(cfg); WSPH_CHECK_PTR(x); WSPH_CHECK_PTR(H); WSPH_CHECK_PTR(m); WSPH_CHECK_PTR(rho); WSPH_CHECK_PTR(v);
     WSPH_CHECK_PTR(dt); WSPH_CHECK_PTR(ws); WSPH_CHECK_PTR(p_out); WSPH_CHECK_PTR(accel_out); WSPH_CHECK_PTR(history);
@@ -445,6 +715,13 @@ static int dfsph_solve(int mode, const SphParams* p, const SphJacobiConfig* cfg,
     if ((rc = check_align_vec(P, x, "x")) || (rc = check_align_vec(P, v, "v")) || (rc = check_align_vec(P, dvdt, "dvdt")) ||
         (rc = check_align_vec(P, accel_out, "accel_out")))
         return rc;
+    if (gradients) {
+        if (entries < 0 || entries > 0x7fffffff) return set_error(SPH_ERR_BAD_ARG, "jacobi: entries out of range");
+        if (gradient_bytes < dfsph_grad_bytes(n, entries, P.dim))
+            return set_error(SPH_ERR_WORKSPACE, "jacobi: gradient buffer %lld < %lld bytes", (long long)gradient_bytes,
+                             (long long)dfsph_grad_bytes(n, entries, P.dim));
+        if (reinterpret_cast<uintptr_t>(gradients) & 255) return set_error(SPH_ERR_BAD_ARG, "jacobi: the gradient buffer must be 256-byte aligned");
+    }
     char* w = static_cast<char*>(ws);
     JacobiCtl* ctl = reinterpret_cast<JacobiCtl*>(w);
     const size_t nb = align256((size_t)n * sizeof(float));
@@ -454,10 +731,42 @@ static int dfsph_solve(int mode, const SphParams* p, const SphJacobiConfig* cfg,
     cudaError_t e = cudaMemsetAsync(ctl, 0, kCtlBytes, s);
     if (e != cudaSuccess) return set_error(SPH_ERR_CUDA, "jacobi: memset: %s", cudaGetErrorString(e));
     const float rho0 = (float)cfg->rest_density;
+    float2* pq = nullptr;
+    float4* a4 = nullptr;
+    float* grads = nullptr;
+    if (gradients) {
+        char* gb = static_cast<char*>(gradients) + kSumsBytes;
+        pq = reinterpret_cast<float2*>(gb);
+        gb += align256((size_t)n * sizeof(float2));
+        a4 = reinterpret_cast<float4*>(gb);
+        grads = reinterpret_cast<float*>(gb + align256((size_t)n * sizeof(float4)));
+    }
     count_launch();
     WSPH_DISPATCH_KDS(*p, (k_dfsph_prep<KF, D, G_LIGHT><<<grid_g<G_LIGHT>(n), PAIR_BLOCK, 0, s>>>(
-        (int)n, P, mode, rho0, x, H, m, rho, v, dvdt, dt, offs, cnt, list, nullptr, nullptr, p_init, cfg->init_mode, src, diag, praw)));
+        (int)n, P, mode, rho0, x, H, m, rho, v, dvdt, dt, offs, cnt, list, nullptr, nullptr, p_init, cfg->init_mode, src, diag, praw, grads, pq)));
     if ((rc = check_launch("jacobi prep"))) return rc;
+    const unsigned long long barrier_ns = cfg->barrier_timeout_us > 0 ? 1000ull * (unsigned long long)cfg->barrier_timeout_us : kBarrierLimitNs;
+    if (gradients) {
+        JacobiGradArgs a;
+        a.n = (int)n; a.mode = mode; a.min_it = cfg->min_iterations; a.max_it = cfg->max_iterations;
+        a.omega = (float)cfg->relaxation; a.tol = (float)cfg->tolerance;
+        a.rho = rho; a.src = src; a.diag = diag; a.dtp = dt; a.grads = grads;
+        a.offs = offs; a.cnt = cnt; a.list = list; a.pq = pq; a.a4 = a4; a.sums = static_cast<JacobiSums*>(gradients);
+        a.p_out = p_out; a.acc = accel_out; a.hist = history; a.iters_out = iterations; a.status_out = status; a.ctl = ctl;
+        a.barrier_ns = barrier_ns;
+        rc = SPH_ERR_UNSUPPORTED;
+        
+#define JACOBI_GRAD(G, U, MINB, HOLD) WSPH_DISPATCH_DIM(P.dim, \
+        (rc = launch_persistent<k_jacobi_grad<D, G, U, JAC_BLOCK, MINB, HOLD>, JAC_BLOCK, JAC_BLOCK / G>(a, s)))
+        // The split by size (see k_jacobi_grad): one block of 8 lanes per particle on each SM, two
+        // blocks of 4 lanes, or a loop over particles.
+        const int sms = device_sms();
+        if (n <= (int64_t)sms * (JAC_BLOCK / 8)) { JACOBI_GRAD(8, 6, 2, true); }
+        else if (n <= (int64_t)sms * 2 * (JAC_BLOCK / 4)) { JACOBI_GRAD(4, 10, 2, true); }
+        else { JACOBI_GRAD(4, 5, 4, false); }
+#undef JACOBI_GRAD
+        return rc;
+    }
     JacobiArgs a;
     a.n = (int)n; a.mode = mode; a.min_it = cfg->min_iterations; a.max_it = cfg->max_iterations;
     a.omega = (float)cfg->relaxation; a.tol = (float)cfg->tolerance; a.P = P;
@@ -465,9 +774,9 @@ static int dfsph_solve(int mode, const SphParams* p, const SphJacobiConfig* cfg,
     a.offs = offs; a.cnt = cnt; a.list = list;
     a.praw = praw; a.p_out = p_out; a.acc = accel_out; a.hist = history;
     a.iters_out = iterations; a.status_out = status; a.ctl = ctl;
-    a.barrier_ns = cfg->barrier_timeout_us > 0 ? 1000ull * (unsigned long long)cfg->barrier_timeout_us : kBarrierLimitNs;
+    a.barrier_ns = barrier_ns;
     rc = SPH_ERR_UNSUPPORTED;
-    WSPH_DISPATCH_KD(P.kernel, P.dim, (rc = launch_jacobi<KF, D>(a, s)));
+    WSPH_DISPATCH_KD(P.kernel, P.dim, (rc = launch_persistent<k_jacobi<KF, D>, JAC_BLOCK, JAC_PPB>(a, s)));
     return rc;
 }
 
@@ -645,6 +954,21 @@ int sph_dfsph_div_solve(const SphParams* p, const SphJacobiConfig* cfg, int64_t 
                         float* p_out, float* accel_out, float* history, int32_t* iterations, int32_t* status, void* stream) {
     return dfsph_solve(0, p, cfg, n, x, H, m, rho, v, dvdt, p_init, dt, offs, cnt, list, workspace, workspace_bytes, p_out,
                        accel_out, history, iterations, status, stream);
+}
+
+int64_t sph_dfsph_gradient_bytes(int64_t n, int64_t entries, int32_t dim) {
+    return n < 0 || entries < 0 || dim < 1 || dim > 3 ? -1 : dfsph_grad_bytes(n, entries, dim);
+}
+
+int sph_dfsph_solve_cached(int32_t mode, const SphParams* p, const SphJacobiConfig* cfg, int64_t n, int64_t entries, const float* x,
+                           const float* H, const float* m, const float* rho, const float* v, const float* dvdt, const float* p_init,
+                           const float* dt, const int32_t* offs, const int32_t* cnt, const int32_t* list, void* workspace,
+                           int64_t workspace_bytes, void* gradients, int64_t gradient_bytes, float* p_out, float* accel_out,
+                           float* history, int32_t* iterations, int32_t* status, void* stream) {
+    if (mode != 0 && mode != 1) return set_error(SPH_ERR_BAD_ARG, "sph_dfsph_solve_cached: mode must be 0 or 1");
+    if (n > 0) WSPH_CHECK_PTR(gradients);
+    return dfsph_solve(mode, p, cfg, n, x, H, m, rho, v, dvdt, p_init, dt, offs, cnt, list, workspace, workspace_bytes, p_out,
+                       accel_out, history, iterations, status, stream, entries, gradients, gradient_bytes);
 }
 
 int sph_dfsph_density_solve(const SphParams* p, const SphJacobiConfig* cfg, int64_t n, const float* x, const float* H,

@@ -4,6 +4,12 @@
 // default; the Jacobi solves take the limit from their launch arguments) or 2^26 polls,
 // sets SPH_STATUS_TIMEOUT in the control block and makes every block return, so a
 // failure ends the kernel instead of hanging the GPU.
+//
+// The arrival counter only ever grows: block b's k-th wait ends when it has reached
+// k * gridDim.x, so no block resets it and no second word is published (at most
+// 2^21 waits x 2^11 blocks in a solve, compared modulo 2^32).  One thread arrives with a
+// release and polls with an acquire; the block barriers on both sides extend that order to
+// the whole block, so plain loads after the barrier see every write made before it.
 #pragma once
 #include <cuda_runtime.h>
 #include "sph_common.cuh"
@@ -11,8 +17,8 @@
 namespace wsph {
 
 struct BarrierCtl {
-    unsigned int count;        // arrivals in the current generation
-    unsigned int gen;          // barrier generation
+    unsigned int count;        // arrivals since the control block was zeroed
+    unsigned int pad0;
     int status;                // SPH_STATUS_* bits
     int pad;
 };
@@ -25,39 +31,35 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 constexpr unsigned long long kBarrierLimitNs = 2000000000ull;
 
-// Returns false when any block gave up (SPH_STATUS_TIMEOUT); the caller then returns.
-static __device__ __noinline__ bool grid_barrier(BarrierCtl* c, unsigned long long limit_ns = kBarrierLimitNs) {
+static __device__ __noinline__ bool grid_wait(BarrierCtl* c, unsigned int arrived, unsigned long long limit_ns) {
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned int* vgen = &c->gen;
-        volatile int* vstat = &c->status;
-        const unsigned int g = *vgen;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&c->count) : "memory");
+        const unsigned long long t0 = global_ns();
+        unsigned int spins = 0, now;
         int good = 1;
-        __threadfence();
-        const unsigned int arrived = atomicAdd(&c->count, 1u) + 1u;
-        if (arrived == gridDim.x) {
-            atomicExch(&c->count, 0u);
-            __threadfence();
-            atomicAdd(&c->gen, 1u);
-        } else {
-            const unsigned long long t0 = global_ns();
-            unsigned int spins = 0;
-            while (*vgen == g) {
-                if (*vstat & SPH_STATUS_TIMEOUT) { good = 0; break; }
-                if (++spins > (1u << 26) || global_ns() - t0 > limit_ns) {
-                    atomicOr(&c->status, SPH_STATUS_TIMEOUT);
-                    good = 0;
-                    break;
-                }
-                __nanosleep(64);
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&c->count) : "memory");
+            if (static_cast<int>(now - arrived) >= 0) break;
+            if (*reinterpret_cast<volatile int*>(&c->status) & SPH_STATUS_TIMEOUT) { good = 0; break; }
+            if (++spins > (1u << 26) || global_ns() - t0 > limit_ns) {
+                atomicOr(&c->status, SPH_STATUS_TIMEOUT);
+                good = 0;
+                break;
             }
         }
-        __threadfence();
         ok = good;
     }
     __syncthreads();
     return ok != 0;
+}
+// `arrived` counts the arrivals this block waits for; it starts at 0 with the zeroed control
+// block and is the same in every thread.  Returns false when any block gave up
+// (SPH_STATUS_TIMEOUT); the caller then returns.
+__device__ __forceinline__ bool grid_barrier(BarrierCtl* c, unsigned int& arrived, unsigned long long limit_ns = kBarrierLimitNs) {
+    arrived += gridDim.x;
+    return grid_wait(c, arrived, limit_ns);
 }
 
 }  // namespace wsph

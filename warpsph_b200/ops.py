@@ -965,12 +965,29 @@ def jacobi_solve(params, mode: int, cfg, x, H, m, rho, v, dvdt, p_init, dt, adj:
     acc = _empty((n, d), m)
     hist = torch.zeros((max(int(cfg.max_iterations), 1), 4), device=m.device, dtype=torch.float32)
     flags = torch.zeros(2, device=m.device, dtype=torch.int32)
-    fn = _capi.lib().sph_dfsph_div_solve if mode == DIVERGENCE_FREE else _capi.lib().sph_dfsph_density_solve
+    L = _capi.lib()
     with _timed("dfsph_div_solve" if mode == DIVERGENCE_FREE else "dfsph_density_solve"):
+        grads = _gradient_buffer(n, adj.nnz, d, m.device)
+        if grads is not None:
+            check(L.sph_dfsph_solve_cached(mode, _p(params), C.cast(C.pointer(cfg), C.c_void_p), n, adj.nnz, fptr(x), fptr(H), fptr(m),
+                                           fptr(rho), fptr(v), fptr(dvdt), fptr(p_init), ptr(dt_tensor(dt, m.device)),
+                                           *_lists(params, adj, True), ptr(ws), int(ws.numel()), ptr(grads), int(grads.numel()), ptr(pr),
+                                           ptr(acc), ptr(hist), ptr(flags), ptr(flags[1:]), stream_ptr(m.device)), "jacobi solve")
+            return pr, acc, hist, flags[:1], flags[1:]
+        fn = L.sph_dfsph_div_solve if mode == DIVERGENCE_FREE else L.sph_dfsph_density_solve
         check(fn(_p(params), C.cast(C.pointer(cfg), C.c_void_p), n, fptr(x), fptr(H), fptr(m), fptr(rho), fptr(v), fptr(dvdt),
                  fptr(p_init), ptr(dt_tensor(dt, m.device)), *_lists(params, adj, True), ptr(ws), int(ws.numel()), ptr(pr), ptr(acc),
                  ptr(hist), ptr(flags), ptr(flags[1:]), stream_ptr(m.device)), "jacobi solve")
     return pr, acc, hist, flags[:1], flags[1:]
+
+
+def _gradient_buffer(n: int, entries: int, d: int, device) -> Optional[torch.Tensor]:
+    """The cached pair gradients of one solve (16 bytes per row entry in 3D), or None when the
+    device has no room for them: the solve then forms each gradient in every iteration."""
+    try:
+        return torch.empty(int(_capi.lib().sph_dfsph_gradient_bytes(n, entries, d)), dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
 
 
 def _jacobi_workspace(n: int, d: int, device) -> torch.Tensor:
