@@ -49,6 +49,20 @@ def test_step_matches_oracle(cuda, switch):
         assert_close(S.alphas.cpu().numpy(), st["alphas"], 1e-3, 1e-3, f"alpha step {k}")
 
 
+def test_odd_particle_count_matches_oracle(cuda):
+    """An odd number of particles in 2D: the compatible-energy finalize keeps its half-step
+    velocities behind n floats, where pairs of them do not start on an 8-byte boundary."""
+    cfg, sch, integ, step, system = sedov(33, cuda)
+    st = state_to_numpy(system.state)
+    orc = CRKSPHOracle(ws.make_params(cfg, sch), "f32", switch=SWITCH_CULLEN)
+    res = integ.function(state=system, f=step, dt=2e-4, config=cfg, compParams=sch)
+    st, _, _ = orc.step(st, 2e-4, "rungeKutta2")
+    S = res.state.state
+    assert_close(S.positions.cpu().numpy(), st["positions"], 1e-6, 1e-6, "x")
+    assert_close(S.velocities.cpu().numpy(), st["velocities"], 2e-4, 2e-4, "v")
+    assert_close(S.internalEnergies.cpu().numpy(), st["internalEnergies"], 2e-4, 2e-4, "u")
+
+
 def test_rk4_step_matches_oracle(cuda):
     cfg, sch, integ, step, system = sedov(24, cuda, scheme=ws.IntegrationSchemeType.rungeKutta4)
     st = state_to_numpy(system.state)

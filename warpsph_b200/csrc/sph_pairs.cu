@@ -1249,7 +1249,9 @@ __global__ void k_vhalf(int n, int ns, StagePtrs S, const float* __restrict__ dt
         vh[(size_t)i * D + a] = v0[(size_t)i * D + a] + 0.5f * fa * dt;
     }
 }
-template <int D, int G>
+// PAIRS: the half-step velocities may be read as float2 (2D).  They follow n floats of du_out, so
+// in 2D an odd n leaves them 4 bytes off an 8-byte boundary, and they are read word by word.
+template <int D, int G, bool PAIRS>
 __global__ void __launch_bounds__(PAIR_BLOCK)
 k_finalize(int n, int ns, StagePtrs S, int pdv, const float* __restrict__ dtp, const float* __restrict__ vh,
            const float* __restrict__ u0, float* __restrict__ u_out, float* __restrict__ du_out) {
@@ -1257,7 +1259,17 @@ k_finalize(int n, int ns, StagePtrs S, int pdv, const float* __restrict__ dtp, c
     Grp<G> g(n);
     float du = 0.f;
     if (g.valid) {
-        Vec<D> vi = load_vec<D>(vh, g.i);
+        auto half = [&](int i) {
+            if constexpr (PAIRS) {
+                return load_vec<D>(vh, i);
+            } else {
+                Vec<D> r;
+                #pragma unroll
+                for (int a = 0; a < D; ++a) r.v[a] = __ldg(vh + (size_t)i * D + a);
+                return r;
+            }
+        };
+        Vec<D> vi = half(g.i);
         for (int s = 0; s < ns; ++s) {
             const int32_t* __restrict__ lst = S.list[s];
             const float* __restrict__ f = S.f[s];
@@ -1268,7 +1280,7 @@ k_finalize(int n, int ns, StagePtrs S, int pdv, const float* __restrict__ dtp, c
             float acc = 0.f;
             for (int q = b + g.lane; q < e; q += G) {
                 int j, k; entry(lst, q, j, k);
-                Vec<D> vj = load_vec<D>(vh, j);
+                Vec<D> vj = half(j);
                 Vec<D> a1 = load_vec<D>(ap, k), a2 = load_vec<D>(av, k);
                 float fk = __ldg(f + k);
                 float d1 = 0.f, d2 = 0.f;
@@ -1752,7 +1764,12 @@ int sph_finalize_compatible_energy(const SphParams* p, int64_t n, int32_t nstage
     int pdv = P.energy_scheme == SPH_ENERGY_PDV;
     wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, (launch_pdl(k_vhalf<D>, grid_for(n, 256), 256, 0, s, (int)n, nstages, S, dt, v0, vh)));
     wsph::count_launch();
-    WSPH_DISPATCH_DS(*p, (launch_pdl(k_finalize<D, G_LIGHT>, grid_g<G_LIGHT>(n), PAIR_BLOCK, 0, s, (int)n, nstages, S, pdv, dt, vh, u0, u_out, du_out)));
+    const bool pairs = P.dim != 2 || !(reinterpret_cast<uintptr_t>(vh) & 7);
+    if (pairs) {
+        WSPH_DISPATCH_DS(*p, (launch_pdl(k_finalize<D, G_LIGHT, true>, grid_g<G_LIGHT>(n), PAIR_BLOCK, 0, s, (int)n, nstages, S, pdv, dt, vh, u0, u_out, du_out)));
+    } else {
+        launch_pdl(k_finalize<2, G_LIGHT, false>, grid_g<G_LIGHT>(n), PAIR_BLOCK, 0, s, (int)n, nstages, S, pdv, dt, vh, u0, u_out, du_out);
+    }
     return check_launch("sph_finalize_compatible_energy");
 }
 
