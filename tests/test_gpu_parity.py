@@ -48,6 +48,54 @@ def test_neighbors_bit_exact(cuda, dim, n_side, periodic):
     assert np.array_equal(j, ref["list"]) and np.array_equal(np.bincount(i, minlength=len(ref["counts"])), ref["counts"])
 
 
+@pytest.mark.parametrize("dim,n_side,keep", [(1, 700, 0.6), (2, 61, 1.0), (2, 44, 0.35), (3, 22, 1.0), (3, 18, 0.4)])
+@pytest.mark.parametrize("periodic", [True, False])
+def test_neighbors_bit_exact_uneven_cells(cuda, dim, n_side, keep, periodic):
+    """Cells from empty to several work items (the lattice squeezed towards one corner and
+    thinned), supports that differ by up to a factor of two: full and partial chunks, items of
+    at most 16 particles, shifted and unshifted stencils."""
+    cfg, sch, p = make_params(dim, periodic=periodic)
+    P = make_particles(dim, n_side, seed=70 + dim, jitter=0.5, h_spread=0.33, periodic=periodic)
+    rng = np.random.default_rng(7)
+    on = rng.random(len(P["supports"])) < keep
+    u = (P["positions"][on] + 0.5).astype(np.float64)
+    x = np.ascontiguousarray((0.45 * u + 0.55 * u ** 3 - 0.5).astype(np.float32))
+    H = np.ascontiguousarray(P["supports"][on])
+    adj = ops.buildVerletList(torch.from_numpy(x).to(cuda), torch.from_numpy(H).to(cuda), p, p.verlet_scale)
+    ref = oracle.get("f32").neighbors(p, x, H, cell_capacity_for(len(H), dim))
+    assert ref["grid"][:dim].min() >= 3
+    assert adj.nnz == ref["nnz"]
+    assert np.array_equal(adj.neighborOffsets.cpu().numpy(), ref["offsets"])
+    assert np.array_equal(adj.numNeighbors.cpu().numpy(), ref["counts"])
+    assert np.array_equal(adj.neighborList.cpu().numpy(), ref["list"])
+    assert np.array_equal(adj.interCounts.cpu().numpy(), ref["inter_counts"])
+
+
+@pytest.mark.parametrize("dim,n_side", [(2, 60), (3, 20)])
+@pytest.mark.parametrize("test", ["verlet", "interacting"])
+def test_neighbors_bit_exact_at_the_bound(cuda, dim, n_side, test):
+    """Supports chosen so that every particle has a pair whose rounded squared distance is the
+    bound itself to the last bit or two: a contracted or reordered square would decide some of
+    them the other way."""
+    cfg, sch, p = make_params(dim)
+    P = make_particles(dim, n_side, seed=80 + dim, jitter=0.3, h_spread=0.0)
+    x, n = P["positions"], len(P["supports"])
+    H0 = float(P["supports"][0])
+    rng = np.random.default_rng(3)
+    j = (np.arange(n) + rng.choice([1, 2, n_side, n_side + 1, 2 * n_side, 2 * n_side + 1], n)) % n
+    d = x - x[j]
+    d = np.where(d > 0.5, d - np.float32(1), np.where(d < -0.5, d + np.float32(1), d)).astype(np.float32)
+    r = np.sqrt((d.astype(np.float64) ** 2).sum(1))
+    near = r < 1.4 * H0
+    H = np.where(near, r / (float(np.float32(p.verlet_scale)) if test == "verlet" else 1.0), 0.7 * H0).astype(np.float32)
+    H = np.maximum(H, np.float32(0.3 * H0))
+    adj = ops.buildVerletList(torch.from_numpy(x).to(cuda), torch.from_numpy(H).to(cuda), p, p.verlet_scale)
+    ref = oracle.get("f32").neighbors(p, x, H, cell_capacity_for(n, dim))
+    assert np.array_equal(adj.numNeighbors.cpu().numpy(), ref["counts"])
+    assert np.array_equal(adj.interCounts.cpu().numpy(), ref["inter_counts"])
+    assert np.array_equal(adj.neighborList.cpu().numpy(), ref["list"])
+
+
 @pytest.mark.parametrize("dim,n_side", [(1, 12), (1, 20), (2, 9), (2, 12), (3, 8)])
 def test_neighbors_bit_exact_small_periodic_grids(cuda, dim, n_side):
     """One or two cells along a periodic axis: a cell is reached through two periodic

@@ -9,12 +9,11 @@
 //      atomic scatter, then a per-cell insertion sort by particle index, so the
 //      permutation equals a stable sort by (key, index) -- deterministic and
 //      bit-identical to the CPU oracle.
-//   3. Verlet list as CSR: count pass, exclusive scan, fill pass.  One warp per
-//      particle (in sorted order, over position/support records gathered in sorted
-//      order) visits the 3^d stencil cells in offset order with lanes over the
-//      candidates, keeps j when |x_i - x_j|^2 < (verlet_scale * max(H_i, H_j))^2
-//      (explicit round-to-nearest operations, so the oracle reproduces it exactly)
-//      and writes each row with ballot-compacted, coalesced stores.
+//   3. Verlet list as CSR: count pass, exclusive scan, fill pass.  One warp per 32
+//      particles of a cell (in sorted order, over position records gathered in sorted
+//      order) visits the 3^d stencil cells in offset order, keeps j when
+//      |x_i - x_j|^2 < (verlet_scale * max(H_i, H_j))^2 (explicit round-to-nearest
+//      operations, so the oracle reproduces it exactly) and writes each row compacted.
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -420,17 +419,32 @@ __global__ void k_scatter(const uint32_t* __restrict__ keys, int n, int32_t* __r
     sort_index[pos] = i;
 }
 
+// The smallest float s with fl(sqrt(s)) >= h: the square root is monotone, so
+// fl(sqrt(r2)) < h exactly when r2 < s.  Starts at fl(h^2), a few floats away at most.
+__device__ __forceinline__ float inter_threshold(float h) {
+    if (!(h > 0.f)) return 0.f;
+    float s = __fmul_rn(h, h);
+    for (int k = 0; k < 4 && s > 0.f; ++k) {
+        const float t = __uint_as_float(__float_as_uint(s) - 1u);
+        if (!(sqrtf(t) >= h)) break;
+        s = t;
+    }
+    for (int k = 0; k < 4 && sqrtf(s) < h; ++k) s = __uint_as_float(__float_as_uint(s) + 1u);
+    return s;
+}
+
 // Canonical order inside a cell: ascending particle index.  After the atomic
 // scatter each cell holds its particles in arbitrary order; every particle's final
 // slot is begin[cell] + (number of cell members with a smaller index).  The pass
-// also writes the sorted keys and packs (x, H) into sorted float4 records that the
-// Verlet walk reads contiguously.
+// also writes the sorted keys and packs (x, fl(fl(vs H)^2)) into sorted float4 records that
+// the Verlet walk reads contiguously, with the interacting test's threshold beside them.
 template <int D>
 __global__ void k_rank_sort(const int32_t* __restrict__ tmp, const uint32_t* __restrict__ keys,
                             const int32_t* __restrict__ begin, const int32_t* __restrict__ end, int n,
                             const float* __restrict__ x, const float* __restrict__ H,
                             int32_t* __restrict__ sort_index, uint32_t* __restrict__ sorted_keys, float4* __restrict__ recs,
-                            int32_t* __restrict__ tasks, int32_t* __restrict__ ntasks, const unsigned int* __restrict__ gate) {
+                            float* __restrict__ inter, float vs, int32_t* __restrict__ tasks, int32_t* __restrict__ ntasks,
+                            const unsigned int* __restrict__ gate) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n || gate_closed(gate)) return;
     int i = tmp[k];
@@ -447,8 +461,9 @@ __global__ void k_rank_sort(const int32_t* __restrict__ tmp, const uint32_t* __r
     sort_index[slot] = i;
     sorted_keys[slot] = c;
     Vec<D> xi = load_vec<D>(x, i);
-    float4 r = make_float4(xi.v[0], D > 1 ? xi.v[D > 1 ? 1 : 0] : 0.f, D > 2 ? xi.v[D > 2 ? 2 : 0] : 0.f, H[i]);
-    recs[slot] = r;
+    const float h = H[i], R = __fmul_rn(vs, h);
+    recs[slot] = make_float4(xi.v[0], D > 1 ? xi.v[D > 1 ? 1 : 0] : 0.f, D > 2 ? xi.v[D > 2 ? 2 : 0] : 0.f, h > 0.f ? __fmul_rn(R, R) : 0.f);
+    inter[slot] = inter_threshold(h);
 }
 
 template <int D> __device__ __forceinline__ Vec<D> rec_pos(const float4& r) {
@@ -459,15 +474,9 @@ template <int D> __device__ __forceinline__ Vec<D> rec_pos(const float4& r) {
     return v;
 }
 
-// Stencil of neighbour cell keys in offset order (x fastest, offsets -1, 0, +1 per
-// axis), periodic axes wrapped, cells outside a non-periodic grid skipped, and a cell
-// reached twice (fewer than three cells along a periodic axis) kept only once.
-// shift[q*3+a] is the periodic image offset of stencil cell q along axis a (-L, 0, +L):
-// with at least three cells per axis, x_i - x_j - shift is the minimum-image
-// difference for every pair within one cell width, bit-identical to the per-pair test
-// of dist_vec (x - 0 = x exactly).  With fewer than three cells along an axis one cell
-// is reached through two images and a single shift cannot serve every pair in it; the
-// walk then takes the minimum image pair by pair (see grid_needs_min_image).
+// With fewer than three cells along a periodic axis one cell is reached through two images
+// and a single shift cannot serve every pair in it; the walk then takes the minimum image
+// pair by pair.
 template <int D>
 __device__ __forceinline__ bool grid_needs_min_image(const GridDev& g, const DomainF& dom) {
     bool r = false;
@@ -476,69 +485,59 @@ __device__ __forceinline__ bool grid_needs_min_image(const GridDev& g, const Dom
     return r;
 }
 
-template <int D>
-__device__ __forceinline__ int stencil_keys(const int* c, const GridDev& g, const DomainF& dom, uint32_t* out, float* shift) {
-    int cnt = 0;
-    constexpr int NS = D == 1 ? 3 : (D == 2 ? 9 : 27);
-    bool dedupe = false;
-    #pragma unroll
-    for (int a = 0; a < D; ++a) dedupe |= g.G[a] < 3;
-    #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-        const int o[3] = {s % 3 - 1, (s / 3) % 3 - 1, (s / 9) % 3 - 1};
-        int cc[3];
-        float sh[3] = {0.f, 0.f, 0.f};
-        bool ok = true;
-        #pragma unroll
-        for (int a = 0; a < D; ++a) {
-            int v = c[a] + o[a];
-            if (v < 0) {
-                if (dom.periodic[a]) { v += g.G[a]; sh[a] = -dom.L[a]; } else ok = false;
-            } else if (v >= g.G[a]) {
-                if (dom.periodic[a]) { v -= g.G[a]; sh[a] = dom.L[a]; } else ok = false;
-            }
-            cc[a] = v;
-        }
-        uint32_t k = morton<D>(cc);
-        if (ok && dedupe) {
-            for (int q = 0; q < cnt; ++q) ok = ok && out[q] != k;
-        }
-        if (ok) {
-            #pragma unroll
-            for (int a = 0; a < 3; ++a) shift[cnt * 3 + a] = sh[a];
-            out[cnt++] = k;
-        }
-    }
-    return cnt;
-}
-
 // Verlet list walk, one warp per work item: up to 32 particles of one cell, lane l
-// owning sorted position start+l.  All lanes share the cell and hence the 3^d stencil
-// and every loop bound (no divergence).  Candidate records of each stencil cell are
-// staged through shared memory 32 at a time (one coalesced load, broadcast reads).
-// A Verlet entry needs r^2 < (verlet_scale*max(H_i,H_j))^2.
+// owning sorted position start+l.  All lanes share the cell and hence the 3^d stencil.
+// Lane q < 3^d looks up stencil cell q (offsets -1, 0, +1 per axis, x fastest; periodic axes
+// wrapped, cells outside a non-periodic grid empty, a cell reached twice kept once), and the
+// candidates of all cells form one sequence in that order, taken 32 at a time whatever the
+// cells' sizes: each chunk is staged through shared memory and tested by every lane.
 //
-// Row layout (when interacting counts are requested): the interacting entries --
-// fl(sqrt(r^2))/max(H_i,H_j) < 1, exactly the pairs some support scheme gives W != 0 --
-// come first, then the rest of the Verlet entries, each part in walk order (stencil
-// cells in offset order, candidates by sorted position).  The pair passes walk only
-// the prefix [offset, offset + interacting count): plain int32 indices, and pairwise
-// outputs written contiguously at their Verlet entry.  The count pass counts both
-// parts, so the fill pass knows where each row's tail starts.  Rows are staged in
-// shared memory (VS entries per lane and part) and flushed by the warp cooperatively,
-// so they are written with contiguous stores.
+// A Verlet entry needs r^2 < fl(fl(vs max(H_i, H_j))^2).  Rounding is monotone, so that bound is
+// the larger of the two particles' own bounds, which the sorted records carry; likewise the
+// interacting test fl(sqrt(r^2)) < max(H_i, H_j) against the thresholds of inter_threshold.  A
+// test takes the larger bound from r^2 (a difference of floats never rounds across zero) and
+// shifts the sign bit into a word: the half-rate integer pipe then has two instructions per
+// test (a comparison with a predicated or makes three) and the multiply-add pipe one, which
+// fills both about equally.  r^2 takes explicit round-to-nearest steps without contraction, so
+// the CPU oracle reproduces it bit for bit; two candidates share each packed add and multiply.
+// An item of at most 16 particles gives each two lanes, one per half of the chunk.
+//
+// Periodic images: with at least three cells per axis, (x_i - x_j) - shift is the minimum-image
+// difference for every pair within one cell width, bit-identical to dist_vec (x - 0 = x
+// exactly); items whose stencil crosses no boundary skip the shift.
+//
+// Row layout (when interacting counts are requested): the interacting entries -- exactly the
+// pairs some support scheme gives W != 0 -- come first, then the rest of the Verlet entries,
+// each part in walk order (stencil cells in offset order, candidates by sorted position).  The
+// pair passes walk only the prefix [offset, offset + interacting count).
+//
+// The count pass keeps each lane's 32 acceptance bits and 32 interacting bits per chunk in a
+// bounded pool; the fill pass reads them back (an item that found the pool exhausted tests
+// again) and writes row by row: the 32 lanes hold the chunk's 32 candidates, and the ones in a
+// row's bits store themselves at the popcount of the lower bits.
+//
+// The count pass is bound by the arithmetic pipes, the fill pass by the latency of its row loop (47 %
+// of issue slots).  1,030,301 particles in 3D with 128 neighbours (about 2,000 candidates for 251
+// entries each): count 1.35 ms against 2.65 ms with both thresholds formed per pair and one
+// candidate per instruction, fill 1.38 ms against 2.85 ms with entries staged per lane and
+// flushed; 262,144 particles in 2D: 48 and 65 us against 127 and 143 us.
 constexpr int VW_WARPS = 4;
 constexpr int VW_BLOCK = 32 * VW_WARPS;
-constexpr int VS = 16;
-// Row pitch of the staging buffers: one word more than VS, so that the 32 lanes'
-// stores of their next entry fall in 32 different banks (with a pitch of 16 words the
-// even and the odd lanes would each share one bank, a 16-way conflict per store).
-constexpr int VP = VS + 1;
+constexpr int VW_ROWS = 4;       // rows the fill pass writes together
+struct alignas(16) VerletStage {
+    float x[3][32];          // -x_j of the chunk's candidates, by axis
+    float sh[3][32];         // image shifts (items that need them)
+    float T[32], S[32];      // minus the Verlet bound and the interacting threshold
+    int first[32];           // sequence number of each stencil cell's first candidate
+    int begin[32];           // its sorted position
+    int code[32];            // image of the cell: two bits per axis (1: -L, 2: +L)
+    uint4 row[32];           // fill: interacting bits, other bits, next entry of each part
+};
 
-// fl(sqrt(r2)) / Hm < 1, with the square root only inside a narrow band around r = Hm
-// (outside it the comparison of r2 with Hm^2 decides the same way).  For positive finite
-// a and b, fl(a / b) < 1 exactly when a < b (a < b gives a / b <= 1 - 2^-24, the float
-// next below 1, so a / b never rounds up to 1), so the test is fl(sqrt(r2)) < Hm.
+// fl(sqrt(r2)) < Hm, with the square root only inside a narrow band around r = Hm (outside it the
+// comparison of r2 with Hm^2 decides the same way).  For positive finite a and b,
+// fl(a / b) < 1 exactly when a < b (a < b gives a / b <= 1 - 2^-24, the float next below 1,
+// so a / b never rounds up to 1), so the oracle's test fl(sqrt(r2)) / Hm < 1 is this one.
 __device__ __forceinline__ bool interacting_pair(float r2, float Hm) {
     const float h2 = Hm * Hm;
     if (r2 < 0.9998f * h2) return true;
@@ -546,120 +545,151 @@ __device__ __forceinline__ bool interacting_pair(float r2, float Hm) {
     return sqrtf(r2) < Hm;
 }
 
-// Writes every lane's staged entries of one part: lanes pair up per owner row (16
-// entries per half warp), base_o + e for the owner's base.
-__device__ __forceinline__ void verlet_flush_part(int lane, int wib, int& nb, int& written, int base,
-                                                  int32_t (*buf)[32][VP], int32_t* __restrict__ list) {
-    const int half = lane >> 4, e = lane & 15;
-    #pragma unroll 4
-    for (int r = 0; r < 32; r += 2) {
-        const int owner = r + half;
-        const int n_o = __shfl_sync(0xffffffffu, nb, owner);
-        const int b_o = __shfl_sync(0xffffffffu, base + written, owner);
-        if (e < n_o) list[b_o + e] = buf[wib][owner][e];
-    }
-    written += nb;
-    nb = 0;
+// Packed pairs of floats: one instruction per operation on two candidates, each rounded as the
+// scalar operation.  The compiler contracts a packed multiply with the add behind it, rounding
+// modes or not, so a product that must be rounded is a multiply-add with a -0 that it cannot see
+// (a kernel argument): rn(a b - 0) = rn(a b).
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add2_rn(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+constexpr unsigned long long NEG_ZERO2 = 0x8000000080000000ull;
+__device__ __forceinline__ unsigned long long mul2_rn(unsigned long long a, unsigned long long b, unsigned long long neg0) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(neg0));
+    return r;
 }
 
-// One work item of the walk (32 particles of one cell against its stencil).  MI: the grid
-// has fewer than three cells along a periodic axis, and every pair takes its minimum image
-// (rare, tiny grids; kept out of line so the common loop stays compact).  Candidate slots
-// past the end of a cell hold a record at 3e38, which no test accepts, so the unrolled
-// candidate loop needs no bound check.
-//
-// Acceptance bits (masks non-null, not MI): the count pass reserves 64 words per candidate
-// chunk of its work item from a bounded pool and stores each lane's 32 acceptance bits and 32
-// interacting bits per chunk; the fill pass then walks the candidates that some lane accepted,
-// in the same order, and files each into the interacting prefix or the rest from the bits,
-// without distance arithmetic.  A work item that found the pool exhausted tests every
-// candidate again.
-template <int D, bool MI, bool SH = true>
-__device__ __forceinline__ void verlet_pair(const Vec<D>& xi, float Hi, const float4& rj, const float* sh, const DomainF& dom,
-                                            float vs, float& r2, float& Hm, float& R) {
-    Hm = fmaxf(Hi, rj.w);
-    R = __fmul_rn(vs, Hm);
-    Vec<D> dv;
+enum { VERLET_PLAIN = 0, VERLET_SHIFT = 1, VERLET_MIN_IMAGE = 2 };
+
+// Acceptance and interacting bits of the lane's particle against the staged candidates (padded
+// to a multiple of 8 with records at 3e38, which no test accepts).
+template <int D, int MODE>
+__device__ __forceinline__ void verlet_test_chunk(const Vec<D>& xi, float Ti, float Si, const VerletStage& st, const DomainF& dom,
+                                                  int base, int mcount, unsigned long long neg0, uint32_t& hm, uint32_t& im) {
+    unsigned long long x2[D];
     #pragma unroll
-    for (int a = 0; a < D; ++a) {
-        const float xj = a == 0 ? rj.x : (a == 1 ? rj.y : rj.z);
-        if (MI) {
-            float d = __fsub_rn(xi.v[a], xj);
-            if (dom.periodic[a]) {
-                if (d > dom.halfL[a]) d = __fsub_rn(d, dom.L[a]);
-                else if (d < -dom.halfL[a]) d = __fadd_rn(d, dom.L[a]);
-            }
-            dv.v[a] = d;
-        } else if (SH) {
-            dv.v[a] = __fsub_rn(__fsub_rn(xi.v[a], xj), sh[a]);
-        } else {
-            dv.v[a] = __fsub_rn(xi.v[a], xj);     // equal to the above with sh = 0 (x - 0 = x exactly)
-        }
-    }
-    r2 = dist2_rn<D>(dv);
-}
-
-// The count pass over one staged chunk: acceptance and interacting bits of the lane's
-// particle against the (up to 32) staged candidates; padded slots never match.
-template <int D, bool MI, bool SH>
-__device__ __forceinline__ void verlet_count_chunk(const Vec<D>& xi, float Hi, bool active, bool part, const float4* __restrict__ sr,
-                                                   const float* sh, const DomainF& dom, float vs, int mcount, uint32_t& hm,
-                                                   uint32_t& im) {
-    for (int u0 = 0; u0 < mcount; u0 += 8) {
+    for (int a = 0; a < D; ++a) x2[a] = pack2(xi.v[a], xi.v[a]);
+    hm = 0u; im = 0u;
+    // 8 candidates at a time, last first: each shifts its sign bits into the words' low ends
+    for (int u0 = (mcount - 1) & ~7; u0 >= 0; u0 -= 8) {
         #pragma unroll
-        for (int du = 0; du < 8; ++du) {
-            const int u = u0 + du;
-            float r2, Hm, R;
-            verlet_pair<D, MI, SH>(xi, Hi, sr[u], sh, dom, vs, r2, Hm, R);
-            const bool hit = active & (r2 < __fmul_rn(R, R));
-            hm |= hit ? (1u << u) : 0u;
-            if (part) im |= (hit && interacting_pair(r2, Hm)) ? (1u << u) : 0u;
+        for (int h = 6; h >= 0; h -= 2) {
+            const int u = base + u0 + h;
+            unsigned long long r2;
+            if (MODE == VERLET_MIN_IMAGE) {
+                float r[2];
+                #pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    Vec<D> xj;
+                    #pragma unroll
+                    for (int a = 0; a < D; ++a) xj.v[a] = -st.x[a][u + k];
+                    r[k] = dist2_rn<D>(dist_vec<D>(xi, xj, dom));
+                }
+                r2 = pack2(r[0], r[1]);
+            } else {
+                #pragma unroll
+                for (int a = 0; a < D; ++a) {
+                    unsigned long long d = add2_rn(x2[a], *reinterpret_cast<const unsigned long long*>(&st.x[a][u]));
+                    if (MODE == VERLET_SHIFT) d = add2_rn(d, *reinterpret_cast<const unsigned long long*>(&st.sh[a][u]));
+                    const unsigned long long q = mul2_rn(d, d, neg0);
+                    r2 = a == 0 ? q : add2_rn(r2, q);
+                }
+            }
+            float t[2], i[2];
+            unpack2(add2_rn(r2, pack2(fminf(-Ti, st.T[u]), fminf(-Ti, st.T[u + 1]))), t[0], t[1]);
+            unpack2(add2_rn(r2, pack2(fminf(-Si, st.S[u]), fminf(-Si, st.S[u + 1]))), i[0], i[1]);
+            #pragma unroll
+            for (int k = 1; k >= 0; --k) {
+                hm = __funnelshift_l(__float_as_uint(t[k]), hm, 1);
+                im = __funnelshift_l(__float_as_uint(i[k]), im, 1);
+            }
         }
     }
+    im &= hm;
 }
 
 template <int D, bool FILL, bool MI>
-__device__ __forceinline__ void verlet_task(int task, int lane, int wib, const float4* __restrict__ recs,
-                                            const uint32_t* __restrict__ sorted_keys, const int32_t* __restrict__ tasks,
-                                            const GridDev& g, const DevParams& P, const int32_t* __restrict__ sort_index,
-                                            const int32_t* __restrict__ cell_begin, const int32_t* __restrict__ cell_end,
-                                            int32_t* __restrict__ counts, int32_t* __restrict__ icounts,
-                                            const int32_t* __restrict__ offsets, int32_t* __restrict__ list, long long& itotal,
-                                            float4 (*srec)[32], int32_t (*sidx)[32], int32_t (*sbuf)[32][VP],
-                                            int32_t (*sibuf)[32][VP], uint32_t* __restrict__ masks,
-                                            int32_t* __restrict__ mask_base, unsigned long long* __restrict__ mask_cursor,
-                                            long long mask_words) {
+__device__ __forceinline__ int verlet_task(int task, int lane, VerletStage& st, const float4* __restrict__ recs,
+                                           const float* __restrict__ inter, const uint32_t* __restrict__ sorted_keys,
+                                           const int32_t* __restrict__ tasks, const GridDev& g, const DevParams& P,
+                                           const int32_t* __restrict__ sort_index, const int32_t* __restrict__ cell_begin,
+                                           const int32_t* __restrict__ cell_end, int32_t* __restrict__ counts,
+                                           int32_t* __restrict__ icounts, const int32_t* __restrict__ offsets,
+                                           int32_t* __restrict__ list, uint32_t* __restrict__ masks, int32_t* __restrict__ mask_base,
+                                           unsigned long long* __restrict__ mask_cursor, long long mask_words,
+                                           unsigned long long neg0) {
+    constexpr int NS = D == 1 ? 3 : (D == 2 ? 9 : 27);
     const bool part = icounts != nullptr;
     const DomainF& dom = P.dom;
-    const float vs = P.verlet_scale;
     const int start = tasks[task];
-    const uint32_t ckey = sorted_keys[start];
-    const int stop = min(start + 32, cell_end[ckey]);
-    const int t = start + lane;
-    const bool active = t < stop;
-    const float4 ri = recs[active ? t : start];
+    const int stop = min(start + 32, cell_end[sorted_keys[start]]);
+    const bool halves = stop - start <= 16;
+    const int t = start + (halves ? lane & 15 : lane);
+    const bool active = start + lane < stop;
+    const int ts = t < stop ? t : start;
+    const float4 ri = recs[ts];
     const Vec<D> xi = rec_pos<D>(ri);
-    const float Hi = ri.w;
-    int c[3];
-    cell_coords<D>(rec_pos<D>(recs[start]), g, dom, c);
-    uint32_t keys[D == 1 ? 3 : (D == 2 ? 9 : 27)];
-    float shifts[3 * (D == 1 ? 3 : (D == 2 ? 9 : 27))];
-    const int nk = stencil_keys<D>(c, g, dom, keys, shifts);
+    const float Ti = ri.w, Si = inter[ts];
     const int i = active ? sort_index[t] : 0;
-    int cnt = 0, icnt = 0;
-    int row = 0, tail = 0, nb = 0, nib = 0, written = 0, iwritten = 0;
-    if (FILL && active) {
-        row = offsets[i];
-        tail = row + (part ? icounts[i] : 0);
+
+    // ---- stencil cell of this lane
+    int first = 0, cb = 0, code = 0;
+    {
+        int c[3], cc[3];
+        cell_coords<D>(rec_pos<D>(recs[start]), g, dom, c);
+        const int o[3] = {lane % 3 - 1, (lane / 3) % 3 - 1, lane / 9 - 1};
+        bool ok = lane < NS, dup = false;
+        #pragma unroll
+        for (int a = 0; a < D; ++a) {
+            int v = c[a] + o[a];
+            dup |= g.G[a] < 3;
+            if (v < 0) {
+                if (dom.periodic[a]) { v += g.G[a]; code |= 1 << (2 * a); } else ok = false;
+            } else if (v >= g.G[a]) {
+                if (dom.periodic[a]) { v -= g.G[a]; code |= 2 << (2 * a); } else ok = false;
+            }
+            cc[a] = v;
+        }
+        const uint32_t key = ok ? morton<D>(cc) : 0u;
+        if (dup) {      // a cell that an earlier offset reached is left to that one
+            const unsigned int same = __match_any_sync(0xffffffffu, ok ? key : 0xffffff00u + lane);
+            ok = ok && __ffs(same) - 1 == lane;
+        }
+        int cnt = 0;
+        if (ok) { cb = cell_begin[key]; cnt = cell_end[key] - cb; }
+        if (cnt == 0) code = 0;
+        int incl = cnt;
+        #pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, s);
+            if (lane >= s) incl += y;
+        }
+        first = incl - cnt;
     }
-    // the work item's slice of the acceptance-bit pool
+    const int total = __shfl_sync(0xffffffffu, first, 31);       // lanes past the stencil hold no cell
+    const bool shifted = !MI && __any_sync(0xffffffffu, code != 0);
+    __syncwarp();
+    st.first[lane] = first;
+    st.begin[lane] = cb;
+    st.code[lane] = code;
+    __syncwarp();
+
+    // ---- the item's slice of the acceptance-bit pool
     int mbase = -1;
     if (!MI && masks != nullptr) {
         if (!FILL) {
-            int nch = 0;
-            for (int q = 0; q < nk; ++q) nch += (cell_end[keys[q]] - cell_begin[keys[q]] + 31) >> 5;
             if (lane == 0) {
-                const unsigned long long need = 64ull * (unsigned long long)nch;
+                const unsigned long long need = 64ull * (unsigned long long)((total + 31) >> 5);
                 const unsigned long long o = atomicAdd(mask_cursor, need);
                 mbase = o + need <= (unsigned long long)mask_words ? (int)o : -1;
                 mask_base[task] = mbase;
@@ -669,147 +699,152 @@ __device__ __forceinline__ void verlet_task(int task, int lane, int wib, const f
             mbase = mask_base[task];
         }
     }
+
+    int cnt = 0, icnt = 0, inext = 0, rnext = 0;
+    if (FILL && active) {
+        inext = offsets[i];
+        rnext = inext + (part ? icounts[i] : 0);
+    }
+    const bool retest = !FILL || mbase < 0;
     const float4 far = make_float4(3e38f, 3e38f, 3e38f, 0.f);
-    int ch = 0;
-    for (int q = 0; q < nk; ++q) {
-        const int b = cell_begin[keys[q]], e = cell_end[keys[q]];
-        const float sh[3] = {shifts[3 * q], shifts[3 * q + 1], shifts[3 * q + 2]};
-        for (int k0 = b; k0 < e; k0 += 32, ++ch) {
-            if (FILL && mbase >= 0) {
-                const uint32_t m = active ? masks[mbase + 64 * ch + lane] : 0u;
-                const uint32_t im = active ? masks[mbase + 64 * ch + 32 + lane] : 0u;
-                uint32_t U = __reduce_or_sync(0xffffffffu, m);
-                if (U == 0u) continue;
-                __syncwarp();
-                if (k0 + lane < e) sidx[wib][lane] = sort_index[k0 + lane];
-                __syncwarp();
-                // the candidates some lane accepted, in candidate order; each lane files at
-                // most one entry per candidate, so 8 candidates fit between two flushes
-                for (int r = 0; U != 0u; ++r) {
-                    if ((r & 7) == 0 && __any_sync(0xffffffffu, nb > VS - 8 || nib > VS - 8)) {
-                        __syncwarp();
-                        verlet_flush_part(lane, wib, nib, iwritten, row, sibuf, list);
-                        verlet_flush_part(lane, wib, nb, written, tail, sbuf, list);
-                        __syncwarp();
-                    }
-                    const int u = __ffs(U) - 1;
-                    U &= U - 1u;
-                    if ((m >> u) & 1u) {
-                        const int j = sidx[wib][u];
-                        if ((im >> u) & 1u) sibuf[wib][lane][nib++] = j;
-                        else sbuf[wib][lane][nb++] = j;
-                    }
+    // the lane's candidate of a chunk: its sorted position, one chunk ahead of the tests
+    int q = 0;
+    auto locate = [&](int c) {
+        if (c >= total) return -1;
+        while (q < NS - 1 && c >= st.first[q + 1]) ++q;
+        return st.begin[q] + (c - st.first[q]);
+    };
+    int pos = locate(lane), ccode = st.code[q];
+    float4 rc = far;
+    float sc = 0.f;
+    int jc = 0;
+    uint2 mc = make_uint2(0u, 0u);
+    auto fetch = [&](int ch) {
+        rc = far; sc = 0.f; jc = 0; mc = make_uint2(0u, 0u);
+        if (pos >= 0) {
+            if (retest) { rc = recs[pos]; sc = inter[pos]; }
+            if (FILL) jc = sort_index[pos];
+        }
+        if (!retest) mc = reinterpret_cast<const uint2*>(masks + mbase)[32 * ch + lane];
+    };
+    if (total > 0) fetch(0);
+    for (int c0 = 0, ch = 0; c0 < total; c0 += 32, ++ch) {
+        uint32_t hm = mc.x, im = mc.y;
+        const int jcur = jc;
+        if (retest) {
+            __syncwarp();
+            #pragma unroll
+            for (int a = 0; a < D; ++a) {
+                st.x[a][lane] = -(a == 0 ? rc.x : (a == 1 ? rc.y : rc.z));
+                if (shifted) {
+                    const int k = (ccode >> (2 * a)) & 3;
+                    st.sh[a][lane] = k == 1 ? dom.L[a] : (k == 2 ? -dom.L[a] : 0.f);     // minus the image offset
                 }
-                continue;
             }
+            st.T[lane] = -rc.w;
+            st.S[lane] = -sc;
             __syncwarp();
-            const bool real = k0 + lane < e;
-            srec[wib][lane] = real ? recs[k0 + lane] : far;
-            if (FILL && real) sidx[wib][lane] = sort_index[k0 + lane];
+        }
+        if (c0 + 32 < total) {
+            pos = locate(c0 + 32 + lane);
+            ccode = st.code[q];
+            fetch(ch + 1);
+        }
+        if (retest) {
+            const int base = halves ? lane & 16 : 0, m = halves ? 16 : min(32, total - c0);
+            if (MI) verlet_test_chunk<D, VERLET_MIN_IMAGE>(xi, Ti, Si, st, dom, base, m, neg0, hm, im);
+            else if (shifted) verlet_test_chunk<D, VERLET_SHIFT>(xi, Ti, Si, st, dom, base, m, neg0, hm, im);
+            else verlet_test_chunk<D, VERLET_PLAIN>(xi, Ti, Si, st, dom, base, m, neg0, hm, im);
+            if (halves) {
+                hm |= __shfl_down_sync(0xffffffffu, hm, 16) << 16;
+                im |= __shfl_down_sync(0xffffffffu, im, 16) << 16;
+            }
+            if (!active) hm = im = 0u;
+            if (!part) im = 0u;
+        }
+        if (!FILL) {
+            cnt += __popc(hm);
+            icnt += __popc(im);
+            if (mbase >= 0) reinterpret_cast<uint2*>(masks + mbase)[32 * ch + lane] = make_uint2(hm, im);
+        } else {
+            const uint32_t rm = hm & ~im;
             __syncwarp();
-            const int mcount = min(32, e - k0);
-            if constexpr (!FILL) {
-                uint32_t hm = 0, im = 0;
-                if (!MI && sh[0] == 0.f && sh[1] == 0.f && sh[2] == 0.f)
-                    verlet_count_chunk<D, MI, false>(xi, Hi, active, part, srec[wib], sh, dom, vs, mcount, hm, im);
-                else
-                    verlet_count_chunk<D, MI, true>(xi, Hi, active, part, srec[wib], sh, dom, vs, mcount, hm, im);
-                cnt += __popc(hm);
-                icnt += __popc(im);
-                if (mbase >= 0) {
-                    masks[mbase + 64 * ch + lane] = hm;
-                    masks[mbase + 64 * ch + 32 + lane] = im;
-                }
-            } else {
-            for (int u0 = 0; u0 < mcount; u0 += 8) {
-                // room for the next 8 candidates in every lane's buffers
-                if (FILL && __any_sync(0xffffffffu, nb > VS - 8 || nib > VS - 8)) {
-                    __syncwarp();
-                    verlet_flush_part(lane, wib, nib, iwritten, row, sibuf, list);
-                    verlet_flush_part(lane, wib, nb, written, tail, sbuf, list);
-                    __syncwarp();
-                }
+            st.row[lane] = make_uint4(im, rm, (uint32_t)inext, (uint32_t)rnext);
+            __syncwarp();
+            const uint32_t bit = 1u << lane;
+            const uint32_t rows = __ballot_sync(0xffffffffu, hm != 0u);
+            #pragma unroll
+            for (int p0 = 0; p0 < 32; p0 += VW_ROWS) {
+                if (((rows >> p0) & ((1u << VW_ROWS) - 1u)) == 0u) continue;
                 #pragma unroll
-                for (int du = 0; du < 8; ++du) {
-                    const int u = u0 + du;
-                    float r2, Hm, R;
-                    verlet_pair<D, MI>(xi, Hi, srec[wib][u], sh, dom, vs, r2, Hm, R);
-                    const bool hit = active & (r2 < __fmul_rn(R, R));
-                    const bool inter = part && hit && interacting_pair(r2, Hm);
-                    if (hit) {
-                        const int j = sidx[wib][u];
-                        if (inter) sibuf[wib][lane][nib++] = j;
-                        else sbuf[wib][lane][nb++] = j;
-                    }
+                for (int p = p0; p < p0 + VW_ROWS; ++p) {
+                    const uint4 r = st.row[p];
+                    const bool in = (r.x & bit) != 0u;
+                    const uint32_t set = in ? r.x : r.y;
+                    if (set & bit) list[(in ? r.z : r.w) + __popc(set & (bit - 1u))] = jcur;
                 }
             }
-            }
+            inext += __popc(im);
+            rnext += __popc(rm);
         }
     }
-    if (FILL) {
-        if (__any_sync(0xffffffffu, nb > 0 || nib > 0)) {
-            __syncwarp();
-            verlet_flush_part(lane, wib, nib, iwritten, row, sibuf, list);
-            verlet_flush_part(lane, wib, nb, written, tail, sbuf, list);
-            __syncwarp();
-        }
-    } else if (active) {
+    if (!FILL && active) {
         counts[i] = cnt;
         if (part) icounts[i] = icnt;
-        itotal += icnt;
     }
+    return icnt;
 }
 
 template <int D, bool FILL>
-__device__ __noinline__ void verlet_task_min_image(int task, int lane, int wib, const float4* __restrict__ recs,
-                                                   const uint32_t* __restrict__ sorted_keys, const int32_t* __restrict__ tasks,
-                                                   const GridDev& g, const DevParams& P, const int32_t* __restrict__ sort_index,
-                                                   const int32_t* __restrict__ cell_begin, const int32_t* __restrict__ cell_end,
-                                                   int32_t* __restrict__ counts, int32_t* __restrict__ icounts,
-                                                   const int32_t* __restrict__ offsets, int32_t* __restrict__ list, long long& itotal,
-                                                   float4 (*srec)[32], int32_t (*sidx)[32], int32_t (*sbuf)[32][VP],
-                                                   int32_t (*sibuf)[32][VP]) {
-    verlet_task<D, FILL, true>(task, lane, wib, recs, sorted_keys, tasks, g, P, sort_index, cell_begin, cell_end, counts, icounts,
-                               offsets, list, itotal, srec, sidx, sbuf, sibuf, nullptr, nullptr, nullptr, 0);
+__device__ __noinline__ int verlet_task_min_image(int task, int lane, VerletStage& st, const float4* __restrict__ recs,
+                                                  const float* __restrict__ inter, const uint32_t* __restrict__ sorted_keys,
+                                                  const int32_t* __restrict__ tasks, const GridDev& g, const DevParams& P,
+                                                  const int32_t* __restrict__ sort_index, const int32_t* __restrict__ cell_begin,
+                                                  const int32_t* __restrict__ cell_end, int32_t* __restrict__ counts,
+                                                  int32_t* __restrict__ icounts, const int32_t* __restrict__ offsets,
+                                                  int32_t* __restrict__ list) {
+    return verlet_task<D, FILL, true>(task, lane, st, recs, inter, sorted_keys, tasks, g, P, sort_index, cell_begin, cell_end, counts,
+                                      icounts, offsets, list, nullptr, nullptr, nullptr, 0, NEG_ZERO2);
 }
 
 template <int D, bool FILL>
-__global__ void __launch_bounds__(VW_BLOCK)
-k_verlet(const float4* __restrict__ recs, const uint32_t* __restrict__ sorted_keys, const int32_t* __restrict__ tasks,
-         const int32_t* __restrict__ ntasks, const GridDev* __restrict__ gp, DevParams P,
+__global__ void __launch_bounds__(VW_BLOCK, FILL ? 10 : 8)
+k_verlet(const float4* __restrict__ recs, const float* __restrict__ inter, const uint32_t* __restrict__ sorted_keys,
+         const int32_t* __restrict__ tasks, const int32_t* __restrict__ ntasks, const GridDev* __restrict__ gp,
+         const __grid_constant__ DevParams P,
          const int32_t* __restrict__ sort_index, const int32_t* __restrict__ cell_begin, const int32_t* __restrict__ cell_end,
          int32_t* __restrict__ counts, int32_t* __restrict__ icounts, const int32_t* __restrict__ offsets,
          int32_t* __restrict__ list, long long* __restrict__ innz, const long long* __restrict__ nnz, long long capacity,
          uint32_t* __restrict__ masks, int32_t* __restrict__ mask_base, unsigned long long* __restrict__ mask_cursor,
-         long long mask_words, const unsigned int* __restrict__ gate) {
+         long long mask_words, unsigned long long neg0, const unsigned int* __restrict__ gate) {
     if (gate_closed(gate)) return;
-    __shared__ float4 srec[VW_WARPS][32];
-    __shared__ int32_t sidx[FILL ? VW_WARPS : 1][32];
-    __shared__ int32_t sbuf[FILL ? VW_WARPS : 1][32][VP];     // rest of the row
-    __shared__ int32_t sibuf[FILL ? VW_WARPS : 1][32][VP];    // interacting prefix
+    __shared__ VerletStage stage[VW_WARPS];
+    __shared__ unsigned int itotal;
     const bool part = icounts != nullptr;
     if (FILL && *nnz > capacity) return;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    VerletStage& st = stage[threadIdx.x >> 5];
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const int nt = *ntasks;
     const GridDev g = *gp;
     const bool min_image = grid_needs_min_image<D>(g, P.dom);     // uniform over the grid
-    long long itotal = 0;
+    long long sum = 0;
+    if (!FILL && threadIdx.x == 0) itotal = 0u;
     for (int task = warp; task < nt; task += nwarps) {
-        if (min_image)
-            verlet_task_min_image<D, FILL>(task, lane, wib, recs, sorted_keys, tasks, g, P, sort_index, cell_begin, cell_end, counts,
-                                           icounts, offsets, list, itotal, srec, FILL ? sidx : nullptr, FILL ? sbuf : nullptr,
-                                           FILL ? sibuf : nullptr);
-        else
-            verlet_task<D, FILL, false>(task, lane, wib, recs, sorted_keys, tasks, g, P, sort_index, cell_begin, cell_end, counts,
-                                        icounts, offsets, list, itotal, srec, FILL ? sidx : nullptr, FILL ? sbuf : nullptr,
-                                        FILL ? sibuf : nullptr, masks, mask_base, mask_cursor, mask_words);
+        sum += min_image ? verlet_task_min_image<D, FILL>(task, lane, st, recs, inter, sorted_keys, tasks, *gp, P, sort_index, cell_begin,
+                                                          cell_end, counts, icounts, offsets, list)
+                         : verlet_task<D, FILL, false>(task, lane, st, recs, inter, sorted_keys, tasks, g, P, sort_index, cell_begin,
+                                                       cell_end, counts, icounts, offsets, list, masks, mask_base, mask_cursor,
+                                                       mask_words, neg0);
     }
-    if (!FILL && part) {
+    if (!FILL && part) {        // one global addition per block
         #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) itotal += __shfl_xor_sync(0xffffffffu, itotal, o);
-        if (lane == 0 && itotal) atomicAdd(reinterpret_cast<unsigned long long*>(innz), (unsigned long long)itotal);
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        __syncthreads();
+        if (lane == 0 && sum) atomicAdd(&itotal, (unsigned int)sum);
+        __syncthreads();
+        if (threadIdx.x == 0 && itotal) atomicAdd(reinterpret_cast<unsigned long long*>(innz), (unsigned long long)itotal);
     }
 }
 
@@ -865,6 +900,7 @@ struct NbWs {
     int32_t* counts;
     int32_t* tmp;
     float4* recs;
+    float* inter;                     // interacting-test thresholds in sorted order
     int32_t* tasks;
     int32_t* ntasks;
     char* scan;
@@ -893,6 +929,7 @@ static NbWs carve(char* base, int64_t n, int64_t cap) {
     w.counts = reinterpret_cast<int32_t*>(base + off); off += align256(cap * 4);
     w.tmp = reinterpret_cast<int32_t*>(base + off); off += align256(n * 4);
     w.recs = reinterpret_cast<float4*>(base + off); off += align256(n * 16);
+    w.inter = reinterpret_cast<float*>(base + off); off += align256(n * 4);
     w.tasks = reinterpret_cast<int32_t*>(base + off); off += align256(n * 4);
     w.ntasks = reinterpret_cast<int32_t*>(base + off); off += 256;
     w.scan = base + off;
@@ -1192,23 +1229,25 @@ static void build_rows(const DevParams& P, int64_t n, const float* x, const floa
     wsph::count_launch(); k_scatter<<<grid_for(n, 256), 256, 0, s>>>(w.keys, (int)n, cell_end, w.tmp, gate);
     clear(w.ntasks, sizeof(int32_t));
     wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, (k_rank_sort<D><<<grid_for(n, 256), 256, 0, s>>>(w.tmp, w.keys, cell_begin, cell_end, (int)n, x, H,
-                                                                                                 sort_index, sorted_keys, w.recs, w.tasks, w.ntasks,
+                                                                                                 sort_index, sorted_keys, w.recs, w.inter, P.verlet_scale, w.tasks, w.ntasks,
                                                                                                  gate)));
-    int vblocks = grid_for(n, VW_BLOCK);          // >= one warp per 32 particles; warps stride over the work items
-    if (vblocks > 148 * 32) vblocks = 148 * 32;
+    // one warp per 16 particles, usually one per work item (2D cells hold about 20 particles);
+    // blocks past the last item return at once, and with fuller grids the warps stride
+    int vblocks = grid_for(n, VW_BLOCK / 2);
+    if (vblocks > 1 << 16) vblocks = 1 << 16;
     if (part) clear(inter_nnz_out, sizeof(int64_t));
     clear(w.mask_cursor, sizeof(unsigned long long));
-    wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, (k_verlet<D, false><<<vblocks, VW_BLOCK, 0, s>>>(w.recs, sorted_keys, w.tasks, w.ntasks, w.grid, P, sort_index,
+    wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, (k_verlet<D, false><<<vblocks, VW_BLOCK, 0, s>>>(w.recs, w.inter, sorted_keys, w.tasks, w.ntasks, w.grid, P, sort_index,
                                                                                  cell_begin, cell_end, num_neighbors, inter_counts, nullptr,
                                                                                  nullptr, innz, nullptr, 0, w.masks, w.mask_base,
-                                                                                 w.mask_cursor, (long long)w.mask_words, gate)));
+                                                                                 w.mask_cursor, (long long)w.mask_words, NEG_ZERO2, gate)));
     exclusive_scan_i32(num_neighbors, neighbor_offsets, n, w.scan, reinterpret_cast<long long*>(nnz_out), s, gate);
     wsph::count_launch(); k_check_capacity<<<1, 1, 0, s>>>(reinterpret_cast<long long*>(nnz_out), list_capacity, status, gate);
-    wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, (k_verlet<D, true><<<vblocks, VW_BLOCK, 0, s>>>(w.recs, sorted_keys, w.tasks, w.ntasks, w.grid, P, sort_index,
+    wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, (k_verlet<D, true><<<vblocks, VW_BLOCK, 0, s>>>(w.recs, w.inter, sorted_keys, w.tasks, w.ntasks, w.grid, P, sort_index,
                                                                                 cell_begin, cell_end, nullptr, inter_counts, neighbor_offsets,
                                                                                 neighbor_list, nullptr, reinterpret_cast<long long*>(nnz_out),
                                                                                 list_capacity, w.masks, w.mask_base, w.mask_cursor,
-                                                                                (long long)w.mask_words, gate)));
+                                                                                (long long)w.mask_words, NEG_ZERO2, gate)));
 }
 
 // ---------------------------------------------------------------- rebuild as a graph conditional
