@@ -1,0 +1,21 @@
+"""The pair passes' square root and reciprocal (the hardware approximation with one
+Newton-Raphson step) against 64 bits: the step leaves the error below one unit in the last
+place (the approximations' own bounds are 2 and 1 ulp)."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+from warpsph_b200 import build
+
+pytestmark = pytest.mark.gpu
+
+
+def test_newton_step_is_within_one_ulp(cuda, tmp_path):
+    src = Path(__file__).resolve().parent / "native" / "newton_check.cu"
+    exe = tmp_path / "newton_check"
+    subprocess.run([build.nvcc(), *build.ARCH_FLAGS, "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-I", str(build.INCLUDE), "-I",
+                    str(build.CSRC), str(src), "-o", str(exe)], check=True, capture_output=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    assert float(out[1]) <= 1.0 and float(out[3]) <= 1.0, out
+    assert float(out[5]) == 0.0, out

@@ -13,6 +13,7 @@ namespace wsph {
 // ---------------------------------------------------------------- params
 struct DomainF {
     float min[3], max[3], L[3], halfL[3];
+    float invL[3];          // 1 / L of a periodic axis, else 0
     int periodic[3];
 };
 
@@ -128,6 +129,32 @@ template <int D> __device__ __forceinline__ Vec<D> dist_vec(const Vec<D>& xi, co
         r.v[a] = d;
     }
     return r;
+}
+// The same minimum image for the pair sums, with the image number k = rint(d / L) taken by adding
+// and subtracting 1.5 * 2^23: four multiply-add instructions per axis instead of three and four of
+// the half-rate comparison pipe.  d - k L is rounded once, as above, so the result is the same
+// float unless |d| is within a rounding of L / 2, where both images are equally far.
+template <int D> __device__ __forceinline__ Vec<D> pair_vec(const Vec<D>& xi, const Vec<D>& xj, const DomainF& dom) {
+    Vec<D> r;
+    _Pragma("unroll") for (int a = 0; a < D; ++a) {
+        const float d = __fsub_rn(xi.v[a], xj.v[a]);
+        const float k = __fsub_rn(__fmaf_rn(d, dom.invL[a], 12582912.f), 12582912.f);
+        r.v[a] = __fmaf_rn(-k, dom.L[a], d);
+    }
+    return r;
+}
+// sqrt(x) for 0 <= x and 1 / x for normal x > 0: the hardware's approximation and one Newton-Raphson
+// step, within 1 ulp (pair distances and reciprocals of supports and densities).
+__device__ __forceinline__ float sqrt_newton(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(x, 1e-36f)));
+    const float r = x * y;
+    return fmaf(fmaf(-r, r, x), 0.5f * y, r);
+}
+__device__ __forceinline__ float rcp_newton(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(fmaf(-x, y, 1.f), y, y);
 }
 // Squared distance with explicit round-to-nearest steps (no FMA contraction) so the
 // neighbour criterion is bit-identical to the CPU oracle.

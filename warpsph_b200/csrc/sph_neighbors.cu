@@ -85,6 +85,7 @@ int params_to_dev(const SphParams* p, DevParams* o) {
         o->dom.L[a] = (float)(p->domain_max[a] - p->domain_min[a]);
         o->dom.halfL[a] = 0.5f * o->dom.L[a];
         o->dom.periodic[a] = p->periodic[a] ? 1 : 0;
+        o->dom.invL[a] = p->periodic[a] ? 1.f / o->dom.L[a] : 0.f;
         if (a < p->dim && !(o->dom.L[a] > 0.f)) return set_error(SPH_ERR_BAD_ARG, "domain extent along axis %d must be > 0", a);
     }
     o->verlet_scale = (float)p->verlet_scale;
@@ -1091,7 +1092,7 @@ __global__ void k_refilter(const float* __restrict__ x, const float* __restrict_
         float Hj;
         pipe.take(j, xj, Hj);
         if (in_row) {
-            const Vec<D> d = dist_vec<D>(xi, xj, P.dom);
+            const Vec<D> d = pair_vec<D>(xi, xj, P.dom);
             const float Hm = fmaxf(Hi, Hj);
             keep = interacting_pair(dist2_rn<D>(d), Hm);
         }
@@ -1150,10 +1151,10 @@ __global__ void k_refilter_volume(const float* __restrict__ x, const float* __re
         float Hj;
         pipe.take(j, xj, Hj);
         if (in_row) {
-            const Vec<D> d = dist_vec<D>(xi, xj, P.dom);
+            const Vec<D> d = pair_vec<D>(xi, xj, P.dom);
             const float Hm = fmaxf(Hi, Hj);
             keep = interacting_pair(dist2_rn<D>(d), Hm);
-            wsum += kW_inv<KF, D>(safe_sqrt(dot<D>(d, d)), 1.f / Hj);
+            if (keep) wsum += kW_inv<KF, D>(sqrt_newton(dot<D>(d, d)), rcp_newton(Hj));
         }
         const unsigned int kb = (__ballot_sync(0xffffffffu, keep) >> gshift) & ((1u << RF_G) - 1u);
         const unsigned int rb = (__ballot_sync(0xffffffffu, in_row && !keep) >> gshift) & ((1u << RF_G) - 1u);

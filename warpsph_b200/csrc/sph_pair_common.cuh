@@ -82,6 +82,32 @@ template <int KF, int D> __device__ __forceinline__ void kWG_inv(const Vec<D>& x
     for (int a = 0; a < D; ++a) g.v[a] = s * x.v[a];
 }
 
+// W and s with grad_i W = s x_ij; false (and zeros) outside the support.
+template <int KF, int D> __device__ __forceinline__ bool kWS_inv(float r, float invH, float& W, float& s) {
+    const float q = r * invH;
+    if (!(q < 1.f)) { W = 0.f; s = 0.f; return false; }
+    float k, p; kernel_kp<KF, D>(q, k, p);
+    const float cH = KernelTraits<KF, D>::C * ipow<D>(invH);
+    W = cH * k;
+    s = -cH * p * (invH * invH);
+    return true;
+}
+// crk_grad with grad W = s x and its terms gathered by factor:
+//   A (1 + B.x) s x + W (gA (1 + B.x) + A (B + gB^T x))
+template <int D> __device__ __forceinline__ Vec<D> crk_grad_s(const Vec<D>& x, float W, float s, float A, const Vec<D>& B,
+                                                              const Vec<D>& gA, const Mat<D>& gB) {
+    const float bx = 1.f + dot<D>(B, x), cx = A * bx * s, AW = A * W, bW = bx * W;
+    Vec<D> r;
+    #pragma unroll
+    for (int g = 0; g < D; ++g) {
+        float t = B.v[g];
+        #pragma unroll
+        for (int a = 0; a < D; ++a) t += gB.m[a][g] * x.v[a];
+        r.v[g] = cx * x.v[g] + (gA.v[g] * bW + AW * t);
+    }
+    return r;
+}
+
 // Neumaier-compensated accumulator (DevParams::kahan).
 struct KSum {
     float s, c;
