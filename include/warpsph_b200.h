@@ -255,6 +255,20 @@ int sph_neighbors_rewrite(const SphParams* p, int64_t n, const float* x, const f
                           int32_t* counts_out, int32_t* inter_counts, int64_t* inter_nnz_out,
                           float* V_out, int32_t* status, void* stream);
 
+/* The two rewrites above with their gathers from packed words (sph_pack_xh of the same x and
+ * H; null: from x and H). */
+int sph_neighbors_refresh_volume_packed(const SphParams* p, int64_t n, const float* x, const float* H,
+                                        const float* xh, const float* x0, const float* H0,
+                                        const int32_t* neighbor_offsets, const int32_t* num_neighbors,
+                                        const int32_t* neighbor_list, int32_t* list_out,
+                                        int32_t* inter_counts, uint32_t* scratch, int64_t* inter_nnz_out,
+                                        int32_t* status, float* V_out, void* stream);
+int sph_neighbors_rewrite_packed(const SphParams* p, int64_t n, const float* x, const float* H,
+                                 const float* xh, const int32_t* neighbor_offsets, const int32_t* num_neighbors,
+                                 const int32_t* neighbor_list, int32_t* list_out, int32_t* offsets_out,
+                                 int32_t* counts_out, int32_t* inter_counts, int64_t* inter_nnz_out,
+                                 float* V_out, int32_t* status, void* stream);
+
 /* Expands CSR rows into the reference's AdjacencyList.i / .j int64 arrays
  * (io.py:8-20 field names). */
 int sph_neighbors_expand(int64_t n, const int32_t* neighbor_offsets, const int32_t* num_neighbors,
@@ -295,6 +309,13 @@ int sph_adaptive_h_iter(const SphParams* p, int64_t n, int32_t support_mode,
                         const float* hbounds, float* rho_out, float* H_out, float* ratio_out,
                         void* stream);
 
+/* sph_adaptive_h_iter (gather) with the neighbours' positions and masses from packed words:
+ * xm [n][4], sph_pack_xh of x and m. */
+int sph_adaptive_h_iter_packed(const SphParams* p, int64_t n, const float* x, const float* H, const float* m,
+                               const float* xm, const int32_t* offs, const int32_t* cnt, const int32_t* list,
+                               const float* hbounds, float* rho_out, float* H_out, float* ratio_out,
+                               void* stream);
+
 /* min and max of a device array into out2[0], out2[1] (device). */
 int sph_minmax(int64_t n, const float* a, float* out2, void* stream);
 
@@ -322,6 +343,31 @@ int sph_crk_factors_eos(const SphParams* p, int64_t n, const float* x, const flo
                         const int32_t* list, float* A, float* B, float* gradA, float* gradB,
                         float* rho_out, const float* u, float* entropy_out, float* P_out,
                         float* c_out, void* stream);
+
+/* The CRK right-hand side's passes over packed words: four floats per particle, 16-byte
+ * aligned, so that a pair's gathers are one or two 128-bit loads.
+ *   xh [n][4]   position, the support behind it, and below 3D its reciprocal in word 3
+ *   fv [n][4]   velocity; below 3D V and m / rho in words 2 and 3, in 3D V in word 3 and m / rho in vol [n]
+ *   fc [n][4]   velocity; below 3D c and m sgn(div) in words 2 and 3, in 3D c in word 3 and m sgn(div) in msgn [n]
+ * sph_pack_xh writes xh.  sph_crk_factors_packed is sph_crk_factors_eos reading xh, and writes fv
+ * (vol) from v.  sph_grad_v_packed is sph_grad_v without v_sig reading xh and fv, and with div_out
+ * writes fc (msgn).  sph_switch_cullen_packed is sph_switch_cullen with v_sig from xh and fc over
+ * the Verlet rows. */
+int sph_pack_xh(const SphParams* p, int64_t n, const float* x, const float* H, float* xh, void* stream);
+int sph_crk_factors_packed(const SphParams* p, int64_t n, const float* xh, const float* m, const float* V,
+                           const float* v, const int32_t* offs, const int32_t* cnt, const int32_t* list,
+                           float* A, float* B, float* gradA, float* gradB, float* rho_out, const float* u,
+                           float* entropy_out, float* P_out, float* c_out, float* fv, float* vol,
+                           void* stream);
+int sph_grad_v_packed(const SphParams* p, int64_t n, const float* xh, const float* fv, const float* vol,
+                      const float* m, const float* rho, const float* c, const float* A, const float* B,
+                      const float* gradA, const float* gradB, const int32_t* offs, const int32_t* cnt,
+                      const int32_t* list, float* DvDx_out, float* drhodt_out, float* div_out, float* fc,
+                      float* msgn, void* stream);
+int sph_switch_cullen_packed(const SphParams* p, int64_t n, const float* xh, const float* fc, const float* msgn,
+                             const float* rho, const float* div, const float* div_prev,
+                             const float* alpha0_prev, const float* dt, const int32_t* offs,
+                             const int32_t* cnt, const int32_t* list, float* alpha_out, void* stream);
 
 /* Ideal-gas EOS (modules/eos/idealGas.py:6-38 with u and rho given). */
 int sph_eos_ideal_gas(const SphParams* p, int64_t n, const float* u, const float* rho,
@@ -523,6 +569,14 @@ int sph_compsph_balance(const SphParams* p, int64_t n, const float* m, const flo
                         const int32_t* list, const int32_t* inter_counts,
                         const float* ap_ij, const float* av_ij,
                         float* scratch, float* f_ij_out, void* stream);
+
+/* sph_compsph_balance in 3D with each particle's half-step velocity and entropy packed in one
+ * 16-byte word; words: n * 4 floats of scratch, 16-byte aligned. */
+int sph_compsph_balance_packed(const SphParams* p, int64_t n, const float* m, const float* rho,
+                               const float* P, const float* u, const float* v, const float* dvdt,
+                               const float* dt, const int32_t* offs, const int32_t* cnt, const int32_t* list,
+                               const int32_t* inter_counts, const float* ap_ij, const float* av_ij,
+                               float* words, float* f_ij_out, void* stream);
 
 /* sph_compsph_balance without a scratch argument: no counterpart in the reference,
  * which allocates its temporaries through torch.  For callers that cannot allocate

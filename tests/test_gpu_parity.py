@@ -430,3 +430,73 @@ def test_hopkins_corrected_gradient_rank_deficient(cuda):
     assert_close(s2, r_s2, 1e-3, 1e-5, "corrected |S|^2 on a line")
     # traceless symmetric part of diag(g, 0): |S|^2 = g^2 / 2 with g the divergence
     assert_close(s2, 0.5 * div.astype(np.float64) ** 2, 1e-4, 1e-6, "|S|^2 of a rank-one gradient")
+
+
+# below and above the particle count where the passes change their lanes per particle (9,472)
+PACKED = [(1, 300), (1, 9473), (2, 30), (2, 97), (2, 98), (3, 14), (3, 22)]
+
+
+@pytest.mark.parametrize("dim,n_side", PACKED)
+@pytest.mark.parametrize("kernel", [core.KernelFunctions.Wendland2, core.KernelFunctions.B7])
+def test_packed_passes_match_separate_arrays(cuda, dim, n_side, kernel):
+    """The CRK right-hand side's passes over packed words against the same passes over separate
+    arrays: the same sums from the same values, so rounding only (2e-6 of scale; 1e-5 where a
+    sum cancels; alpha as in the oracle comparison)."""
+    cfg, sch, p = make_params(dim, kernel=kernel)
+    P = make_particles(dim, n_side, seed=60 + dim)
+    G = to_gpu(P, cuda)
+    x, H, m, v, u = (G[k] for k in ("positions", "supports", "masses", "velocities", "internalEnergies"))
+    n = len(P["masses"])
+    adj = ops.buildVerletList(x, H, p, p.verlet_scale)
+    hb = ops.minmax(H)
+    rho1, H1, ratio1 = ops.adaptive_h_iter(p, x, H, m, adj, hb)
+    rho0, H0, ratio0 = (torch.empty(n, device=cuda) for _ in range(3))
+    ptr = ops.ptr
+    _capi.check(_capi.lib().sph_adaptive_h_iter(ops._p(p), n, 0, ptr(x), ptr(H), ptr(m), *ops._lists(p, adj, True), ptr(hb), ptr(rho0), ptr(H0),
+                                                ptr(ratio0), ops.stream_ptr(cuda)), "sph_adaptive_h_iter")
+    for a, b, name in ((rho1, rho0, "rho"), (H1, H0, "H"), (ratio1, ratio0, "ratio")):
+        assert_close(a.cpu().numpy(), b.cpu().numpy(), 2e-6, 2e-6, name)
+    xh = ops.pack_xh(p, x, H)
+    V = ops.crk_volume(p, x, H, adj)
+    crk, rho, A, Pr, c, Gv, dr, div, fc, msgn = ops.crk_rhs_fields(p, xh, m, V, v, u, adj, True)
+    crk0, rho_0, A0, Pr0, c0 = ops.crk_factors_eos(p, x, H, m, V, adj, u)
+    Gv0, dr0, div0, _ = ops.grad_v(p, x, H, m, rho_0, V, crk0, v, c0, adj, True)
+    for a, b, tol, name in ((crk.A, crk0.A, 2e-6, "A"), (crk.B, crk0.B, 1e-5, "B"), (crk.gradA, crk0.gradA, 1e-5, "gradA"),
+                            (crk.gradB, crk0.gradB, 1e-5, "gradB"), (rho, rho_0, 2e-6, "density"), (A, A0, 2e-6, "entropy"),
+                            (Pr, Pr0, 2e-6, "pressure"), (c, c0, 2e-6, "sound speed"), (Gv, Gv0, 1e-5, "gradient"), (dr, dr0, 1e-5, "drhodt"),
+                            (div, div0, 1e-5, "divergence")):
+        assert_close(a.cpu().numpy(), b.cpu().numpy(), tol, tol, name)
+    prev, a0 = 0.5 * div0, torch.full((n,), 0.5, device=cuda)
+    al = ops.switch_cullen_packed(p, xh, fc, msgn, rho, div, prev, a0, 1e-3, adj)
+    al0, _, _ = ops.switch_cullen(p, x, H, m, rho, div, prev, None, a0, 1e-3, adj, v=v, c=c)
+    assert_close(al.cpu().numpy(), al0.cpu().numpy(), 1e-3, 1e-3, "alpha")
+    if dim == 3:
+        dvdt, _, ap, av = ops.crk_accel_dudt(p, x, H, m, rho, V, crk, v, c, Pr, Gv, adj)
+        f = ops.compsph_balance(p, m, rho, Pr, u, v, dvdt, 1e-3, adj, ap, av)
+        f0, scratch = torch.empty_like(f), torch.empty(4 * n, device=cuda)
+        _capi.check(_capi.lib().sph_compsph_balance(ops._p(p), n, ptr(m), ptr(rho), ptr(Pr), ptr(u), ptr(v), ptr(dvdt),
+                                                    ptr(ops.dt_tensor(1e-3, cuda)), *ops._csr(adj), ops.iptr(adj.interCounts), ptr(ap), ptr(av),
+                                                    ptr(scratch), ptr(f0), ops.stream_ptr(cuda)), "sph_compsph_balance")
+        # an entry whose energy rounds to either side of zero takes the other particle's share
+        assert (f - f0).abs().gt(1e-5).float().mean().item() < 1e-4
+
+
+@pytest.mark.parametrize("dim,n_side", [(1, 300), (2, 30), (2, 98), (3, 14)])
+def test_packed_rewrite_matches_separate_arrays(cuda, dim, n_side):
+    """The kept list's row rewrite gathering from packed words: the same rows and counts, and the
+    volumes to rounding (2e-6)."""
+    cfg, sch, p = make_params(dim)
+    P = make_particles(dim, n_side, seed=64 + dim)
+    G = to_gpu(P, cuda)
+    x, H = G["positions"], G["supports"]
+    base = ops.buildVerletList(x, H, p, p.verlet_scale)
+    x1 = (x + 0.002 * H.min() * G["velocities"].reshape(x.shape)).contiguous()
+    x1 = torch.where(x1 >= 0.5, x1 - 1.0, torch.where(x1 < -0.5, x1 + 1.0, x1)).contiguous()
+    out = []
+    for xh in (None, ops.pack_xh(p, x1, H)):
+        adj = ops.buildVerletList(x1, H, p, p.verlet_scale, base)
+        assert adj._pending is not None
+        V = ops.crk_volume(p, x1, H, adj, xh)
+        out.append((adj.neighborList, adj.interCounts, V))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert_close(out[1][2].cpu().numpy(), out[0][2].cpu().numpy(), 2e-6, 2e-6, "V")

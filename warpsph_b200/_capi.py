@@ -105,6 +105,14 @@ _PROTOS = {
                             _P, _P, _P, _P],
     "sph_neighbors_refresh": [_P, _I64] + [_P] * 13,
     "sph_neighbors_refresh_volume": [_P, _I64] + [_P] * 14,
+    "sph_neighbors_refresh_volume_packed": [_P, _I64] + [_P] * 15,
+    "sph_neighbors_rewrite_packed": [_P, _I64] + [_P] * 14,
+    "sph_adaptive_h_iter_packed": [_P, _I64] + [_P] * 12,
+    "sph_compsph_balance_packed": [_P, _I64] + [_P] * 16,
+    "sph_pack_xh": [_P, _I64] + [_P] * 4,
+    "sph_crk_factors_packed": [_P, _I64] + [_P] * 19,
+    "sph_grad_v_packed": [_P, _I64] + [_P] * 19,
+    "sph_switch_cullen_packed": [_P, _I64] + [_P] * 13,
     "sph_neighbors_update": [_P, _I64, _P, _P, _P, _P, _P, _I64, _I64] + [_P] * 8 + [_I64] + [_P] * 5,
     "sph_neighbors_rewrite": [_P, _I64] + [_P] * 13,
     "sph_rk_combine_fields": [_P, _I32, _P, _P, _P, _P, _I32, _P, _P, _P, _P],

@@ -1118,13 +1118,27 @@ __global__ void k_refilter(const float* __restrict__ x, const float* __restrict_
 // Verlet neighbour's position and support, and W(r_ij, H_j) is zero past the interacting
 // prefix (r >= max(H_i, H_j) >= H_j), so the whole row can be summed.  The sum runs in
 // the row's original order, 8 lanes per row.
-template <int KF, int D>
+template <int D, bool PK> struct RewriteSource {
+    RewritePipe<D> pipe;
+    __device__ __forceinline__ RewriteSource(const int32_t* l, const float* x, const float* H, const float4*, int q0, int e) : pipe(l, x, H, q0, e) {}
+    __device__ __forceinline__ void take(int, int& j, Vec<D>& xj, float& Hj, float& invHj) { pipe.take(j, xj, Hj); invHj = rcp_newton(Hj); }
+};
+template <int D> struct RewriteSource<D, true> {
+    WordPipe pipe;
+    __device__ __forceinline__ RewriteSource(const int32_t* l, const float*, const float*, const float4* xh, int q0, int e) : pipe(l, xh, q0, e, RF_G) {}
+    __device__ __forceinline__ void take(int q, int& j, Vec<D>& xj, float& Hj, float& invHj) {
+        float4 t;
+        pipe.take(q, j, t);
+        xj = vec_of_word<D>(t); Hj = support_of<D>(t); invHj = inv_support_of<D>(t);
+    }
+};
+template <int KF, int D, bool PK>
 __global__ void k_refilter_volume(const float* __restrict__ x, const float* __restrict__ H, int n, DevParams P,
                                   const unsigned int* __restrict__ acc3, const int32_t* __restrict__ offs,
                                   const int32_t* __restrict__ cnt, const int32_t* __restrict__ list,
                                   int32_t* __restrict__ list_out, int32_t* __restrict__ icnt,
                                   unsigned long long* __restrict__ innz, int32_t* __restrict__ status, float* __restrict__ V,
-                                  int32_t* __restrict__ offs_out, int32_t* __restrict__ cnt_out) {
+                                  int32_t* __restrict__ offs_out, int32_t* __restrict__ cnt_out, const float4* __restrict__ xh) {
     if (acc3 != nullptr && !refresh_valid(acc3)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status, SPH_STATUS_LIST_STALE);
         return;
@@ -1142,19 +1156,19 @@ __global__ void k_refilter_volume(const float* __restrict__ x, const float* __re
     if (valid) { xi = load_vec<D>(x, i); Hi = H[i]; b = offs[i]; c = cnt[i]; }
     int w = 0, rw = 0;
     float wsum = 0.f;
-    RewritePipe<D> pipe(list, x, H, b + sub, b + c);
+    RewriteSource<D, PK> src(list, x, H, xh, b + sub, b + c);
     for (int base = 0; __any_sync(0xffffffffu, base < c); base += RF_G) {
         const bool in_row = base + sub < c;
         bool keep = false;
         int j;
         Vec<D> xj;
-        float Hj;
-        pipe.take(j, xj, Hj);
+        float Hj, invHj;
+        src.take(b + base + sub, j, xj, Hj, invHj);
         if (in_row) {
             const Vec<D> d = pair_vec<D>(xi, xj, P.dom);
             const float Hm = fmaxf(Hi, Hj);
             keep = interacting_pair(dist2_rn<D>(d), Hm);
-            if (keep) wsum += kW_inv<KF, D>(sqrt_newton(dot<D>(d, d)), rcp_newton(Hj));
+            if (keep) wsum += kW_inv<KF, D>(sqrt_newton(dot<D>(d, d)), invHj);
         }
         const unsigned int kb = (__ballot_sync(0xffffffffu, keep) >> gshift) & ((1u << RF_G) - 1u);
         const unsigned int rb = (__ballot_sync(0xffffffffu, in_row && !keep) >> gshift) & ((1u << RF_G) - 1u);
@@ -1249,6 +1263,24 @@ static void build_rows(const DevParams& P, int64_t n, const float* x, const floa
                                                                                 neighbor_list, nullptr, reinterpret_cast<long long*>(nnz_out),
                                                                                 list_capacity, w.masks, w.mask_base, w.mask_cursor,
                                                                                 (long long)w.mask_words, NEG_ZERO2, gate)));
+}
+
+// The fused rewrite with its gathers from packed words (xh) or from x and H.
+static void launch_refilter_volume(const DevParams& P, int64_t n, const float* x, const float* H, const float* xh, const unsigned int* acc3,
+                                   const int32_t* offs, const int32_t* cnt, const int32_t* list, int32_t* list_out, int32_t* icnt,
+                                   int64_t* innz, int32_t* status, float* V, int32_t* offs_out, int32_t* cnt_out, int blocks,
+                                   cudaStream_t s) {
+    unsigned long long* nz = reinterpret_cast<unsigned long long*>(innz);
+    const float4* w = reinterpret_cast<const float4*>(xh);
+    if (xh) {
+        WSPH_DISPATCH_KD(P.kernel, P.dim, (k_refilter_volume<KF, D, true><<<blocks, 256, 0, s>>>(x, H, (int)n, P, acc3, offs, cnt, list,
+                                                                                                list_out, icnt, nz, status, V, offs_out,
+                                                                                                cnt_out, w)));
+    } else {
+        WSPH_DISPATCH_KD(P.kernel, P.dim, (k_refilter_volume<KF, D, false><<<blocks, 256, 0, s>>>(x, H, (int)n, P, acc3, offs, cnt, list,
+                                                                                                 list_out, icnt, nz, status, V, offs_out,
+                                                                                                 cnt_out, w)));
+    }
 }
 
 // ---------------------------------------------------------------- rebuild as a graph conditional
@@ -1442,6 +1474,14 @@ int sph_neighbors_refresh_volume(const SphParams* p, int64_t n, const float* x, 
                                  const int32_t* neighbor_offsets, const int32_t* num_neighbors, const int32_t* neighbor_list,
                                  int32_t* list_out, int32_t* inter_counts, uint32_t* scratch, int64_t* inter_nnz_out,
                                  int32_t* status, float* V_out, void* stream) {
+    return sph_neighbors_refresh_volume_packed(p, n, x, H, nullptr, x0, H0, neighbor_offsets, num_neighbors, neighbor_list, list_out,
+                                               inter_counts, scratch, inter_nnz_out, status, V_out, stream);
+}
+
+int sph_neighbors_refresh_volume_packed(const SphParams* p, int64_t n, const float* x, const float* H, const float* xh, const float* x0,
+                                 const float* H0, const int32_t* neighbor_offsets, const int32_t* num_neighbors, const int32_t* neighbor_list,
+                                 int32_t* list_out, int32_t* inter_counts, uint32_t* scratch, int64_t* inter_nnz_out,
+                                 int32_t* status, float* V_out, void* stream) {
     DevParams P;
     int rc = params_to_dev(p, &P);
     if (rc) return rc;
@@ -1463,11 +1503,8 @@ int sph_neighbors_refresh_volume(const SphParams* p, int64_t n, const float* x, 
     WSPH_DISPATCH_DIM(P.dim, (k_refresh_check<D><<<cblocks, 256, 0, s>>>(x, H, x0, H0, (int)n, P, scratch)));
     const int rblocks = (int)((n * RF_G + 255) / 256);
     wsph::count_launch();
-    WSPH_DISPATCH_KD(P.kernel, P.dim, (k_refilter_volume<KF, D><<<rblocks, 256, 0, s>>>(x, H, (int)n, P, scratch, neighbor_offsets,
-                                                                                       num_neighbors, neighbor_list, list_out,
-                                                                                       inter_counts,
-                                                                                       reinterpret_cast<unsigned long long*>(inter_nnz_out),
-                                                                                       status, V_out, nullptr, nullptr)));
+    launch_refilter_volume(P, n, x, H, xh, scratch, neighbor_offsets, num_neighbors, neighbor_list, list_out, inter_counts, inter_nnz_out,
+                           status, V_out, nullptr, nullptr, rblocks, s);
     return check_launch("sph_neighbors_refresh_volume");
 }
 
@@ -1524,6 +1561,14 @@ int sph_neighbors_rewrite(const SphParams* p, int64_t n, const float* x, const f
                           const int32_t* neighbor_offsets, const int32_t* num_neighbors, const int32_t* neighbor_list,
                           int32_t* list_out, int32_t* offsets_out, int32_t* counts_out, int32_t* inter_counts,
                           int64_t* inter_nnz_out, float* V_out, int32_t* status, void* stream) {
+    return sph_neighbors_rewrite_packed(p, n, x, H, nullptr, neighbor_offsets, num_neighbors, neighbor_list, list_out, offsets_out,
+                                        counts_out, inter_counts, inter_nnz_out, V_out, status, stream);
+}
+
+int sph_neighbors_rewrite_packed(const SphParams* p, int64_t n, const float* x, const float* H, const float* xh,
+                          const int32_t* neighbor_offsets, const int32_t* num_neighbors, const int32_t* neighbor_list,
+                          int32_t* list_out, int32_t* offsets_out, int32_t* counts_out, int32_t* inter_counts,
+                          int64_t* inter_nnz_out, float* V_out, int32_t* status, void* stream) {
     DevParams P;
     int rc = params_to_dev(p, &P);
     if (rc) return rc;
@@ -1540,11 +1585,8 @@ int sph_neighbors_rewrite(const SphParams* p, int64_t n, const float* x, const f
     const int rblocks = (int)((n * RF_G + 255) / 256);
     wsph::count_launch();
     if (V_out) {
-        WSPH_DISPATCH_KD(P.kernel, P.dim, (k_refilter_volume<KF, D><<<rblocks, 256, 0, s>>>(x, H, (int)n, P, nullptr, neighbor_offsets,
-                                                                                           num_neighbors, neighbor_list, list_out,
-                                                                                           inter_counts,
-                                                                                           reinterpret_cast<unsigned long long*>(inter_nnz_out),
-                                                                                           status, V_out, offsets_out, counts_out)));
+        launch_refilter_volume(P, n, x, H, xh, nullptr, neighbor_offsets, num_neighbors, neighbor_list, list_out, inter_counts,
+                               inter_nnz_out, status, V_out, offsets_out, counts_out, rblocks, s);
     } else {
         WSPH_DISPATCH_DIM(P.dim, (k_refilter<D><<<rblocks, 256, 0, s>>>(x, H, (int)n, P, nullptr, neighbor_offsets, num_neighbors,
                                                                          neighbor_list, list_out, inter_counts,

@@ -62,6 +62,62 @@ template <int D> struct RowPipe {
     }
 };
 
+// The same walk over 16-byte words (positions packed with the support, k_pack_xh).
+struct WordPipe {
+    const int32_t* __restrict__ list;
+    const float4* __restrict__ src;
+    int e, step, j1, j2;
+    float4 v1;
+    __device__ __forceinline__ WordPipe(const int32_t* __restrict__ l, const float4* __restrict__ s, int q0, int e_, int st)
+        : list(l), src(s), e(e_), step(st) {
+        j1 = q0 < e_ ? __ldg(l + q0) : 0;
+        j2 = q0 + st < e_ ? __ldg(l + q0 + st) : 0;
+        v1 = __ldg(s + j1);
+    }
+    __device__ __forceinline__ void take(int q, int& j, float4& t) {
+        j = j1;
+        t = v1;
+        j1 = j2;
+        v1 = __ldg(src + j1);
+        j2 = q + 2 * step < e ? __ldg(list + q + 2 * step) : 0;
+    }
+};
+
+// Packed words of the CRK right-hand side, one 16-byte gather each:
+//   xh   position and, behind it, the support; in 1D and 2D its reciprocal in the last word
+//   fv   velocity, then (1D, 2D) V and m / rho in words 2 and 3; in 3D V in the last word and
+//        m / rho in an array of its own
+//   fc   velocity, then (1D, 2D) the sound speed and m sgn(div v) in words 2 and 3; in 3D the sound
+//        speed in the last word and m sgn(div v) in an array of its own
+__device__ __forceinline__ float word_of(const float4& t, int a) { return a == 0 ? t.x : (a == 1 ? t.y : (a == 2 ? t.z : t.w)); }
+template <int D> __device__ __forceinline__ Vec<D> vec_of_word(const float4& t) {
+    Vec<D> r;
+    #pragma unroll
+    for (int a = 0; a < D; ++a) r.v[a] = word_of(t, a);
+    return r;
+}
+template <int D> __device__ __forceinline__ float support_of(const float4& xh) { return word_of(xh, D); }
+template <int D> __device__ __forceinline__ float inv_support_of(const float4& xh) {
+    if constexpr (D == 3) return rcp_newton(xh.w);
+    else return xh.w;
+}
+template <int D> __device__ __forceinline__ float4 make_xh(const Vec<D>& x, float H) {
+    float w[4] = {0.f, 0.f, 0.f, 0.f};
+    #pragma unroll
+    for (int a = 0; a < D; ++a) w[a] = x.v[a];
+    w[D] = H;
+    if (D < 3) w[3] = 1.f / H;
+    return make_float4(w[0], w[1], w[2], w[3]);
+}
+// (v, s, t) of fv and fc: word 2 and 3 below 3D, else the last word and `third`.
+template <int D> __device__ __forceinline__ float4 make_flow(const Vec<D>& v, float s, float t) {
+    float w[4] = {0.f, 0.f, 0.f, 0.f};
+    #pragma unroll
+    for (int a = 0; a < D; ++a) w[a] = v.v[a];
+    if (D < 3) { w[2] = s; w[3] = t; } else { w[3] = s; }
+    return make_float4(w[0], w[1], w[2], w[3]);
+}
+
 template <int G> __host__ __forceinline__ int grid_g(int64_t n) { return (int)((n * G + PAIR_BLOCK - 1) / PAIR_BLOCK); }
 
 // W and grad_i W with a precomputed 1/H.
@@ -120,7 +176,18 @@ struct KSum {
     }
 };
 
-// group sizes (lanes per particle) of the pair passes (a build may override them)
+// Lanes per particle.  The sums of long rows want few lanes (no lane idles, few shuffles), streams
+// of pair arrays more (contiguous rows), and a particle set that does not fill the chip wants many:
+// below WIDE_LIMIT particles (64 per SM) a pass is a chain of dependent loads, shorter with 16 lanes.
+// Microseconds per launch with 4 / 8 / 16 / 32 lanes (Wendland C4; 2D 32, 3D 128 neighbours):
+//                        2D 262,144              3D 884,736                 2D 4,096
+//   CRK accel            173 / 184 / 234 / 329   3189 / 2832 / 2911 / 3381  12.9 / 8.3 / 6.7 / 7.1
+//   energy partition     103 /  88 /  94 / 114   1731 / 1366 / 1213 / 1255  10.8 / 6.9 / 4.9 / 4.0
+//   velocity gradient     63 /  70 /  99 / 159    688 /  723 /  844 / 1126   6.0 / 4.7 / 4.3 / 4.6
+//   Cullen switch         79 /  85 / 100 / 149   1291 / 1190 / 1135 / 1185   7.7 / 5.4 / 4.5 / 4.5
+//   CRK factors           59 /  78 / 127 / 226    718 /  818 / 1072 / 1628   6.8 / 5.2 / 5.0 / 6.3
+//   adaptive support      47 /  52 /  70 / 108   1014 / 1049 / 1101 / 1288   6.2 / 4.5 / 4.0 / 3.9
+// At 25,600 particles in 2D the first column's choices still win; at 8,000 in 3D 8 to 16 lanes.
 #ifndef G_LIGHT
 #define G_LIGHT 8
 #endif
@@ -130,16 +197,21 @@ struct KSum {
 #ifndef G_CRK
 #define G_CRK 4
 #endif
-// Lanes per particle of the light gather passes that walk long rows (adaptive support,
-// CRK volume, velocity gradient, Cullen switch): in 3D, 4 lanes with twice the
-// iterations each beat 8 (measured on the 128^3 Sedov case: Cullen 13.7 -> 10.8 ms,
-// adaptive support 6.1 -> 5.2, velocity gradient 6.9 -> 6.0 per step).
+// Light gather passes that walk long rows (CRK volume and the unpacked passes).
 #define G_SCAN(D) ((D) == 3 ? 4 : G_LIGHT)
-// Lanes per particle of the CRK accel pass: 4 (measured against 8: 0.241 vs 0.245 ms per
-// launch at 512^2 in 2D, 27.6 vs 28.7 ms per step at 128^3 in 3D).
-#ifndef G_ACCEL
-#define G_ACCEL 4
-#endif
+#define G_ACCEL(D) ((D) == 3 ? 8 : 4)
+#define G_BALANCE(D) ((D) == 3 ? 16 : 8)
+#define G_GRADV(D) 4
+#define G_CULLEN(D) ((D) == 3 ? 16 : 4)
+#define G_ADAPT(D) 4
+constexpr int64_t WIDE_LIMIT = 148 * 64;
+#define G_WIDE 16
+// Runs the launch with LG lanes per particle: BASE, or WIDE for small particle sets.
+#define PAIR_LANES(n, BASE, WIDE, ...)                               \
+    do {                                                             \
+        if ((n) <= WIDE_LIMIT) { constexpr int LG = WIDE; __VA_ARGS__; } \
+        else { constexpr int LG = BASE; __VA_ARGS__; }               \
+    } while (0)
 
 #define WSPH_DISPATCH_KDS(params, ...) WSPH_DISPATCH_KD(P.kernel, P.dim, __VA_ARGS__)
 #define WSPH_DISPATCH_DS(params, ...) WSPH_DISPATCH_DIM(P.dim, __VA_ARGS__)

@@ -276,27 +276,29 @@ def _csr(adj: AdjacencyList):
     return iptr(adj.neighborOffsets), iptr(adj.numNeighbors), iptr(adj.neighborList)
 
 
-def _materialize_inter(adj: AdjacencyList, V_out: Optional[torch.Tensor] = None) -> None:
+def _materialize_inter(adj: AdjacencyList, V_out: Optional[torch.Tensor] = None, xh: Optional[torch.Tensor] = None) -> None:
     """Rewrites the rows of a kept prior list with the interacting entries for the
     current positions first (sph_neighbors_refresh).  The rows go to a new tensor:
     earlier stages keep the old order their pairwise arrays are indexed by.  With V_out
-    the CRK volumes of the rewritten rows are computed in the same pass."""
+    the CRK volumes of the rewritten rows are computed in the same pass, its gathers from
+    the packed words xh (pack_xh of the list's positions and supports) when given."""
     if isinstance(adj._pending, _DevicePending):
-        adj._pending.rewrite(adj, V_out)
+        adj._pending.rewrite(adj, V_out, xh)
         return
     params = adj._pending
     n, dev = adj.numRows, adj.neighborList.device
     icnt = torch.empty(n, dtype=torch.int32, device=dev)
     lst = torch.empty(_list_capacity(adj.nnz), dtype=torch.int32, device=dev)
     flags = torch.zeros(4, dtype=torch.int64, device=dev)   # [inter nnz, status (low half), scratch (2 words)]
-    args = (_p(params), n, ptr(adj.queryPositions), ptr(adj.querySupports), ptr(adj._x0), ptr(adj._h0), ptr(adj.neighborOffsets),
-            ptr(adj.numNeighbors), ptr(adj.neighborList), ptr(lst), ptr(icnt), flags.data_ptr() + 16, flags.data_ptr(),
-            flags.data_ptr() + 8)
+    head = (_p(params), n, ptr(adj.queryPositions), ptr(adj.querySupports))
+    args = (ptr(adj._x0), ptr(adj._h0), ptr(adj.neighborOffsets), ptr(adj.numNeighbors), ptr(adj.neighborList), ptr(lst),
+            ptr(icnt), flags.data_ptr() + 16, flags.data_ptr(), flags.data_ptr() + 8)
     with _timed("neighbors_refresh"):
         if V_out is None:
-            check(_capi.lib().sph_neighbors_refresh(*args, stream_ptr(dev)), "sph_neighbors_refresh")
+            check(_capi.lib().sph_neighbors_refresh(*head, *args, stream_ptr(dev)), "sph_neighbors_refresh")
         else:   # the rewrite fused with the CRK volume sum of the rewritten rows
-            check(_capi.lib().sph_neighbors_refresh_volume(*args, fptr(V_out), stream_ptr(dev)), "sph_neighbors_refresh_volume")
+            check(_capi.lib().sph_neighbors_refresh_volume_packed(*head, fptr(xh), *args, fptr(V_out), stream_ptr(dev)),
+                  "sph_neighbors_refresh_volume_packed")
     adj.neighborList, adj.interCounts = lst[: adj.nnz], icnt
     adj._ij = None
     adj._inter_nnz_dev = flags[:1]
@@ -394,7 +396,7 @@ class _DevicePending:
     def __init__(self, lists: DeviceLists, params, generation: int):
         self.lists, self.params, self.generation = lists, params, generation
 
-    def rewrite(self, adj: AdjacencyList, V_out: Optional[torch.Tensor]) -> None:
+    def rewrite(self, adj: AdjacencyList, V_out: Optional[torch.Tensor], xh: Optional[torch.Tensor] = None) -> None:
         nb = self.lists
         if nb.generation != self.generation:
             raise RuntimeError("a device-decided list was used after a later update of the same rows")
@@ -403,10 +405,10 @@ class _DevicePending:
         offs, cnt, icnt = (torch.empty(n, dtype=torch.int32, device=dev) for _ in range(3))
         innz = torch.empty(1, dtype=torch.int64, device=dev)
         with _timed("neighbors_rewrite"):
-            check(_capi.lib().sph_neighbors_rewrite(_p(self.params), n, ptr(adj.queryPositions), ptr(adj.querySupports),
-                                                    ptr(nb.offsets), ptr(nb.counts), ptr(nb.rows), ptr(lst), ptr(offs), ptr(cnt),
-                                                    ptr(icnt), ptr(innz), fptr(V_out) if V_out is not None else None,
-                                                    ptr(nb.status), stream_ptr(dev)), "sph_neighbors_rewrite")
+            check(_capi.lib().sph_neighbors_rewrite_packed(_p(self.params), n, ptr(adj.queryPositions), ptr(adj.querySupports), fptr(xh),
+                                                           ptr(nb.offsets), ptr(nb.counts), ptr(nb.rows), ptr(lst), ptr(offs),
+                                                           ptr(cnt), ptr(icnt), ptr(innz), fptr(V_out), ptr(nb.status),
+                                                           stream_ptr(dev)), "sph_neighbors_rewrite_packed")
         adj.neighborOffsets, adj.numNeighbors, adj.neighborList, adj.interCounts = offs, cnt, lst, icnt
         adj._inter_nnz_dev = innz
         adj._ij = None
@@ -497,19 +499,30 @@ def adaptive_h_iter(params, x, H, m, adj: AdjacencyList, hbounds: torch.Tensor):
     with _timed("adaptive_h_iter"):
         # the supports change right after this pass: a kept list that has not filtered its
         # interacting subset yet is walked over its Verlet rows (W = 0 beyond the support)
-        check(_capi.lib().sph_adaptive_h_iter(_p(params), n, 0, fptr(x), fptr(H), fptr(m), *_lists(params, adj, adj._pending is None),
-                                              fptr(hbounds), ptr(rho), ptr(Hn),
-                                              ptr(ratio), stream_ptr(H.device)), "sph_adaptive_h_iter")
+        xm = pack_xh(params, x, m)
+        check(_capi.lib().sph_adaptive_h_iter_packed(_p(params), n, fptr(x), fptr(H), fptr(m), ptr(xm),
+                                                     *_lists(params, adj, adj._pending is None), fptr(hbounds), ptr(rho), ptr(Hn),
+                                                     ptr(ratio), stream_ptr(H.device)), "sph_adaptive_h_iter_packed")
     return rho, Hn, ratio
 
 
-def crk_volume(params, x, H, adj: AdjacencyList) -> torch.Tensor:
+def pack_xh(params, x, H) -> torch.Tensor:
+    """Positions and supports (or another scalar field) packed in 16-byte words [n, 4] for the
+    passes' gathers (sph_pack_xh)."""
+    xh = _empty((H.shape[0], 4), H)
+    with _timed("pack_xh"):
+        check(_capi.lib().sph_pack_xh(_p(params), H.shape[0], fptr(x), fptr(H), ptr(xh), stream_ptr(H.device)), "sph_pack_xh")
+    return xh
+
+
+def crk_volume(params, x, H, adj: AdjacencyList, xh: Optional[torch.Tensor] = None) -> torch.Tensor:
     """V_i = 1 / sum_j W(r_ij, H_j).  A kept list whose rows still await their rewrite for
-    (x, H) gets it here, fused with the volume sum (sph_neighbors_refresh_volume)."""
+    (x, H) gets it here, fused with the volume sum (sph_neighbors_refresh_volume), gathering
+    from the packed words xh when given."""
     n = H.shape[0]
     V = _empty(n, H)
     if adj is not None and adj._pending is not None and adj.queryPositions is x and adj.querySupports is H:
-        _materialize_inter(adj, V_out=V)
+        _materialize_inter(adj, V_out=V, xh=xh)
         return V
     with _timed("crk_volume"):
         check(_capi.lib().sph_crk_volume(_p(params), n, fptr(x), fptr(H), *_lists(params, adj, True), ptr(V), stream_ptr(H.device)), "sph_crk_volume")
@@ -536,6 +549,42 @@ def crk_factors_eos(params, x, H, m, V, adj: AdjacencyList, u):
                                               ptr(gA), ptr(gB), ptr(rho), fptr(u), ptr(Ae), ptr(P), ptr(c), stream_ptr(H.device)),
               "sph_crk_factors_eos")
     return CRKState(A=A, B=B, gradA=gA, gradB=gB), rho, Ae, P, c
+
+
+def crk_rhs_fields(params, xh, m, V, v, u, adj: AdjacencyList, cullen: bool):
+    """CRK factors with the ideal-gas EOS, then the velocity gradient (and the Cullen divergence),
+    over packed words (sph_crk_factors_packed, sph_grad_v_packed): crk_factors_eos followed by
+    grad_v.  Returns (crk, rho, entropy, P, c, DvDx, drhodt, div, fc, msgn); fc and msgn are the
+    words switch_cullen_packed reads."""
+    n, d = m.shape[0], int(params.dim)
+    A, B, gA, gB, rho = _empty(n, m), _empty((n, d), m), _empty((n, d), m), _empty((n, d, d), m), _empty(n, m)
+    Ae, P, c = _empty(n, m), _empty(n, m), _empty(n, m)
+    fv = _empty((n, 4), m)
+    vol = _empty(n, m) if d == 3 else None
+    rows = _lists(params, adj, True)
+    L = _capi.lib()
+    with _timed("crk_factors"):
+        check(L.sph_crk_factors_packed(_p(params), n, fptr(xh), fptr(m), fptr(V), fptr(v), *rows, ptr(A), ptr(B), ptr(gA), ptr(gB), ptr(rho),
+                                       fptr(u), ptr(Ae), ptr(P), ptr(c), ptr(fv), ptr(vol), stream_ptr(m.device)), "sph_crk_factors_packed")
+    G, drho = _empty((n, d, d), m), _empty(n, m)
+    div = _empty(n, m) if cullen else None
+    fc = _empty((n, 4), m) if cullen else None
+    msgn = _empty(n, m) if cullen and d == 3 else None
+    with _timed("grad_v"):
+        check(L.sph_grad_v_packed(_p(params), n, ptr(xh), ptr(fv), ptr(vol), fptr(m), ptr(rho), ptr(c), ptr(A), ptr(B), ptr(gA), ptr(gB),
+                                  *rows, ptr(G), ptr(drho), ptr(div), ptr(fc), ptr(msgn), stream_ptr(m.device)), "sph_grad_v_packed")
+    return CRKState(A=A, B=B, gradA=gA, gradB=gB), rho, Ae, P, c, G, drho, div, fc, msgn
+
+
+def switch_cullen_packed(params, xh, fc, msgn, rho, div, div_prev, alpha0, dt, adj: AdjacencyList) -> torch.Tensor:
+    """switch_cullen with the signal velocity, over packed words (sph_switch_cullen_packed)."""
+    n = rho.shape[0]
+    al = _empty(n, rho)
+    with _timed("switch_cullen"):
+        check(_capi.lib().sph_switch_cullen_packed(_p(params), n, ptr(xh), ptr(fc), ptr(msgn), fptr(rho), fptr(div), fptr(_f32(div_prev)),
+                                                   fptr(_f32(alpha0)), fptr(dt_tensor(dt, rho.device)), *_lists(params, adj, False),
+                                                   ptr(al), stream_ptr(rho.device)), "sph_switch_cullen_packed")
+    return al
 
 
 def eos_ideal_gas(params, u, rho):
@@ -811,12 +860,12 @@ def compsph_balance(params, m, rho, P, u, v, dvdt, dt, adj: AdjacencyList, ap, a
     """Energy partition f_ij for every Verlet entry."""
     n, d = m.shape[0], int(params.dim)
     f = _pair_empty(adj.nnz, 0, m)
+    entry = _capi.lib().sph_compsph_balance_packed if d == 3 else _capi.lib().sph_compsph_balance
     scratch = _empty(n * (d + 1), m)
     with _timed("compsph_balance"):
-        check(_capi.lib().sph_compsph_balance(_p(params), n, fptr(m), fptr(rho), fptr(P), fptr(u), fptr(v), fptr(dvdt),
-                                              fptr(dt_tensor(dt, m.device)), *_lists(params, adj, False),
-                                              iptr(adj.interCounts) if adj._pending is None else None, fptr(ap), fptr(av),
-                                              ptr(scratch), ptr(f), stream_ptr(m.device)), "sph_compsph_balance")
+        check(entry(_p(params), n, fptr(m), fptr(rho), fptr(P), fptr(u), fptr(v), fptr(dvdt), fptr(dt_tensor(dt, m.device)),
+                    *_lists(params, adj, False), iptr(adj.interCounts) if adj._pending is None else None, fptr(ap), fptr(av),
+                    ptr(scratch), ptr(f), stream_ptr(m.device)), "sph_compsph_balance")
     return f
 
 

@@ -6,10 +6,10 @@ every SPH operation executed by libwarpsph_b200 kernels:
 
   adaptive support (Monaghan Newton)  crkSPH.py:40  -> sph_adaptive_h_iter + sph_density_gather
   Verlet list                         crkSPH.py:54  -> sph_neighbors_build (unchanged prior reused)
-  CRK volume / coefficients / rho     crkSPH.py:61  -> sph_crk_volume + sph_crk_factors_eos
-  ideal-gas EOS                       crkSPH.py:95  -> the epilogue of sph_crk_factors_eos
-  CRK velocity gradient               crkSPH.py:158 -> sph_grad_v (also the Cullen divergence)
-  viscosity switch                    crkSPH.py:195 -> sph_switch_cullen (R and v_sig) / sph_switch_balsara
+  CRK volume / coefficients / rho     crkSPH.py:61  -> sph_crk_volume + sph_crk_factors_packed
+  ideal-gas EOS                       crkSPH.py:95  -> the epilogue of sph_crk_factors_packed
+  CRK velocity gradient               crkSPH.py:158 -> sph_grad_v_packed (also the Cullen divergence)
+  viscosity switch                    crkSPH.py:195 -> sph_switch_cullen_packed (R and v_sig) / sph_switch_balsara
   momentum + energy RHS, dE/dt        crkSPH.py:241,263,330 -> sph_crk_accel_dudt (one fused pass)
   energy partition f_ij               crkSPH.py:343 -> sph_compsph_balance
 """
@@ -143,21 +143,19 @@ def crkSPH_step(system: CompSPHSystem, dt, config: SimulationConfig, compParams:
     adjacency = ops.buildVerletList(S.positions, S.supports, params, config.verletScale, system.adjacency)
     system.adjacency = adjacency
     # crkSPH.py:61 (computeCRKFactors) with crkSPH.py:95-101 (the ideal-gas EOS of the CRK
-    # density) in the epilogue of the same pass
-    V = ops.crk_volume(params, S.positions, S.supports, adjacency)
-    crk, S.densities, S.entropies, S.pressures, S.soundspeeds = ops.crk_factors_eos(params, S.positions, S.supports, S.masses, V,
-                                                                                   adjacency, S.internalEnergies)
-    if S.divergence is None:
-        S.divergence = torch.zeros_like(S.densities)
+    # density) in the epilogue of the same pass, and crkSPH.py:158-172 (the velocity gradient,
+    # with the Cullen divergence in the same pass)
+    xh = ops.pack_xh(params, S.positions, S.supports)
+    V = ops.crk_volume(params, S.positions, S.supports, adjacency, xh)
     switch = compParams.viscositySwitchParams.scheme
     cullen = switch == ViscositySwitch.CullenDehnen2010
-    # crkSPH.py:158-172 (+ the Cullen divergence in the same pass)
-    DvDx, drhodt, div_cd, _ = ops.grad_v(params, S.positions, S.supports, S.masses, S.densities, V, crk, S.velocities,
-                                         S.soundspeeds, adjacency, cullen)
+    crk, S.densities, S.entropies, S.pressures, S.soundspeeds, DvDx, drhodt, div_cd, fc, msgn = ops.crk_rhs_fields(
+        params, xh, S.masses, V, S.velocities, S.internalEnergies, adjacency, cullen)
+    if S.divergence is None:
+        S.divergence = torch.zeros_like(S.densities)
     # crkSPH.py:195-200 (v_sig over the Verlet set is computed inside the switch pass)
     if cullen:
-        S.alphas, _, _ = ops.switch_cullen(params, S.positions, S.supports, S.masses, S.densities, div_cd, S.divergence, None,
-                                           S.alpha0s, dt, adjacency, v=S.velocities, c=S.soundspeeds)
+        S.alphas = ops.switch_cullen_packed(params, xh, fc, msgn, S.densities, div_cd, S.divergence, S.alpha0s, dt, adjacency)
     elif switch == ViscositySwitch.Balsara1995:
         S.alphas = ops.switch_balsara(params, DvDx, S.soundspeeds)
     elif switch == ViscositySwitch.CullenHopkins:
