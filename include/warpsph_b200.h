@@ -492,6 +492,15 @@ int sph_compsph_prep(const SphParams* p, int64_t n, const float* x, const float*
                      const float* m, const float* rho, const float* v,
                      const int32_t* offs, const int32_t* cnt, const int32_t* list,
                      float* omega_out, float* div_out, float* drhodt_out, void* stream);
+/* The same pass over packed words: a first launch packs position with support and velocity with
+ * m and m/rho into words (n * sph_compsph_prep_floats(dim) floats, 16-byte aligned, caller-owned
+ * scratch), and the pair launch gathers each neighbour from them. */
+int sph_compsph_prep_floats(int32_t dim);
+int sph_compsph_prep_packed(const SphParams* p, int64_t n, const float* x, const float* H,
+                            const float* m, const float* rho, const float* v,
+                            const int32_t* offs, const int32_t* cnt, const int32_t* list,
+                            float* omega_out, float* div_out, float* drhodt_out, float* words,
+                            void* stream);
 /* Omega alone, for callers that bind computeOmegaWarp (wp_omega.py:175). */
 int sph_grad_h_omega(const SphParams* p, int64_t n, const float* x, const float* H,
                      const float* m, const float* rho,
@@ -514,10 +523,10 @@ int sph_compsph_accel_dudt(const SphParams* p, int64_t n, const float* x, const 
                            const int32_t* offs, const int32_t* cnt, const int32_t* list,
                            const int32_t* verlet_cnt, float* dvdt_out, float* dudt_out,
                            float* dEdt_out, float* ap_ij, float* av_ij, void* stream);
-/* The same pass over packed particle records: a first launch copies the fields the pass
- * reads into records [n, R] (R = sph_compsph_record_floats(dim) floats per particle: 12, 12
- * and 16 in 1D, 2D and 3D; 16-byte aligned, caller-owned scratch; null c, alpha, omega take
- * their defaults there), and the pair launch gathers each neighbour from that one record.
+/* The same pass over packed particle records: a first launch packs the fields the pass
+ * reads into records (n * R floats, R = sph_compsph_record_floats(dim): 12, 12 and 16 in 1D,
+ * 2D and 3D; 16-byte aligned, caller-owned scratch whose layout is the library's own; null c,
+ * alpha, omega take their defaults there), and the pair launch gathers each neighbour from them.
  * Outputs and arguments otherwise as sph_compsph_accel_dudt. */
 int sph_compsph_record_floats(int32_t dim);
 int sph_compsph_accel_dudt_packed(const SphParams* p, int64_t n, const float* x, const float* H,

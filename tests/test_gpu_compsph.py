@@ -6,6 +6,7 @@ with compatible energy.
 The GPU replaces repeated divisions by reciprocal multiplications and sums each row in
 G interleaved partial sums, so tolerances are relative to each field's scale (stated at
 each assertion)."""
+import ctypes as C
 from pathlib import Path
 
 import numpy as np
@@ -16,7 +17,7 @@ import warpsph_b200 as ws
 from oracle import oracle
 from oracle.steps import SWITCH_CULLEN, SWITCH_HOPKINS, SWITCH_NONE, CompSPHOracle, MonaghanOracle, cell_capacity_for, state_to_numpy
 from tests.cases import assert_close, make_params, make_particles
-from warpsph_b200 import core, ops
+from warpsph_b200 import _capi, core, ops
 from warpsph_b200.core import AdjacencyList
 
 pytestmark = pytest.mark.gpu
@@ -277,3 +278,32 @@ def test_compsph_energy_conservation(cuda):
     c1 = ops.conservation_sums(p, S.masses, S.velocities, S.internalEnergies).cpu().numpy()
     assert abs(c1[3] - c0[3]) / c0[3] < 2e-6, ("total energy drift", c0[3], c1[3])
     assert np.max(np.abs(c1[4:6])) < 1e-6 * np.sqrt(2 * c1[1] * c1[0]) + 1e-12
+
+
+@pytest.mark.parametrize("dim,n_side,kernel,kahan", CASES + [(2, 101, core.KernelFunctions.Wendland6, False), (3, 22, core.KernelFunctions.Wendland2, False)])
+def test_packed_passes_match_separate_arrays(cuda, dim, n_side, kernel, kahan):
+    """The passes over packed words and records against the entry points over separate arrays, for
+    each choice of outputs, below and above the particle count where the lanes change.  Both sum
+    the same terms in FP32 with different lane counts and quotients: a relative 1e-5 of the
+    field's scale is about a hundred roundings."""
+    p, nb, h, d = case_inputs(dim, n_side, kernel, kahan, cuda)
+    adj = built_adjacency(p, d["x"], d["H"])
+    n = d["H"].shape[0]
+    rows = (adj.neighborOffsets.data_ptr(), adj.numNeighbors.data_ptr(), adj.neighborList.data_ptr())
+    lib, st = _capi.lib(), torch.cuda.current_stream().cuda_stream
+    ptrs = [d[k].data_ptr() for k in ("x", "H", "m", "rho", "v")]
+    out = torch.empty(3, n, device=cuda)
+    for want in ((1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 1, 0), (0, 1, 1), (1, 1, 1)):
+        got = ops.compsph_prep(p, d["x"], d["H"], d["m"], d["rho"], d["v"], adj, *(bool(w) for w in want))
+        _capi.check(lib.sph_compsph_prep(C.byref(p), n, *ptrs, *rows, *(out[k].data_ptr() if w else None for k, w in enumerate(want)), st),
+                    "sph_compsph_prep")
+        for k, w in enumerate(want):
+            assert (got[k] is not None) == bool(w)
+            if w:
+                assert_close(got[k].cpu().numpy(), out[k].cpu().numpy(), 1e-5, 1e-5, f"prep output {k} of {want}")
+    dv, du, dE, ap, av = ops.compsph_accel_dudt(p, d["x"], d["H"], d["m"], d["rho"], d["v"], d["c"], d["alpha"], d["P"], None, adj)
+    ref = [torch.empty_like(t) for t in (dv, du, dE, ap, av)]
+    _capi.check(lib.sph_compsph_accel_dudt(C.byref(p), n, *ptrs, d["c"].data_ptr(), d["alpha"].data_ptr(), d["P"].data_ptr(), None, *rows,
+                                           None, *(t.data_ptr() for t in ref), st), "sph_compsph_accel_dudt")
+    for name, a, b in zip(("dvdt", "dudt", "dEdt", "ap", "av"), (dv, du, dE, ap, av), ref):
+        assert_close(a.cpu().numpy(), b.cpu().numpy(), 1e-5, 1e-5, name)

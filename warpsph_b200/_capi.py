@@ -136,6 +136,8 @@ _PROTOS = {
     "sph_crk_accel": [_P, _I64] + [_P] * 21,
     "sph_crk_dudt": [_P, _I64] + [_P] * 18,
     "sph_compsph_prep": [_P, _I64] + [_P] * 12,
+    "sph_compsph_prep_floats": [_I32],
+    "sph_compsph_prep_packed": [_P, _I64] + [_P] * 13,
     "sph_grad_h_omega": [_P, _I64] + [_P] * 9,
     "sph_compsph_accel_dudt": [_P, _I64] + [_P] * 19,
     "sph_compsph_record_floats": [_I32],

@@ -17,6 +17,9 @@
 
 namespace wsph {
 
+#define G_PREP 4
+#define G_COMP(D) ((D) == 3 ? 16 : 8)
+
 // ---------------------------------------------------------------- Omega, divergence, continuity
 // Omega_i = 1 - sum_j (-H_i / (rho_i d)) m_j dW/dH(r_ij, H_i)
 //   (modules/adaptiveSupport/wp_omega.py:11-78, :140; gather support at schemes/compSPH.py:90-97);
@@ -25,49 +28,84 @@ namespace wsph {
 // d rho_i/dt = -(rho_i / Omega_i) (1 / rho_i) sum_j m_j (v_j - v_i) . grad W(r_ij, max(H_i, H_j))
 //   (modules/momentum/consistent.py:8-35, the consistent divergence weighting each
 //   neighbour by m_j / rho_i, so that rho_i cancels).
-template <int KF, int D, int G>
+//
+// Bound by issue slots in 2D and by L1 in 3D.  With PK the neighbours come as two packed 16-byte
+// words per entry (a scalar more in 3D) instead of 7 to 9 scalar gathers; the factors of H_i are
+// out of the Omega sum; roots and reciprocals by Newton steps.  262,144 particles with 32 neighbours:
+// 85 -> 48 us with 4 lanes (8 lanes 55, 16 lanes 76) after 5 us of packing; 884,736 in 3D with 128
+// neighbours 0.66 ms (16 lanes the same); 4,096 in 2D 4.1 us with 16 lanes against 6.1 with 4.
+template <int D>
+__global__ void k_compsph_pack_prep(int n, const float* __restrict__ x, const float* __restrict__ H, const float* __restrict__ m,
+                                    const float* __restrict__ rho, const float* __restrict__ v, float4* __restrict__ xh,
+                                    float4* __restrict__ vm, float* __restrict__ vol) {
+    pdl_entry();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    xh[i] = make_xh<D>(load_vec<D>(x, i), H[i]);
+    const float Vi = m[i] / rho[i];
+    vm[i] = make_flow<D>(v ? load_vec<D>(v, i) : vzero<D>(), m[i], Vi);
+    if (D == 3) vol[i] = Vi;
+}
+
+template <int KF, int D, int G, bool PK>
 __global__ void __launch_bounds__(PAIR_BLOCK)
 k_compsph_prep(int n, DevParams P, const float* __restrict__ x, const float* __restrict__ H, const float* __restrict__ m,
                const float* __restrict__ rho, const float* __restrict__ v,
+               const float4* __restrict__ xh, const float4* __restrict__ vm, const float* __restrict__ vol,
                const int32_t* __restrict__ offs, const int32_t* __restrict__ cnt, const int32_t* __restrict__ list,
                float* __restrict__ omega, float* __restrict__ div, float* __restrict__ drhodt) {
     pdl_entry();
     Grp<G> g(n);
-    const bool want_om = omega != nullptr, want_div = div != nullptr, want_con = drhodt != nullptr;
+    const bool want_om = omega != nullptr, want_div = div != nullptr, want_con = drhodt != nullptr, want_v = want_div || want_con;
     float sdh = 0.f, sdiv = 0.f, scon = 0.f;
     if (g.valid) {
         const int i = g.i;
-        Vec<D> xi = load_vec<D>(x, i);
-        Vec<D> vi = (want_div || want_con) ? load_vec<D>(v, i) : vzero<D>();
-        const float Hi = H[i];
-        int b = offs[i], e = b + cnt[i];
-        RowPipe<D> rp(list, x, b + g.lane, e, G);
+        const Vec<D> xi = load_vec<D>(x, i), vi = want_v ? load_vec<D>(v, i) : vzero<D>();
+        const float invHi = 1.f / H[i];
+        const int b = offs[i], e = b + cnt[i];
+        typename PairPipe<D, PK>::T rp(list, PairPipe<D, PK>::src(x, xh), b + g.lane, e, G);
         for (int q = b + g.lane; q < e; q += G) {
-            int j; Vec<D> xj; rp.take(q, j, xj);
+            int j;
+            Vec<D> xj, vj = vzero<D>();
+            float invHj, mj, Vj = 0.f;
             // every gather of the entry issued together, ahead of the tests that select them
-            const float Hj = __ldg(H + j), mj = __ldg(m + j);
-            const float rhoj = want_div ? __ldg(rho + j) : 1.f;
-            const Vec<D> vj = (want_div || want_con) ? load_vec<D>(v, j) : vzero<D>();
-            Vec<D> xij = dist_vec<D>(xi, xj, P.dom);
-            float r2 = dot<D>(xij, xij);
-            float Hs = wmax(Hi, Hj);
-            if (!(r2 < Hs * Hs)) continue;
-            float r = safe_sqrt(r2);
-            if (want_om && r < Hi) {
-                float W, dWdH;
-                kernelWdH<KF, D>(r, Hi, W, dWdH);
-                sdh += mj * dWdH;
+            if constexpr (PK) {
+                float4 t;
+                rp.take(q, j, t);
+                const float4 f = __ldg(vm + j);
+                if (D == 3 && want_div) Vj = __ldg(vol + j);
+                xj = vec_of_word<D>(t);
+                invHj = inv_support_of<D>(t);
+                vj = vec_of_word<D>(f);
+                mj = D == 3 ? f.w : f.z;
+                if (D < 3) Vj = f.w;
+            } else {
+                rp.take(q, j, xj);
+                const float Hj = __ldg(H + j);
+                mj = __ldg(m + j);
+                if (want_v) vj = load_vec<D>(v, j);
+                if (want_div) Vj = mj * rcp_newton(__ldg(rho + j));
+                invHj = rcp_newton(Hj);
             }
-            if (want_div || want_con) {
-                float W; Vec<D> gS;
-                kWG_inv<KF, D>(xij, r, 1.f / Hs, W, gS);
-                float s = 0.f;
+            const Vec<D> xij = pair_vec<D>(xi, xj, P.dom);
+            const float r = sqrt_newton(dot<D>(xij, xij)), q1 = r * invHi;
+            if (want_om && q1 < 1.f) {
+                // dW/dH = -C / H^(d+1) (d k - q^2 p)
+                float k, p;
+                kernel_kp<KF, D>(q1, k, p);
+                sdh += mj * ((float)D * k - q1 * q1 * p);
+            }
+            float W, s;
+            if (want_v && kWS_inv<KF, D>(r, fminf(invHi, invHj), W, s)) {
+                float dv = 0.f;
                 #pragma unroll
-                for (int a = 0; a < D; ++a) s += (vj.v[a] - vi.v[a]) * gS.v[a];
-                if (want_div) sdiv += mj / rhoj * s;
-                scon += mj * s;
+                for (int a = 0; a < D; ++a) dv += (vj.v[a] - vi.v[a]) * xij.v[a];
+                const float sg = s * dv;
+                sdiv += Vj * sg;
+                scon += mj * sg;
             }
         }
+        sdh *= -(KernelTraits<KF, D>::C * ipow<D>(invHi)) * invHi;
     }
     if (want_om) sdh = gsum<G>(sdh);
     if (want_div) sdiv = gsum<G>(sdiv);
@@ -93,14 +131,20 @@ k_compsph_prep(int n, DevParams P, const float* __restrict__ x, const float* __r
 // (accel.py:195-198).  Walking the interacting prefix of each Verlet row (cnt =
 // interacting counts) with vcnt = the Verlet counts, the ap_ij / av_ij entries of the
 // rest of the row are written as zeros.
-// Packed per-particle record of the CompSPH accel pass: position and support first (read
-// before the distance test), then velocity, mass, density, pressure, sound speed, switch
-// and grad-h factor, in one block of R floats (16-byte granules), so a neighbour is R/4
-// 128-bit loads from one record instead of 2D + 8 scalar loads from as many arrays.  The
-// optional fields take their defaults at pack time (sound speed c_s, switch 1, Omega 1).
+// Packed per-particle record of the CompSPH accel pass: position and support, then velocity,
+// mass, density, pressure, sound speed, switch, the pressure term P / rho^2 / Omega and
+// 1 / rho (both formed once per particle, not once per pair), in R floats, so a neighbour is
+// R/4 128-bit loads instead of 2D + 8 scalar loads from as many arrays.  The optional fields
+// take their defaults at pack time (sound speed c_s, switch 1, Omega 1).  Granule k of
+// particle i is word k n + i: consecutive row entries are mostly consecutive particles, so a
+// load of the lanes covers contiguous words.  Latency bound at 72 registers (40 %
+// of the warps): held to 64 in 2D.  262,144 particles with 32 neighbours: 182 -> 121 us with 8
+// lanes (4 lanes 142, 16 lanes 160; the next record loaded ahead 133, for its registers); 3D,
+// 884,736 with 128 neighbours: 16 lanes 1.97 ms, 8 lanes 2.69, 4 lanes 4.20; 4,096 in 2D: 16
+// lanes 5.2 us, 8 lanes 6.3.
 template <int D> struct CompRec {
-    static constexpr int X = 0, H = D, V = D + 1, M = 2 * D + 1, RHO = M + 1, P = M + 2, C = M + 3, AL = M + 4, OM = M + 5,
-                         END = M + 6, R = (END + 3) / 4 * 4, K1 = (H + 1 + 3) / 4, K2 = R / 4;
+    static constexpr int X = 0, H = D, V = D + 1, M = 2 * D + 1, RHO = M + 1, P = M + 2, C = M + 3, AL = M + 4, PT = M + 5,
+                         IR = M + 6, END = M + 7, R = (END + 3) / 4 * 4;
 };
 
 template <int D>
@@ -116,25 +160,28 @@ __global__ void k_compsph_pack(int n, DevParams P, const float* __restrict__ x, 
     #pragma unroll
     for (int a = 0; a < D; ++a) { r[L::X + a] = x[(size_t)i * D + a]; r[L::V + a] = v[(size_t)i * D + a]; }
     r[L::H] = H[i]; r[L::M] = m[i]; r[L::RHO] = rho[i]; r[L::P] = Pr[i];
-    r[L::C] = c ? c[i] : P.c_s; r[L::AL] = alpha ? alpha[i] : 1.f; r[L::OM] = omega ? omega[i] : 1.f;
+    r[L::C] = c ? c[i] : P.c_s; r[L::AL] = alpha ? alpha[i] : 1.f;
+    r[L::PT] = Pr[i] / (rho[i] * rho[i]) / (omega ? omega[i] : 1.f);
+    r[L::IR] = 1.f / rho[i];
     #pragma unroll
     for (int a = L::END; a < L::R; ++a) r[a] = 0.f;
-    float4* dst = reinterpret_cast<float4*>(rec + (size_t)i * L::R);
+    float4* dst = reinterpret_cast<float4*>(rec) + i;
     #pragma unroll
-    for (int k = 0; k < L::R / 4; ++k) dst[k] = make_float4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+    for (int k = 0; k < L::R / 4; ++k) dst[(size_t)k * n] = make_float4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
 }
 
-template <int D, int K0, int K1>
-__device__ __forceinline__ void comp_granules(const float4* __restrict__ src, float (&r)[CompRec<D>::R]) {
+template <int D>
+__device__ __forceinline__ void comp_record(const float* __restrict__ rec, int n, int j, float (&r)[CompRec<D>::R]) {
+    const float4* src = reinterpret_cast<const float4*>(rec) + j;
     #pragma unroll
-    for (int k = K0; k < K1; ++k) {
-        const float4 t = __ldg(src + k);
+    for (int k = 0; k < CompRec<D>::R / 4; ++k) {
+        const float4 t = __ldg(src + (size_t)k * n);
         r[4 * k] = t.x; r[4 * k + 1] = t.y; r[4 * k + 2] = t.z; r[4 * k + 3] = t.w;
     }
 }
 
 template <int KF, int D, int G, bool REC>
-__global__ void __launch_bounds__(PAIR_BLOCK)
+__global__ void __launch_bounds__(PAIR_BLOCK, D == 3 ? 1 : 8)
 k_compsph_accel_dudt(int n, DevParams P, const float* __restrict__ x, const float* __restrict__ H, const float* __restrict__ m,
                      const float* __restrict__ rho, const float* __restrict__ v, const float* __restrict__ c,
                      const float* __restrict__ alpha, const float* __restrict__ Pr, const float* __restrict__ omega,
@@ -153,31 +200,34 @@ k_compsph_accel_dudt(int n, DevParams P, const float* __restrict__ x, const floa
         const int i = g.i;
         using L = CompRec<D>;
         Vec<D> xi, vi;
-        float Hi, rhoi, Pi, ci, ai, omi;
+        float Hi, rhoi, Pi, ci, ai, pTi, irhoi;
         if constexpr (REC) {
             float r[L::R];
-            comp_granules<D, 0, L::K2>(reinterpret_cast<const float4*>(rec + (size_t)i * L::R), r);
+            comp_record<D>(rec, n, i, r);
             #pragma unroll
             for (int a = 0; a < D; ++a) { xi.v[a] = r[L::X + a]; vi.v[a] = r[L::V + a]; }
-            Hi = r[L::H]; rhoi = r[L::RHO]; Pi = r[L::P]; ci = r[L::C]; ai = r[L::AL]; omi = r[L::OM];
+            Hi = r[L::H]; rhoi = r[L::RHO]; Pi = r[L::P]; ci = r[L::C]; ai = r[L::AL];
+            pTi = r[L::PT]; irhoi = r[L::IR];
         } else {
             xi = load_vec<D>(x, i); vi = load_vec<D>(v, i);
             Hi = H[i]; rhoi = rho[i]; Pi = Pr[i];
-            ci = c ? c[i] : P.c_s; ai = alpha ? alpha[i] : 1.f; omi = omega ? omega[i] : 1.f;
+            ci = c ? c[i] : P.c_s; ai = alpha ? alpha[i] : 1.f;
+            pTi = Pi / (rhoi * rhoi) / (omega ? omega[i] : 1.f);
+            irhoi = 1.f / rhoi;
         }
         const float invHi = 1.f / Hi;
-        const float pTi = Pi / (rhoi * rhoi) / omi;
         int b = offs[i], e = b + cnt[i];
+        int jn = b + g.lane < e ? __ldg(list + b + g.lane) : 0;   // the neighbour index one entry ahead
         for (int q = b + g.lane; q < e; q += G) {
-            int j, k; entry(list, q, j, k);
+            const int j = jn, k = q;
+            if (q + G < e) jn = __ldg(list + q + G);
             float rj[L::R];
-            const float4* sj = REC ? reinterpret_cast<const float4*>(rec + (size_t)j * L::R) : nullptr;
             Vec<D> xj;
             float Hj;
             if constexpr (REC) {
-                // the first two groups issued together (walked rows are interacting prefixes, so
-                // the range test below almost never discards the second)
-                comp_granules<D, 0, L::K2>(sj, rj);
+                // the whole record at once (walked rows are interacting prefixes, so the range test
+                // below almost never discards it)
+                comp_record<D>(rec, n, j, rj);
                 #pragma unroll
                 for (int a = 0; a < D; ++a) xj.v[a] = rj[L::X + a];
                 Hj = rj[L::H];
@@ -185,7 +235,7 @@ k_compsph_accel_dudt(int n, DevParams P, const float* __restrict__ x, const floa
                 xj = load_vec<D>(x, j);
                 Hj = __ldg(H + j);
             }
-            Vec<D> xij = dist_vec<D>(xi, xj, P.dom);
+            Vec<D> xij = pair_vec<D>(xi, xj, P.dom);
             float r2 = dot<D>(xij, xij);
             float Hm = wmax(Hi, Hj);
             if (!(r2 < Hm * Hm)) {
@@ -193,41 +243,41 @@ k_compsph_accel_dudt(int n, DevParams P, const float* __restrict__ x, const floa
                 if (av) store_vec<D>(av, k, vzero<D>());
                 continue;
             }
-            float r = safe_sqrt(r2);
+            float r = sqrt_newton(r2);
             Vec<D> vj;
-            float mj, rhoj, Pj, cj, aj, omj;
+            float mj, rhoj, Pj, cj, aj, pTj, irhoj;
             if constexpr (REC) {
                 #pragma unroll
                 for (int a = 0; a < D; ++a) vj.v[a] = rj[L::V + a];
-                mj = rj[L::M]; rhoj = rj[L::RHO]; Pj = rj[L::P]; cj = rj[L::C]; aj = rj[L::AL]; omj = rj[L::OM];
+                mj = rj[L::M]; rhoj = rj[L::RHO]; Pj = rj[L::P]; cj = rj[L::C]; aj = rj[L::AL]; pTj = rj[L::PT]; irhoj = rj[L::IR];
             } else {
                 vj = load_vec<D>(v, j);
                 mj = __ldg(m + j); rhoj = __ldg(rho + j); Pj = __ldg(Pr + j);
-                cj = c ? __ldg(c + j) : P.c_s; aj = alpha ? __ldg(alpha + j) : 1.f; omj = omega ? __ldg(omega + j) : 1.f;
+                cj = c ? __ldg(c + j) : P.c_s; aj = alpha ? __ldg(alpha + j) : 1.f;
+                irhoj = rcp_newton(rhoj);
+                pTj = Pj * irhoj * irhoj * (omega ? rcp_newton(__ldg(omega + j)) : 1.f);
             }
-            const float Vj = mj / rhoj;
+            const float Vj = mj * irhoj;
             const float rho_bar = 0.5f * (rhoi + rhoj);
             float ux = 0.f;
             #pragma unroll
             for (int a = 0; a < D; ++a) ux += (vi.v[a] - vj.v[a]) * xij.v[a];
-            const float pi_i = pi_actual(P, D, r, ux, Hi, Hj, rhoi, rhoj, Pi, Pj, true, ci, cj, ai, aj, false, false) * (rho_bar / rhoi);
-            const float pi_j = pi_actual(P, D, r, ux, Hi, Hj, rhoi, rhoj, Pi, Pj, true, ci, cj, ai, aj, true, false) * (rho_bar / rhoj);
-            float Wi, Wj; Vec<D> gi, gj;
-            kWG_inv<KF, D>(xij, r, invHi, Wi, gi);
-            kWG_inv<KF, D>(xij, r, 1.f / Hj, Wj, gj);
-            const float pTj = Pj / (rhoj * rhoj) / omj;
+            const float pi_i = pi_actual(P, D, r, ux, Hi, Hj, rhoi, rhoj, Pi, Pj, true, ci, cj, ai, aj, false, false) * (rho_bar * irhoi);
+            const float pi_j = pi_actual(P, D, r, ux, Hi, Hj, rhoi, rhoj, Pi, Pj, true, ci, cj, ai, aj, true, false) * (rho_bar * irhoj);
+            float Wi, Wj, si, sj;                        // grad W(H_i) = s_i x_ij, grad W(H_j) = s_j x_ij
+            kWS_inv<KF, D>(r, invHi, Wi, si);
+            kWS_inv<KF, D>(r, rcp_newton(Hj), Wj, sj);
             // (v_j - v_i) . x_ij / (r + 1e-14 H_i)
-            const float mu = -ux / (r + 1.0e-14f * Hi);
+            const float mu = -ux * rcp_newton(r + 1.0e-14f * Hi);
+            const float sk = 0.5f * (si + sj), cp = -(pTi + pTj) * mj * sk, cv = -0.5f * (pi_i + pi_j) * Vj * mu * sk;
             Vec<D> pt, vt;
-            float dotg = 0.f;
             #pragma unroll
             for (int a = 0; a < D; ++a) {
-                const float gw = 0.5f * (gi.v[a] + gj.v[a]);
-                pt.v[a] = -(pTi * gw + pTj * gw) * mj;
-                vt.v[a] = -0.5f * (pi_i * gw + pi_j * gw) * Vj * mu;
+                pt.v[a] = cp * xij.v[a];
+                vt.v[a] = cv * xij.v[a];
                 acc[a].add(pt.v[a] + vt.v[a], comp);
-                dotg += (vj.v[a] - vi.v[a]) * gi.v[a];
             }
+            const float dotg = -si * ux;
             if (ap) store_vec<D>(ap, k, pt);
             if (av) store_vec<D>(av, k, vt);
             const float pTerm = -Vj * pTi * rhoj * dotg;
@@ -257,9 +307,11 @@ k_compsph_accel_dudt(int n, DevParams P, const float* __restrict__ x, const floa
         Vec<D> vi;
         float mi;
         if constexpr (REC) {
+            float r[CompRec<D>::R];
+            comp_record<D>(rec, n, i, r);
             #pragma unroll
-            for (int a = 0; a < D; ++a) vi.v[a] = __ldg(rec + (size_t)i * CompRec<D>::R + CompRec<D>::V + a);
-            mi = __ldg(rec + (size_t)i * CompRec<D>::R + CompRec<D>::M);
+            for (int a = 0; a < D; ++a) vi.v[a] = r[CompRec<D>::V + a];
+            mi = r[CompRec<D>::M];
         } else {
             vi = load_vec<D>(v, i);
             mi = m[i];
@@ -392,9 +444,31 @@ int sph_compsph_prep(const SphParams* p, int64_t n, const float* x, const float*
     if (!omega_out && !div_out && !drhodt_out) return SPH_OK;
     if ((rc = check_align_vec(P, x, "x")) || (rc = check_align_vec(P, v, "v"))) return rc;
     wsph::count_launch();
-    WSPH_DISPATCH_KDS(*p, (launch_pdl(k_compsph_prep<KF, D, G_LIGHT>, grid_g<G_LIGHT>(n), PAIR_BLOCK, 0, s, (int)n, P, x, H, m, rho, v, offs, cnt, list,
+    WSPH_DISPATCH_KDS(*p, (launch_pdl(k_compsph_prep<KF, D, G_LIGHT, false>, grid_g<G_LIGHT>(n), PAIR_BLOCK, 0, s, (int)n, P, x, H, m, rho, v, nullptr, nullptr, nullptr, offs, cnt, list,
                                                                                                         omega_out, div_out, drhodt_out)));
     return check_launch("sph_compsph_prep");
+}
+
+int sph_compsph_prep_floats(int32_t dim) { return dim == 3 ? 9 : dim == 1 || dim == 2 ? 8 : 0; }
+
+int sph_compsph_prep_packed(const SphParams* p, int64_t n, const float* x, const float* H, const float* m, const float* rho,
+                            const float* v, const int32_t* offs, const int32_t* cnt, const int32_t* list, float* omega_out,
+                            float* div_out, float* drhodt_out, float* words, void* stream) {
+    PAIR_PRELUDE();
+    WSPH_CHECK_PTR(x); WSPH_CHECK_PTR(H); WSPH_CHECK_PTR(m); WSPH_CHECK_PTR(rho); WSPH_CHECK_PTR(words); CHECK_CSR();
+    if (div_out || drhodt_out) WSPH_CHECK_PTR(v);
+    if (!omega_out && !div_out && !drhodt_out) return SPH_OK;
+    if ((rc = check_align_vec(P, x, "x")) || (rc = check_align_vec(P, v, "v"))) return rc;
+    if (reinterpret_cast<uintptr_t>(words) & 15) return set_error(SPH_ERR_BAD_ARG, "sph_compsph_prep_packed: words must be 16-byte aligned");
+    float4* xh = reinterpret_cast<float4*>(words);
+    float4* vm = xh + n;
+    float* vol = reinterpret_cast<float*>(vm + n);           // 3D only
+    wsph::count_launch();
+    WSPH_DISPATCH_DS(*p, (launch_pdl(k_compsph_pack_prep<D>, (unsigned)((n + 255) / 256), 256, 0, s, (int)n, x, H, m, rho, v, xh, vm, vol)));
+    wsph::count_launch();
+    PAIR_LANES(n, G_PREP, G_WIDE, WSPH_DISPATCH_KDS(*p, (launch_pdl(k_compsph_prep<KF, D, LG, true>, grid_g<LG>(n), PAIR_BLOCK, 0, s, (int)n, P, x, H, m, rho, v, xh, vm, vol,
+                                                                    offs, cnt, list, omega_out, div_out, drhodt_out))));
+    return check_launch("sph_compsph_prep_packed");
 }
 
 int sph_grad_h_omega(const SphParams* p, int64_t n, const float* x, const float* H, const float* m, const float* rho,
@@ -440,8 +514,8 @@ int sph_compsph_accel_dudt_packed(const SphParams* p, int64_t n, const float* x,
     WSPH_DISPATCH_DS(*p, (launch_pdl(k_compsph_pack<D>, (unsigned)((n + 255) / 256), 256, 0, s, (int)n, P, x, H, m, rho, v, c, alpha, Pr, omega,
                                                                                         records)));
     wsph::count_launch();
-    WSPH_DISPATCH_KDS(*p, (launch_pdl(k_compsph_accel_dudt<KF, D, G_HEAVY, true>, grid_g<G_HEAVY>(n), PAIR_BLOCK, 0, s, (int)n, P, x, H, m, rho, v, c, alpha, Pr, omega, records, offs, cnt, list, verlet_cnt, dvdt_out, dudt_out,
-                              dEdt_out, ap_ij, av_ij)));
+    WSPH_DISPATCH_KDS(*p, PAIR_LANES(n, G_COMP(D), G_WIDE, launch_pdl(k_compsph_accel_dudt<KF, D, LG, true>, grid_g<LG>(n), PAIR_BLOCK, 0, s, (int)n, P, x, H, m, rho, v, c, alpha, Pr, omega, records, offs, cnt, list, verlet_cnt,
+                                                                    dvdt_out, dudt_out, dEdt_out, ap_ij, av_ij)));
     return check_launch("sph_compsph_accel_dudt_packed");
 }
 

@@ -83,6 +83,16 @@ struct WordPipe {
     }
 };
 
+// The row walk of a pass over packed words or over separate arrays.
+template <int D, bool PK> struct PairPipe {
+    using T = RowPipe<D>;
+    static __device__ __forceinline__ const float* src(const float* x, const float4*) { return x; }
+};
+template <int D> struct PairPipe<D, true> {
+    using T = WordPipe;
+    static __device__ __forceinline__ const float4* src(const float*, const float4* xh) { return xh; }
+};
+
 // Packed words of the CRK right-hand side, one 16-byte gather each:
 //   xh   position and, behind it, the support; in 1D and 2D its reciprocal in the last word
 //   fv   velocity, then (1D, 2D) V and m / rho in words 2 and 3; in 3D V in the last word and

@@ -63,15 +63,6 @@ template <int D> __device__ __forceinline__ float volume_to_support(float V, flo
     else return powf(nH * V / 3.14159265358979f * 3.f / 4.f, 1.f / 3.f);
 }
 
-// The row walk of a pass over packed words or over separate arrays.
-template <int D, bool PK> struct PairPipe {
-    using T = RowPipe<D>;
-    static __device__ __forceinline__ const float* src(const float* x, const float4*) { return x; }
-};
-template <int D> struct PairPipe<D, true> {
-    using T = WordPipe;
-    static __device__ __forceinline__ const float4* src(const float*, const float4* xh) { return xh; }
-};
 // One Newton iteration of modules/adaptiveSupport/optimalSupportMonaghan.py:87-125
 // with Omega of modules/adaptiveSupport/wp_omega.py:40-60 (gather support).
 // The neighbours' positions and masses come packed in one 16-byte word each (xm: sph_pack_xh of

@@ -23,15 +23,16 @@ __device__ __forceinline__ float pi_actual(const DevParams& P, int dim, float r,
     const int term = thermal ? P.conductivity_term : P.viscosity_term;
     // compute_mu_ij (util.py:6-38)
     const float den = r + 1e-14f * h_bar;
-    const float mu0 = ux / den;
-    const float sfac = h_bar / xi / den;
+    const float rden = rcp_newton(den), rxi = rcp_newton(xi);      // quotients as products with 1-ulp reciprocals
+    const float mu0 = ux * rden;
+    const float sfac = h_bar * rxi * rden;
     float mu, sf;
     switch (term) {
         case SPH_VISC_CLEARY1998: case SPH_VISC_MONAGHAN1997A: case SPH_VISC_MONAGHAN1997B: case SPH_VISC_DUKOWICZ:
         case SPH_VISC_PRICE2012_98: case SPH_VISC_PRICE2012: case SPH_VISC_PRICE2008: case SPH_VISC_WADSLEY2008:
             mu = mu0; sf = 1.f; break;
         case SPH_VISC_MONAGHAN1992: mu = mu0 * sfac; sf = 1.f * sfac; break;
-        default: mu = mu0 * sfac; sf = h_bar / xi; break;      // Default, MonaghanGingold1983, DeltaSPH
+        default: mu = mu0 * sfac; sf = h_bar * rxi; break;      // Default, MonaghanGingold1983, DeltaSPH
     }
     // compute_bars (util.py:40-134)
     bool ub_rho = true, ub_c = true, ub_h = true;
@@ -62,7 +63,7 @@ __device__ __forceinline__ float pi_actual(const DevParams& P, int dim, float r,
         case SPH_VISC_WADSLEY2008: v_sig = C_l * fabsf(mu); break;
         default: v_sig = C_l * c - C_q * mu; break;          // DeltaSPH, Default
     }
-    float val = rhoj * 1.f / rho * v_sig * sf;
+    float val = rhoj * rcp_newton(rho) * v_sig * sf;
     if (P.monaghan_switch && !thermal && ux > 0.f) val = 0.f;
     return val;
 }

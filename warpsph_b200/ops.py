@@ -809,9 +809,11 @@ def compsph_prep(params, x, H, m, rho, v, adj: AdjacencyList, grad_h: bool = Tru
     om = _empty(n, H) if grad_h else None
     div = _empty(n, H) if want_div else None
     dr = _empty(n, H) if want_drhodt else None
+    words = _empty(n * int(_capi.lib().sph_compsph_prep_floats(int(params.dim))), H)
     with _timed("compsph_prep"):
-        check(_capi.lib().sph_compsph_prep(_p(params), n, fptr(x), fptr(H), fptr(m), fptr(rho), fptr(v), *_lists(params, adj, True),
-                                           ptr(om), ptr(div), ptr(dr), stream_ptr(H.device)), "sph_compsph_prep")
+        check(_capi.lib().sph_compsph_prep_packed(_p(params), n, fptr(x), fptr(H), fptr(m), fptr(rho), fptr(v),
+                                                  *_lists(params, adj, True), ptr(om), ptr(div), ptr(dr), ptr(words),
+                                                  stream_ptr(H.device)), "sph_compsph_prep_packed")
     return om, div, dr
 
 
