@@ -194,3 +194,23 @@ def test_learned_warm_start_gain(cuda):
     d = tot["density"]
     assert d["learned"][2] == 0 and d["plain"][2] == 0, d
     assert d["learned"][0] <= 0.7 * d["plain"][0], d
+
+
+@pytest.mark.parametrize("tiles", [1, 147, 148, 149, 2 * 148, 3 * 148 + 1, 4 * 148 - 1, 7 * 148 + 5])
+def test_mlp_gradient_adds_up(cuda, tiles):
+    """The gradient over 2 m samples against the mean of those over its halves, m = 128 x tiles, for
+    every number of tiles per SM modulo the three in flight.  dy of a half is exactly twice that of
+    the whole, so all BF16 roundings agree and only the FP32 sums are ordered differently: 2e-4 of
+    a block's largest entry is 3000 roundings of it."""
+    m = 128 * tiles
+    rng = np.random.default_rng(tiles)
+    th = torch.from_numpy(random_net(3)).to(cuda)
+    x = torch.from_numpy(rng.standard_normal((2 * m, 8)).astype(np.float32)).to(cuda)
+    t = torch.from_numpy(rng.standard_normal(2 * m).astype(np.float32)).to(cuda)
+    g, loss = ops.mlp_grad(th, x, t, tensor_cores="tcgen05")
+    (ga, la), (gb, lb) = (ops.mlp_grad(th, x[s], t[s], tensor_cores="tcgen05") for s in (slice(0, m), slice(m, 2 * m)))
+    assert int(ops.mlp_status(cuda).item()) == 0
+    ref = 0.5 * (ga.double() + gb.double())
+    for name, a, b in BLOCKS:
+        assert_close(g[a:b].cpu().numpy(), ref[a:b].cpu().numpy(), 2e-4, 2e-4, f"d loss / d {name}")
+    assert abs(float(loss) - (float(la) + float(lb))) <= 1e-6 * float(loss)        # the loss is a sum

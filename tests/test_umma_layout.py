@@ -35,3 +35,17 @@ def test_umma_layout_matches_cute(tmp_path):
     assert r.returncode == 0, r.stderr[-3000:]
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0 and out.stdout.strip().endswith("ok"), out.stdout + out.stderr
+
+
+def test_umma_mn_major_matches_cute(tmp_path):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    inc = _cutlass_include()
+    if not os.path.exists(nvcc) or inc is None:
+        pytest.skip("nvcc or a CUTLASS header tree with the sm100 UMMA traits is not available")
+    exe = tmp_path / "umma_mn_check"
+    src = os.path.join(ROOT, "tests", "native", "umma_mn_check.cu")
+    r = subprocess.run([nvcc, "-std=c++17", "-w", "-I", inc, "-I", os.path.join(ROOT, "warpsph_b200", "csrc"), "-I",
+                        os.path.join(ROOT, "include"), "-o", str(exe), src], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0 and out.stdout.strip().endswith("ok"), out.stdout + out.stderr

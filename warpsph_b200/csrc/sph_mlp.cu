@@ -549,349 +549,450 @@ k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restri
 
 // ---------------------------------------------------------------- training on tcgen05
 // The gradient of the mean squared error with every GEMM on the tensor cores.  One CTA per
-// SM (4 warps, one sample per thread and TMEM lane) loops over 128-sample tiles:
+// SM: three warpgroups, each with a 128-sample tile of its own in flight (one sample per
+// thread and TMEM lane), and one warp of a fourth that issues every MMA and gives its
+// registers to the others.
 //   forward   the three hidden layers as in k_mlp_forward_tc (TS form, biases in the
-//             contraction), keeping each layer's BF16 input transposed in shared memory
-//             (XT, H1T, H2T: rows = input unit, K = sample) and the ReLU masks in registers;
-//   output    y = h3 . w4 + b4 in FP32, dy = 2 (y - t) / n; the w4 and b4 gradients are
-//             warp-reduced FP32 sums;
-//   backward  dZ3 = dy w4 * [z3 > 0]; then per layer l = 3, 2, 1 two MMA chains:
-//               G_l (+)= H_{l-1}^T dZ_l^T   (SS form, M = 128 input rows, N = 64 outputs,
-//                                           K = 128 samples; accumulated in TMEM over the
-//                                           CTA's tiles; the ones row of H^T gives db_l)
-//               dH_{l-1} = dZ_l W_l          (TS form, A = dZ_l in TMEM, B = W_l^T)
+//             contraction), keeping each layer's BF16 input in shared memory (X, H1, H2) and
+//             the ReLU masks in registers;
+//   output    y = h3 . w4 + b4 in FP32, dy = 2 (y - t) / n; the w4 and b4 gradients and the loss
+//             are sums in registers over the thread's samples, reduced once at the end;
+//   backward  dZ3 = dy w4 * [z3 > 0]; then per layer l = 3, 2, 1
+//               dH_{l-1} = dZ_l W_l          (TS form, A = dZ_l in TMEM)
+//               G_l (+)= dZ_l^T H_{l-1}      (SS form, M = 64 outputs, N = the inputs and a ones
+//                                           column for db_l, K = 128 samples; accumulated in TMEM
+//                                           over all tiles of the CTA)
 //             and dZ_{l-1} = dH_{l-1} * [z_{l-1} > 0] in the epilogue.
-// At the end each thread adds its TMEM lane of G_1..G_3 (one input unit, all outputs) to the
-// global gradient with FP32 atomics.  Rounding points: BF16 inputs, weights, activations and
+// At the end G_1..G_3 are added to the global gradient with FP32 atomics.  Rounding points: BF16 inputs, weights, activations and
 // dZ, FP32 accumulation, as the oracle's BF16 gradient (oracle/mlp.py); the bias gradients
 // come from the BF16 dZ, which the oracle sums unrounded.
 //
+// The samples are the contraction of G_l, and a thread holds all units of one sample, so the
+// operands of G_l are MN-major: 8 units of a sample are 16 contiguous bytes, stored at once and
+// without bank conflicts (a K-major operand took 64 two-byte stores per layer with four-way
+// conflicts).  The same reading of W (stored once, K-major for the forward pass) gives the
+// B operand of dH without a transposed copy.
+//
+// A tile is a chain of five MMA round trips (about 900 cycles of waiting and 1000 of epilogue each),
+// so the chain and not the tensor pipe (a third busy) bounds a single tile: three tiles in flight are
+// what TMEM (3 x 104 columns beside G) and shared memory (3 x 60 KB) hold.  The chains that the
+// epilogues wait for are issued by one warp and the G_l by another; an epilogue waits for G_l only
+// before it overwrites dZ.  Each warp takes the warpgroups in turn, so the additions into G keep
+// the order of the tiles.  4,194,304 samples: 2.23 -> 0.37 ms (one tile in flight with two-byte
+// transposed stores before; 0.80 with one diverged issuing thread, 0.46 with the w4 sums spilled
+// at 128 registers).  Starting the second half's tcgen05.ld ahead of the first half's arithmetic
+// changes nothing (0.37 to 0.38).
+//
 // TMEM columns (512, one CTA per SM):
-//   0..63     D: layer outputs in the forward pass, dH in the backward pass (FP32)
-//   64..103   H: the hidden A operand; in the backward pass columns 64..95 hold dZ (BF16)
-//   104..111  X: the layer-1 A operand
-//   128..191, 192..255, 256..319   G_1, G_2, G_3 (lane = input unit, column = output unit)
-constexpr int GT_TMEM_COLS = 512;
-constexpr uint32_t GT_COL_G1 = 128, GT_COL_G2 = 192, GT_COL_G3 = 256;
+//   0..15, 32..103, 104..175   G_1, G_2, G_3: column = input unit, the ones column behind the last;
+//             output unit o in lane 32 (o / 16) + o % 16, as an accumulator of M = 64 lies
+//   192..383  D of each warpgroup: layer outputs in the forward pass, dH in the backward pass (FP32)
+//   384..503  H of each warpgroup (40 columns): the A operand; X and its ones use the first 8
+//             columns before layer 1, dZ the first 32 in the backward pass, the last 8 hold the
+//             constant ones of the bias columns
+//
+// Shared memory of a warpgroup: 2 KB chunks of 8 units x 128 samples,
+//   H1 (8 chunks) ones X0 ones X1 ones H2 (8 chunks) ones dZ (8 chunks);
+// X alternates between two chunks because G_1 of a tile is issued after the next tile's X is
+// written.
+constexpr int GT_WGS = 3, GT_THREADS = (GT_WGS + 1) * TC_M, GT_TMEM_COLS = 512;
+// registers per thread after the launch with 128: the w4 sums do not fit in 128
+constexpr int GT_REGS = 160, GT_REGS_MMA = 32;
+static_assert(TC_M * (GT_WGS * GT_REGS + GT_REGS_MMA) <= GT_THREADS * 128, "the shares add up to the launch's registers");
+constexpr uint32_t GT_COL_D = 192, GT_COL_H = 384, GT_H_COLS = TC_K2 / 2;
+static_assert(GT_COL_D + GT_WGS * MLP_H <= GT_COL_H && GT_COL_H + GT_WGS * GT_H_COLS <= GT_TMEM_COLS, "TMEM column plan");
+constexpr int GT_CHUNK = TC_M * 16;
+constexpr int GT_H1 = 0, GT_X = 9, GT_X_STEP = 2, GT_H2 = 13, GT_DZ = 22, GT_CHUNKS = 30;
+constexpr int GT_N = MLP_H + 8, GT_N1 = MLP_IN + 8;      // columns of G_2, G_3 and of G_1: inputs, then the ones chunk
+constexpr uint32_t GT_COL_G1 = 0, GT_COL_G2 = 32, GT_COL_G3 = GT_COL_G2 + GT_N;
+static_assert(GT_COL_G3 + GT_N <= GT_COL_D, "TMEM column plan");
+constexpr uint32_t GT_IDESC_G = umma_idesc_bf16_f32<MLP_H, GT_N, true, true>(), GT_IDESC_G1 = umma_idesc_bf16_f32<MLP_H, GT_N1, true, true>();
+constexpr uint32_t GT_IDESC_DH = umma_idesc_bf16_f32<TC_M, MLP_H, false, true>();    // A in TMEM, B MN-major
+constexpr int GT_STAGE = 73;      // floats per output of G_l staged in shared memory (odd: no bank conflicts)
 
 struct MlpGradTcSmem {
     __nv_bfloat16 W1[MLP_H * K1];      // B of layer 1 [64 x 16]: W1 | b1 hi | b1 lo | 0
     __nv_bfloat16 W2[MLP_H * TC_K2];   // B of layer 2 [64 x 80]
     __nv_bfloat16 W3[MLP_H * TC_K2];
-    __nv_bfloat16 W2T[MLP_H * MLP_H];  // B of dH1 = dZ2 W2: rows = input unit, K = output unit
-    __nv_bfloat16 W3T[MLP_H * MLP_H];
-    __nv_bfloat16 XT[TC_M * TC_M];     // A of the weight GEMMs: rows = input unit (+ a ones row), K = sample
-    __nv_bfloat16 H1T[TC_M * TC_M];
-    __nv_bfloat16 H2T[TC_M * TC_M];
-    __nv_bfloat16 DZT[MLP_H * TC_M];   // B of the weight GEMMs: rows = output unit, K = sample
-    float w4[MLP_H];
+    uint4 act[GT_WGS][GT_CHUNKS][TC_M];
+    float4 feats[GT_WGS][TC_M][2];     // the next tile's rows, copied while a tile is computed
+    float4 w4[MLP_H / 4];
     float gw4[MLP_H];
+    double loss;
+    unsigned long long ready[GT_WGS];  // the warpgroup's operands of the next chain are in place (128 arrivals)
+    unsigned long long gready[GT_WGS]; // those of the next G_l
+    unsigned long long chain[GT_WGS];  // the chain that its epilogue waits for is complete
+    unsigned long long wgrad[GT_WGS];  // G_l of its tile is complete
+    unsigned long long done;           // every MMA of the CTA is complete
     float gb4;
     float b4;
-    double loss;
-    unsigned long long bar;
     uint32_t tmem_base;
     int abort;
 };
 static_assert(sizeof(MlpGradTcSmem) + 128 <= 227 * 1024, "one CTA per SM");
+static_assert(sizeof(__nv_bfloat16) * MLP_H * (K1 + 2 * TC_K2) % 128 == 0, "128 B aligned operands");
 
-__device__ __forceinline__ float bf16_lo(uint32_t p) { return __uint_as_float(p << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
-__device__ __forceinline__ __nv_bfloat16 bf16_bits(uint32_t b) { return __ushort_as_bfloat16(static_cast<unsigned short>(b)); }
+// 0xffff in the low and high half if bit j, j + 16 of m is set: prmt replicates the signs of bytes 1 and 3
+__device__ __forceinline__ uint32_t mask_halves(uint32_t m, int j) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, 0, 0xbb99;" : "=r"(d) : "r"(m << (15 - j)));
+    return d;
+}
 
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(GT_THREADS, 1)
 k_mlp_grad_tc(const float* __restrict__ prm, int64_t n, const float* __restrict__ feats, const float* __restrict__ target,
               float* __restrict__ grad, double* __restrict__ loss_out, int32_t* __restrict__ status) {
     extern __shared__ unsigned char gt_dyn[];
     MlpGradTcSmem& s = *reinterpret_cast<MlpGradTcSmem*>((reinterpret_cast<uintptr_t>(gt_dyn) + 127) & ~static_cast<uintptr_t>(127));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (warp == 0) {
         tmem_alloc(smem_u32(&s.tmem_base), GT_TMEM_COLS);
         tmem_relinquish();
     }
     if (tid == 0) {
-        mbar_init(smem_u32(&s.bar), 1);
+        for (int w = 0; w < GT_WGS; ++w) {
+            mbar_init(smem_u32(&s.ready[w]), TC_M);
+            mbar_init(smem_u32(&s.gready[w]), TC_M);
+            mbar_init(smem_u32(&s.chain[w]), 1);
+            mbar_init(smem_u32(&s.wgrad[w]), 1);
+        }
+        mbar_init(smem_u32(&s.done), 2);
         s.abort = 0;
         s.gb4 = 0.f;
         s.loss = 0.0;
+        s.b4 = prm[OFF_B4];
         fence_mbar_init();
     }
-    for (int t = tid; t < MLP_H * K1; t += TC_THREADS) {
+    for (int t = tid; t < MLP_H * K1; t += GT_THREADS) {
         const int r = t / K1, k = t % K1;
         s.W1[umma_k_index(r, k, MLP_H)] = k < MLP_IN ? __float2bfloat16_rn(prm[OFF_W1 + r * MLP_IN + k])
                                                      : bias_part(prm[OFF_B1 + r], k - MLP_IN);
     }
-    for (int t = tid; t < MLP_H * TC_K2; t += TC_THREADS) {
+    for (int t = tid; t < MLP_H * TC_K2; t += GT_THREADS) {
         const int r = t / TC_K2, k = t % TC_K2;
         const bool w = k < MLP_H;
         s.W2[umma_k_index(r, k, MLP_H)] = w ? __float2bfloat16_rn(prm[OFF_W2 + r * MLP_H + k]) : bias_part(prm[OFF_B2 + r], k - MLP_H);
         s.W3[umma_k_index(r, k, MLP_H)] = w ? __float2bfloat16_rn(prm[OFF_W3 + r * MLP_H + k]) : bias_part(prm[OFF_B3 + r], k - MLP_H);
     }
-    for (int t = tid; t < MLP_H * MLP_H; t += TC_THREADS) {
-        const int o = t / MLP_H, i = t % MLP_H;      // W[o][i]
-        s.W2T[umma_k_index(i, o, MLP_H)] = __float2bfloat16_rn(prm[OFF_W2 + t]);
-        s.W3T[umma_k_index(i, o, MLP_H)] = __float2bfloat16_rn(prm[OFF_W3 + t]);
+    const uint4 one_chunk = make_uint4(pack_bf16(1.f, 0.f), 0u, 0u, 0u);
+    for (int t = tid; t < GT_WGS * TC_M; t += GT_THREADS) {
+        const int w = t / TC_M, r = t % TC_M;
+        s.act[w][GT_H1 + 8][r] = one_chunk;
+        s.act[w][GT_X + 1][r] = one_chunk;
+        s.act[w][GT_X + GT_X_STEP + 1][r] = one_chunk;
+        s.act[w][GT_H2 + 8][r] = one_chunk;
     }
-    {   // the ones rows of the transposed inputs (row MLP_IN of XT, row MLP_H of H1T and H2T)
-        const __nv_bfloat16 one = __float2bfloat16_rn(1.f);
-        s.XT[umma_k_index(MLP_IN, tid, TC_M)] = one;
-        s.H1T[umma_k_index(MLP_H, tid, TC_M)] = one;
-        s.H2T[umma_k_index(MLP_H, tid, TC_M)] = one;
-    }
-    if (tid < MLP_H) { s.w4[tid] = prm[OFF_W4 + tid]; s.gw4[tid] = 0.f; }
-    if (tid == 0) s.b4 = prm[OFF_B4];
+    if (tid < MLP_H) { reinterpret_cast<float*>(s.w4)[tid] = prm[OFF_W4 + tid]; s.gw4[tid] = 0.f; }
     fence_proxy_async_smem();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
 
     const uint32_t tbase = s.tmem_base;
-    const uint32_t tlane = tbase + (static_cast<uint32_t>(warp * 32) << 16);
-    {
-        const uint32_t one2 = pack_bf16(1.f, 1.f);
-        const uint32_t hb[8] = {one2, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-        tmem_st_32x32b_x8(tlane + TC_COL_H + MLP_H / 2, hb);
-        tmem_st_32x32b_x4(tlane + TC_COL_X + MLP_IN / 2, one2, 0u, 0u, 0u);
-        tmem_st_wait();
-    }
-    const uint32_t bar = smem_u32(&s.bar);
-    const uint32_t aW1 = smem_u32(s.W1), aW2 = smem_u32(s.W2), aW3 = smem_u32(s.W3), aW2T = smem_u32(s.W2T),
-                   aW3T = smem_u32(s.W3T), aXT = smem_u32(s.XT), aH1T = smem_u32(s.H1T), aH2T = smem_u32(s.H2T),
-                   aDZT = smem_u32(s.DZT);
-    constexpr uint32_t LBO_64 = MLP_H * 16, LBO_128 = TC_M * 16, SBO = 128;
     const float inv_n = 2.f / static_cast<float>(n);
+    // the CTA's tiles are blockIdx.x + k gridDim.x, k < ktiles; warpgroup w takes k = w, w + 3, ...
     const int64_t ntiles = (n + TC_M - 1) / TC_M;
-    uint32_t phase = 0;
-    bool first = true;
-    int64_t tile = blockIdx.x;
+    const int ktiles = static_cast<int>((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
 
-    // one MMA phase: issue (thread 0), commit, bounded wait, then every thread may read TMEM
-    auto sync_mma = [&](auto issue) -> bool {
-        if (tid == 0) {
+    if (warp >= GT_WGS * 4) {
+        setmaxnreg_dec<GT_REGS_MMA>();
+        // The loops are uniform over the warp, so that descriptors and addresses stay in uniform registers
+        // (one diverged thread spent 85 cycles on moving them per MMA); one elected lane issues.
+        const uint32_t aAct = smem_u32(s.act);
+        constexpr uint32_t CORE = 128, LBO_W = MLP_H * 16, WG_BYTES = GT_CHUNKS * GT_CHUNK;
+        uint32_t rphase = 0u;          // parity of each ready barrier
+        bool ok = true;
+        auto wait_ready = [&](uint32_t bars, int w) -> bool {
+            ok = mbar_wait_bounded(bars + 8 * w, (rphase >> w) & 1u, TC_WAIT_CYCLES);
+            rphase ^= 1u << w;
             tc_fence_after_sync();
-            issue();
-            umma_commit(bar);
-        }
-        const bool done = mbar_wait_bounded(bar, phase, TC_WAIT_CYCLES);
-        phase ^= 1u;
-        if (!done) s.abort = 1;
-        __syncthreads();
-        tc_fence_after_sync();
-        return s.abort == 0;
-    };
-    // this thread's BF16 value of input unit c for sample tid into a transposed operand
-    auto put_t = [&](__nv_bfloat16* dstT, int rows, int c, __nv_bfloat16 v) { dstT[umma_k_index(c, tid, rows)] = v; };
-    auto finish_epilogue = [&]() {
-        tmem_st_wait();
-        fence_proxy_async_smem();
-        tc_fence_before_sync();
-        __syncthreads();
-    };
-
-    for (; tile < ntiles; tile += gridDim.x) {
-        const int64_t row = tile * TC_M + tid;
-        const bool valid = row < n;
-        {
-            float4 f0 = make_float4(0.f, 0.f, 0.f, 0.f), f1 = f0;
-            if (valid) {
-                f0 = __ldg(reinterpret_cast<const float4*>(feats + row * MLP_IN));
-                f1 = __ldg(reinterpret_cast<const float4*>(feats + row * MLP_IN) + 1);
-            }
-            const uint32_t x01 = pack_bf16(f0.x, f0.y), x23 = pack_bf16(f0.z, f0.w), x45 = pack_bf16(f1.x, f1.y),
-                           x67 = pack_bf16(f1.z, f1.w);
-            tmem_st_32x32b_x4(tlane + TC_COL_X, x01, x23, x45, x67);
-            const uint32_t xp[4] = {x01, x23, x45, x67};
-            #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                put_t(s.XT, TC_M, 2 * j, bf16_bits(xp[j]));
-                put_t(s.XT, TC_M, 2 * j + 1, bf16_bits(xp[j] >> 16));
-            }
-            finish_epilogue();
-        }
-        // ---- forward
-        uint32_t mask[2][2] = {{0u, 0u}, {0u, 0u}};     // [layer][32-column half]: z > 0
-        float dy = 0.f;
-        #pragma unroll 1
-        for (int layer = 0; layer < 3; ++layer) {
-            const bool ok = sync_mma([&] {
-                if (layer == 0) {
-                    umma_bf16_ts(tbase + TC_COL_D, tbase + TC_COL_X, umma_desc_kmajor(aW1, LBO_64, SBO), TC_IDESC, 0u);
-                } else {
-                    const uint32_t aW = layer == 1 ? aW2 : aW3;
-                    #pragma unroll
-                    for (int ks = 0; ks < TC_K2 / 16; ++ks)
-                        umma_bf16_ts(tbase + TC_COL_D, tbase + TC_COL_H + ks * 8, umma_desc_kmajor(aW + ks * 2 * LBO_64, LBO_64, SBO),
-                                     TC_IDESC, ks > 0 ? 1u : 0u);
-                }
-            });
-            if (!ok) break;
-            float y = 0.f;
-            #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int cb = 32 * half;
-                uint32_t v[32];
-                tmem_ld_32x32b_x32(tlane + TC_COL_D + cb, v);
-                tmem_ld_wait(v);
-                if (layer < 2) {
-                    uint32_t h[16], m = 0u;
-                    #pragma unroll
-                    for (int j = 0; j < 16; ++j) h[j] = relu_bf16x2(v[2 * j], v[2 * j + 1]);
-                    #pragma unroll
-                    for (int j = 0; j < 32; ++j) m |= (__uint_as_float(v[j]) > 0.f ? 1u : 0u) << j;
-                    mask[layer][half] = m;
-                    const uint32_t (&h0)[8] = *reinterpret_cast<const uint32_t(*)[8]>(h);
-                    const uint32_t (&h1)[8] = *reinterpret_cast<const uint32_t(*)[8]>(h + 8);
-                    tmem_st_32x32b_x8(tlane + TC_COL_H + cb / 2, h0);
-                    tmem_st_32x32b_x8(tlane + TC_COL_H + cb / 2 + 8, h1);
-                    __nv_bfloat16* dstT = layer == 0 ? s.H1T : s.H2T;
-                    #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        put_t(dstT, TC_M, cb + 2 * j, bf16_bits(h[j]));
-                        put_t(dstT, TC_M, cb + 2 * j + 1, bf16_bits(h[j] >> 16));
+            return ok;
+        };
+        if (warp == GT_WGS * 4) {
+            // the chains that the epilogues wait for: layers 1, 2, 3, dH2, dH1
+            const uint32_t aW1 = smem_u32(s.W1), aW2 = smem_u32(s.W2), aW3 = smem_u32(s.W3), aReady = smem_u32(s.ready), aChain = smem_u32(s.chain);
+            #pragma unroll 1
+            for (int k0 = 0; ok && k0 < ktiles; k0 += GT_WGS) {
+                #pragma unroll 1
+                for (int phase = 0; ok && phase < 5; ++phase) {
+                    #pragma unroll 1
+                    for (int w = 0; w < GT_WGS && k0 + w < ktiles; ++w) {
+                        if (!wait_ready(aReady, w)) break;
+                        const uint32_t tD = tbase + GT_COL_D + w * MLP_H, tH = tbase + GT_COL_H + w * GT_H_COLS;
+                        if (elect_one()) {
+                            if (phase == 0) {
+                                umma_bf16_ts(tD, tH, umma_desc_kmajor(aW1, LBO_W, CORE), TC_IDESC, 0u);
+                            } else if (phase <= 2) {
+                                const uint64_t dW = umma_desc_kmajor(phase == 1 ? aW2 : aW3, LBO_W, CORE);
+                                #pragma unroll
+                                for (int ks = 0; ks < TC_K2 / 16; ++ks)
+                                    umma_bf16_ts(tD, tH + ks * 8, dW + ks * (2 * LBO_W / 16), TC_IDESC, ks > 0 ? 1u : 0u);
+                            } else {
+                                const uint64_t dW = umma_desc_mnmajor(phase == 3 ? aW3 : aW2, CORE, LBO_W);
+                                #pragma unroll
+                                for (int ks = 0; ks < MLP_H / 16; ++ks)
+                                    umma_bf16_ts(tD, tH + ks * 8, dW + ks * (2 * CORE / 16), GT_IDESC_DH, ks > 0 ? 1u : 0u);
+                            }
+                            umma_commit(aChain + 8 * w);
+                        }
+                        __syncwarp();
                     }
-                } else {
-                    #pragma unroll
-                    for (int j = 0; j < 32; ++j) y = fmaf(fmaxf(__uint_as_float(v[j]), 0.f), s.w4[cb + j], y);
                 }
             }
-            if (layer < 2) {
-                finish_epilogue();
-            } else {
-                // ---- output layer and dZ3
-                y += s.b4;
-                const float e = valid ? y - __ldg(target + row) : 0.f;
-                dy = e * inv_n;
-                double le = static_cast<double>(e) * static_cast<double>(e);
-                float gb = dy;
-                #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    le += __shfl_xor_sync(0xffffffffu, le, o);
-                    gb += __shfl_xor_sync(0xffffffffu, gb, o);
+        } else if (warp == GT_WGS * 4 + 1) {
+            // G_3, G_2, G_1 of each tile, in the order of the tiles
+            const uint32_t aReady = smem_u32(s.gready), aWgrad = smem_u32(s.wgrad);
+            uint32_t x = GT_X;
+            #pragma unroll 1
+            for (int k0 = 0; ok && k0 < ktiles; k0 += GT_WGS) {
+                #pragma unroll 1
+                for (int l = 3; ok && l >= 1; --l) {
+                    const uint32_t tG = tbase + (l == 3 ? GT_COL_G3 : (l == 2 ? GT_COL_G2 : GT_COL_G1));
+                    const uint32_t idesc = l == 1 ? GT_IDESC_G1 : GT_IDESC_G;
+                    #pragma unroll 1
+                    for (int w = 0; w < GT_WGS && k0 + w < ktiles; ++w) {
+                        if (!wait_ready(aReady, w)) break;
+                        const uint32_t act = aAct + w * WG_BYTES;
+                        const uint64_t dA = umma_desc_mnmajor(act + GT_DZ * GT_CHUNK, CORE, GT_CHUNK);
+                        const uint64_t dB = umma_desc_mnmajor(act + (l == 3 ? GT_H2 : (l == 2 ? GT_H1 : x)) * GT_CHUNK, CORE, GT_CHUNK);
+                        if (elect_one()) {
+                            umma_bf16_ss(tG, dA, dB, idesc, k0 + w > 0);
+                            #pragma unroll
+                            for (int ks = 1; ks < TC_M / 16; ++ks) umma_bf16_ss(tG, dA + ks * (2 * CORE / 16), dB + ks * (2 * CORE / 16), idesc, 1u);
+                            umma_commit(aWgrad + 8 * w);
+                        }
+                        __syncwarp();
+                    }
                 }
-                if (lane == 0) { atomicAdd(&s.loss, le); atomicAdd(&s.gb4, gb); }
+                x = 2 * GT_X + GT_X_STEP - x;
+            }
+        }
+        if (warp <= GT_WGS * 4 + 1) {
+            if (elect_one()) umma_commit(smem_u32(&s.done));
+            // also after a timeout: nothing may be in flight when the TMEM columns are released
+            if (!mbar_wait_bounded(smem_u32(&s.done), 0u, TC_WAIT_CYCLES) || !ok) s.abort = 1;
+        }
+    } else {
+        setmaxnreg_inc<GT_REGS>();
+        const int wg = warp >> 2, r = tid & (TC_M - 1);
+        const uint32_t tlane = tbase + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        const uint32_t tD = tlane + GT_COL_D + wg * MLP_H, tH = tlane + GT_COL_H + wg * GT_H_COLS;
+        const uint32_t ready = smem_u32(&s.ready[wg]), gready = smem_u32(&s.gready[wg]), chain = smem_u32(&s.chain[wg]), wgrad = smem_u32(&s.wgrad[wg]);
+        const uint32_t one2 = pack_bf16(1.f, 1.f);
+        uint4 (*act)[TC_M] = s.act[wg];
+        uint32_t cphase = 0u, gphase = 0u;
+        bool ok = true;
+        float gw[MLP_H];
+        #pragma unroll
+        for (int j = 0; j < MLP_H; ++j) gw[j] = 0.f;
+        float gb = 0.f;
+        double lsum = 0.0;
+        // operands of a chain, of a G_l, or of both are in place
+        auto signal = [&](bool to_chain, bool to_g) {
+            tmem_st_wait();
+            fence_proxy_async_smem();
+            tc_fence_before_sync();
+            if (to_chain) mbar_arrive(ready);
+            if (to_g) mbar_arrive(gready);
+        };
+        auto wait_on = [&](uint32_t bar, uint32_t& phase) -> bool {
+            ok = mbar_wait_bounded(bar, phase, TC_WAIT_CYCLES);
+            phase ^= 1u;
+            tc_fence_after_sync();
+            return ok;
+        };
+        // this thread's row of tile k into shared memory, without a register held meanwhile
+        auto fetch_row = [&](int k) {
+            const int64_t row = (blockIdx.x + static_cast<int64_t>(k) * gridDim.x) * TC_M + r;
+            const bool in = k < ktiles && row < n;
+            const float* src = in ? feats + row * MLP_IN : feats;
+            cp_async_16(smem_u32(&s.feats[wg][r][0]), src, in ? 16 : 0);
+            cp_async_16(smem_u32(&s.feats[wg][r][1]), src + 4, in ? 16 : 0);
+        };
+        auto put_x = [&](int parity) {
+            cp_async_wait();
+            const float4 f0 = s.feats[wg][r][0], f1 = s.feats[wg][r][1];
+            const uint4 x = make_uint4(pack_bf16(f0.x, f0.y), pack_bf16(f0.z, f0.w), pack_bf16(f1.x, f1.y), pack_bf16(f1.z, f1.w));
+            const uint32_t xw[8] = {x.x, x.y, x.z, x.w, one2, 0u, 0u, 0u};
+            tmem_st_32x32b_x8(tH, xw);
+            act[GT_X + GT_X_STEP * parity][r] = x;
+        };
+        // 32 units (a half) as BF16 pairs: into the A operand and, 8 units at a time, the chunks from c0
+        auto put_tmem = [&](int half, const uint32_t (&h)[16]) {
+            const uint32_t (&h0)[8] = *reinterpret_cast<const uint32_t(*)[8]>(h);
+            const uint32_t (&h1)[8] = *reinterpret_cast<const uint32_t(*)[8]>(h + 8);
+            tmem_st_32x32b_x8(tH + 16 * half, h0);
+            tmem_st_32x32b_x8(tH + 16 * half + 8, h1);
+        };
+        auto put_chunks = [&](int c0, int half, const uint32_t (&h)[16]) {
+            #pragma unroll
+            for (int q = 0; q < 4; ++q) act[c0 + 4 * half + q][r] = make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+        };
+        {
+            const uint32_t hb[8] = {one2, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+            tmem_st_32x32b_x8(tH + MLP_H / 2, hb);
+        }
+        if (wg < ktiles) {
+            fetch_row(wg);
+            put_x(0);
+            signal(true, false);
+        }
+        int parity = 0;
+        #pragma unroll 1
+        for (int k = wg; k < ktiles; k += GT_WGS) {
+            const int64_t row = (blockIdx.x + static_cast<int64_t>(k) * gridDim.x) * TC_M + r;
+            const bool valid = row < n;
+            const float tgt = valid ? __ldg(target + row) : 0.f;
+            fetch_row(k + GT_WGS);
+            // ---- forward
+            uint32_t mask[2][2];     // [layer][32-unit half]: z > 0, units 2 j and 2 j + 1 in bits j and j + 16
+            #pragma unroll
+            for (int layer = 0; layer < 2; ++layer) {
+                if (!wait_on(chain, cphase)) break;
                 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    const int cb = 32 * half;
-                    uint32_t v[32];      // z3 of this half, read again now that dy is known
-                    tmem_ld_32x32b_x32(tlane + TC_COL_D + cb, v);
+                    uint32_t v[32], h[16], m = 0u;
+                    tmem_ld_32x32b_x32(tD + 32 * half, v);
                     tmem_ld_wait(v);
-                    uint32_t p[16];
-                    {   // d loss / d w4_j summed over the warp's samples: a butterfly that
-                        // halves the values per lane each round leaves lane l with column l
-                        float g[32];
-                        #pragma unroll
-                        for (int j = 0; j < 32; ++j) g[j] = dy * fmaxf(__uint_as_float(v[j]), 0.f);
-                        #pragma unroll
-                        for (int off = 16; off >= 1; off >>= 1) {
-                            const bool upper = (lane & off) != 0;
-                            #pragma unroll
-                            for (int t = 0; t < off; ++t) {
-                                const float send = upper ? g[t] : g[t + off];
-                                const float keep = upper ? g[t + off] : g[t];
-                                g[t] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-                            }
-                        }
-                        atomicAdd(&s.gw4[cb + lane], g[0]);
-                    }
                     #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        const float d0 = __uint_as_float(v[2 * j]) > 0.f ? dy * s.w4[cb + 2 * j] : 0.f;
-                        const float d1 = __uint_as_float(v[2 * j + 1]) > 0.f ? dy * s.w4[cb + 2 * j + 1] : 0.f;
-                        p[j] = pack_bf16(d0, d1);
-                        put_t(s.DZT, MLP_H, cb + 2 * j, bf16_bits(p[j]));
-                        put_t(s.DZT, MLP_H, cb + 2 * j + 1, bf16_bits(p[j] >> 16));
+                        h[j] = relu_bf16x2(v[2 * j], v[2 * j + 1]);
+                        m |= __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&h[j]), __float2bfloat162_rn(0.f)) & (0x00010001u << j);
                     }
-                    const uint32_t (&p0)[8] = *reinterpret_cast<const uint32_t(*)[8]>(p);
-                    const uint32_t (&p1)[8] = *reinterpret_cast<const uint32_t(*)[8]>(p + 8);
-                    tmem_st_32x32b_x8(tlane + TC_COL_H + cb / 2, p0);
-                    tmem_st_32x32b_x8(tlane + TC_COL_H + cb / 2 + 8, p1);
+                    mask[layer][half] = m;
+                    put_tmem(half, h);
+                    put_chunks(layer == 0 ? GT_H1 : GT_H2, half, h);
                 }
-                finish_epilogue();
+                signal(true, false);
             }
-        }
-        if (s.abort) break;
-        // ---- backward: l = 3, 2, 1
-        #pragma unroll 1
-        for (int l = 3; l >= 1; --l) {
-            const uint32_t aA = l == 3 ? aH2T : (l == 2 ? aH1T : aXT);
-            const uint32_t colG = l == 3 ? GT_COL_G3 : (l == 2 ? GT_COL_G2 : GT_COL_G1);
-            const uint32_t aWT = l == 3 ? aW3T : aW2T;
-            const bool acc0 = !first;
-            const bool ok = sync_mma([&] {
+            if (!ok || !wait_on(chain, cphase)) break;
+            // ---- output layer and dZ3
+            float dy;
+            {
+                float y = 0.f;
                 #pragma unroll
-                for (int ks = 0; ks < TC_M / 16; ++ks)
-                    umma_bf16_ss(tbase + colG, umma_desc_kmajor(aA + ks * 2 * LBO_128, LBO_128, SBO),
-                                 umma_desc_kmajor(aDZT + ks * 2 * LBO_64, LBO_64, SBO), TC_IDESC, (acc0 || ks > 0) ? 1u : 0u);
-                if (l > 1) {
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t v[32];
+                    tmem_ld_32x32b_x32(tD + 32 * half, v);
+                    tmem_ld_wait(v);
                     #pragma unroll
-                    for (int ks = 0; ks < MLP_H / 16; ++ks)
-                        umma_bf16_ts(tbase + TC_COL_D, tbase + TC_COL_H + ks * 8, umma_desc_kmajor(aWT + ks * 2 * LBO_64, LBO_64, SBO),
-                                     TC_IDESC, ks > 0 ? 1u : 0u);
+                    for (int q = 0; q < 8; ++q) {
+                        const float4 w = s.w4[8 * half + q];
+                        y = fmaf(fmaxf(__uint_as_float(v[4 * q]), 0.f), w.x, y);
+                        y = fmaf(fmaxf(__uint_as_float(v[4 * q + 1]), 0.f), w.y, y);
+                        y = fmaf(fmaxf(__uint_as_float(v[4 * q + 2]), 0.f), w.z, y);
+                        y = fmaf(fmaxf(__uint_as_float(v[4 * q + 3]), 0.f), w.w, y);
+                    }
                 }
-            });
-            if (!ok) break;
-            if (l == 1) break;
-            // dZ_{l-1} = dH_{l-1} * [z_{l-1} > 0]
+                const float e = valid ? y + s.b4 - tgt : 0.f;
+                dy = e * inv_n;
+                lsum += static_cast<double>(e) * static_cast<double>(e);
+                gb += dy;
+            }
+            if (k != wg && !wait_on(wgrad, gphase)) break;      // G_1 of the tile before has read dZ1
             #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                const int cb = 32 * half;
-                const uint32_t m = mask[l - 2][half];
-                uint32_t v[32];
-                tmem_ld_32x32b_x32(tlane + TC_COL_D + cb, v);
+                uint32_t v[32], p[16];      // z3 of this half, read again now that dy is known
+                tmem_ld_32x32b_x32(tD + 32 * half, v);
                 tmem_ld_wait(v);
-                uint32_t p[16];
                 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float d0 = ((m >> (2 * j)) & 1u) ? __uint_as_float(v[2 * j]) : 0.f;
-                    const float d1 = ((m >> (2 * j + 1)) & 1u) ? __uint_as_float(v[2 * j + 1]) : 0.f;
-                    p[j] = pack_bf16(d0, d1);
-                    put_t(s.DZT, MLP_H, cb + 2 * j, bf16_bits(p[j]));
-                    put_t(s.DZT, MLP_H, cb + 2 * j + 1, bf16_bits(p[j] >> 16));
+                for (int q = 0; q < 8; ++q) {
+                    const float4 w = s.w4[8 * half + q];
+                    const float z[4] = {__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]),
+                                        __uint_as_float(v[4 * q + 3])};
+                    #pragma unroll
+                    for (int t = 0; t < 4; ++t) gw[32 * half + 4 * q + t] = fmaf(dy, fmaxf(z[t], 0.f), gw[32 * half + 4 * q + t]);
+                    p[2 * q] = pack_bf16(z[0] > 0.f ? dy * w.x : 0.f, z[1] > 0.f ? dy * w.y : 0.f);
+                    p[2 * q + 1] = pack_bf16(z[2] > 0.f ? dy * w.z : 0.f, z[3] > 0.f ? dy * w.w : 0.f);
                 }
-                if (l == 3) {     // dZ2 is the A operand of dH1 = dZ2 W2
-                    const uint32_t (&p0)[8] = *reinterpret_cast<const uint32_t(*)[8]>(p);
-                    const uint32_t (&p1)[8] = *reinterpret_cast<const uint32_t(*)[8]>(p + 8);
-                    tmem_st_32x32b_x8(tlane + TC_COL_H + cb / 2, p0);
-                    tmem_st_32x32b_x8(tlane + TC_COL_H + cb / 2 + 8, p1);
+                put_tmem(half, p);
+                put_chunks(GT_DZ, half, p);
+            }
+            signal(true, true);
+            // ---- backward: dZ_{l-1} = dH_{l-1} * [z_{l-1} > 0] for l = 3, 2
+            #pragma unroll
+            for (int l = 3; l >= 2; --l) {
+                if (!wait_on(chain, cphase)) break;
+                const bool more = l == 3 || k + GT_WGS < ktiles;
+                if (l == 2) {
+                    parity ^= 1;
+                    if (more) put_x(parity);
+                }
+                uint32_t p[2][16];
+                #pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const uint32_t m = mask[l - 2][half];
+                    uint32_t v[32];
+                    tmem_ld_32x32b_x32(tD + 32 * half, v);
+                    tmem_ld_wait(v);
+                    #pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        p[half][j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])) & mask_halves(m, j);
+                    if (l == 3) put_tmem(half, p[half]);     // dZ2 is the A operand of dH1 = dZ2 W2
+                }
+                if (!wait_on(wgrad, gphase)) break;          // G_l has read dZ_l
+                put_chunks(GT_DZ, 0, p[0]);
+                put_chunks(GT_DZ, 1, p[1]);
+                signal(more, true);
+            }
+            if (!ok) break;
+        }
+        if (ok) ok = mbar_wait_bounded(smem_u32(&s.done), 0u, TC_WAIT_CYCLES);
+        if (!ok) s.abort = 1;
+        tc_fence_after_sync();
+        // the thread's sums over its samples: a butterfly that halves the values per lane each
+        // round leaves lane l with column l
+        #pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float g[32];
+            #pragma unroll
+            for (int j = 0; j < 32; ++j) g[j] = gw[32 * half + j];
+            #pragma unroll
+            for (int off = 16; off >= 1; off >>= 1) {
+                const bool upper = (lane & off) != 0;
+                #pragma unroll
+                for (int t = 0; t < off; ++t) {
+                    const float send = upper ? g[t] : g[t + off];
+                    const float keep = upper ? g[t + off] : g[t];
+                    g[t] = keep + __shfl_xor_sync(0xffffffffu, send, off);
                 }
             }
-            finish_epilogue();
+            atomicAdd(&s.gw4[32 * half + lane], g[0]);
         }
-        if (s.abort) break;
-        first = false;
-    }
-    if (s.abort) {
-        if (tid == 0) {
-            (void)mbar_wait_bounded(bar, phase ^ 1u, TC_WAIT_CYCLES);
-            if (status) atomicOr(status, SPH_STATUS_TIMEOUT);
+        #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+            gb += __shfl_xor_sync(0xffffffffu, gb, o);
         }
-    } else if (!first) {
-        // this thread's TMEM lane of G_1..G_3: input unit r = tid, every output unit
-        const int r = tid;
-        #pragma unroll 1
-        for (int l = 1; l <= 3; ++l) {
-            const uint32_t colG = l == 3 ? GT_COL_G3 : (l == 2 ? GT_COL_G2 : GT_COL_G1);
+        if (lane == 0) { atomicAdd(&s.loss, lsum); atomicAdd(&s.gb4, gb); }
+        bar_sync_named(GT_WGS + 1, GT_WGS * TC_M);       // every warpgroup's sums and abort flag
+        if (s.abort) {
+            if (tid == 0 && status) atomicOr(status, SPH_STATUS_TIMEOUT);
+        } else {
+            // each warpgroup brings one G_l through shared memory, so that the atomics run along its rows
+            const int l = wg + 1;
+            const uint32_t tG = tlane + (l == 1 ? GT_COL_G1 : (l == 2 ? GT_COL_G2 : GT_COL_G3));
             const int nin = l == 1 ? MLP_IN : MLP_H;
             const int offW = l == 1 ? OFF_W1 : (l == 2 ? OFF_W2 : OFF_W3), offB = l == 1 ? OFF_B1 : (l == 2 ? OFF_B2 : OFF_B3);
-            #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t v[32];
-                tmem_ld_32x32b_x32(tlane + colG + 32 * half, v);
-                tmem_ld_wait(v);
-                if (r < nin) {
-                    #pragma unroll 4
-                    for (int j = 0; j < 32; ++j) atomicAdd(&grad[offW + (32 * half + j) * nin + r], __uint_as_float(v[j]));
-                } else if (r == nin) {
-                    #pragma unroll 4
-                    for (int j = 0; j < 32; ++j) atomicAdd(&grad[offB + 32 * half + j], __uint_as_float(v[j]));
+            float* stage = reinterpret_cast<float*>(s.act[wg]);
+            const int o = (warp & 3) * 16 + lane;
+            #pragma unroll 1
+            for (int c = 0; c <= nin; c += 8) {
+                uint32_t v[8];
+                tmem_ld_32x32b_x8(tG + c, v);
+                if (lane < 16) {
+                    #pragma unroll
+                    for (int j = 0; j < 8; ++j) stage[o * GT_STAGE + c + j] = __uint_as_float(v[j]);
                 }
             }
-        }
-        __syncthreads();
-        if (tid < MLP_H) atomicAdd(&grad[OFF_W4 + tid], s.gw4[tid]);
-        if (tid == 0) {
-            atomicAdd(&grad[OFF_B4], s.gb4);
-            atomicAdd(loss_out, s.loss);
+            bar_sync_named(wg + 1, TC_M);
+            for (int t = r; t < MLP_H * nin; t += TC_M) atomicAdd(&grad[offW + t], stage[(t / nin) * GT_STAGE + t % nin]);
+            for (int t = r; t < MLP_H; t += TC_M) atomicAdd(&grad[offB + t], stage[t * GT_STAGE + nin]);
+            if (tid < MLP_H) atomicAdd(&grad[OFF_W4 + tid], s.gw4[tid]);
+            if (tid == 0) {
+                atomicAdd(&grad[OFF_B4], s.gb4);
+                atomicAdd(loss_out, s.loss);
+            }
         }
     }
     tc_fence_before_sync();
@@ -981,7 +1082,7 @@ int sph_mlp_grad_tc(const float* params, int64_t n, const float* feats, const fl
     const int64_t tiles = (n + TC_M - 1) / TC_M;
     const int grid = (int)(tiles < 148 ? tiles : 148);
     count_launch();
-    k_mlp_grad_tc<<<grid, TC_THREADS, grad_tc_smem_bytes(), s>>>(params, n, feats, target, grad, loss, status);
+    k_mlp_grad_tc<<<grid, GT_THREADS, grad_tc_smem_bytes(), s>>>(params, n, feats, target, grad, loss, status);
     return check_launch("sph_mlp_grad_tc");
 }
 

@@ -10,6 +10,11 @@
 // so core matrices that are adjacent along R are 128 B apart (stride byte offset) and
 // those adjacent along K are R * 16 B apart (leading byte offset).  One kind::f16 MMA
 // consumes K = 16, i.e. two core-matrix columns; the k-th step starts k * R * 32 bytes in.
+//
+// An MN-major operand has 8 elements along R contiguous in the 16 bytes of a core-matrix row and
+// the rows along K: there the stride byte offset separates the groups of 8 along R and the leading
+// byte offset those along K.  The bytes of a K-major [R x K] operand read as the MN-major
+// [K x R] one, so one copy of a matrix serves both it and its transpose.
 #pragma once
 #include <cstdint>
 
@@ -20,12 +25,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast
 __host__ __device__ constexpr int umma_k_index(int r, int k, int R) { return ((k >> 3) * (R >> 3) + (r >> 3)) * 64 + (r & 7) * 8 + (k & 7); }
 
 // Instruction descriptor of tcgen05.mma kind::f16: FP32 accumulator (bits 4-5 = 1),
-// BF16 A and B (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0), N / 8 in
+// BF16 A and B (bits 7-9 = 1, 10-12 = 1), A and B K-major or MN-major (bits 15, 16), N / 8 in
 // bits 17-22 and M / 16 in bits 24-28.
-template <int M, int N>
+template <int M, int N, bool A_MN = false, bool B_MN = false>
 __host__ __device__ constexpr uint32_t umma_idesc_bf16_f32() {
-    static_assert(M == 128 && N % 16 == 0 && N >= 16 && N <= 256, "single-CTA M = 128 tile");
-    return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
+    static_assert((M == 128 && N % 16 == 0 && N >= 16 && N <= 256) || (M == 64 && N % 8 == 0 && N >= 8 && N <= 256), "single-CTA tile");
+    return (1u << 4) | (1u << 7) | (1u << 10) | (A_MN ? 1u << 15 : 0u) | (B_MN ? 1u << 16 : 0u) | (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
 }
 
 // Shared-memory matrix descriptor, no swizzle: start address >> 4 in bits 0-13, leading
@@ -34,6 +39,12 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16_f32() {
 __host__ __device__ __forceinline__ uint64_t umma_desc_kmajor(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
     return static_cast<uint64_t>((saddr >> 4) & 0x3FFFu) | (static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16) |
            (static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+}
+
+// The same for an MN-major operand: k_group_bytes between groups of 8 along K, mn_group_bytes
+// between groups of 8 along R.
+__host__ __device__ __forceinline__ uint64_t umma_desc_mnmajor(uint32_t saddr, uint32_t k_group_bytes, uint32_t mn_group_bytes) {
+    return umma_desc_kmajor(saddr, k_group_bytes, mn_group_bytes);
 }
 
 // ---- TMEM allocation (one full warp executes each of these)
@@ -47,17 +58,43 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
+// True in one lane of a converged warp, the same one at every call.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
+
 // ---- ordering
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // Makes this thread's generic-proxy shared-memory writes visible to the tensor core.
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// ---- warpgroups: registers taken from and given to the block's pool, a barrier of some of its warps
+template <int R> __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R> __device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+__device__ __forceinline__ void bar_sync_named(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// ---- copies of 16 bytes from global into shared memory (bytes beyond `size` are zero), and the wait
+// for all of this thread's
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, int size) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ---- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -117,6 +154,15 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)
           "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
           "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
           "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr)
+        : "memory");
+}
+// Eight columns, loaded and waited for.
+__device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
         : "r"(taddr)
         : "memory");
 }
