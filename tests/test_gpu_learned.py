@@ -214,3 +214,17 @@ def test_mlp_gradient_adds_up(cuda, tiles):
     for name, a, b in BLOCKS:
         assert_close(g[a:b].cpu().numpy(), ref[a:b].cpu().numpy(), 2e-4, 2e-4, f"d loss / d {name}")
     assert abs(float(loss) - (float(la) + float(lb))) <= 1e-6 * float(loss)        # the loss is a sum
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 5 * 148 * 128 + 1, 6 * 148 * 128 - 5, 11 * 148 * 128 + 300])
+def test_mlp_forward_is_per_row(cuda, n):
+    """The tcgen05 forward of n rows against the same rows evaluated in slices: a row's output
+    does not depend on the tile, the warpgroup or the SM that computes it, so they are equal."""
+    rng = np.random.default_rng(n % 1000)
+    th = torch.from_numpy(random_net(4)).to(cuda)
+    x = torch.from_numpy(rng.standard_normal((n, 8)).astype(np.float32)).to(cuda)
+    y = ops.mlp_forward(th, x)
+    step = 1000 if n < 10**5 else 200_000
+    ref = torch.cat([ops.mlp_forward(th, x[a:a + step]) for a in range(0, n, step)])
+    assert int(ops.mlp_status(cuda).item()) == 0
+    assert torch.equal(y, ref)

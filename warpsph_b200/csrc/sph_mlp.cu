@@ -350,16 +350,17 @@ __global__ void k_mlp_adam(float* __restrict__ prm, const float* __restrict__ gr
 }
 
 // ---------------------------------------------------------------- inference on tcgen05
-// One CTA of 4 warps takes 128 samples per tile.  Each layer is one chain of
+// One CTA per SM: five warpgroups with a 128-sample tile each in flight (one sample per thread and
+// TMEM lane), each issuing its own MMAs from one warp.  Each layer is one chain of
 //   D[128 x 64] (TMEM, FP32) = A[128 x K] (TMEM, BF16) x W[64 x K]^T (shared, BF16)
-// of K/16 tcgen05.mma kind::f16 instructions with A read from tensor memory, issued by one
-// thread and completed through tcgen05.commit on an mbarrier.  Warp w then reads TMEM
-// lanes 32w..32w+31 of D (one sample per thread, tcgen05.ld 32x32b), applies ReLU while
-// rounding to BF16 (cvt.rn.relu) and stores the packed pairs straight back into the A
-// columns of the next layer (tcgen05.st 32x32b).  Activations never pass through shared
-// memory, which holds only the weights: with A in shared memory every MMA re-read its
-// activations from there (about 98 KB of shared-memory traffic per tile, the limit).
-// The 64 -> 1 output layer is an FP32 dot product in registers.
+// of K/16 tcgen05.mma kind::f16 instructions with A read from tensor memory, completed
+// through tcgen05.commit on the warpgroup's mbarrier.  Warp w then reads TMEM lanes
+// 32 (w % 4)..+31 of D (tcgen05.ld 32x32b), applies ReLU while rounding to BF16 (cvt.rn.relu)
+// and stores the packed pairs straight back into the A columns of the next layer
+// (tcgen05.st 32x32b).  Activations never pass through shared memory, which holds only the
+// weights: with A in shared memory every MMA re-read its activations from there (about 98 KB
+// of shared-memory traffic per tile, the limit).  The 64 -> 1 output layer is an FP32 dot product
+// in registers.
 //
 // The biases ride in the contraction: A carries two constant-one columns after its real K
 // columns (X columns 8, 9; H columns 64, 65) and W the bias split into BF16 hi + lo parts
@@ -368,36 +369,39 @@ __global__ void k_mlp_adam(float* __restrict__ prm, const float* __restrict__ gr
 // Rounding points otherwise match k_mlp_forward: BF16 features, weights and hidden
 // activations, FP32 accumulation, FP32 output layer.
 //
-// TMEM columns of a CTA (128 allocated, 32-bit each):
-//   0..63    D, the FP32 accumulator
-//   64..103  H, the hidden-layer A operand: 64 BF16 activations (64..95), then 1, 1, 0... (96..103)
-//   104..111 X, the layer-1 A operand: 8 BF16 features (104..107), then 1, 1, 0... (108..111)
-constexpr int TC_M = 128, TC_THREADS = 128, TC_TMEM_COLS = 128, TC_CTAS_PER_SM = 4;
+// A tile is three MMA round trips, latency bound (no pipe above 55 %): the tiles in flight decide, and
+// TMEM holds five, because X lies in the first columns of H (which layer 1 has read when H1 is
+// written) and the ones of the hidden layers are one block that the last k-step of every warpgroup
+// reads.  An MMA costs its issuing warp about 73 cycles against 32 in the tensor pipe, so one issuing
+// warp for all tiles was the limit.  16,777,216 samples: 545 us with four CTAs of a tile each and a
+// diverged issuing thread, 490 with five tiles and one issuing warp, 374 with two, 350 with one per
+// warpgroup; four partial sums of y or an earlier second tcgen05.ld change nothing (353 to 356).
+// Back to back for longer than 0.1 s the GPU reaches its power limit and 350 becomes 410.
+//
+// TMEM columns (512 allocated, 32-bit each):
+//   0..319    D of each warpgroup, the FP32 accumulator
+//   320..479  H of each warpgroup: 64 BF16 activations, or X: 8 BF16 features (4 columns), 1, 1, 0...
+//   480..487  1, 1, 0...: the bias columns of the hidden layers
+constexpr int TC_M = 128, FT_WGS = 5, FT_THREADS = FT_WGS * TC_M, FT_TMEM_COLS = 512;
 constexpr int TC_K2 = MLP_H + 16;   // hidden-layer K with the bias columns
-constexpr uint32_t TC_COL_D = 0, TC_COL_H = 64, TC_COL_X = 104;
+constexpr uint32_t FT_COL_D = 0, FT_COL_H = FT_WGS * MLP_H, FT_H_COLS = MLP_H / 2, FT_COL_ONES = FT_COL_H + FT_WGS * FT_H_COLS;
 constexpr uint32_t TC_IDESC = umma_idesc_bf16_f32<TC_M, MLP_H>();
 static_assert(TC_IDESC == 0x08100490u, "kind::f16 descriptor: BF16 x BF16 -> FP32, M = 128, N = 64, K-major");
-static_assert(TC_COL_H >= TC_COL_D + MLP_H && TC_COL_X >= TC_COL_H + TC_K2 / 2 && TC_COL_X + K1 / 2 <= TC_TMEM_COLS,
-              "TMEM column plan");
+static_assert(FT_COL_ONES + 8 <= FT_TMEM_COLS, "TMEM column plan");
 constexpr long long TC_WAIT_CYCLES = 1ll << 31;   // about a second at B200 clocks
 
 struct MlpTcSmem {
     __nv_bfloat16 W1[MLP_H * K1];      // [64 x 16]: W1 | b1 hi | b1 lo | 0
     __nv_bfloat16 W2[MLP_H * TC_K2];   // [64 x 80]: W2 | b2 hi | b2 lo | 0
     __nv_bfloat16 W3[MLP_H * TC_K2];
-    float w4[MLP_H];
-    unsigned long long bar;
+    float4 feats[FT_WGS][2][TC_M];     // the next tile's rows, copied while a tile is computed
+    float4 w4[MLP_H / 4];
+    unsigned long long chain[FT_WGS];  // the warpgroup's chain is complete
     float b4;
     uint32_t tmem_base;
-    int abort;
-    // keeps the CTA above a fifth of the SM's shared memory, so that no more than the 4
-    // CTAs whose 128 TMEM columns fit in 512 are resident on one SM
-    unsigned char occupancy_pad[24 * 1024];
 };
 static_assert((sizeof(__nv_bfloat16) * MLP_H * K1) % 128 == 0 && (sizeof(__nv_bfloat16) * MLP_H * TC_K2) % 128 == 0,
               "128 B aligned operands");
-static_assert(4 * (sizeof(MlpTcSmem) + 1024) <= 228 * 1024 && 5 * (sizeof(MlpTcSmem) + 1024) > 228 * 1024 &&
-              4 * TC_TMEM_COLS <= 512, "4 resident CTAs per SM, within the SM's TMEM columns");
 
 // relu of (lo, hi) rounded to BF16 and packed, lo in the low half
 __device__ __forceinline__ uint32_t relu_bf16x2(uint32_t lo, uint32_t hi) {
@@ -412,138 +416,176 @@ __device__ __forceinline__ __nv_bfloat16 bias_part(float b, int part) {
     return part == 0 ? hi : part == 1 ? __float2bfloat16_rn(b - __bfloat162float(hi)) : __float2bfloat16_rn(0.f);
 }
 
-__global__ void __launch_bounds__(TC_THREADS, TC_CTAS_PER_SM)
+__global__ void __launch_bounds__(FT_THREADS, 1)
 k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restrict__ feats, const float* __restrict__ scale,
                  float* __restrict__ out, int32_t* __restrict__ status) {
-    __shared__ __align__(128) MlpTcSmem s;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    extern __shared__ unsigned char ft_dyn[];
+    MlpTcSmem& s = *reinterpret_cast<MlpTcSmem*>((reinterpret_cast<uintptr_t>(ft_dyn) + 127) & ~static_cast<uintptr_t>(127));
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     if (warp == 0) {
-        tmem_alloc(smem_u32(&s.tmem_base), TC_TMEM_COLS);
+        tmem_alloc(smem_u32(&s.tmem_base), FT_TMEM_COLS);
         tmem_relinquish();
     }
     if (tid == 0) {
-        mbar_init(smem_u32(&s.bar), 1);
-        s.abort = 0;
+        for (int w = 0; w < FT_WGS; ++w) {
+            mbar_init(smem_u32(&s.chain[w]), 1);
+        }
+        s.b4 = prm[OFF_B4];
         fence_mbar_init();
     }
     // weights in the K-major core-matrix layout (B operands: rows = output units)
-    for (int t = tid; t < MLP_H * K1; t += TC_THREADS) {
+    for (int t = tid; t < MLP_H * K1; t += FT_THREADS) {
         const int r = t / K1, k = t % K1;
         s.W1[umma_k_index(r, k, MLP_H)] = k < MLP_IN ? __float2bfloat16_rn(prm[OFF_W1 + r * MLP_IN + k])
                                                      : bias_part(prm[OFF_B1 + r], k - MLP_IN);
     }
-    for (int t = tid; t < MLP_H * TC_K2; t += TC_THREADS) {
+    for (int t = tid; t < MLP_H * TC_K2; t += FT_THREADS) {
         const int r = t / TC_K2, k = t % TC_K2;
         const bool w = k < MLP_H;
         s.W2[umma_k_index(r, k, MLP_H)] = w ? __float2bfloat16_rn(prm[OFF_W2 + r * MLP_H + k]) : bias_part(prm[OFF_B2 + r], k - MLP_H);
         s.W3[umma_k_index(r, k, MLP_H)] = w ? __float2bfloat16_rn(prm[OFF_W3 + r * MLP_H + k]) : bias_part(prm[OFF_B3 + r], k - MLP_H);
     }
-    if (tid < MLP_H) s.w4[tid] = prm[OFF_W4 + tid];
-    if (tid == 0) s.b4 = prm[OFF_B4];
+    if (tid < MLP_H) reinterpret_cast<float*>(s.w4)[tid] = prm[OFF_W4 + tid];
     fence_proxy_async_smem();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
 
     const uint32_t tbase = s.tmem_base;
-    const uint32_t tlane = tbase + (static_cast<uint32_t>(warp * 32) << 16);   // this warp's 32 lanes
-    {   // the constant columns of this thread's row of H and X, the same for every tile
-        const uint32_t one2 = pack_bf16(1.f, 1.f);
+    const int wg = warp >> 2, r = tid & (TC_M - 1);
+    const uint32_t tlane = tbase + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const uint32_t one2 = pack_bf16(1.f, 1.f);
+    if (wg == 0) {
         const uint32_t hb[8] = {one2, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-        tmem_st_32x32b_x8(tlane + TC_COL_H + MLP_H / 2, hb);
-        tmem_st_32x32b_x4(tlane + TC_COL_X + MLP_IN / 2, one2, 0u, 0u, 0u);
+        tmem_st_32x32b_x8(tlane + FT_COL_ONES, hb);
         tmem_st_wait();
     }
-    const uint32_t bar = smem_u32(&s.bar);
-    const uint32_t aW1 = smem_u32(s.W1), aW2 = smem_u32(s.W2), aW3 = smem_u32(s.W3);
-    const uint32_t LBO_B = MLP_H * 16, SBO = 128;
-    const float sc = scale ? *scale : 1.f;
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    // the CTA's tiles are blockIdx.x + k gridDim.x, k < ktiles; warpgroup w takes k = w, w + 5, ...
     const int64_t ntiles = (n + TC_M - 1) / TC_M;
-    uint32_t phase = 0;
-    int64_t tile = blockIdx.x;
-    for (; tile < ntiles; tile += gridDim.x) {
-        const int64_t row = tile * TC_M + tid;
-        {   // layer-1 operand: this thread's sample, 8 features -> 4 packed BF16 pairs
-            float4 f0 = make_float4(0.f, 0.f, 0.f, 0.f), f1 = f0;
-            if (row < n) {
-                f0 = __ldg(reinterpret_cast<const float4*>(feats + row * MLP_IN));
-                f1 = __ldg(reinterpret_cast<const float4*>(feats + row * MLP_IN) + 1);
-            }
-            tmem_st_32x32b_x4(tlane + TC_COL_X, pack_bf16(f0.x, f0.y), pack_bf16(f0.z, f0.w), pack_bf16(f1.x, f1.y),
-                              pack_bf16(f1.z, f1.w));
+    const int ktiles = static_cast<int>((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+    // the issuing warps of the warpgroups lie on different sub-cores
+    const bool issuer = (warp & 3) == (wg & 3);
+    const uint32_t tDw = tbase + FT_COL_D + wg * MLP_H, tHw = tbase + FT_COL_H + wg * FT_H_COLS;
+    const uint32_t tD = tlane + FT_COL_D + wg * MLP_H, tH = tlane + FT_COL_H + wg * FT_H_COLS, chain = smem_u32(&s.chain[wg]);
+    constexpr uint32_t LBO_W = MLP_H * 16, SBO = 128;
+    const uint64_t dW1 = umma_desc_kmajor(smem_u32(s.W1), LBO_W, SBO), dW2 = umma_desc_kmajor(smem_u32(s.W2), LBO_W, SBO),
+                   dW3 = umma_desc_kmajor(smem_u32(s.W3), LBO_W, SBO);
+    const float sc = scale ? *scale : 1.f;
+    {
+        uint32_t phase = 0u;
+        bool ok = true;
+        auto row_of = [&](int k) { return (blockIdx.x + static_cast<int64_t>(k) * gridDim.x) * TC_M + r; };
+        // the A operand is in place: issue the chain of a layer
+        auto issue = [&](int layer) {
             tmem_st_wait();
-        }
-        tc_fence_before_sync();
-        __syncthreads();
-        float y = 0.f;
-        #pragma unroll 1
-        for (int layer = 0; layer < 3; ++layer) {
-            if (tid == 0) {
+            tc_fence_before_sync();
+            bar_sync_named(wg + 1, TC_M);
+            if (issuer) {
                 tc_fence_after_sync();
-                if (layer == 0) {
-                    umma_bf16_ts(tbase + TC_COL_D, tbase + TC_COL_X, umma_desc_kmajor(aW1, LBO_B, SBO), TC_IDESC, 0u);
-                } else {
-                    const uint32_t aW = layer == 1 ? aW2 : aW3;
-                    #pragma unroll
-                    for (int ks = 0; ks < TC_K2 / 16; ++ks)
-                        umma_bf16_ts(tbase + TC_COL_D, tbase + TC_COL_H + ks * 8, umma_desc_kmajor(aW + ks * 2 * LBO_B, LBO_B, SBO),
-                                     TC_IDESC, ks > 0 ? 1u : 0u);
+                if (elect_one()) {
+                    if (layer == 0) {
+                        umma_bf16_ts(tDw, tHw, dW1, TC_IDESC, 0u);
+                    } else {
+                        const uint64_t dW = layer == 1 ? dW2 : dW3;
+                        #pragma unroll
+                        for (int ks = 0; ks < MLP_H / 16; ++ks)
+                            umma_bf16_ts(tDw, tHw + ks * 8, dW + ks * (2 * LBO_W / 16), TC_IDESC, ks > 0 ? 1u : 0u);
+                        umma_bf16_ts(tDw, tbase + FT_COL_ONES, dW + (MLP_H / 16) * (2 * LBO_W / 16), TC_IDESC, 1u);
+                    }
+                    umma_commit(chain);
                 }
-                umma_commit(bar);
+                __syncwarp();
             }
-            const bool done = mbar_wait_bounded(bar, phase, TC_WAIT_CYCLES);
+        };
+        auto wait_chain = [&]() -> bool {
+            ok = mbar_wait_bounded(chain, phase, TC_WAIT_CYCLES);
             phase ^= 1u;
-            if (!done) s.abort = 1;
-            __syncthreads();
-            if (s.abort) break;
             tc_fence_after_sync();
-            #pragma unroll
-            for (int cb = 0; cb < MLP_H; cb += 32) {
-                uint32_t v[32];
-                tmem_ld_32x32b_x32(tlane + TC_COL_D + cb, v);
-                tmem_ld_wait(v);
-                if (layer < 2) {
-                    uint32_t h[16];
+            return ok;
+        };
+        // this thread's row of tile k into shared memory, without a register held meanwhile
+        auto fetch_row = [&](int k) {
+            const int64_t row = row_of(k);
+            const bool in = k < ktiles && row < n;
+            const float* src = in ? feats + row * MLP_IN : feats;
+            cp_async_16(smem_u32(&s.feats[wg][0][r]), src, in ? 16 : 0);
+            cp_async_16(smem_u32(&s.feats[wg][1][r]), src + 4, in ? 16 : 0);
+        };
+        auto put_x = [&]() {
+            cp_async_wait();
+            const float4 f0 = s.feats[wg][0][r], f1 = s.feats[wg][1][r];
+            const uint32_t xw[8] = {pack_bf16(f0.x, f0.y), pack_bf16(f0.z, f0.w), pack_bf16(f1.x, f1.y), pack_bf16(f1.z, f1.w), one2, 0u, 0u, 0u};
+            tmem_st_32x32b_x8(tH, xw);
+        };
+        if (wg < ktiles) {
+            fetch_row(wg);
+            put_x();
+            issue(0);
+        }
+        int k = wg;
+        #pragma unroll 1
+        for (; k < ktiles; k += FT_WGS) {
+            fetch_row(k + FT_WGS);
+            #pragma unroll 1
+            for (int layer = 0; layer < 2; ++layer) {
+                if (!wait_chain()) break;
+                #pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t v[32], h[16];
+                    tmem_ld_32x32b_x32(tD + 32 * half, v);
+                    tmem_ld_wait(v);
                     #pragma unroll
                     for (int j = 0; j < 16; ++j) h[j] = relu_bf16x2(v[2 * j], v[2 * j + 1]);
                     const uint32_t (&h0)[8] = *reinterpret_cast<const uint32_t(*)[8]>(h);
                     const uint32_t (&h1)[8] = *reinterpret_cast<const uint32_t(*)[8]>(h + 8);
-                    tmem_st_32x32b_x8(tlane + TC_COL_H + cb / 2, h0);
-                    tmem_st_32x32b_x8(tlane + TC_COL_H + cb / 2 + 8, h1);
-                } else {
-                    #pragma unroll
-                    for (int j = 0; j < 32; ++j) y = fmaf(fmaxf(__uint_as_float(v[j]), 0.f), s.w4[cb + j], y);
+                    tmem_st_32x32b_x8(tH + 16 * half, h0);
+                    tmem_st_32x32b_x8(tH + 16 * half + 8, h1);
+                }
+                issue(layer + 1);
+            }
+            if (!ok || !wait_chain()) break;
+            // the next tile's first chain runs while the second half of the output layer is summed
+            float y = 0.f;
+            #pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(tD + 32 * half, v);
+                tmem_ld_wait(v);
+                if (half == 1 && k + FT_WGS < ktiles) {
+                    put_x();
+                    issue(0);
+                }
+                #pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const float4 w = s.w4[8 * half + q];
+                    y = fmaf(fmaxf(__uint_as_float(v[4 * q]), 0.f), w.x, y);
+                    y = fmaf(fmaxf(__uint_as_float(v[4 * q + 1]), 0.f), w.y, y);
+                    y = fmaf(fmaxf(__uint_as_float(v[4 * q + 2]), 0.f), w.z, y);
+                    y = fmaf(fmaxf(__uint_as_float(v[4 * q + 3]), 0.f), w.w, y);
                 }
             }
-            if (layer < 2) {
-                tmem_st_wait();
-                tc_fence_before_sync();
-                __syncthreads();
-            }
+            const int64_t row = row_of(k);
+            if (row < n) out[row] = (y + s.b4) * sc;
         }
-        if (s.abort) break;
-        if (row < n) out[row] = (y + s.b4) * sc;
-    }
-    if (s.abort) {
-        // a chain did not complete in time: the samples of this and later tiles get NaN.
-        // The MMA chain and its commit may still be in flight, so the issuing thread waits
-        // once more (bounded) for that commit before the TMEM columns are released; the
-        // timeout status tells the host that the context is suspect, and the host stops
-        // issuing work to this device's MLP after it.
-        for (; tile < ntiles; tile += gridDim.x) {
-            const int64_t row = tile * TC_M + tid;
-            if (row < n) out[row] = __int_as_float(0x7fc00000);
-        }
-        if (tid == 0) {
-            (void)mbar_wait_bounded(bar, phase ^ 1u, TC_WAIT_CYCLES);
-            if (status) atomicOr(status, SPH_STATUS_TIMEOUT);
+        if (!ok) {
+            // A chain did not complete in time: the samples of this and later tiles get NaN.  Its MMAs may
+            // still be in flight, so the issuing warp waits once more (bounded) before the TMEM columns
+            // are released; the status tells the host that the context is suspect, and the host stops
+            // issuing work to this device's MLP after it.
+            if (issuer) (void)mbar_wait_bounded(chain, phase ^ 1u, TC_WAIT_CYCLES);
+            if (r == 0 && status) atomicOr(status, SPH_STATUS_TIMEOUT);
+            for (; k < ktiles; k += FT_WGS)
+                if (row_of(k) < n) out[row_of(k)] = __int_as_float(0x7fc00000);
         }
     }
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after_sync();
-        tmem_dealloc(tbase, TC_TMEM_COLS);
+        tmem_dealloc(tbase, FT_TMEM_COLS);
     }
 }
 
@@ -1003,6 +1045,8 @@ k_mlp_grad_tc(const float* __restrict__ prm, int64_t n, const float* __restrict_
     }
 }
 
+static int forward_tc_smem_bytes() { return (int)sizeof(MlpTcSmem) + 128; }
+
 static int grad_tc_smem_bytes() { return (int)sizeof(MlpGradTcSmem) + 128; }
 
 static int train_smem_bytes() { return (int)sizeof(MlpSmemTrain); }
@@ -1034,10 +1078,16 @@ int sph_mlp_forward_tc(const float* params, int64_t n, const float* feats, const
     WSPH_CHECK_PTR(params); WSPH_CHECK_PTR(feats); WSPH_CHECK_PTR(out);
     if (reinterpret_cast<uintptr_t>(feats) & 15) return set_error(SPH_ERR_BAD_ARG, "sph_mlp_forward_tc: feats must be 16-byte aligned");
     const int64_t tiles = (n + TC_M - 1) / TC_M;
-    const int64_t cap = 148 * TC_CTAS_PER_SM;
-    const int grid = (int)(tiles < cap ? tiles : cap);
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(k_mlp_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, forward_tc_smem_bytes());
+    });
+    if (attr_err != cudaSuccess)
+        return set_error(SPH_ERR_CUDA, "sph_mlp_forward_tc: shared memory opt-in: %s", cudaGetErrorString(attr_err));
+    const int grid = (int)(tiles < 148 ? tiles : 148);
     count_launch();
-    k_mlp_forward_tc<<<grid, TC_THREADS, 0, WSPH_STREAM(stream)>>>(params, n, feats, scale, out, status);
+    k_mlp_forward_tc<<<grid, FT_THREADS, forward_tc_smem_bytes(), WSPH_STREAM(stream)>>>(params, n, feats, scale, out, status);
     return check_launch("sph_mlp_forward_tc");
 }
 
