@@ -12,13 +12,15 @@ Ensemble checks:
     own lists, at 1e-3 of scale;
   * graph: replaying a captured CUDA graph is bit-identical to the same launches issued
     one by one."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 from oracle import oracle
-from tests.cases import assert_close, make_params
-from warpsph_b200 import core, ops
+from tests.cases import assert_close, make_params, make_particles
+from warpsph_b200 import _capi, core, ops
 from warpsph_b200.configurations import WeaklyCompressibleSPHConfig, wc_params
 from warpsph_b200.ensemble import TILE_CANDIDATES, BoxSet, Ensemble
 
@@ -130,3 +132,52 @@ def test_autotune_chooses_a_measured_candidate(cuda):
         outs.append((x, v, r))
     for x, v, r in outs[1:]:
         assert_close(v.cpu().numpy(), outs[0][1].cpu().numpy(), 1e-5, 1e-5, "v across tile shapes")
+
+
+@pytest.mark.parametrize("lanes", [4, 8, 16])
+@pytest.mark.parametrize("dim,n_side,verlet,terms", [(1, 60, 1.5, (0, 0)), (2, 24, 1.5, (2, 0)), (2, 64, 4.5, (0, 3)), (2, 31, 1.4, (5, 2)),
+                                                     (3, 12, 1.3, (2, 0)), (3, 18, 1.9, (1, 0))])
+def test_ensemble_step_matches_single_rhs(cuda, dim, n_side, verlet, terms, lanes):
+    """One sph_ensemble_step against Heun's method over the single-list right-hand side on the same
+    Verlet rows: 1D to 3D, varying supports, all forms of pressure and density term, rows longer than
+    the 256 entries whose reach is precomputed (verlet 4.5 and 1.9), and particles that move
+    by a tenth of a support within the step, so that pairs come into range at the second stage.  The
+    terms are the same; sums in another lane order differ by FP32 rounding, 2e-5 of each
+    field's scale."""
+    P = make_particles(dim, n_side, seed=5, jitter=0.4, h_spread=0.15)
+    cfg, _, p = make_params(dim)
+    p.verlet_scale = verlet
+    wc = wc_params(WeaklyCompressibleSPHConfig())
+    wc.pressure_term, wc.density_scheme = terms
+    x, H, m, v = (torch.from_numpy(P[k]).to(cuda) for k in ("positions", "supports", "masses", "velocities"))
+    n = H.shape[0]
+    rho = 1.0 + 0.01 * torch.from_numpy(np.random.default_rng(1).standard_normal(n).astype(np.float32)).to(cuda)
+    built = ops.buildVerletList(x, H, p, verlet)
+    rows = core.AdjacencyList(neighborOffsets=built.neighborOffsets, numNeighbors=built.numNeighbors, neighborList=built.neighborList,
+                              numRows=n, numCols=n, nnz=built.nnz)
+    dt = torch.full((1,), 0.1 * float(H.min()) / float(v.abs().max()), device=cuda)
+    L = 1.0
+
+    def wrap(y):
+        return torch.where(y >= 0.5 * L, y - L, torch.where(y < -0.5 * L, y + L, y))
+
+    k1v, k1r, _, _ = ops.deltasph_rhs(p, wc, x, H, m, rho, v, rows)
+    x1, v1, r1 = wrap(x + dt * v), v + dt * k1v, rho + dt * k1r
+    k2v, k2r, _, _ = ops.deltasph_rhs(p, wc, x1, H, m, r1, v1, rows)
+    h = 0.5 * dt
+    ref = (wrap(x + h * (v + v1)), v + h * (k1v + k2v), rho + h * (k1r + k2r))
+    got = [t.clone() for t in (x, v, rho)]
+    lib = _capi.lib()
+    ws = torch.empty(int(lib.sph_ensemble_step_workspace_size(n, dim)), dtype=torch.uint8, device=cuda)
+    flags = torch.zeros(2, dtype=torch.int32, device=cuda)
+    box = torch.zeros(n, dtype=torch.int32, device=cuda)
+    rc = lib.sph_ensemble_step(C.byref(p), C.cast(C.pointer(wc), C.c_void_p), n, box.data_ptr(), dt.data_ptr(), H.data_ptr(), m.data_ptr(),
+                               got[0].data_ptr(), got[1].data_ptr(), got[2].data_ptr(), x.data_ptr(), rows.neighborOffsets.data_ptr(),
+                               rows.numNeighbors.data_ptr(), rows.neighborList.data_ptr(), ws.data_ptr(), ws.numel(), lanes, 128,
+                               flags.data_ptr(), flags.data_ptr() + 4, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and int(flags[1]) == 0
+    assert (int(rows.numNeighbors.max()) > 256) == (verlet > 1.5)
+    d = (got[0] - ref[0]).cpu().numpy()
+    assert np.abs(d - np.round(d)).max() < 1e-6
+    for name, a, b, y0 in zip(("v", "rho"), got[1:], ref[1:], (v, rho)):
+        assert_close((a - y0).cpu().numpy(), (b - y0).cpu().numpy(), 2e-5, 2e-5, f"change of {name}")

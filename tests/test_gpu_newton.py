@@ -19,3 +19,14 @@ def test_newton_step_is_within_one_ulp(cuda, tmp_path):
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
     assert float(out[1]) <= 1.0 and float(out[3]) <= 1.0, out
     assert float(out[5]) == 0.0, out
+
+
+def test_markstein_quotients_are_rounded(cuda, tmp_path):
+    """The reciprocal over every significand but the all-ones one, and 76 million quotients, equal
+    those of the rounded division."""
+    src = Path(__file__).resolve().parent / "native" / "div_check.cu"
+    exe = tmp_path / "div_check"
+    subprocess.run([build.nvcc(), *build.ARCH_FLAGS, "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-I", str(build.INCLUDE), "-I",
+                    str(build.CSRC), str(src), "-o", str(exe)], check=True, capture_output=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    assert out == ["rcp", "0", "div", "0", "div2", "0"], out

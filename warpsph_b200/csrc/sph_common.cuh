@@ -156,6 +156,22 @@ __device__ __forceinline__ float rcp_newton(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return fmaf(fmaf(-x, y, 1.f), y, y);
 }
+// a / b rounded to nearest, with r = 1 / b rounded to nearest: the second residual correction starts
+// from a quotient within an ulp, where its result is the rounded quotient (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990).  No underflow of the residuals.
+__device__ __forceinline__ float div_markstein(float a, float b, float r) {
+    float q = a * r;
+    q = fmaf(fmaf(-b, q, a), r, q);
+    return fmaf(fmaf(-b, q, a), r, q);
+}
+// 1 / b rounded to nearest: two Newton steps from the hardware approximation, of which the second starts
+// within an ulp (Markstein; a divisor whose significand is all ones may be an ulp off).
+__device__ __forceinline__ float rcp_markstein(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    y = fmaf(fmaf(-b, y, 1.f), y, y);
+    return fmaf(fmaf(-b, y, 1.f), y, y);
+}
 // Squared distance with explicit round-to-nearest steps (no FMA contraction) so the
 // neighbour criterion is bit-identical to the CPU oracle.
 template <int D> __device__ __forceinline__ float dist2_rn(const Vec<D>& d) {

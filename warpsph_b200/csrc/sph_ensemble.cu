@@ -9,11 +9,10 @@
 // table) never pairs particles of different boxes.
 //
 // One time step of every box is ONE cooperative persistent launch (k_ens_step): Heun
-// RK2 with two right-hand sides, four phases separated by three bounded grid barriers:
-//   A(y0) | B(y0), y1 = y0 + dt k1 | A(y1) | B(y1), y = y0 + dt/2 (k1 + k2)
+// RK2 with two right-hand sides, five phases separated by four bounded grid barriers:
+//   pack y0 | A(y0) | B(y0), y1 = y0 + dt k1 | A(y1) | B(y1), y = y0 + dt/2 (k1 + k2)
 // where A is the renormalised density gradient + EOS and B the delta-SPH right-hand side.
-// dt is per box (box_dt).  Arrays that other blocks rewrite between phases are read
-// with ld.global.cg.  The step also reduces the largest displacement since the list
+// dt is per box (box_dt).  The step also reduces the largest displacement since the list
 // was built, so the caller can tell when the Verlet skin is used up.
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -73,6 +72,17 @@ __global__ void k_ens_sort_cells(int64_t ncells, const int32_t* __restrict__ sta
     }
 }
 
+// Position and support of the particles in cell order: the search below reads candidates as
+// consecutive 16-byte words instead of an index, a position and a support each.
+template <int D>
+__global__ void k_ens_pack_sorted(int n, const float* __restrict__ x, const float* __restrict__ H, const int32_t* __restrict__ sorted,
+                                  float4* __restrict__ words) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const int j = sorted[s];
+    words[s] = make_xh<D>(load_vec<D>(x, j), H[j]);
+}
+
 // Count (FILL = false) or fill the Verlet rows: j in the 3^dim stencil cells of i's box
 // grid (periodic wrap, x fastest), ascending index within a cell, kept when
 // |x_i - x_j|^2 < (verlet_scale max(H_i, H_j))^2 with the minimum-image distance.
@@ -80,7 +90,8 @@ template <int D, int G, bool FILL>
 __global__ void __launch_bounds__(128)
 k_ens_verlet(int n, DevParams P, const float* __restrict__ x, const float* __restrict__ H, const int32_t* __restrict__ box_of,
              const int32_t* __restrict__ box_grid, const int32_t* __restrict__ box_base, const int32_t* __restrict__ start,
-             const int32_t* __restrict__ counts, const int32_t* __restrict__ sorted, int32_t* __restrict__ num,
+             const int32_t* __restrict__ counts, const int32_t* __restrict__ sorted, const float4* __restrict__ words,
+             int32_t* __restrict__ num,
              const int32_t* __restrict__ offs, int32_t* __restrict__ list, const long long* __restrict__ nnz, int64_t cap) {
     Grp<G> g(n);
     if (FILL && *nnz > cap) return;            // uniform over the grid
@@ -110,7 +121,11 @@ k_ens_verlet(int n, DevParams P, const float* __restrict__ x, const float* __res
         if (g.valid) {
             int cc[D], t = sidx;
             #pragma unroll
-            for (int a = 0; a < D; ++a) { cc[a] = (c[a] + (t % 3) - 1 + Gb) % Gb; t /= 3; }
+            for (int a = 0; a < D; ++a) {
+                cc[a] = c[a] + (t % 3) - 1;                       // periodic: one wrap at most
+                cc[a] = cc[a] < 0 ? cc[a] + Gb : (cc[a] >= Gb ? cc[a] - Gb : cc[a]);
+                t /= 3;
+            }
             const int key = ens_key<D>(cc, Gb, base);
             s0 = start[key];
             cn = counts[key];
@@ -118,15 +133,14 @@ k_ens_verlet(int n, DevParams P, const float* __restrict__ x, const float* __res
         for (int q0 = 0; __any_sync(0xffffffffu, q0 < cn); q0 += G) {
             const int q = q0 + g.lane;
             bool keep = false;
-            int j = 0;
             if (q < cn) {
-                j = sorted[s0 + q];
-                const Vec<D> d = dist_vec<D>(xi, load_vec<D>(x, j), P.dom);
-                const float R = __fmul_rn(P.verlet_scale, wmax(Hi, __ldg(H + j)));
+                const float4 t = __ldg(words + s0 + q);
+                const Vec<D> d = dist_vec<D>(xi, vec_of_word<D>(t), P.dom);
+                const float R = __fmul_rn(P.verlet_scale, wmax(Hi, support_of<D>(t)));
                 keep = dist2_rn<D>(d) < __fmul_rn(R, R);
             }
             const unsigned int bits = (__ballot_sync(0xffffffffu, keep) >> gshift) & lanes;
-            if (FILL && keep) list[row + w + __popc(bits & ((1u << g.lane) - 1u))] = j;
+            if (FILL && keep) list[row + w + __popc(bits & ((1u << g.lane) - 1u))] = __ldg(sorted + s0 + q);
             w += __popc(bits);
         }
     }
@@ -139,6 +153,7 @@ __global__ void k_ens_check(const long long* __restrict__ nnz, int64_t cap, int3
 
 struct EnsNbWs {
     int32_t *keys, *slot, *counts, *start, *sorted;
+    float4* words;
     long long* total;
     char* scan;
     int64_t bytes;
@@ -151,6 +166,9 @@ static EnsNbWs ens_carve(char* base, int64_t n, int64_t ncells) {
     w.keys = reinterpret_cast<int32_t*>(base + o); o += al256(n * 4);
     w.slot = reinterpret_cast<int32_t*>(base + o); o += al256(n * 4);
     w.sorted = reinterpret_cast<int32_t*>(base + o); o += al256(n * 4);
+    // 16-byte aligned whatever the base's alignment
+    w.words = reinterpret_cast<float4*>((reinterpret_cast<uintptr_t>(base) + o + 15) & ~static_cast<uintptr_t>(15));
+    o += al256(n * 16 + 16);
     w.counts = reinterpret_cast<int32_t*>(base + o); o += al256(ncells * 4);
     w.start = reinterpret_cast<int32_t*>(base + o); o += al256(ncells * 4);
     w.scan = base + o;
@@ -160,6 +178,12 @@ static EnsNbWs ens_carve(char* base, int64_t n, int64_t ncells) {
 }
 
 // ---------------------------------------------------------------- persistent step
+// What the pair passes gather of a particle, in 16-byte words written by the phase that computes
+// them.  Other blocks read them after a grid barrier, with plain loads (never the read-only path).
+//   xv  position, then velocity (1D, 2D: one word; 3D: one word each)          one set per stage:
+//   sv  density, V = m / rho, H                                                the first is still read
+//   gp  renormalised density gradient, then the pressure                       while the second is written
+struct EnsSet { float4 *xv, *sv; };
 struct EnsArgs {
     int n;
     DevParams P;
@@ -167,8 +191,10 @@ struct EnsArgs {
     const int32_t *box_of;
     const float *box_dt, *H, *m, *x_build;
     float *x, *v, *rho;                    // state y0 (updated in place at the end of the step)
-    float *x1, *v1, *rho1, *dv1, *drho1;   // stage state and first right-hand side
-    float *gL, *Pr;                        // pass-A outputs of the current stage
+    float *dv1, *drho1;                    // first right-hand side
+    EnsSet set[2];
+    float4* gp;
+    void* near;                            // ENS_NEAR bits per particle: see EnsWalk
     const int32_t *offs, *cnt, *list;
     BarrierCtl* ctl;
     unsigned int* disp;                    // max |x - x_build| / H since the list was built (ordered float)
@@ -189,29 +215,277 @@ template <int D> __device__ __forceinline__ Vec<D> wrap_pos(Vec<D> x, const Doma
     return x;
 }
 
-// 2D: 9 blocks of 128 threads per SM (56 registers); one block fewer costs the step 9 %.
+template <int D> __device__ __forceinline__ void put_xv(const EnsSet& s, int i, const Vec<D>& x, const Vec<D>& v) {
+    float w[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    constexpr int V0 = D == 3 ? 4 : D;
+    #pragma unroll
+    for (int a = 0; a < D; ++a) { w[a] = x.v[a]; w[V0 + a] = v.v[a]; }
+    constexpr int NW = D == 3 ? 2 : 1;
+    #pragma unroll
+    for (int k = 0; k < NW; ++k) s.xv[(size_t)i * NW + k] = make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+}
+template <int D> __device__ __forceinline__ float4 get_x_word(const EnsSet& s, int i) { return s.xv[D == 3 ? 2 * (size_t)i : (size_t)i]; }
+template <int D> __device__ __forceinline__ Vec<D> get_v(const EnsSet& s, int i, const float4& xw) {
+    if constexpr (D == 3) return vec_of_word<3>(s.xv[2 * (size_t)i + 1]);
+    Vec<D> v;
+    #pragma unroll
+    for (int a = 0; a < D; ++a) v.v[a] = word_of(xw, D + a);
+    return v;
+}
+
+// The entries of a row that are inside the support at y0 or at y1 = y0 + dt v0 are known before the
+// first pair pass (y1 moves with the velocities of y0), so the four passes of a step walk
+// those alone: half of a Verlet row.  ENS_NEAR bits per particle say which, each lane of the G
+// holding the bits of its own entries (lane, lane + G, ...), in order: a lane adds the terms it
+// would add without them in the same order, the others being exact zeros, so the sums are the
+// same to the bit.  Entries behind the first ENS_NEAR of a row are always walked.
+constexpr int ENS_NEAR = 256;
+template <int G> struct NearWord;
+template <> struct NearWord<4> { using T = unsigned long long; };
+template <> struct NearWord<8> { using T = unsigned int; };
+template <> struct NearWord<16> { using T = unsigned short; };
+
+// One lane's walk: the entry index and the neighbour two entries ahead, its position word one ahead.
+template <int D, int G> struct EnsWalk {
+    static constexpr int KM = ENS_NEAR / G;
+    const int32_t* __restrict__ row;       // this lane's first entry
+    const EnsSet& st;
+    unsigned int bits, more;               // near entries from `base` on; with 64 per lane, the second half
+    int base, tail, nk, j1, j2;            // j < 0: no entry
+    float4 w1;
+    __device__ __forceinline__ int next() {
+        int k;
+        if (KM > 32 && !bits) { bits = more; more = 0; base += 32; }
+        if (bits) {
+            k = base + __ffs((int)bits) - 1;
+            bits &= bits - 1;
+        } else {
+            k = tail++;
+        }
+        return k < nk ? __ldg(row + k * G) : -1;
+    }
+    __device__ __forceinline__ EnsWalk(const EnsArgs& a, const EnsSet& s, int i, int lane) : st(s) {
+        row = a.list + a.offs[i] + lane;
+        nk = (a.cnt[i] - lane + G - 1) / G;
+        tail = KM;
+        const auto near = static_cast<const typename NearWord<G>::T*>(a.near)[(size_t)i * G + lane];
+        bits = (unsigned int)near;
+        more = KM > 32 ? (unsigned int)((unsigned long long)near >> 32) : 0u;
+        base = 0;
+        j1 = next();
+        j2 = next();
+        w1 = get_x_word<D>(st, j1 < 0 ? 0 : j1);
+    }
+    __device__ __forceinline__ bool take(int& j, float4& w) {
+        j = j1;
+        w = w1;
+        j1 = j2;
+        if (j >= 0) {
+            w1 = get_x_word<D>(st, j1 < 0 ? 0 : j1);
+            j2 = j1 < 0 ? -1 : next();
+        }
+        return j >= 0;
+    }
+};
+
+// The bits of this lane's entries.  x1_ij = x_ij + dt (v_i - v_j) up to the rounding of the positions,
+// which the limit allows for.
+template <int D, int G>
+__device__ __forceinline__ void ens_near(int i, int lane, const EnsArgs& a, const EnsSet& st) {
+    using T = typename NearWord<G>::T;
+    const float4 wi = get_x_word<D>(st, i);
+    const Vec<D> xi = vec_of_word<D>(wi), vi = get_v<D>(st, i, wi);
+    const float Hi = a.H[i], dt = a.box_dt[a.box_of[i]];
+    float scale = 0.f;
+    #pragma unroll
+    for (int c = 0; c < D; ++c) scale = fmaxf(scale, fabsf(xi.v[c]) + a.P.dom.L[c]);
+    const float slack = 1e-6f * scale;
+    const int nk = min((a.cnt[i] - lane + G - 1) / G, ENS_NEAR / G);
+    const int32_t* row = a.list + a.offs[i] + lane;
+    T bits = 0;
+    int jn = nk > 0 ? __ldg(row) : 0;
+    #pragma unroll 2
+    for (int k = 0; k < nk; ++k) {
+        const int j = jn;
+        if (k + 1 < nk) jn = __ldg(row + (k + 1) * G);
+        const float4 wj = get_x_word<D>(st, j);
+        const Vec<D> vj = get_v<D>(st, j, wj);
+        const float lim = fmaf(fmaxf(Hi, __ldg(a.H + j)), 1.0001f, slack), lim2 = lim * lim;
+        const Vec<D> d0 = pair_vec<D>(xi, vec_of_word<D>(wj), a.P.dom);
+        Vec<D> d1;
+        #pragma unroll
+        for (int c = 0; c < D; ++c) d1.v[c] = fmaf(dt, vi.v[c] - vj.v[c], d0.v[c]);
+        const bool far = dot<D>(d0, d0) >= lim2 && dot<D>(d1, d1) >= lim2;       // NaN is near
+        bits |= (T)((T)(!far) << k);
+    }
+    static_cast<T*>(a.near)[(size_t)i * G + lane] = bits;
+}
+
+// What a pair needs of the larger support.
+template <int KF, int D> struct EnsSupport {
+    float H, rH, HH, rHH, cH;
+    __device__ __forceinline__ explicit EnsSupport(float h)
+        : H(h), rH(1.f / h), HH(h * h), rHH(1.f / (h * h)), cH(KernelTraits<KF, D>::C / ipow<D>(h)) {}
+};
+// gradW(x_ij, max(H_i, H_j)) as kernelWG gives it; false outside the support.
+template <int KF, int D>
+__device__ __forceinline__ bool ens_grad(const Vec<D>& xij, float r, const EnsSupport<KF, D>& hi, float Hj, Vec<D>& gW) {
+    EnsSupport<KF, D> h = hi;
+    if (Hj > hi.H) h = EnsSupport<KF, D>(Hj);
+    const float q = div_markstein(r, h.H, h.rH);
+    if (q >= 1.f) return false;
+    float k, p;
+    kernel_kp<KF, D>(q, k, p);
+    const float s = div_markstein(-h.cH * p, h.HH, h.rHH);
+    #pragma unroll
+    for (int a = 0; a < D; ++a) gW.v[a] = s * xij.v[a];
+    return true;
+}
+
+// Pass A (passA_partial over the near entries).
+template <int KF, int D, int G>
+__device__ __forceinline__ void ens_passA(int i, int lane, const EnsArgs& a, const EnsSet& st, Mat<D>& M, Vec<D>& g) {
+    const Vec<D> xi = vec_of_word<D>(get_x_word<D>(st, i));
+    const float4 si = st.sv[i];
+    const float rhoi = si.x;
+    const EnsSupport<KF, D> hi(si.z);
+    EnsWalk<D, G> walk(a, st, i, lane);
+    int j;
+    float4 w;
+    while (walk.take(j, w)) {
+        const float4 sj = st.sv[j];
+        const Vec<D> xij = pair_vec<D>(xi, vec_of_word<D>(w), a.P.dom);
+        const float r = safe_sqrt(dot<D>(xij, xij));
+        Vec<D> gW;
+        if (!ens_grad<KF, D>(xij, r, hi, sj.z, gW)) continue;
+        const float Vj = sj.y;
+        const float dr = sj.x - rhoi;
+        #pragma unroll
+        for (int c = 0; c < D; ++c) {
+            g.v[c] += Vj * dr * gW.v[c];
+            #pragma unroll
+            for (int e = 0; e < D; ++e) M.m[c][e] += Vj * gW.v[c] * (-xij.v[e]);
+        }
+    }
+}
+
+// Pass B (passB_partial over the near entries, without a free-surface indicator).
+template <int KF, int D, int G, bool USUAL>
+__device__ __forceinline__ void ens_passB(int i, int lane, const EnsArgs& a, const EnsSet& st, float& cont, float& dd, Vec<D>& pf,
+                                          Vec<D>& visc) {
+    const WcDev& W = a.W;
+    const float4 wi = get_x_word<D>(st, i), si = st.sv[i], gi = a.gp[i];
+    const Vec<D> xi = vec_of_word<D>(wi), vi = get_v<D>(st, i, wi), gLi = vec_of_word<D>(gi);
+    const float rhoi = si.x, Pi = word_of(gi, D), Hi = si.z;
+    const EnsSupport<KF, D> hi(Hi);
+    const float eps = 1.0e-14f * Hi;
+    const float factor = W.inviscid ? W.alpha * W.c0 * Hi / W.xi : W.visc_nu;
+    EnsWalk<D, G> walk(a, st, i, lane);
+    int j;
+    float4 w;
+    while (walk.take(j, w)) {
+        const float4 sj = st.sv[j], gj = a.gp[j];
+        const Vec<D> xij = pair_vec<D>(xi, vec_of_word<D>(w), a.P.dom);
+        const float r2 = dot<D>(xij, xij);
+        const float r = safe_sqrt(r2);
+        Vec<D> gW;
+        if (!ens_grad<KF, D>(xij, r, hi, sj.z, gW)) continue;
+        const float rj = sj.x, Vj = sj.y;
+        const Vec<D> vj = get_v<D>(st, j, w), gLj = vec_of_word<D>(gj);
+        // continuity (inconsistent.py:19-31): V_j (v_j - v_i).gW
+        float t = 0.f;
+        #pragma unroll
+        for (int c = 0; c < D; ++c) t += (vj.v[c] - vi.v[c]) * gW.v[c];
+        cont += Vj * t;
+        // density diffusion (wp_densityDelta.py:88-117)
+        {
+            const float inv = rcp_markstein(r + eps);
+            const float s = 2.f * (rj - rhoi) * inv * inv;      // 2 (rho_j - rho_i) n_ij / (r + eps), n_ij = x_ij / (r + eps)
+            float pd = 0.f;
+            #pragma unroll
+            for (int c = 0; c < D; ++c) {
+                float psi;
+                if (USUAL || W.density_scheme == SPH_DENSITY_DIFFUSION_DELTA) psi = (gLi.v[c] + gLj.v[c]) - s * xij.v[c];
+                else if (W.density_scheme == SPH_DENSITY_DIFFUSION_DENSITY_ONLY) psi = -(s * xij.v[c]);
+                else psi = gLi.v[c] + gLj.v[c];
+                pd += psi * gW.v[c];
+            }
+            dd += Vj * pd;
+        }
+        // pressure (wp_surfaceAware.py:48-102)
+        {
+            const float Pj = word_of(gj, D);
+            float pij;
+            if (USUAL) pij = (Pi >= 0.f || Pj >= 0.f) ? Pj + Pi : Pj - Pi;
+            else switch (W.pressure_term) {
+                case SPH_PRESSURE_CONSERVATIVE: pij = Pj - Pi; break;
+                case SPH_PRESSURE_NONCONSERVATIVE: pij = Pj + Pi; break;
+                case SPH_PRESSURE_ANTUONO: pij = (Pi >= 0.f || Pj >= 0.f) ? Pj + Pi : Pj - Pi; break;
+                case SPH_PRESSURE_I: pij = Pi; break;
+                case SPH_PRESSURE_J: pij = Pj; break;
+                default: pij = (Pj / (rj * rj) + Pi / (rhoi * rhoi)) * rj; break;
+            }
+            #pragma unroll
+            for (int c = 0; c < D; ++c) pf.v[c] += Vj * pij * gW.v[c];
+        }
+        // velocity diffusion (wp_viscosityDelta.py:86-106)
+        {
+            float vx = 0.f;
+            #pragma unroll
+            for (int c = 0; c < D; ++c) vx += (vi.v[c] - vj.v[c]) * xij.v[c];
+            const float rr = fmaxf(r2 + eps * Hi, 1.2e-38f);
+            float mu = div_markstein(vx, rr, rcp_markstein(rr));
+            mu = mu > 0.f ? 0.f : mu;
+            const float rho_bar = (rj + rhoi) / 2.f;
+            const float ww = div_markstein(Vj * mu * factor, rho_bar, rcp_markstein(rho_bar));
+            #pragma unroll
+            for (int c = 0; c < D; ++c) visc.v[c] += ww * gW.v[c];
+        }
+    }
+}
+
+// Bound by issue slots (64 %) and the latency of the gathers.  1.3 M particles in 64 boxes, 99 entries
+// per row of which 50 interact: 5.84 -> 3.17 ms per step; of that the walk of the near entries, packed
+// words and quotients hoisted to the particle give 2.2 ms, divisions without the general case's
+// branches 0.3 and the usual terms as constants 0.1.  Rows reordered by distance were faster still
+// (2.14 ms) but change the order of the sums: the Antuono pressure switch jumps where P_j crosses 0, so
+// a rounding there moves whole pair terms.  64 registers: 8 blocks of 128 threads per SM.
 template <int KF, int D, int G, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, (D == 3 ? 1 : 1152 / BLOCK))
-k_ens_step(EnsArgs a) {
+__global__ void __launch_bounds__(BLOCK, (D == 3 ? 1 : 1024 / BLOCK))
+k_ens_step(const __grid_constant__ EnsArgs a) {
     constexpr int PPB = BLOCK / G;
     const int lane = threadIdx.x & (G - 1);
     const int rounds = (a.n + (int)gridDim.x * PPB - 1) / ((int)gridDim.x * PPB);
     unsigned int dmax = 0u, arrived = 0;
+    const bool usual = a.W.density_scheme == SPH_DENSITY_DIFFUSION_DELTA && a.W.pressure_term == SPH_PRESSURE_ANTUONO;
+    // ---- the first stage's words
+    for (int i = blockIdx.x * BLOCK + threadIdx.x; i < a.n; i += gridDim.x * BLOCK) {
+        const float r = a.rho[i];
+        put_xv<D>(a.set[0], i, load_vec<D>(a.x, i), load_vec<D>(a.v, i));
+        a.set[0].sv[i] = make_float4(r, a.m[i] / r, a.H[i], 0.f);
+    }
+    if (!grid_barrier(a.ctl, arrived)) { if (threadIdx.x == 0) atomicOr(a.status, SPH_STATUS_TIMEOUT); return; }
     for (int stage = 0; stage < 2; ++stage) {
-        const float* xs = stage == 0 ? a.x : a.x1;
-        const float* vs = stage == 0 ? a.v : a.v1;
-        const float* rs = stage == 0 ? a.rho : a.rho1;
+        const EnsSet& st = a.set[stage];
         // ---- pass A: renormalised density gradient and EOS
         for (int rd = 0; rd < rounds; ++rd) {
             const int i = (rd * (int)gridDim.x + (int)blockIdx.x) * PPB + (int)threadIdx.x / G;
             const bool valid = i < a.n;
             Mat<D> M = mzero<D>();
             Vec<D> s = vzero<D>();
-            if (valid) passA_partial<KF, D, G, true>(i, lane, a.P, xs, a.H, a.m, rs, a.offs, a.cnt, a.list, M, s);
+            if (valid) {
+                if (stage == 0) ens_near<D, G>(i, lane, a, st);
+                ens_passA<KF, D, G>(i, lane, a, st, M, s);
+            }
             passA_reduce<D, G>(M, s);
             if (valid && lane == 0) {
-                store_vec<D>(a.gL, i, renormalise<D>(M, s));
-                a.Pr[i] = wc_eos(a.W, __ldcg(rs + i));
+                const Vec<D> g = renormalise<D>(M, s);
+                const float Pr = wc_eos(a.W, st.sv[i].x);
+                float w[4] = {0.f, 0.f, 0.f, 0.f};
+                #pragma unroll
+                for (int c = 0; c < D; ++c) w[c] = g.v[c];
+                w[D] = Pr;
+                a.gp[i] = make_float4(w[0], w[1], w[2], w[3]);
             }
         }
         if (!grid_barrier(a.ctl, arrived)) { if (threadIdx.x == 0) atomicOr(a.status, SPH_STATUS_TIMEOUT); return; }
@@ -221,28 +495,31 @@ k_ens_step(EnsArgs a) {
             const bool valid = i < a.n;
             float cont = 0.f, dd = 0.f;
             Vec<D> pf = vzero<D>(), visc = vzero<D>();
-            if (valid) passB_partial<KF, D, G, true>(i, lane, a.P, a.W, xs, a.H, a.m, rs, vs, a.gL, a.Pr, nullptr, a.offs, a.cnt,
-                                                        a.list, cont, dd, pf, visc);
+            if (valid) {
+                if (usual) ens_passB<KF, D, G, true>(i, lane, a, st, cont, dd, pf, visc);
+                else ens_passB<KF, D, G, false>(i, lane, a, st, cont, dd, pf, visc);
+            }
             cont = gsum<G>(cont); dd = gsum<G>(dd);
             #pragma unroll
             for (int c = 0; c < D; ++c) { pf.v[c] = gsum<G>(pf.v[c]); visc.v[c] = gsum<G>(visc.v[c]); }
             if (valid && lane == 0) {
                 float dr; Vec<D> dv;
-                passB_finish<D>(a.W, __ldcg(rs + i), a.H[i], cont, dd, pf, visc, dr, dv);
+                passB_finish<D>(a.W, st.sv[i].x, a.H[i], cont, dd, pf, visc, dr, dv);
                 const float dt = a.box_dt[a.box_of[i]];
-                const Vec<D> x0 = ldv<D, true>(a.x, i), v0 = ldv<D, true>(a.v, i);
-                const float r0 = __ldcg(a.rho + i);
+                const float4 w0 = get_x_word<D>(a.set[0], i);
+                const Vec<D> x0 = vec_of_word<D>(w0), v0 = get_v<D>(a.set[0], i, w0);
+                const float r0 = a.set[0].sv[i].x;
                 if (stage == 0) {
                     Vec<D> xn, vn;
                     #pragma unroll
                     for (int c = 0; c < D; ++c) { xn.v[c] = x0.v[c] + dt * v0.v[c]; vn.v[c] = v0.v[c] + dt * dv.v[c]; }
-                    store_vec<D>(a.x1, i, wrap_pos<D>(xn, a.P.dom));
-                    store_vec<D>(a.v1, i, vn);
-                    a.rho1[i] = r0 + dt * dr;
+                    const float rn = r0 + dt * dr;
+                    put_xv<D>(a.set[1], i, wrap_pos<D>(xn, a.P.dom), vn);
+                    a.set[1].sv[i] = make_float4(rn, a.m[i] / rn, a.H[i], 0.f);
                     store_vec<D>(a.dv1, i, dv);
                     a.drho1[i] = dr;
                 } else {
-                    const Vec<D> v1 = ldv<D, true>(a.v1, i), k1 = ldv<D, true>(a.dv1, i);
+                    const Vec<D> v1 = get_v<D>(st, i, get_x_word<D>(st, i)), k1 = ldv<D, true>(a.dv1, i);
                     const float h = 0.5f * dt;
                     Vec<D> xn, vn;
                     #pragma unroll
@@ -331,24 +608,26 @@ int sph_ensemble_neighbors_build(const SphParams* p, int64_t n, int32_t nbox, co
     k_ens_scatter<<<grid_for(n, 256), 256, 0, s>>>((int)n, w.keys, w.slot, w.start, w.sorted);
     count_launch();
     k_ens_sort_cells<<<grid_for(total_cells, 256), 256, 0, s>>>(total_cells, w.start, w.counts, w.sorted);
+    count_launch();
+    WSPH_DISPATCH_DIM(P.dim, (k_ens_pack_sorted<D><<<grid_for(n, 256), 256, 0, s>>>((int)n, x, H, w.sorted, w.words)));
     constexpr int GE = 8;
     count_launch();
     WSPH_DISPATCH_DIM(P.dim, (k_ens_verlet<D, GE, false><<<grid_for(n * GE, 128), 128, 0, s>>>(
-        (int)n, P, x, H, box_of, box_grid, box_cell_base, w.start, w.counts, w.sorted, cnt, nullptr, nullptr, nullptr, 0)));
+        (int)n, P, x, H, box_of, box_grid, box_cell_base, w.start, w.counts, w.sorted, w.words, cnt, nullptr, nullptr, nullptr, 0)));
     exclusive_scan_i32(cnt, offs, n, w.scan, reinterpret_cast<long long*>(nnz_out), s);
     count_launch();
     k_ens_check<<<1, 1, 0, s>>>(reinterpret_cast<long long*>(nnz_out), list_capacity, status);
     count_launch();
     WSPH_DISPATCH_DIM(P.dim, (k_ens_verlet<D, GE, true><<<grid_for(n * GE, 128), 128, 0, s>>>(
-        (int)n, P, x, H, box_of, box_grid, box_cell_base, w.start, w.counts, w.sorted, nullptr, offs, list,
+        (int)n, P, x, H, box_of, box_grid, box_cell_base, w.start, w.counts, w.sorted, w.words, nullptr, offs, list,
         reinterpret_cast<long long*>(nnz_out), list_capacity)));
     return check_launch("sph_ensemble_neighbors_build");
 }
 
 int64_t sph_ensemble_step_workspace_size(int64_t n, int32_t dim) {
     if (n < 0 || dim < 1 || dim > 3) return -1;
-    // control block, x1 v1 dv1 gL (n*dim each), rho1 drho1 Pr (n each)
-    return 256 + 4 * al256(n * dim * 4) + 3 * al256(n * 4);
+    // control block, xv (twice in 3D) and sv of two stages, gp, the near bits, dv1 (n*dim), drho1 (n)
+    return 256 + ((dim == 3 ? 4 : 2) + 2 + 1) * al256(n * 16) + al256(n * (ENS_NEAR / 8)) + al256(n * dim * 4) + al256(n * 4);
 }
 
 int sph_ensemble_step(const SphParams* p, const SphWcParams* wc, int64_t n, const int32_t* box_of, const float* box_dt,
@@ -375,14 +654,15 @@ int sph_ensemble_step(const SphParams* p, const SphWcParams* wc, int64_t n, cons
     a.n = (int)n; a.P = P; a.W = W; a.box_of = box_of; a.box_dt = box_dt; a.H = H; a.m = m; a.x_build = x_build;
     a.x = x; a.v = v; a.rho = rho;
     int64_t o = 256;
-    const int64_t vb = al256(n * P.dim * 4), sb = al256(n * 4);
-    a.x1 = reinterpret_cast<float*>(w + o); o += vb;
-    a.v1 = reinterpret_cast<float*>(w + o); o += vb;
-    a.dv1 = reinterpret_cast<float*>(w + o); o += vb;
-    a.gL = reinterpret_cast<float*>(w + o); o += vb;
-    a.rho1 = reinterpret_cast<float*>(w + o); o += sb;
-    a.drho1 = reinterpret_cast<float*>(w + o); o += sb;
-    a.Pr = reinterpret_cast<float*>(w + o); o += sb;
+    const int64_t qb = al256(n * 16);
+    for (EnsSet& q : a.set) {
+        q.xv = reinterpret_cast<float4*>(w + o); o += P.dim == 3 ? 2 * qb : qb;
+        q.sv = reinterpret_cast<float4*>(w + o); o += qb;
+    }
+    a.gp = reinterpret_cast<float4*>(w + o); o += qb;
+    a.near = w + o; o += al256(n * (ENS_NEAR / 8));
+    a.dv1 = reinterpret_cast<float*>(w + o); o += al256(n * P.dim * 4);
+    a.drho1 = reinterpret_cast<float*>(w + o);
     a.offs = offs; a.cnt = cnt; a.list = list;
     a.ctl = reinterpret_cast<BarrierCtl*>(w);
     a.disp = disp_max; a.status = status;
