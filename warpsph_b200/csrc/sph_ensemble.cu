@@ -226,11 +226,14 @@ template <int D> __device__ __forceinline__ void put_xv(const EnsSet& s, int i, 
 }
 template <int D> __device__ __forceinline__ float4 get_x_word(const EnsSet& s, int i) { return s.xv[D == 3 ? 2 * (size_t)i : (size_t)i]; }
 template <int D> __device__ __forceinline__ Vec<D> get_v(const EnsSet& s, int i, const float4& xw) {
-    if constexpr (D == 3) return vec_of_word<3>(s.xv[2 * (size_t)i + 1]);
-    Vec<D> v;
-    #pragma unroll
-    for (int a = 0; a < D; ++a) v.v[a] = word_of(xw, D + a);
-    return v;
+    if constexpr (D == 3) {
+        return vec_of_word<3>(s.xv[2 * (size_t)i + 1]);
+    } else {
+        Vec<D> v;
+        #pragma unroll
+        for (int a = 0; a < D; ++a) v.v[a] = word_of(xw, D + a);
+        return v;
+    }
 }
 
 // The entries of a row that are inside the support at y0 or at y1 = y0 + dt v0 are known before the

@@ -294,6 +294,7 @@ k_crk_factors(int n, DevParams P, const float* __restrict__ x, const float* __re
         const Vec<D> xi = PK ? vec_of_word<D>(__ldg(fw.xh + g.i)) : load_vec<D>(x, g.i);
         int b = offs[g.i], e = b + cnt[g.i];
         typename PairPipe<D, PK>::T rp(list, PairPipe<D, PK>::src(x, fw.xh), b + g.lane, e, G);
+        float Vn = __ldg(V + rp.j1), mn = __ldg(m + rp.j1);
         for (int q = b + g.lane; q < e; q += G) {
             int j;
             Vec<D> xj;
@@ -306,7 +307,9 @@ k_crk_factors(int n, DevParams P, const float* __restrict__ x, const float* __re
                 rp.take(q, j, xj);
                 invHj = rcp_newton(__ldg(H + j));
             }
-            const float Vj = __ldg(V + j), mj = __ldg(m + j);   // gathers issued together
+            const float Vj = Vn, mj = mn;
+            Vn = __ldg(V + rp.j1);
+            mn = __ldg(m + rp.j1);
             const Vec<D> xij = pair_vec<D>(xi, xj, P.dom);
             const float q1 = sqrt_newton(dot<D>(xij, xij)) * invHj;
             if (!(q1 < 1.f)) continue;
@@ -646,11 +649,13 @@ k_grad_v_packed(int n, DevParams P, const float4* __restrict__ xh, const float4*
         const Mat<D> gBi = load_mat<D>(gB, i);
         const int b = offs[i], e = b + cnt[i];
         WordPipe rp(list, xh, b + g.lane, e, G);
+        float4 fn = __ldg(fv + rp.j1);         // 3D: a second word ahead (0.68 -> 0.67 ms; 2D: 65 -> 67 us)
         for (int q = b + g.lane; q < e; q += G) {
             int j;
             float4 t;
             rp.take(q, j, t);
-            const float4 f = __ldg(fv + j);
+            const float4 f = D == 3 ? fn : __ldg(fv + j);
+            if (D == 3) fn = __ldg(fv + rp.j1);
             const float vol3 = D == 3 && want_div ? __ldg(volume + j) : 0.f;
             const Vec<D> xij = pair_vec<D>(xi, vec_of_word<D>(t), P.dom), vj = vec_of_word<D>(f);
             const float r = sqrt_newton(dot<D>(xij, xij)), invHj = inv_support_of<D>(t);
@@ -951,20 +956,15 @@ __device__ __forceinline__ float limiter_vl(float x) {
     float vL = __fdividef(2.f, 1.f + x);
     return x * vL * vL;
 }
-__device__ __forceinline__ float sgn_pos(float x) { return x >= 0.f ? 1.f : -1.f; }
 
-// modules/crk/limiter.py:27-86 (quadratic-form Van Leer) with g = (G h).h, h = x_ij / 2,
-// from the products G_i x_ij and G_j x_ij the pass needs anyway: halving is exact in
-// floating point, so (G h).h = (G x_ij).x_ij / 4 (outside the subnormal range).
-template <int D>
-__device__ __forceinline__ float van_leer(const Vec<D>& xij_, const Vec<D>& Gix, const Vec<D>& Gjx) {
-    float gi = 0.25f * dot<D>(Gix, xij_);
-    float gj = 0.25f * dot<D>(Gjx, xij_);
-    float ri = __fdividef(gi, sgn_pos(gj) * fabsf(gj));
-    float rj = __fdividef(gj, sgn_pos(gi) * fabsf(gi));
-    if (ri != ri) ri = 1.f;
-    if (rj != rj) rj = 1.f;
-    return limiter_vl(wmin(ri, rj));
+// modules/crk/limiter.py:27-86 (quadratic-form Van Leer) from g_i = x_ij.(G_i x_ij) and g_j, whose
+// quarters are the reference's (G h).h, h = x_ij / 2.  The limiter's argument min(g_i / g_j, g_j / g_i)
+// is the quotient of the smaller by the larger where their signs agree, and not positive where they differ.
+__device__ __forceinline__ float van_leer(float gi, float gj) {
+    const bool less = fabsf(gi) < fabsf(gj);
+    float x = __fdividef(less ? gi : gj, less ? gj : gi);
+    if (x != x) x = 1.f;
+    return limiter_vl(x);
 }
 
 // Zero pairwise outputs of the entries [offs + cnt, offs + vcnt) of a row: the Verlet
@@ -986,9 +986,9 @@ __device__ __forceinline__ void zero_row_tail(int lane, int e, int te, float* __
 // (before the distance test), velocity, gradient, sound speed and pressure (the limiter
 // and Q), and the rest (the corrected gradient of W_ji), which keeps fewer of them live.
 template <int D> struct CrkRec {
-    static constexpr int X = 0, H = D, RHO = D + 1, V = D + 2, G = 2 * D + 2, C = 2 * D + 2 + D * D, P = C + 1,
-                         VOL = C + 2, A = C + 3, B = C + 4, GA = B + D, GB = GA + D, END = GB + D * D,
-                         R = (END + 3) / 4 * 4;
+    static constexpr int NS = D * (D + 1) / 2;
+    static constexpr int X = 0, H = D, QQ = D + 1, V = D + 2, S = 2 * D + 2, QL = S + NS, P = QL + 1, VOL = P + 1, A = P + 2,
+                         C = P + 3, E = C + D, F = E + D, END = F + D * D, R = (END + 3) / 4 * 4;
     static constexpr int K1 = (H + 1 + 3) / 4;      // granules of the first group
     static constexpr int K2 = (P + 1 + 3) / 4;      // ... of the first two groups
     static constexpr int K3 = R / 4;
@@ -1002,45 +1002,51 @@ __device__ __forceinline__ void rec_granules(const float4* __restrict__ rec, int
     }
 }
 
+// The fields of one particle as the accel pass uses them, with what depends on it alone formed once:
+//   grad W^R = A (1 + B.x) s x + W (gA (1 + B.x) + A (B + gB^T x)) = s (A + C.x) x + W (E + F x),
+//              C = A B, E = gA + A B, F = gA B^T + A gB^T (x = x_ij, grad W = s x)
+//   x.(G x)  = S over the products x_a x_b, a <= b (the velocity gradient enters the pass through it alone)
+//   rho (-C_l c mu + C_q mu^2) = mu (qq mu - ql), qq = rho C_q, ql = rho C_l c
+template <int D> struct CrkPart {
+    Vec<D> x, v, C, E;
+    Mat<D> F;
+    float S[D * (D + 1) / 2];
+    float H, V, P, A, qq, ql;
+};
 template <int D>
-__global__ void k_crk_pack(int n, const float* __restrict__ x, const float* __restrict__ H, const float* __restrict__ rho,
-                           const float* __restrict__ V, const float* __restrict__ A, const float* __restrict__ B,
-                           const float* __restrict__ gA, const float* __restrict__ gB, const float* __restrict__ v,
-                           const float* __restrict__ c, const float* __restrict__ Pr, const float* __restrict__ DvDx,
-                           float* __restrict__ rec) {
-    pdl_entry();
-    using L = CrkRec<D>;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float r[L::R];
+__device__ __forceinline__ void crk_part(const DevParams& P, float rho, float c, float A, const Vec<D>& B, const Vec<D>& gA, const Mat<D>& gB,
+                                         const Mat<D>& G, CrkPart<D>& o) {
+    o.A = A;
     #pragma unroll
     for (int a = 0; a < D; ++a) {
-        r[L::X + a] = x[(size_t)i * D + a];
-        r[L::V + a] = v[(size_t)i * D + a];
-        r[L::B + a] = B[(size_t)i * D + a];
-        r[L::GA + a] = gA[(size_t)i * D + a];
+        o.C.v[a] = A * B.v[a];
+        o.E.v[a] = gA.v[a] + o.C.v[a];
+        #pragma unroll
+        for (int b = 0; b < D; ++b) o.F.m[a][b] = gA.v[a] * B.v[b] + A * gB.m[b][a];
     }
+    int k = 0;
     #pragma unroll
-    for (int a = 0; a < D * D; ++a) {
-        r[L::GB + a] = gB[(size_t)i * D * D + a];
-        r[L::G + a] = DvDx[(size_t)i * D * D + a];
-    }
-    r[L::H] = H[i]; r[L::RHO] = rho[i]; r[L::VOL] = V[i]; r[L::C] = c[i]; r[L::P] = Pr[i]; r[L::A] = A[i];
-    #pragma unroll
-    for (int a = L::END; a < L::R; ++a) r[a] = 0.f;
-    float4* dst = reinterpret_cast<float4*>(rec) + i;
-    #pragma unroll
-    for (int k = 0; k < L::R / 4; ++k) dst[(size_t)k * n] = make_float4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+    for (int a = 0; a < D; ++a)
+        #pragma unroll
+        for (int b = a; b < D; ++b) o.S[k++] = a == b ? G.m[a][a] : G.m[a][b] + G.m[b][a];
+    o.qq = rho * P.C_q;
+    o.ql = rho * P.C_l * c;
 }
-
-// The fields of one particle as the accel pass uses them.
-template <int D> struct CrkPart {
-    Vec<D> x, v, B, gA;
-    Mat<D> gB, G;
-    float H, rho, V, c, P, A;
-};
-// Group 1: position and support; group 2: velocity, velocity gradient, density, sound
-// speed, pressure; group 3: volume and the CRK correction fields.
+// s (A + C.x) x + W (E + F x)
+template <int D> __device__ __forceinline__ Vec<D> crk_part_grad(const CrkPart<D>& p, const Vec<D>& x, float W, float s) {
+    const float cx = s * (p.A + dot<D>(p.C, x));
+    Vec<D> r;
+    #pragma unroll
+    for (int g = 0; g < D; ++g) {
+        float t = p.E.v[g];
+        #pragma unroll
+        for (int a = 0; a < D; ++a) t += p.F.m[g][a] * x.v[a];
+        r.v[g] = cx * x.v[g] + W * t;
+    }
+    return r;
+}
+// Group 1: position and support; group 2: velocity, velocity gradient, viscosity factors and
+// pressure; group 3: volume and the corrections.
 template <int D> __device__ __forceinline__ void crk_unpack1(const float (&r)[CrkRec<D>::R], CrkPart<D>& o) {
     using L = CrkRec<D>;
     #pragma unroll
@@ -1052,20 +1058,46 @@ template <int D> __device__ __forceinline__ void crk_unpack2(const float (&r)[Cr
     #pragma unroll
     for (int a = 0; a < D; ++a) o.v.v[a] = r[L::V + a];
     #pragma unroll
-    for (int a = 0; a < D; ++a)
-        #pragma unroll
-        for (int b = 0; b < D; ++b) o.G.m[a][b] = r[L::G + a * D + b];
-    o.rho = r[L::RHO]; o.c = r[L::C]; o.P = r[L::P];
+    for (int a = 0; a < L::NS; ++a) o.S[a] = r[L::S + a];
+    o.qq = r[L::QQ]; o.ql = r[L::QL]; o.P = r[L::P];
 }
 template <int D> __device__ __forceinline__ void crk_unpack3(const float (&r)[CrkRec<D>::R], CrkPart<D>& o) {
     using L = CrkRec<D>;
     #pragma unroll
-    for (int a = 0; a < D; ++a) { o.B.v[a] = r[L::B + a]; o.gA.v[a] = r[L::GA + a]; }
+    for (int a = 0; a < D; ++a) { o.C.v[a] = r[L::C + a]; o.E.v[a] = r[L::E + a]; }
     #pragma unroll
-    for (int a = 0; a < D; ++a)
-        #pragma unroll
-        for (int b = 0; b < D; ++b) o.gB.m[a][b] = r[L::GB + a * D + b];
+    for (int a = 0; a < D * D; ++a) o.F.m[a / D][a % D] = r[L::F + a];
     o.V = r[L::VOL]; o.A = r[L::A];
+}
+
+template <int D>
+__global__ void k_crk_pack(int n, DevParams P, const float* __restrict__ x, const float* __restrict__ H, const float* __restrict__ rho,
+                           const float* __restrict__ V, const float* __restrict__ A, const float* __restrict__ B,
+                           const float* __restrict__ gA, const float* __restrict__ gB, const float* __restrict__ v,
+                           const float* __restrict__ c, const float* __restrict__ Pr, const float* __restrict__ DvDx,
+                           float* __restrict__ rec) {
+    pdl_entry();
+    using L = CrkRec<D>;
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    CrkPart<D> o;
+    o.x = load_vec<D>(x, i);
+    o.v = load_vec<D>(v, i);
+    o.H = H[i]; o.V = V[i]; o.P = Pr[i];
+    crk_part<D>(P, rho[i], c[i], A[i], load_vec<D>(B, i), load_vec<D>(gA, i), load_mat<D>(gB, i), load_mat<D>(DvDx, i), o);
+    float r[L::R];
+    #pragma unroll
+    for (int a = 0; a < D; ++a) { r[L::X + a] = o.x.v[a]; r[L::V + a] = o.v.v[a]; r[L::C + a] = o.C.v[a]; r[L::E + a] = o.E.v[a]; }
+    #pragma unroll
+    for (int a = 0; a < L::NS; ++a) r[L::S + a] = o.S[a];
+    #pragma unroll
+    for (int a = 0; a < D * D; ++a) r[L::F + a] = o.F.m[a / D][a % D];
+    r[L::H] = o.H; r[L::QQ] = o.qq; r[L::QL] = o.ql; r[L::P] = o.P; r[L::VOL] = o.V; r[L::A] = o.A;
+    #pragma unroll
+    for (int a = L::END; a < L::R; ++a) r[a] = 0.f;
+    float4* dst = reinterpret_cast<float4*>(rec) + i;
+    #pragma unroll
+    for (int k = 0; k < L::R / 4; ++k) dst[(size_t)k * n] = make_float4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
 }
 
 // modules/crk/accel.py:65-250 and modules/crk/dudt.py:62-229 in one pass.  The pair
@@ -1105,13 +1137,13 @@ k_crk_accel_dudt(int n, DevParams P, const float* __restrict__ x, const float* _
             rec_granules<D, 0, CrkRec<D>::K3>(reinterpret_cast<const float4*>(rec), n, i, r);
             crk_unpack1<D>(r, pi); crk_unpack2<D>(r, pi); crk_unpack3<D>(r, pi);
         } else {
-            pi.x = load_vec<D>(x, i); pi.v = load_vec<D>(v, i); pi.B = load_vec<D>(B, i); pi.gA = load_vec<D>(gA, i);
-            pi.gB = load_mat<D>(gB, i); pi.G = load_mat<D>(DvDx, i);
-            pi.H = H[i]; pi.rho = rho[i]; pi.V = V[i]; pi.c = c[i]; pi.P = Pr[i]; pi.A = A[i];
+            pi.x = load_vec<D>(x, i); pi.v = load_vec<D>(v, i);
+            pi.H = H[i]; pi.V = V[i]; pi.P = Pr[i];
+            crk_part<D>(P, rho[i], c[i], A[i], load_vec<D>(B, i), load_vec<D>(gA, i), load_mat<D>(gB, i), load_mat<D>(DvDx, i), pi);
         }
-        const float Hi = pi.H, rhoi = pi.rho, ci = pi.c, Pi = pi.P;
+        const float Hi = pi.H, Pi = pi.P;
         const float invHi = 1.f / Hi;
-        const float Vi_m = pi.V / m[i];          // V_i / m_i
+        const float hVi_m = 0.5f * (pi.V / m[i]);
         const float ks = P.kscale;
         const float inv_smooth_i = ks * invHi;   // 1 / (H_i / ks)
         const float sm_i = Hi / ks;
@@ -1142,72 +1174,80 @@ k_crk_accel_dudt(int n, DevParams P, const float* __restrict__ x, const float* _
                 crk_unpack2<D>(rj, pj);
             } else {
                 pj.v = load_vec<D>(v, j);
-                pj.rho = __ldg(rho + j); pj.c = __ldg(c + j); pj.P = __ldg(Pr + j);
-                pj.G = load_mat<D>(DvDx, j);
+                pj.P = __ldg(Pr + j);
+                pj.V = __ldg(V + j);
+                crk_part<D>(P, __ldg(rho + j), __ldg(c + j), __ldg(A + j), load_vec<D>(B, j), load_vec<D>(gA, j), load_mat<D>(gB, j),
+                            load_mat<D>(DvDx, j), pj);
             }
             float r = sqrt_newton(r2);
             const float invHj = rcp_newton(Hj);
-            const float rhoj = pj.rho, cj = pj.c, Pj = pj.P;
+            const float Pj = pj.P;
             // CRK limiter (limiter.py:89-128), eta measured in supports
             float factor = 1.f;
             if (P.enable_crk_limiter) {
                 float eta = r * wmin(invHi, invHj);
                 if (eta < P.eta_crit) { float t = (eta - P.eta_crit) / P.eta_fold; factor = expf(-(t * t)); }
             }
-            Vec<D> Gix = matvec<D>(pi.G, xij), Gjx = matvec<D>(pj.G, xij);
+            float gi = 0.f, gj = 0.f;
+            {
+                int u = 0;
+                #pragma unroll
+                for (int a = 0; a < D; ++a)
+                    #pragma unroll
+                    for (int b = a; b < D; ++b) {
+                        const float xx = xij.v[a] * xij.v[b];
+                        gi += pi.S[u] * xx;
+                        gj += pj.S[u] * xx;
+                        ++u;
+                    }
+            }
             float phi = 0.f;
-            if (P.enable_vanleer) phi = van_leer<D>(xij, Gix, Gjx) * factor;
+            if (P.enable_vanleer) phi = van_leer(gi, gj) * factor;
             if (P.force_vl_off) phi = 0.f;
             if (P.force_vl_on) phi = 1.f;
             phi = wmax(wmin(phi, 1.f), 0.f);
-            float hp = 0.5f * phi;
-            // v_dot_i - v_dot_j (accel.py:137-141; dudt.py:122-126 uses gradV_j . (-x_ij))
-            Vec<D> da, dd;
-            #pragma unroll
-            for (int a = 0; a < D; ++a) {
-                float vdi = pi.v.v[a] - hp * Gix.v[a];
-                da.v[a] = vdi - (pj.v.v[a] + hp * Gjx.v[a]);
-                dd.v[a] = vdi - (pj.v.v[a] - hp * Gjx.v[a]);
-            }
+            const float hp = 0.5f * phi;
             // corrected gradients (accel.py:170-187, dudt.py:155-170)
             float Wi, si;
             kWS_inv<KF, D>(r, invHj, Wi, si);
-            Vec<D> gradw_i = crk_grad_s<D>(xij, Wi, si, pi.A, pi.B, pi.gA, pi.gB);
+            const Vec<D> gradw_i = crk_part_grad<D>(pi, xij, Wi, si);
             if constexpr (REC) {
                 rec_granules<D, CrkRec<D>::K2, CrkRec<D>::K3>(sj, n, j, rj); crk_unpack3<D>(rj, pj);
-            } else {
-                pj.V = __ldg(V + j);
-                pj.A = __ldg(A + j); pj.B = load_vec<D>(B, j); pj.gA = load_vec<D>(gA, j); pj.gB = load_mat<D>(gB, j);
             }
             Vec<D> xji;
             #pragma unroll
             for (int a = 0; a < D; ++a) xji.v[a] = -xij.v[a];
             float Wj, sj_;
             kWS_inv<KF, D>(r, invHi, Wj, sj_);
-            Vec<D> gradw_j = crk_grad_s<D>(xji, Wj, sj_, pj.A, pj.B, pj.gA, pj.gB);
-            Vec<D> gij;
+            const Vec<D> gradw_j = crk_part_grad<D>(pj, xji, Wj, sj_);
+            Vec<D> gij;                            // twice the mean gradient; the half is in w
             #pragma unroll
-            for (int a = 0; a < D; ++a) gij.v[a] = 0.5f * (gradw_i.v[a] - gradw_j.v[a]);
+            for (int a = 0; a < D; ++a) gij.v[a] = gradw_i.v[a] - gradw_j.v[a];
             // mu_ij, mu_ji and Q (accel.py:189-206): eta = x_ij / smoothing length
             const float inv_smooth_j = ks * invHj;
             const float sm_j = Hj / ks;
             const float eps_j = 1.0e-7f * sm_j * sm_j;
             float den_i = r2 * (inv_smooth_i * inv_smooth_i) + eps_i;
             float den_j = r2 * (inv_smooth_j * inv_smooth_j) + eps_j;
-            float xa = dot<D>(da, xij), xd = dot<D>(dd, xij);
+            // (v_dot_i - v_dot_j).x_ij with the half gradients taken off (accel.py:137-141; dudt.py:122-126 uses
+            // gradV_j . (-x_ij))
+            float vx = 0.f;
+            #pragma unroll
+            for (int a = 0; a < D; ++a) vx += (pi.v.v[a] - pj.v.v[a]) * xij.v[a];
+            const float xa = vx - hp * (gi + gj), xd = vx - hp * (gi - gj);
             float idi = __fdividef(inv_smooth_i, den_i), idj = __fdividef(inv_smooth_j, den_j);
             float mia = wmin(0.f, xa * idi), mja = wmin(0.f, xa * idj);
             float mid = wmin(0.f, xd * idi), mjd = wmin(0.f, xd * idj);
-            float Qa = rhoi * (-P.C_l * ci * mia + P.C_q * mia * mia) + rhoj * (-P.C_l * cj * mja + P.C_q * mja * mja);
-            float Qd = rhoi * (-P.C_l * ci * mid + P.C_q * mid * mid) + rhoj * (-P.C_l * cj * mjd + P.C_q * mjd * mjd);
+            const float Qa = mia * (pi.qq * mia - pi.ql) + mja * (pj.qq * mja - pj.ql);
+            const float Qd = mid * (pi.qq * mid - pi.ql) + mjd * (pj.qq * mjd - pj.ql);
             // accel.py:228-249 (mu_ij = 1 there)
-            const float w = pj.V * Vi_m;   // V_i V_j / m_i
+            const float w = pj.V * hVi_m, cp = -(Pi + Pj) * w, cv = -Qa * w;   // V_i V_j / (2 m_i)
             Vec<D> pt, vt;
             float dotu = 0.f;
             #pragma unroll
             for (int a = 0; a < D; ++a) {
-                pt.v[a] = -(Pi + Pj) * gij.v[a] * w;
-                vt.v[a] = -Qa * gij.v[a] * w;
+                pt.v[a] = cp * gij.v[a];
+                vt.v[a] = cv * gij.v[a];
                 acc[a].add(pt.v[a] + vt.v[a], comp);
                 dotu += (pi.v.v[a] - pj.v.v[a]) * gij.v[a];
             }
@@ -1310,12 +1350,10 @@ k_balance(int n, DevParams P, const float* __restrict__ m, const float* __restri
         float f = 0.5f;
         if (scheme == SPH_ENERGY_CRK) {
             const float sj = sj_crk;
-            float smin = wmin(fabsf(si), fabsf(sj)), smax = wmax(fabsf(si), fabsf(sj));
-            bool mA = fabsf(si - sj) == 0.f;
-            bool mB = (dE >= 0.f && si >= sj) || (dE < 0.f && si < sj);
-            bool mC = (dE >= 0.f && si < sj) || (dE < 0.f && si >= sj);
-            if (!mA && mB) f = smin / (smin + smax + 1.0e-14f);
-            if (!mA && !mB && mC) f = smax / (smin + smax + 1.0e-14f);
+            const float smin = wmin(fabsf(si), fabsf(sj)), smax = wmax(fabsf(si), fabsf(sj));
+            const bool mB = (dE >= 0.f && si >= sj) || (dE < 0.f && si < sj);
+            const bool mC = (dE >= 0.f && si < sj) || (dE < 0.f && si >= sj);
+            if (fabsf(si - sj) != 0.f && (mB || mC)) f = (mB ? smin : smax) * rcp_newton(smin + smax + 1.0e-14f);
             f = wmax(0.f, wmin(1.f, f));
         } else if (scheme == SPH_ENERGY_PDV) {
             float rhoj = __ldg(rho + j), Pj = __ldg(Pr + j);
@@ -1482,6 +1520,7 @@ k_finalize(int n, int ns, StagePtrs S, int pdv, const float* __restrict__ dtp, c
             const float w = S.w[s];
             int b = S.offs[s][g.i], e = b + S.cnt[s][g.i];
             float acc = 0.f;
+            #pragma unroll 4
             for (int q = b + g.lane; q < e; q += G) {
                 int j, k; entry(lst, q, j, k);
                 Vec<D> vj = half(j);
@@ -1860,7 +1899,7 @@ static int crk_accel_dudt_impl(const SphParams* p, int64_t n, const float* x, co
         return set_error(SPH_ERR_BAD_ARG, "%s: records must be 16-byte aligned", name);
     if (records) {
         wsph::count_launch();
-        WSPH_DISPATCH_DS(*p, (launch_pdl(k_crk_pack<D>, (unsigned)((n + 255) / 256), 256, 0, s, (int)n, x, H, rho, V, A, B, gradA, gradB, v, c,
+        WSPH_DISPATCH_DS(*p, (launch_pdl(k_crk_pack<D>, (unsigned)((n + 255) / 256), 256, 0, s, (int)n, P, x, H, rho, V, A, B, gradA, gradB, v, c,
                                                                                        Pr, DvDx, records)));
         wsph::count_launch();
         WSPH_DISPATCH_KDS(*p, PAIR_LANES(n, G_ACCEL(D), G_WIDE, launch_pdl(k_crk_accel_dudt<KF, D, LG, true>, grid_g<LG>(n), PAIR_BLOCK, 0, s, (int)n, P, x, H, m, rho, V, A, B, gradA, gradB, v, c, Pr, DvDx, records, offs, cnt, list,
