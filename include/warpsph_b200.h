@@ -350,8 +350,8 @@ int sph_crk_factors_eos(const SphParams* p, int64_t n, const float* x, const flo
  *   fv [n][4]   velocity; below 3D V and m / rho in words 2 and 3, in 3D V in word 3 and m / rho in vol [n]
  *   fc [n][4]   velocity; below 3D c and m sgn(div) in words 2 and 3, in 3D c in word 3 and m sgn(div) in msgn [n]
  * sph_pack_xh writes xh.  sph_crk_factors_packed is sph_crk_factors_eos reading xh, and writes fv
- * (vol) from v.  sph_grad_v_packed is sph_grad_v without v_sig reading xh and fv, and with div_out
- * writes fc (msgn).  sph_switch_cullen_packed is sph_switch_cullen with v_sig from xh and fc over
+ * (vol) from v.  sph_grad_v_packed is sph_grad_v without v_sig reading xh and fv; with
+ * divergence_out it writes -drhodt / rho (schemes/crkSPH.py:324), and with div_out fc (msgn).  sph_switch_cullen_packed is sph_switch_cullen with v_sig from xh and fc over
  * the Verlet rows. */
 int sph_pack_xh(const SphParams* p, int64_t n, const float* x, const float* H, float* xh, void* stream);
 int sph_crk_factors_packed(const SphParams* p, int64_t n, const float* xh, const float* m, const float* V,
@@ -362,8 +362,8 @@ int sph_crk_factors_packed(const SphParams* p, int64_t n, const float* xh, const
 int sph_grad_v_packed(const SphParams* p, int64_t n, const float* xh, const float* fv, const float* vol,
                       const float* m, const float* rho, const float* c, const float* A, const float* B,
                       const float* gradA, const float* gradB, const int32_t* offs, const int32_t* cnt,
-                      const int32_t* list, float* DvDx_out, float* drhodt_out, float* div_out, float* fc,
-                      float* msgn, void* stream);
+                      const int32_t* list, float* DvDx_out, float* drhodt_out, float* divergence_out,
+                      float* div_out, float* fc, float* msgn, void* stream);
 int sph_switch_cullen_packed(const SphParams* p, int64_t n, const float* xh, const float* fc, const float* msgn,
                              const float* rho, const float* div, const float* div_prev,
                              const float* alpha0_prev, const float* dt, const int32_t* offs,

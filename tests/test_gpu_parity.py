@@ -500,3 +500,17 @@ def test_packed_rewrite_matches_separate_arrays(cuda, dim, n_side):
         out.append((adj.neighborList, adj.interCounts, V))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
     assert_close(out[1][2].cpu().numpy(), out[0][2].cpu().numpy(), 2e-6, 2e-6, "V")
+
+
+@pytest.mark.parametrize("dim,n_side", [(1, 301), (2, 33), (3, 9)])
+@pytest.mark.parametrize("cullen", [True, False])
+def test_velocity_gradient_writes_the_divergence(cuda, dim, n_side, cullen):
+    """divergence = -drhodt / rho from the velocity-gradient pass: the same two roundings, so equal."""
+    cfg, sch, p = make_params(dim)
+    G = to_gpu(make_particles(dim, n_side, seed=3), cuda)
+    x, H, m, v, u = (G[k] for k in ("positions", "supports", "masses", "velocities", "internalEnergies"))
+    adj = ops.buildVerletList(x, H, p, p.verlet_scale)
+    V = ops.crk_volume(p, x, H, adj)
+    divergence = torch.full_like(V, float("nan"))
+    _, rho, *_, dr, _, _, _ = ops.crk_rhs_fields(p, ops.pack_xh(p, x, H), m, V, v, u, adj, cullen, divergence)
+    assert torch.equal(divergence, -dr / rho)

@@ -111,7 +111,7 @@ _PROTOS = {
     "sph_compsph_balance_packed": [_P, _I64] + [_P] * 16,
     "sph_pack_xh": [_P, _I64] + [_P] * 4,
     "sph_crk_factors_packed": [_P, _I64] + [_P] * 19,
-    "sph_grad_v_packed": [_P, _I64] + [_P] * 19,
+    "sph_grad_v_packed": [_P, _I64] + [_P] * 20,
     "sph_switch_cullen_packed": [_P, _I64] + [_P] * 13,
     "sph_neighbors_update": [_P, _I64, _P, _P, _P, _P, _P, _I64, _I64] + [_P] * 8 + [_I64] + [_P] * 5,
     "sph_neighbors_rewrite": [_P, _I64] + [_P] * 13,

@@ -633,8 +633,8 @@ k_grad_v_packed(int n, DevParams P, const float4* __restrict__ xh, const float4*
                 const float* __restrict__ m, const float* __restrict__ rho, const float* __restrict__ c, const float* __restrict__ A,
                 const float* __restrict__ B, const float* __restrict__ gA, const float* __restrict__ gB,
                 const int32_t* __restrict__ offs, const int32_t* __restrict__ cnt, const int32_t* __restrict__ list,
-                float* __restrict__ DvDx, float* __restrict__ drhodt, float* __restrict__ div_out, float4* __restrict__ fc,
-                float* __restrict__ msgn) {
+                float* __restrict__ DvDx, float* __restrict__ drhodt, float* __restrict__ divergence_out, float* __restrict__ div_out,
+                float4* __restrict__ fc, float* __restrict__ msgn) {
     pdl_entry();
     Grp<G> g(n);
     const bool want_div = div_out != nullptr;
@@ -688,7 +688,9 @@ k_grad_v_packed(int n, DevParams P, const float4* __restrict__ xh, const float4*
     float tr = Gm.m[0][0];
     #pragma unroll
     for (int a = 1; a < D; ++a) tr += Gm.m[a][a];
-    drhodt[i] = -tr * rho[i];
+    const float rhoi = rho[i], dr = -tr * rhoi;
+    drhodt[i] = dr;
+    if (divergence_out) divergence_out[i] = -dr / rhoi;
     if (want_div) {
         div_out[i] = div;
         const float ms = m[i] * (div > 0.f ? 1.f : (div < 0.f ? -1.f : 0.f));
@@ -1769,8 +1771,8 @@ int sph_crk_factors_packed(const SphParams* p, int64_t n, const float* xh, const
 
 int sph_grad_v_packed(const SphParams* p, int64_t n, const float* xh, const float* fv, const float* vol, const float* m, const float* rho,
                       const float* c, const float* A, const float* B, const float* gradA, const float* gradB, const int32_t* offs,
-                      const int32_t* cnt, const int32_t* list, float* DvDx_out, float* drhodt_out, float* div_out, float* fc,
-                      float* msgn, void* stream) {
+                      const int32_t* cnt, const int32_t* list, float* DvDx_out, float* drhodt_out, float* divergence_out,
+                      float* div_out, float* fc, float* msgn, void* stream) {
     PAIR_PRELUDE();
     WSPH_CHECK_PTR(xh); WSPH_CHECK_PTR(fv); WSPH_CHECK_PTR(rho); WSPH_CHECK_PTR(A); WSPH_CHECK_PTR(B); WSPH_CHECK_PTR(gradA);
     WSPH_CHECK_PTR(gradB); WSPH_CHECK_PTR(DvDx_out); WSPH_CHECK_PTR(drhodt_out); CHECK_CSR();
@@ -1782,7 +1784,7 @@ int sph_grad_v_packed(const SphParams* p, int64_t n, const float* xh, const floa
     wsph::count_launch();
     WSPH_DISPATCH_KDS(*p, PAIR_LANES(n, G_GRADV(D), G_WIDE, launch_pdl(k_grad_v_packed<KF, D, LG>, grid_g<LG>(n), PAIR_BLOCK, 0, s, (int)n, P,
                                       reinterpret_cast<const float4*>(xh), reinterpret_cast<const float4*>(fv), vol, m, rho, c, A, B, gradA,
-                                      gradB, offs, cnt, list, DvDx_out, drhodt_out, div_out, reinterpret_cast<float4*>(fc), msgn)));
+                                      gradB, offs, cnt, list, DvDx_out, drhodt_out, divergence_out, div_out, reinterpret_cast<float4*>(fc), msgn)));
     return check_launch("sph_grad_v_packed");
 }
 

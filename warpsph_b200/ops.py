@@ -551,11 +551,11 @@ def crk_factors_eos(params, x, H, m, V, adj: AdjacencyList, u):
     return CRKState(A=A, B=B, gradA=gA, gradB=gB), rho, Ae, P, c
 
 
-def crk_rhs_fields(params, xh, m, V, v, u, adj: AdjacencyList, cullen: bool):
+def crk_rhs_fields(params, xh, m, V, v, u, adj: AdjacencyList, cullen: bool, divergence=None):
     """CRK factors with the ideal-gas EOS, then the velocity gradient (and the Cullen divergence),
     over packed words (sph_crk_factors_packed, sph_grad_v_packed): crk_factors_eos followed by
     grad_v.  Returns (crk, rho, entropy, P, c, DvDx, drhodt, div, fc, msgn); fc and msgn are the
-    words switch_cullen_packed reads."""
+    words switch_cullen_packed reads.  divergence [n], when given, receives -drhodt / rho."""
     n, d = m.shape[0], int(params.dim)
     A, B, gA, gB, rho = _empty(n, m), _empty((n, d), m), _empty((n, d), m), _empty((n, d, d), m), _empty(n, m)
     Ae, P, c = _empty(n, m), _empty(n, m), _empty(n, m)
@@ -572,7 +572,8 @@ def crk_rhs_fields(params, xh, m, V, v, u, adj: AdjacencyList, cullen: bool):
     msgn = _empty(n, m) if cullen and d == 3 else None
     with _timed("grad_v"):
         check(L.sph_grad_v_packed(_p(params), n, ptr(xh), ptr(fv), ptr(vol), fptr(m), ptr(rho), ptr(c), ptr(A), ptr(B), ptr(gA), ptr(gB),
-                                  *rows, ptr(G), ptr(drho), ptr(div), ptr(fc), ptr(msgn), stream_ptr(m.device)), "sph_grad_v_packed")
+                                  *rows, ptr(G), ptr(drho), ptr(divergence), ptr(div), ptr(fc), ptr(msgn), stream_ptr(m.device)),
+              "sph_grad_v_packed")
     return CRKState(A=A, B=B, gradA=gA, gradB=gB), rho, Ae, P, c, G, drho, div, fc, msgn
 
 

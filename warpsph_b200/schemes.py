@@ -149,8 +149,9 @@ def crkSPH_step(system: CompSPHSystem, dt, config: SimulationConfig, compParams:
     V = ops.crk_volume(params, S.positions, S.supports, adjacency, xh)
     switch = compParams.viscositySwitchParams.scheme
     cullen = switch == ViscositySwitch.CullenDehnen2010
+    divergence = torch.empty_like(V)            # -drhodt / rho (crkSPH.py:324), written with the velocity gradient
     crk, S.densities, S.entropies, S.pressures, S.soundspeeds, DvDx, drhodt, div_cd, fc, msgn = ops.crk_rhs_fields(
-        params, xh, S.masses, V, S.velocities, S.internalEnergies, adjacency, cullen)
+        params, xh, S.masses, V, S.velocities, S.internalEnergies, adjacency, cullen, divergence)
     if S.divergence is None:
         S.divergence = torch.zeros_like(S.densities)
     # crkSPH.py:195-200 (v_sig over the Verlet set is computed inside the switch pass)
@@ -170,7 +171,7 @@ def crkSPH_step(system: CompSPHSystem, dt, config: SimulationConfig, compParams:
                                                             S.velocities, S.soundspeeds, S.pressures, DvDx, adjacency,
                                                             want_dEdt=True, reference_layout=False)
     # crkSPH.py:324-337
-    S.divergence = -drhodt / S.densities
+    S.divergence = divergence
     update = CompressibleSystemUpdate(dxdt=S.velocities, dvdt=dvdt, dudt=dudt, drhodt=drhodt, dEdt=dEdt, passive=None)
     # crkSPH.py:341-363
     S.f_ij = ops.compsph_balance(params, S.masses, S.densities, S.pressures, S.internalEnergies, S.velocities, dvdt, dt, adjacency,
