@@ -197,6 +197,7 @@ struct EnsArgs {
     void* near;                            // ENS_NEAR bits per particle: see EnsWalk
     const int32_t *offs, *cnt, *list;
     BarrierCtl* ctl;
+    int* work;                             // next particle of each pair pass
     unsigned int* disp;                    // max |x - x_build| / H since the list was built (ordered float)
     int32_t* status;
 };
@@ -448,18 +449,26 @@ __device__ __forceinline__ void ens_passB(int i, int lane, const EnsArgs& a, con
 }
 
 // Bound by issue slots (64 %) and the latency of the gathers.  1.3 M particles in 64 boxes, 99 entries
-// per row of which 50 interact: 5.84 -> 3.17 ms per step; of that the walk of the near entries, packed
+// per row of which 50 interact: 5.84 -> 2.78 ms per step; of that the walk of the near entries, packed
 // words and quotients hoisted to the particle give 2.2 ms, divisions without the general case's
-// branches 0.3 and the usual terms as constants 0.1.  Rows reordered by distance were faster still
-// (2.14 ms) but change the order of the sums: the Antuono pressure switch jumps where P_j crosses 0, so
-// a rounding there moves whole pair terms.  64 registers: 8 blocks of 128 threads per SM.
+// branches 0.3, the usual terms as constants 0.1, particles handed to free warps (1, 2 or 4 warpfuls
+// at a time: 0.27, 0.21, 0.21) and 9 blocks of 128 threads per SM (56 registers; 8: 0.1 more, 10: 0.06
+// more) the rest.  Rows reordered by distance were faster still (2.14 ms with static shares) but change
+// the order of the sums: the Antuono pressure switch jumps where P_j crosses 0, so a rounding there
+// moves whole pair terms.
 template <int KF, int D, int G, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, (D == 3 ? 1 : 1024 / BLOCK))
+__global__ void __launch_bounds__(BLOCK, (D == 3 ? 1 : 1152 / BLOCK))
 k_ens_step(const __grid_constant__ EnsArgs a) {
-    constexpr int PPB = BLOCK / G;
-    const int lane = threadIdx.x & (G - 1);
-    const int rounds = (a.n + (int)gridDim.x * PPB - 1) / ((int)gridDim.x * PPB);
+    constexpr int PPW = 32 / G;            // particles of a warp at a time
+    const int lane = threadIdx.x & (G - 1), sub = (threadIdx.x & 31) / G;
     unsigned int dmax = 0u, arrived = 0;
+    // The particles of a pass go to the warps as they become free (rows differ in length, and a grid
+    // barrier waits for the last), PPW at a time.
+    auto take = [&](int pass) {
+        int base = 0;
+        if ((threadIdx.x & 31) == 0) base = atomicAdd(a.work + pass, PPW);
+        return __shfl_sync(0xffffffffu, base, 0);
+    };
     const bool usual = a.W.density_scheme == SPH_DENSITY_DIFFUSION_DELTA && a.W.pressure_term == SPH_PRESSURE_ANTUONO;
     // ---- the first stage's words
     for (int i = blockIdx.x * BLOCK + threadIdx.x; i < a.n; i += gridDim.x * BLOCK) {
@@ -471,8 +480,8 @@ k_ens_step(const __grid_constant__ EnsArgs a) {
     for (int stage = 0; stage < 2; ++stage) {
         const EnsSet& st = a.set[stage];
         // ---- pass A: renormalised density gradient and EOS
-        for (int rd = 0; rd < rounds; ++rd) {
-            const int i = (rd * (int)gridDim.x + (int)blockIdx.x) * PPB + (int)threadIdx.x / G;
+        for (int base = take(2 * stage); base < a.n; base = take(2 * stage)) {
+            const int i = base + sub;
             const bool valid = i < a.n;
             Mat<D> M = mzero<D>();
             Vec<D> s = vzero<D>();
@@ -493,8 +502,8 @@ k_ens_step(const __grid_constant__ EnsArgs a) {
         }
         if (!grid_barrier(a.ctl, arrived)) { if (threadIdx.x == 0) atomicOr(a.status, SPH_STATUS_TIMEOUT); return; }
         // ---- pass B: right-hand side, stage update
-        for (int rd = 0; rd < rounds; ++rd) {
-            const int i = (rd * (int)gridDim.x + (int)blockIdx.x) * PPB + (int)threadIdx.x / G;
+        for (int base = take(2 * stage + 1); base < a.n; base = take(2 * stage + 1)) {
+            const int i = base + sub;
             const bool valid = i < a.n;
             float cont = 0.f, dd = 0.f;
             Vec<D> pf = vzero<D>(), visc = vzero<D>();
@@ -668,8 +677,10 @@ int sph_ensemble_step(const SphParams* p, const SphWcParams* wc, int64_t n, cons
     a.drho1 = reinterpret_cast<float*>(w + o);
     a.offs = offs; a.cnt = cnt; a.list = list;
     a.ctl = reinterpret_cast<BarrierCtl*>(w);
+    a.work = reinterpret_cast<int*>(w + 128);
+    static_assert(sizeof(BarrierCtl) <= 128, "the control block's two halves");
     a.disp = disp_max; a.status = status;
-    cudaError_t e = cudaMemsetAsync(a.ctl, 0, sizeof(BarrierCtl), s);
+    cudaError_t e = cudaMemsetAsync(a.ctl, 0, 128 + 4 * sizeof(int), s);
     if (e != cudaSuccess) return set_error(SPH_ERR_CUDA, "sph_ensemble_step: memset: %s", cudaGetErrorString(e));
     if (!(lanes == 4 || lanes == 8 || lanes == 16) || !(block == 128 || block == 256))
         return set_error(SPH_ERR_BAD_ARG, "sph_ensemble_step: lanes must be 4, 8 or 16 and block 128 or 256");
