@@ -169,7 +169,8 @@ __device__ __forceinline__ long long block_exclusive_scan(long long v, long long
 
 // in -> out (exclusive, local to tile), tile totals -> sums
 __global__ void k_scan_tiles(const int32_t* __restrict__ in, int64_t n, long long* __restrict__ out_ll,
-                             int32_t* __restrict__ out32, long long* __restrict__ sums, const unsigned int* __restrict__ gate) {
+                             int32_t* __restrict__ out32, int32_t* __restrict__ copy32, long long* __restrict__ sums,
+                             const unsigned int* __restrict__ gate) {
     if (gate_closed(gate)) return;
     __shared__ long long sw[SCAN_THREADS / 32];
     int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
@@ -188,6 +189,7 @@ __global__ void k_scan_tiles(const int32_t* __restrict__ in, int64_t n, long lon
         int64_t idx = base + k;
         if (idx < n) {
             if (out_ll) out_ll[idx] = off; else out32[idx] = (int32_t)off;
+            if (copy32) copy32[idx] = (int32_t)off;
         }
         off += vals[k];
     }
@@ -217,13 +219,16 @@ __global__ void k_scan_tiles_ll(const long long* in, int64_t n, long long* out, 
     }
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
-__global__ void k_scan_add(long long* __restrict__ out_ll, int32_t* __restrict__ out32, int64_t n,
+__global__ void k_scan_add(long long* __restrict__ out_ll, int32_t* __restrict__ out32, int32_t* __restrict__ copy32, int64_t n,
                            const long long* __restrict__ tile_off, const unsigned int* __restrict__ gate) {
     if (gate_closed(gate)) return;
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
     long long o = tile_off[idx / SCAN_TILE];
-    if (out_ll) out_ll[idx] += o; else out32[idx] = (int32_t)((long long)out32[idx] + o);
+    if (out_ll) { out_ll[idx] += o; return; }
+    const int32_t r = (int32_t)((long long)out32[idx] + o);
+    out32[idx] = r;
+    if (copy32) copy32[idx] = r;
 }
 
 // Workspace: for each level the tile sums and their scanned offsets.
@@ -239,50 +244,31 @@ int64_t scan_ws_bytes(int64_t n) {
     return bytes + 256;
 }
 
-__global__ void k_copy_total(long long* __restrict__ total, const long long* __restrict__ sums, const unsigned int* __restrict__ gate) {
-    if (!gate_closed(gate)) *total = *sums;
-}
-
-// The single-tile total: a device copy, or under a gate a one-thread kernel (a copy
-// cannot be skipped by the GPU).
-static void copy_total(long long* total, const long long* sums, const unsigned int* gate, cudaStream_t s) {
-    if (gate) {
-        wsph::count_launch(); k_copy_total<<<1, 1, 0, s>>>(total, sums, gate);
-    } else {
-        cudaMemcpyAsync(total, sums, sizeof(long long), cudaMemcpyDeviceToDevice, s);
-    }
-}
-
 // Scans a level of long long values in place (exclusive) and writes the total to *total.
 static void scan_ll_inplace(long long* data, int64_t n, char* ws, long long* total, cudaStream_t s, const unsigned int* gate) {
     int64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (tiles < 1) tiles = 1;
     long long* sums = reinterpret_cast<long long*>(ws);
     char* next = ws + ((tiles * 8 + 255) / 256) * 256 * 2;
-    wsph::count_launch(); k_scan_tiles_ll<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(data, n, data, sums, gate);
-    if (tiles == 1) {
-        copy_total(total, sums, gate, s);
-        return;
-    }
+    wsph::count_launch(); k_scan_tiles_ll<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(data, n, data, tiles == 1 ? total : sums, gate);
+    if (tiles == 1) return;
     scan_ll_inplace(sums, tiles, next, total, s, gate);
-    wsph::count_launch(); k_scan_add<<<grid_for(n, 256), 256, 0, s>>>(data, nullptr, n, sums, gate);
+    wsph::count_launch(); k_scan_add<<<grid_for(n, 256), 256, 0, s>>>(data, nullptr, nullptr, n, sums, gate);
 }
 
-// Exclusive scan int32 -> int32, total (int64, device).  Under a gate every launch
+// Exclusive scan int32 -> int32 (twice with `copy`), total (int64, device).  Under a gate every launch
 // returns at once when the gate is closed, leaving out and total as they were.
 void exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, char* ws, long long* total, cudaStream_t s,
-                        const unsigned int* gate) {
+                        const unsigned int* gate, int32_t* copy) {
     int64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (tiles < 1) tiles = 1;
     long long* sums = reinterpret_cast<long long*>(ws);
     char* next = ws + ((tiles * 8 + 255) / 256) * 256 * 2;
-    wsph::count_launch(); k_scan_tiles<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(in, n, nullptr, out, sums, gate);
-    if (tiles == 1) {
-        copy_total(total, sums, gate, s);
-        return;
-    }
+    wsph::count_launch(); k_scan_tiles<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(in, n, nullptr, out, tiles == 1 ? copy : nullptr,
+                                                                                 tiles == 1 ? total : sums, gate);
+    if (tiles == 1) return;
     scan_ll_inplace(sums, tiles, next, total, s, gate);
-    wsph::count_launch(); k_scan_add<<<grid_for(n, 256), 256, 0, s>>>(nullptr, out, n, sums, gate);
+    wsph::count_launch(); k_scan_add<<<grid_for(n, 256), 256, 0, s>>>(nullptr, out, copy, n, sums, gate);
 }
 
 // ---------------------------------------------------------------- min / max
@@ -373,8 +359,13 @@ __global__ void k_hmax(const float* __restrict__ H, int64_t n, float* out, int32
 
 // One thread: derive the grid from max H and the cell-table capacity.
 template <int D>
-__global__ void k_grid(const float* hmax, DevParams P, int max_bits, GridDev* g, int32_t* grid_out, const unsigned int* __restrict__ gate) {
+__global__ void k_grid(const float* hmax, DevParams P, int max_bits, GridDev* g, int32_t* grid_out, int32_t* ntasks, long long* innz,
+                       unsigned long long* mask_cursor, const unsigned int* __restrict__ gate) {
     if (gate_closed(gate)) return;
+    // the counters of the passes behind it
+    *ntasks = 0;
+    *mask_cursor = 0ull;
+    if (innz) *innz = 0;
     float h = *hmax;
     float Lmax = 0.f;
     for (int a = 0; a < D; ++a) Lmax = fmaxf(Lmax, P.dom.L[a]);
@@ -817,12 +808,15 @@ k_verlet(const float4* __restrict__ recs, const float* __restrict__ inter, const
          int32_t* __restrict__ counts, int32_t* __restrict__ icounts, const int32_t* __restrict__ offsets,
          int32_t* __restrict__ list, long long* __restrict__ innz, const long long* __restrict__ nnz, long long capacity,
          uint32_t* __restrict__ masks, int32_t* __restrict__ mask_base, unsigned long long* __restrict__ mask_cursor,
-         long long mask_words, unsigned long long neg0, const unsigned int* __restrict__ gate) {
+         long long mask_words, unsigned long long neg0, int32_t* __restrict__ status, const unsigned int* __restrict__ gate) {
     if (gate_closed(gate)) return;
     __shared__ VerletStage stage[VW_WARPS];
     __shared__ unsigned int itotal;
     const bool part = icounts != nullptr;
-    if (FILL && *nnz > capacity) return;
+    if (FILL && *nnz > capacity) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status, SPH_STATUS_LIST_OVERFLOW);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     VerletStage& st = stage[threadIdx.x >> 5];
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -847,11 +841,6 @@ k_verlet(const float4* __restrict__ recs, const float* __restrict__ inter, const
         __syncthreads();
         if (threadIdx.x == 0 && itotal) atomicAdd(reinterpret_cast<unsigned long long*>(innz), (unsigned long long)itotal);
     }
-}
-
-__global__ void k_check_capacity(const long long* nnz, long long capacity, int32_t* status, const unsigned int* __restrict__ gate) {
-    if (gate_closed(gate)) return;
-    if (*nnz > capacity) atomicOr(status, SPH_STATUS_LIST_OVERFLOW);
 }
 
 // After a gated rebuild that overflowed the list (the fill pass wrote nothing), each row
@@ -1195,11 +1184,6 @@ __global__ void k_fill_gated(uint32_t* __restrict__ p, int64_t count, uint32_t v
     if (gate_closed(gate)) return;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
-__global__ void k_copy_gated(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, int64_t count,
-                             const unsigned int* __restrict__ gate) {
-    if (gate_closed(gate)) return;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) dst[i] = src[i];
-}
 static int word_blocks(int64_t words) {
     int64_t b = (words + 255) / 256;
     return (int)(b < 1 ? 1 : (b > 148 * 8 ? 148 * 8 : b));
@@ -1230,19 +1214,11 @@ static void build_rows(const DevParams& P, int64_t n, const float* x, const floa
     int rblocks = (int)((n + 1023) / 1024);
     if (rblocks > 148 * 4) rblocks = 148 * 4;
     wsph::count_launch(); k_hmax<<<rblocks, 256, 0, s>>>(H, n, w.hmax, status, gate);
-    wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, k_grid<D><<<1, 1, 0, s>>>(w.hmax, P, mb, w.grid, grid_out, gate));
+    wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, k_grid<D><<<1, 1, 0, s>>>(w.hmax, P, mb, w.grid, grid_out, w.ntasks, innz, w.mask_cursor, gate));
     clear(w.counts, ncells * sizeof(int32_t));
     wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, k_keys<D><<<grid_for(n, 256), 256, 0, s>>>(x, (int)n, w.grid, P.dom, w.keys, w.counts, gate));
-    exclusive_scan_i32(w.counts, cell_begin, ncells, w.scan, w.total, s, gate);
-    if (gate) {
-        wsph::count_launch();
-        k_copy_gated<<<word_blocks(ncells), 256, 0, s>>>(reinterpret_cast<uint32_t*>(cell_end), reinterpret_cast<const uint32_t*>(cell_begin),
-                                                          ncells, gate);
-    } else {
-        cudaMemcpyAsync(cell_end, cell_begin, ncells * sizeof(int32_t), cudaMemcpyDeviceToDevice, s);
-    }
+    exclusive_scan_i32(w.counts, cell_begin, ncells, w.scan, w.total, s, gate, cell_end);
     wsph::count_launch(); k_scatter<<<grid_for(n, 256), 256, 0, s>>>(w.keys, (int)n, cell_end, w.tmp, gate);
-    clear(w.ntasks, sizeof(int32_t));
     wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, (k_rank_sort<D><<<grid_for(n, 256), 256, 0, s>>>(w.tmp, w.keys, cell_begin, cell_end, (int)n, x, H,
                                                                                                  sort_index, sorted_keys, w.recs, w.inter, P.verlet_scale, w.tasks, w.ntasks,
                                                                                                  gate)));
@@ -1250,19 +1226,16 @@ static void build_rows(const DevParams& P, int64_t n, const float* x, const floa
     // blocks past the last item return at once, and with fuller grids the warps stride
     int vblocks = grid_for(n, VW_BLOCK / 2);
     if (vblocks > 1 << 16) vblocks = 1 << 16;
-    if (part) clear(inter_nnz_out, sizeof(int64_t));
-    clear(w.mask_cursor, sizeof(unsigned long long));
     wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, (k_verlet<D, false><<<vblocks, VW_BLOCK, 0, s>>>(w.recs, w.inter, sorted_keys, w.tasks, w.ntasks, w.grid, P, sort_index,
                                                                                  cell_begin, cell_end, num_neighbors, inter_counts, nullptr,
                                                                                  nullptr, innz, nullptr, 0, w.masks, w.mask_base,
-                                                                                 w.mask_cursor, (long long)w.mask_words, NEG_ZERO2, gate)));
+                                                                                 w.mask_cursor, (long long)w.mask_words, NEG_ZERO2, status, gate)));
     exclusive_scan_i32(num_neighbors, neighbor_offsets, n, w.scan, reinterpret_cast<long long*>(nnz_out), s, gate);
-    wsph::count_launch(); k_check_capacity<<<1, 1, 0, s>>>(reinterpret_cast<long long*>(nnz_out), list_capacity, status, gate);
     wsph::count_launch(); WSPH_DISPATCH_DIM(P.dim, (k_verlet<D, true><<<vblocks, VW_BLOCK, 0, s>>>(w.recs, w.inter, sorted_keys, w.tasks, w.ntasks, w.grid, P, sort_index,
                                                                                 cell_begin, cell_end, nullptr, inter_counts, neighbor_offsets,
                                                                                 neighbor_list, nullptr, reinterpret_cast<long long*>(nnz_out),
                                                                                 list_capacity, w.masks, w.mask_base, w.mask_cursor,
-                                                                                (long long)w.mask_words, NEG_ZERO2, gate)));
+                                                                                (long long)w.mask_words, NEG_ZERO2, status, gate)));
 }
 
 // The fused rewrite with its gathers from packed words (xh) or from x and H.

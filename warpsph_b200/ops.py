@@ -229,7 +229,8 @@ def buildVerletList(x: torch.Tensor, H: torch.Tensor, params, verletScale: float
     ce = torch.empty(cap, dtype=torch.int32, device=dev)
     grid = torch.empty(8, dtype=torch.int32, device=dev)
     icnt = torch.empty(n, dtype=torch.int32, device=dev)
-    flags = torch.zeros(3, dtype=torch.int64, device=dev)   # [nnz, status (int32 in the low half), interacting nnz]
+    flags = torch.empty(3, dtype=torch.int64, device=dev)   # [nnz, status (int32 in the low half), interacting nnz]
+    x0, h0 = x.clone(), H.clone()                           # build-time state for the validity check
     hint = _nb_cache.cap_hint.get((dev.index, n, dim))
     list_cap = hint if hint is not None else _list_capacity(n * 64)
     for attempt in range(2):
@@ -257,7 +258,7 @@ def buildVerletList(x: torch.Tensor, H: torch.Tensor, params, verletScale: float
                         interCounts=icnt, interNnz=innz)
     adj._x_version = _version(x)
     adj._h_version = _version(H)
-    adj._x0, adj._h0, adj._dim = x.clone(), H.clone(), dim   # build-time state for the validity check
+    adj._x0, adj._h0, adj._dim = x0, h0, dim
     return adj
 
 
