@@ -263,16 +263,6 @@ template <int KF, int D> __device__ __forceinline__ void kernelWG(const Vec<D>& 
     float s = -cH * p / (H * H);
     _Pragma("unroll") for (int a = 0; a < D; ++a) g.v[a] = s * xij.v[a];
 }
-// W and dW/dH.
-template <int KF, int D> __device__ __forceinline__ void kernelWdH(float r, float H, float& W, float& dWdH) {
-    float q = r / H;
-    if (!(q < 1.f)) { W = 0.f; dWdH = 0.f; return; }
-    float k, p; kernel_kp<KF, D>(q, k, p);
-    float cH = KernelTraits<KF, D>::C / ipow<D>(H);
-    W = cH * k;
-    dWdH = -cH / H * ((float)D * k - q * q * p);
-}
-
 // Pair kernel value for a support scheme.
 template <int KF, int D> __device__ __forceinline__ float kernelW_mode(float r, float Hi, float Hj, int mode) {
     switch (mode) {
@@ -297,22 +287,6 @@ template <int KF, int D> __device__ __forceinline__ void kernelWG_mode(const Vec
             _Pragma("unroll") for (int a = 0; a < D; ++a) g.v[a] = 0.5f * (ga.v[a] + gb.v[a]);
         }
     }
-}
-
-// CRK-corrected kernel gradient (Frontiere, Raskin & Owen 2017, eq. for d W^R_ij):
-//   W^R = A (1 + B.x) W,  x = x_ij
-//   d_g W^R = A (1+B.x) d_g W + A B_g W + d_g A (1+B.x) W + A (sum_a dB^a/dx^g x^a) W
-// gB[a][g] = dB^a/dx^g.
-template <int D> __device__ __forceinline__ Vec<D> crk_grad(const Vec<D>& x, float W, const Vec<D>& gW,
-                                                            float A, const Vec<D>& B, const Vec<D>& gA, const Mat<D>& gB) {
-    float bx = 1.f + dot<D>(B, x);
-    Vec<D> r;
-    _Pragma("unroll") for (int g = 0; g < D; ++g) {
-        float gbx = gB.m[0][g] * x.v[0];
-        _Pragma("unroll") for (int a = 1; a < D; ++a) gbx += gB.m[a][g] * x.v[a];
-        r.v[g] = A * bx * gW.v[g] + A * B.v[g] * W + gA.v[g] * bx * W + A * gbx * W;
-    }
-    return r;
 }
 
 // ---------------------------------------------------------------- dispatch helpers

@@ -158,7 +158,8 @@ template <int KF, int D> __device__ __forceinline__ bool kWS_inv(float r, float 
     s = -cH * p * (invH * invH);
     return true;
 }
-// crk_grad with grad W = s x and its terms gathered by factor:
+// CRK-corrected kernel gradient (Frontiere, Raskin & Owen 2017, eq. for d W^R_ij) of
+// W^R = A (1 + B.x) W, x = x_ij, with grad W = s x and gB[a][g] = dB^a/dx^g:
 //   A (1 + B.x) s x + W (gA (1 + B.x) + A (B + gB^T x))
 template <int D> __device__ __forceinline__ Vec<D> crk_grad_s(const Vec<D>& x, float W, float s, float A, const Vec<D>& B,
                                                               const Vec<D>& gA, const Mat<D>& gB) {
