@@ -478,12 +478,13 @@ k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restri
         uint32_t phase = 0u;
         bool ok = true;
         auto row_of = [&](int k) { return (blockIdx.x + static_cast<int64_t>(k) * gridDim.x) * TC_M + r; };
-        // the A operand is in place: issue the chain of a layer
+        // The A operand is in place: issue the chain of a layer, unless a wait before ran out in some thread
+        // (one that gave up still comes to this barrier, so the warpgroup decides as one).
         auto issue = [&](int layer) {
             tmem_st_wait();
             tc_fence_before_sync();
-            bar_sync_named(wg + 1, TC_M);
-            if (issuer) {
+            ok = bar_and_named(wg + 1, TC_M, ok);
+            if (issuer && ok) {
                 tc_fence_after_sync();
                 if (elect_one()) {
                     if (layer == 0) {
@@ -500,11 +501,10 @@ k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restri
                 __syncwarp();
             }
         };
-        auto wait_chain = [&]() -> bool {
+        auto wait_chain = [&]() {
             ok = mbar_wait_bounded(chain, phase, TC_WAIT_CYCLES);
             phase ^= 1u;
             tc_fence_after_sync();
-            return ok;
         };
         // this thread's row of tile k into shared memory, without a register held meanwhile
         auto fetch_row = [&](int k) {
@@ -531,7 +531,7 @@ k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restri
             fetch_row(k + FT_WGS);
             #pragma unroll 1
             for (int layer = 0; layer < 2; ++layer) {
-                if (!wait_chain()) break;
+                wait_chain();
                 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     uint32_t v[32], h[16];
@@ -545,8 +545,10 @@ k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restri
                     tmem_st_32x32b_x8(tH + 16 * half + 8, h1);
                 }
                 issue(layer + 1);
+                if (!ok) break;
             }
-            if (!ok || !wait_chain()) break;
+            if (!ok) break;
+            wait_chain();
             // the next tile's first chain runs while the second half of the output layer is summed
             float y = 0.f;
             #pragma unroll
@@ -567,6 +569,7 @@ k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restri
                     y = fmaf(fmaxf(__uint_as_float(v[4 * q + 3]), 0.f), w.w, y);
                 }
             }
+            if (!ok) break;
             const int64_t row = row_of(k);
             if (row < n) out[row] = (y + s.b4) * sc;
         }
@@ -745,7 +748,7 @@ k_mlp_grad_tc(const float* __restrict__ prm, int64_t n, const float* __restrict_
         uint32_t rphase = 0u;          // parity of each ready barrier
         bool ok = true;
         auto wait_ready = [&](uint32_t bars, int w) -> bool {
-            ok = mbar_wait_bounded(bars + 8 * w, (rphase >> w) & 1u, TC_WAIT_CYCLES);
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(bars + 8 * w, (rphase >> w) & 1u, TC_WAIT_CYCLES));
             rphase ^= 1u << w;
             tc_fence_after_sync();
             return ok;
@@ -837,8 +840,9 @@ k_mlp_grad_tc(const float* __restrict__ prm, int64_t n, const float* __restrict_
             if (to_chain) mbar_arrive(ready);
             if (to_g) mbar_arrive(gready);
         };
+        // a warp gives up as one, so that it stays converged for the tensor-memory instructions
         auto wait_on = [&](uint32_t bar, uint32_t& phase) -> bool {
-            ok = mbar_wait_bounded(bar, phase, TC_WAIT_CYCLES);
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, TC_WAIT_CYCLES));
             phase ^= 1u;
             tc_fence_after_sync();
             return ok;
