@@ -135,3 +135,22 @@ def test_fused_entries_equal_separate_calls(cuda):
     fused = ops.rk_combine_fields(params, fields, w, dt)
     for (y0, kf, wrap), y in zip(fields, fused):
         assert torch.equal(ops.rk_combine(params, y0, kf, w, dt, wrap), y)
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 4097, 151551, 151553, 303105])
+@pytest.mark.parametrize("dim", [1, 2, 3])
+def test_field_combination_equals_one_field_at_a_time(cuda, n, dim):
+    """sph_rk_combine_fields against sph_rk_combine per field, on both sides of the size where a thread
+    takes several elements, with fields of unequal length: the same operations, so equal bits."""
+    from tests.cases import make_params
+    from warpsph_b200 import ops
+    _, _, p = make_params(dim)
+    g = torch.Generator(device=cuda).manual_seed(n + dim)
+    x = torch.rand((n, dim), device=cuda, generator=g) - 0.5
+    fields = [(x, [torch.randn((n, dim), device=cuda, generator=g) for _ in range(3)], dim),
+              (torch.randn((n, dim), device=cuda, generator=g), [torch.randn((n, dim), device=cuda, generator=g) for _ in range(3)], 0),
+              (torch.randn(n, device=cuda, generator=g), [torch.randn(n, device=cuda, generator=g) for _ in range(3)], 0)]
+    w, dt = [0.25, 0.5, 0.125], torch.full((1,), 0.3, device=cuda)
+    outs = ops.rk_combine_fields(p, fields, w, dt)
+    for (y0, ks, wrap), y in zip(fields, outs):
+        assert torch.equal(y, ops.rk_combine(p, y0, ks, w, dt, wrap))

@@ -1445,27 +1445,43 @@ struct FieldPtrs {
     int wrap[RKF_MAX];
     float w[8];
 };
-__global__ void k_rk_combine_fields(int nf, int nk, FieldPtrs F, const float* __restrict__ dtp, DomainF dom) {
+// One row of blocks per field, ITEMS elements per thread with their loads together: with the field found per
+// element and the domain indexed through local memory a launch of 1.3 M elements took 25 us against 13 now.
+// Below 303,104 elements (8 blocks of 256 per SM) one element per thread fills the chip better.
+template <int ITEMS>
+__global__ void __launch_bounds__(256)
+k_rk_combine_fields(int nk, const __grid_constant__ FieldPtrs F, const float* __restrict__ dtp, const __grid_constant__ DomainF dom) {
     pdl_entry();
-    int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= F.end[nf - 1]) return;
-    int f = 0;
-    #pragma unroll
-    for (int q = 0; q < RKF_MAX - 1; ++q) f += (q < nf - 1 && g >= F.end[q]) ? 1 : 0;
-    const int64_t idx = g - (f > 0 ? F.end[f - 1] : 0);
+    const int f = blockIdx.y;
+    const int64_t count = F.end[f] - (f > 0 ? F.end[f - 1] : 0), base = (int64_t)blockIdx.x * (256 * ITEMS) + threadIdx.x;
+    if (base >= count) return;
+    const float* y0 = F.y0[f];
     const float dt = *dtp;
-    float s = 0.f;
-    for (int q = 0; q < nk; ++q) s = __fadd_rn(s, __fmul_rn(F.w[q], F.k[f][q][idx]));
-    float val = __fadd_rn(F.y0[f][idx], __fmul_rn(dt, s));
-    const int wd = F.wrap[f];
-    if (wd > 0) {
-        int a = (int)(idx % wd);
-        if (dom.periodic[a]) {
-            if (val >= dom.max[a]) val = __fsub_rn(val, dom.L[a]);
-            else if (val < dom.min[a]) val = __fadd_rn(val, dom.L[a]);
-        }
+    float s[ITEMS], y[ITEMS];
+    #pragma unroll
+    for (int u = 0; u < ITEMS; ++u) { s[u] = 0.f; y[u] = base + 256 * u < count ? y0[base + 256 * u] : 0.f; }
+    for (int q = 0; q < nk; ++q) {
+        const float* k = F.k[f][q];
+        const float w = F.w[q];
+        #pragma unroll
+        for (int u = 0; u < ITEMS; ++u)
+            if (base + 256 * u < count) s[u] = __fadd_rn(s[u], __fmul_rn(w, k[base + 256 * u]));
     }
-    F.y[f][idx] = val;
+    const int wd = F.wrap[f];
+    #pragma unroll
+    for (int u = 0; u < ITEMS; ++u) {
+        const int64_t idx = base + 256 * u;
+        if (idx >= count) break;
+        float val = __fadd_rn(y[u], __fmul_rn(dt, s[u]));
+        if (wd > 0) {
+            const int a = wd == 1 ? 0 : (wd == 2 ? (int)(idx & 1) : (int)(idx % 3));
+            if (dom.periodic[a]) {
+                if (val >= dom.max[a]) val = __fsub_rn(val, dom.L[a]);
+                else if (val < dom.min[a]) val = __fadd_rn(val, dom.L[a]);
+            }
+        }
+        F.y[f][idx] = val;
+    }
 }
 
 // ---------------------------------------------------------------- compatible energy
@@ -2074,8 +2090,9 @@ int sph_rk_combine_fields(const SphParams* p, int32_t nfields, const int64_t* co
     if (nk > 0) { WSPH_CHECK_PTR(k_ptrs); WSPH_CHECK_PTR(weights); }
     FieldPtrs F;
     memset(&F, 0, sizeof(F));
-    int64_t total = 0;
+    int64_t total = 0, largest = 0;
     for (int f = 0; f < nfields; ++f) {
+        if (counts[f] > largest) largest = counts[f];
         if (counts[f] < 0) return set_error(SPH_ERR_BAD_ARG, "sph_rk_combine_fields: count %d < 0", f);
         if (counts[f] > 0 && (!y0s[f] || !y_outs[f])) return set_error(SPH_ERR_BAD_ARG, "sph_rk_combine_fields: null field %d", f);
         if (wrap_dims[f] < 0 || wrap_dims[f] > 3) return set_error(SPH_ERR_BAD_ARG, "sph_rk_combine_fields: wrap_dim %d out of range", f);
@@ -2091,7 +2108,10 @@ int sph_rk_combine_fields(const SphParams* p, int32_t nfields, const int64_t* co
     for (int q = 0; q < nk; ++q) F.w[q] = (float)weights[q];
     if (total == 0) return SPH_OK;
     wsph::count_launch();
-    launch_pdl(k_rk_combine_fields, grid_for(total, 256), 256, 0, WSPH_STREAM(stream), nfields, nk, F, dt, P.dom);
+    if (largest <= 148 * 2048) launch_pdl(k_rk_combine_fields<1>, dim3((unsigned)((largest + 255) / 256), (unsigned)nfields), 256, 0,
+                                          WSPH_STREAM(stream), (int)nk, F, dt, P.dom);
+    else launch_pdl(k_rk_combine_fields<4>, dim3((unsigned)((largest + 1023) / 1024), (unsigned)nfields), 256, 0, WSPH_STREAM(stream), (int)nk, F,
+                    dt, P.dom);
     return check_launch("sph_rk_combine_fields");
 }
 
