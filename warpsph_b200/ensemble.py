@@ -28,7 +28,6 @@ No counterpart in the reference, which runs one simulation per process.
 """
 from __future__ import annotations
 
-import ctypes as C
 import math
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
@@ -186,7 +185,7 @@ class Ensemble:
     # -------------------------------------------------------------- stepping
     def _launch(self, tile=None, x=None, v=None, rho=None):
         lanes, block = tile or self.tile
-        check(_capi.lib().sph_ensemble_step(ops._p(self.params), C.cast(C.pointer(self.wc), C.c_void_p), self.n, ptr(self.box_of),
+        check(_capi.lib().sph_ensemble_step(ops._p(self.params), ops._p(self.wc), self.n, ptr(self.box_of),
                                             ptr(self.box_dt), ptr(self.H), ptr(self.m), ptr(self.x if x is None else x),
                                             ptr(self.v if v is None else v), ptr(self.rho if rho is None else rho), ptr(self.x_build),
                                             ptr(self.offs), ptr(self.cnt), ptr(self.list), ptr(self.step_ws), self.step_ws.numel(),

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes as C
+import functools
 from typing import Optional
 
 import torch
@@ -65,8 +66,11 @@ _SUPPORT = {SupportScheme.Gather: 0, SupportScheme.Scatter: 1, SupportScheme.Sym
             SupportScheme.SuperSymmetric: 3, SupportScheme.KernelMeanSymmetric: 4}
 
 
-def _p(params) -> C.c_void_p:
-    return C.cast(C.pointer(params), C.c_void_p)
+def _p(params) -> int:
+    """Address of a ctypes structure for one library call, which the caller's reference outlives.
+    (A pointer object cast to void* costs 1.4 us per call against 0.03, and below about 60,000
+    particles the host sets the time of a right-hand side.)"""
+    return C.addressof(params)
 
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
@@ -78,7 +82,15 @@ def _f32(t: torch.Tensor) -> torch.Tensor:
 
 
 def _empty(shape, like: torch.Tensor, dtype=torch.float32) -> torch.Tensor:
+    if isinstance(shape, tuple):      # unpacked: torch reads a tuple of sizes 1 us slower than separate ones
+        return torch.empty(*shape, device=like.device, dtype=dtype)
     return torch.empty(shape, device=like.device, dtype=dtype)
+
+
+@functools.lru_cache(maxsize=None)
+def _floats_of(entry: str, dim: int) -> int:
+    """A per-particle scratch size that the library states for a dimension."""
+    return int(getattr(_capi.lib(), entry)(dim))
 
 
 _dt_cache: dict = {}
@@ -142,7 +154,7 @@ def _pair_empty(nnz: int, d: int, like: torch.Tensor) -> torch.Tensor:
     from storage rounded up to whole list granules, so that successive steps request the
     same few sizes from the caching allocator."""
     cap = _list_capacity(nnz)
-    base = torch.empty((cap, d) if d else cap, dtype=like.dtype, device=like.device)
+    base = _empty((cap, d) if d else cap, like, like.dtype)
     return base[:nnz]
 
 
@@ -777,7 +789,7 @@ def crk_accel_dudt(params, x, H, m, rho, V, crk: CRKState, v, c, P, DvDx, adj: A
 
 def crk_record_floats(dim: int) -> int:
     """Floats per particle of the packed record of the CRK accel pass."""
-    return int(_capi.lib().sph_crk_record_floats(int(dim)))
+    return _floats_of("sph_crk_record_floats", int(dim))
 
 
 def pair_reference_layout(adj: AdjacencyList, *arrays):
@@ -811,7 +823,7 @@ def compsph_prep(params, x, H, m, rho, v, adj: AdjacencyList, grad_h: bool = Tru
     om = _empty(n, H) if grad_h else None
     div = _empty(n, H) if want_div else None
     dr = _empty(n, H) if want_drhodt else None
-    words = _empty(n * int(_capi.lib().sph_compsph_prep_floats(int(params.dim))), H)
+    words = _empty(n * _floats_of("sph_compsph_prep_floats", params.dim), H)
     with _timed("compsph_prep"):
         check(_capi.lib().sph_compsph_prep_packed(_p(params), n, fptr(x), fptr(H), fptr(m), fptr(rho), fptr(v),
                                                   *_lists(params, adj, True), ptr(om), ptr(div), ptr(dr), ptr(words),
@@ -831,7 +843,7 @@ def compsph_accel_dudt(params, x, H, m, rho, v, c, alpha, P, omega, adj: Adjacen
     dEdt = _empty(n, H) if want_dEdt else None
     ap = _pair_empty(adj.nnz, d, H) if pair_arrays else None
     av = _pair_empty(adj.nnz, d, H) if pair_arrays else None
-    recs = _empty(n * int(_capi.lib().sph_compsph_record_floats(d)), H)
+    recs = _empty(n * _floats_of("sph_compsph_record_floats", d), H)
     with _timed("compsph_accel_dudt"):
         rows = _lists(params, adj, True)
         check(_capi.lib().sph_compsph_accel_dudt_packed(_p(params), n, fptr(x), fptr(H), fptr(m), fptr(rho), fptr(v), fptr(c),
@@ -1022,13 +1034,13 @@ def jacobi_solve(params, mode: int, cfg, x, H, m, rho, v, dvdt, p_init, dt, adj:
     with _timed("dfsph_div_solve" if mode == DIVERGENCE_FREE else "dfsph_density_solve"):
         grads = _gradient_buffer(n, adj.nnz, d, m.device)
         if grads is not None:
-            check(L.sph_dfsph_solve_cached(mode, _p(params), C.cast(C.pointer(cfg), C.c_void_p), n, adj.nnz, fptr(x), fptr(H), fptr(m),
+            check(L.sph_dfsph_solve_cached(mode, _p(params), _p(cfg), n, adj.nnz, fptr(x), fptr(H), fptr(m),
                                            fptr(rho), fptr(v), fptr(dvdt), fptr(p_init), ptr(dt_tensor(dt, m.device)),
                                            *_lists(params, adj, True), ptr(ws), int(ws.numel()), ptr(grads), int(grads.numel()), ptr(pr),
                                            ptr(acc), ptr(hist), ptr(flags), ptr(flags[1:]), stream_ptr(m.device)), "jacobi solve")
             return pr, acc, hist, flags[:1], flags[1:]
         fn = L.sph_dfsph_div_solve if mode == DIVERGENCE_FREE else L.sph_dfsph_density_solve
-        check(fn(_p(params), C.cast(C.pointer(cfg), C.c_void_p), n, fptr(x), fptr(H), fptr(m), fptr(rho), fptr(v), fptr(dvdt),
+        check(fn(_p(params), _p(cfg), n, fptr(x), fptr(H), fptr(m), fptr(rho), fptr(v), fptr(dvdt),
                  fptr(p_init), ptr(dt_tensor(dt, m.device)), *_lists(params, adj, True), ptr(ws), int(ws.numel()), ptr(pr), ptr(acc),
                  ptr(hist), ptr(flags), ptr(flags[1:]), stream_ptr(m.device)), "jacobi solve")
     return pr, acc, hist, flags[:1], flags[1:]
@@ -1064,7 +1076,7 @@ def dfsph_features(params, mode: int, cfg, x, H, m, rho, v, dvdt, p_prev, dt, ad
     feats = torch.empty((n, 8), device=m.device, dtype=torch.float32)
     scale = torch.empty(1, device=m.device, dtype=torch.float32)
     with _timed("dfsph_features"):
-        check(_capi.lib().sph_dfsph_features(_p(params), C.cast(C.pointer(cfg), C.c_void_p), int(mode), n, fptr(x), fptr(H), fptr(m),
+        check(_capi.lib().sph_dfsph_features(_p(params), _p(cfg), int(mode), n, fptr(x), fptr(H), fptr(m),
                                              fptr(rho), fptr(v), fptr(dvdt), fptr(p_prev), ptr(dt_tensor(dt, m.device)),
                                              *_lists(params, adj, True), ptr(ws), int(ws.numel()), ptr(feats), ptr(scale),
                                              stream_ptr(m.device)), "sph_dfsph_features")
@@ -1156,7 +1168,7 @@ def deltasph_rhs(params, wc, x, H, m, rho, v, adj: AdjacencyList, surface_mask=N
     dvdt, drhodt = _empty((n, d), m), _empty(n, m)
     sm = None if surface_mask is None else surface_mask.to(torch.int32).contiguous()
     with _timed("deltasph_rhs"):
-        check(_capi.lib().sph_deltasph_rhs(_p(params), C.cast(C.pointer(wc), C.c_void_p), n, fptr(x), fptr(H), fptr(m), fptr(rho),
+        check(_capi.lib().sph_deltasph_rhs(_p(params), _p(wc), n, fptr(x), fptr(H), fptr(m), fptr(rho),
                                            fptr(v), iptr(sm), *_lists(params, adj, True), ptr(scratch), ptr(dvdt), ptr(drhodt),
                                            stream_ptr(m.device)), "sph_deltasph_rhs")
     return dvdt, drhodt, scratch[: n * d].view(n, d), scratch[n * d:]
@@ -1167,7 +1179,7 @@ def wc_visc_continuity(params, wc, x, H, m, rho, v, adj: AdjacencyList):
     n, d = m.shape[0], int(params.dim)
     dvdt, drhodt = _empty((n, d), m), _empty(n, m)
     with _timed("wc_visc_continuity"):
-        check(_capi.lib().sph_wc_visc_continuity(_p(params), C.cast(C.pointer(wc), C.c_void_p), n, fptr(x), fptr(H), fptr(m), fptr(rho),
+        check(_capi.lib().sph_wc_visc_continuity(_p(params), _p(wc), n, fptr(x), fptr(H), fptr(m), fptr(rho),
                                                  fptr(v), *_lists(params, adj, True), ptr(dvdt), ptr(drhodt), stream_ptr(m.device)),
               "sph_wc_visc_continuity")
     return dvdt, drhodt
@@ -1189,7 +1201,7 @@ def delta_shift(params, x, H, m, rho, v, kinds, adj: AdjacencyList, cfl: float, 
 
 def wc_eos(wc, rho) -> torch.Tensor:
     out = torch.empty_like(rho)
-    check(_capi.lib().sph_wc_eos(C.cast(C.pointer(wc), C.c_void_p), rho.shape[0], fptr(rho), ptr(out), stream_ptr(rho.device)),
+    check(_capi.lib().sph_wc_eos(_p(wc), rho.shape[0], fptr(rho), ptr(out), stream_ptr(rho.device)),
           "sph_wc_eos")
     return out
 
