@@ -514,3 +514,9 @@ def test_velocity_gradient_writes_the_divergence(cuda, dim, n_side, cullen):
     divergence = torch.full_like(V, float("nan"))
     _, rho, *_, dr, _, _, _ = ops.crk_rhs_fields(p, ops.pack_xh(p, x, H), m, V, v, u, adj, cullen, divergence)
     assert torch.equal(divergence, -dr / rho)
+
+
+# both sides of the particle count up to which the 4-lane passes run with 8 lanes (16,576)
+@pytest.mark.parametrize("dim,n_side", [(2, 128), (2, 129), (3, 25), (3, 26)])
+def test_packed_passes_at_the_middle_lane_split(cuda, dim, n_side):
+    test_packed_passes_match_separate_arrays(cuda, dim, n_side, core.KernelFunctions.Wendland4)

@@ -198,7 +198,18 @@ struct KSum {
 //   Cullen switch         79 /  85 / 100 / 149   1291 / 1190 / 1135 / 1185   7.7 / 5.4 / 4.5 / 4.5
 //   CRK factors           59 /  78 / 127 / 226    718 /  818 / 1072 / 1628   6.8 / 5.2 / 5.0 / 6.3
 //   adaptive support      47 /  52 /  70 / 108   1014 / 1049 / 1101 / 1288   6.2 / 4.5 / 4.0 / 3.9
-// At 25,600 particles in 2D the first column's choices still win; at 8,000 in 3D 8 to 16 lanes.
+// Up to MID_LIMIT particles (112 per SM) the passes that take 4 lanes above it run with 8, for twice the
+// warps.  Microseconds with 4 / 8 / 16 lanes (3D: 64 neighbours):
+//                        2D 10,000            2D 16,384            2D 25,600            3D 10,648
+//   CRK accel            13.5 /  9.7 / 11.7   14.9 / 11.6 / 14.7   17.1 / 18.2 / 21.8
+//   velocity gradient     6.5 /  5.6 /  6.0    7.0 /  6.6 /  8.3    8.3 /  9.7 / 11.2    9.6 / 9.0 /  9.9
+//   Cullen switch         8.2 /  6.0 /  6.1    8.4 /  7.3 /  9.7    9.7 / 10.3 / 12.4
+//   CRK factors           7.1 /  6.1 /  7.6    7.8 /  7.6 / 10.6    8.8 / 11.3 / 15.2   10.9 / 9.8 / 12.7
+//   adaptive support      6.5 /  4.7 /  4.9    6.8 /  5.6 /  6.5    7.0 /  7.3 /  9.2    9.7 / 6.9 /  7.4
+//   CompSPH prep          6.6 /  4.9 /  5.0    6.6 /  5.6 /  7.4    7.1 /  7.3 /  9.1    9.4 / 7.2 /  7.2
+// Six recorded steps in 2D, 4 against 8 lanes, with 20 / 32 / 50 neighbours: 14,400 particles 1209 / 1345 / 1653
+// against 1214 / 1307 / 1547 us, 16,384 particles 1233 / 1512 / 1737 against 1237 / 1450 / 1564, 17,956 particles
+// 1267 / 1550 / 1770 against 1286 / 1535 / 1635.
 #ifndef G_LIGHT
 #define G_LIGHT 8
 #endif
@@ -216,11 +227,15 @@ struct KSum {
 #define G_CULLEN(D) ((D) == 3 ? 16 : 4)
 #define G_ADAPT(D) 4
 constexpr int64_t WIDE_LIMIT = 148 * 64;
+constexpr int64_t MID_LIMIT = 148 * 112;
 #define G_WIDE 16
-// Runs the launch with LG lanes per particle: BASE, or WIDE for small particle sets.
+#define G_MID 8
+// Runs the launch with LG lanes per particle: BASE, at least G_MID up to MID_LIMIT particles, or WIDE
+// for small particle sets.
 #define PAIR_LANES(n, BASE, WIDE, ...)                               \
     do {                                                             \
         if ((n) <= WIDE_LIMIT) { constexpr int LG = WIDE; __VA_ARGS__; } \
+        else if ((n) <= MID_LIMIT) { constexpr int LG = (BASE) < G_MID ? G_MID : (BASE); __VA_ARGS__; } \
         else { constexpr int LG = BASE; __VA_ARGS__; }               \
     } while (0)
 
