@@ -30,3 +30,14 @@ def test_markstein_quotients_are_rounded(cuda, tmp_path):
                     str(build.CSRC), str(src), "-o", str(exe)], check=True, capture_output=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
     assert out == ["rcp", "0", "div", "0", "div2", "0"], out
+
+
+def test_newton_bounds_hold_up_to_the_ends_of_the_range(cuda, tmp_path):
+    """Every exponent from the subnormals up, zeros, infinities and NaN: zero results outside the
+    stated bounds (a reciprocal of 0 is infinite and of an infinity 0, as the division's)."""
+    src = Path(__file__).resolve().parent / "native" / "newton_domain_check.cu"
+    exe = tmp_path / "newton_domain_check"
+    subprocess.run([build.nvcc(), *build.ARCH_FLAGS, "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-I", str(build.INCLUDE), "-I",
+                    str(build.CSRC), str(src), "-o", str(exe)], check=True, capture_output=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    assert out == ["sqrt", "0", "rcp", "0", "special", "0"], out

@@ -520,3 +520,30 @@ def test_velocity_gradient_writes_the_divergence(cuda, dim, n_side, cullen):
 @pytest.mark.parametrize("dim,n_side", [(2, 128), (2, 129), (3, 25), (3, 26)])
 def test_packed_passes_at_the_middle_lane_split(cuda, dim, n_side):
     test_packed_passes_match_separate_arrays(cuda, dim, n_side, core.KernelFunctions.Wendland4)
+
+
+@pytest.mark.parametrize("dim,n_side", [(1, 60), (2, 12), (3, 8)])
+def test_energy_partition_with_an_infinite_entropy(cuda, dim, n_side):
+    """P / rho^gamma overflows where a density all but vanishes: the other particle of a pair then takes
+    the share 0, as the quotient of the smaller entropy by the sum gives it (NaN where the oracle has NaN)."""
+    cfg, sch, p = make_params(dim)
+    p.energy_scheme = int(EnergyScheme.CRK.value)
+    P = make_particles(dim, n_side, seed=80 + dim)
+    G = to_gpu(P, cuda)
+    adj = ops.buildVerletList(G["positions"], G["supports"], p, p.verlet_scale)
+    n, nnz = len(P["masses"]), adj.nnz
+    rng = np.random.default_rng(5)
+    rho, Pr = (1.0 + 0.1 * rng.random(n)).astype(np.float32), (1.0 + 0.1 * rng.random(n)).astype(np.float32)
+    rho[:: 7] = 1e-30
+    dvdt = rng.standard_normal((n, dim)).astype(np.float32)
+    ap, av = (rng.standard_normal((nnz, dim)).astype(np.float32) for _ in range(2))
+    d = to_gpu(dict(rho=rho, P=Pr, dvdt=dvdt, ap=ap, av=av), cuda)
+    # every Verlet entry carries an acceleration here, so every entry is walked
+    adj.interCounts = adj.numNeighbors
+    f = ops.compsph_balance(p, G["masses"], d["rho"], d["P"], G["internalEnergies"], G["velocities"], d["dvdt"], 1e-3, adj, d["ap"], d["av"])
+    want = oracle.get("f32").balance(p, P["masses"], rho, Pr, P["internalEnergies"], P["velocities"], dvdt, 1e-3, nb_numpy(adj), ap, av)
+    got = f.cpu().numpy()
+    assert np.isnan(want).any() and (want == 0).any()
+    wrong = ~((got == want) | (np.isnan(got) & np.isnan(want)) | (np.abs(got - want) <= 1e-5))
+    # an entry whose energy rounds to either side of zero takes the other particle's share
+    assert wrong.mean() < 1e-4, (wrong.sum(), got[wrong][:5], want[wrong][:5])

@@ -143,29 +143,37 @@ template <int D> __device__ __forceinline__ Vec<D> pair_vec(const Vec<D>& xi, co
     }
     return r;
 }
-// sqrt(x) for 0 <= x and 1 / x for normal x > 0: the hardware's approximation and one Newton-Raphson
-// step, within 1 ulp (pair distances and reciprocals of supports and densities).
+// sqrt(x) and 1 / x for the pair sums: the hardware's approximation and one Newton-Raphson step.
+//   sqrt_newton   within 1 ulp from 2^-100 up and 2 ulp down to FLT_MIN, 0 at 0; a subnormal argument gives
+//                 less than its root (by less than 1.1e-19); NaN at +inf, which like an infinite distance
+//                 compares false with every support
+//   rcp_newton    within 1 ulp for normal |x| <= 2^126, above that 0 or the subnormal quotient; 0 and the
+//                 subnormals give an infinity, an infinity 0 of its sign.  There the residual 1 - x y is NaN,
+//                 which fminf replaces by its bound (every other residual lies below 2^-20)
 __device__ __forceinline__ float sqrt_newton(float x) {
     float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(x, 1e-36f)));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(x, 1.17549435e-38f)));
     const float r = x * y;
     return fmaf(fmaf(-r, r, x), 0.5f * y, r);
 }
 __device__ __forceinline__ float rcp_newton(float x) {
-    float y;
+    float y, e;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return fmaf(fmaf(-x, y, 1.f), y, y);
+    asm("fma.rn.ftz.f32 %0, %1, %2, 0f3F800000;" : "=f"(e) : "f"(-x), "f"(y));
+    return fmaf(fminf(e, 9.5367432e-7f), y, y);
 }
 // a / b rounded to nearest, with r = 1 / b rounded to nearest: the second residual correction starts
 // from a quotient within an ulp, where its result is the rounded quotient (Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", 1990).  No underflow of the residuals.
+// elementary functions on the IBM RISC System/6000 processor", 1990).  For finite a and quotients and
+// residuals in the normal range (|a| >= 2^-102 or a = 0); outside it the result may be an ulp off, and
+// an infinite quotient is NaN.
 __device__ __forceinline__ float div_markstein(float a, float b, float r) {
     float q = a * r;
     q = fmaf(fmaf(-b, q, a), r, q);
     return fmaf(fmaf(-b, q, a), r, q);
 }
-// 1 / b rounded to nearest: two Newton steps from the hardware approximation, of which the second starts
-// within an ulp (Markstein; a divisor whose significand is all ones may be an ulp off).
+// 1 / b rounded to nearest for normal |b| <= 2^126: two Newton steps from the hardware approximation, of which
+// the second starts within an ulp (Markstein; a divisor whose significand is all ones may be an ulp off).
 __device__ __forceinline__ float rcp_markstein(float b) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
