@@ -1,0 +1,62 @@
+"""Host side of the DFSPH pressure solves (no GPU): memory of the cached pair gradients."""
+import pytest
+import torch
+
+from warpsph_b200 import _capi, ops
+from warpsph_b200.core import AdjacencyList
+
+
+class FakeLib:
+    """Records the solves that reach the library, with their arguments."""
+
+    def __init__(self):
+        self.calls = []
+
+    def sph_dfsph_gradient_bytes(self, n, entries, dim):
+        return 16 * (n + entries)
+
+    def __getattr__(self, name):
+        return lambda *args: self.calls.append((name, args)) or 0
+
+
+@pytest.fixture
+def host(monkeypatch):
+    lib = FakeLib()
+    monkeypatch.setattr(_capi, "lib", lambda: lib)
+    for name in ("ptr", "fptr", "iptr"):
+        monkeypatch.setattr(ops, name, lambda t: None if t is None else t.data_ptr())
+    monkeypatch.setattr(ops, "stream_ptr", lambda device: 0)
+    monkeypatch.setattr(ops, "_jacobi_workspace", lambda n, d, device: torch.empty(256, dtype=torch.uint8))
+    return lib
+
+
+def solve(adj, n=5):
+    cfg = _capi.SphJacobiConfig()
+    cfg.max_iterations = 2
+    params = _capi.SphParams()
+    params.dim = 3
+    f, f3 = torch.zeros(n), torch.zeros(n, 3)
+    return ops.jacobi_solve(params, ops.DENSITY, cfg, f3, f, f, f, f3, f3, f, 1e-3, adj)
+
+
+def rows_of(n=5, nnz=20, length=20):
+    return AdjacencyList(neighborOffsets=torch.arange(0, 4 * n, 4, dtype=torch.int32), numNeighbors=torch.full((n,), 4, dtype=torch.int32),
+                         neighborList=torch.zeros(length, dtype=torch.int32), numRows=n, numCols=n, nnz=nnz)
+
+
+def test_kept_rows_are_rewritten_before_the_optional_buffer(host, monkeypatch):
+    """On a device that is nearly full the rewrite of a kept list must not find its memory taken by the
+    gradients, without which the solve still runs."""
+    order = []
+    adj = rows_of()
+    adj._pending = object()
+
+    def rewrite(a, *rest):
+        order.append("rows")
+        a._pending = None
+
+    monkeypatch.setattr(ops, "_materialize_inter", rewrite)
+    monkeypatch.setattr(ops, "_gradient_buffer", lambda *a: order.append("gradients"))
+    solve(adj)
+    assert order == ["rows", "gradients"]
+    assert [name for name, _ in host.calls] == ["sph_dfsph_density_solve"]

@@ -1032,16 +1032,17 @@ def jacobi_solve(params, mode: int, cfg, x, H, m, rho, v, dvdt, p_init, dt, adj:
     flags = torch.zeros(2, device=m.device, dtype=torch.int32)
     L = _capi.lib()
     with _timed("dfsph_div_solve" if mode == DIVERGENCE_FREE else "dfsph_density_solve"):
+        rows = _lists(params, adj, True)      # a kept list is rewritten here, with the memory it needs, before the optional buffer
         grads = _gradient_buffer(n, adj.nnz, d, m.device)
         if grads is not None:
             check(L.sph_dfsph_solve_cached(mode, _p(params), _p(cfg), n, adj.nnz, fptr(x), fptr(H), fptr(m),
                                            fptr(rho), fptr(v), fptr(dvdt), fptr(p_init), ptr(dt_tensor(dt, m.device)),
-                                           *_lists(params, adj, True), ptr(ws), int(ws.numel()), ptr(grads), int(grads.numel()), ptr(pr),
+                                           *rows, ptr(ws), int(ws.numel()), ptr(grads), int(grads.numel()), ptr(pr),
                                            ptr(acc), ptr(hist), ptr(flags), ptr(flags[1:]), stream_ptr(m.device)), "jacobi solve")
             return pr, acc, hist, flags[:1], flags[1:]
         fn = L.sph_dfsph_div_solve if mode == DIVERGENCE_FREE else L.sph_dfsph_density_solve
         check(fn(_p(params), _p(cfg), n, fptr(x), fptr(H), fptr(m), fptr(rho), fptr(v), fptr(dvdt),
-                 fptr(p_init), ptr(dt_tensor(dt, m.device)), *_lists(params, adj, True), ptr(ws), int(ws.numel()), ptr(pr), ptr(acc),
+                 fptr(p_init), ptr(dt_tensor(dt, m.device)), *rows, ptr(ws), int(ws.numel()), ptr(pr), ptr(acc),
                  ptr(hist), ptr(flags), ptr(flags[1:]), stream_ptr(m.device)), "jacobi solve")
     return pr, acc, hist, flags[:1], flags[1:]
 
