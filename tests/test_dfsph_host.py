@@ -60,3 +60,14 @@ def test_kept_rows_are_rewritten_before_the_optional_buffer(host, monkeypatch):
     solve(adj)
     assert order == ["rows", "gradients"]
     assert [name for name, _ in host.calls] == ["sph_dfsph_density_solve"]
+
+
+def test_the_buffer_covers_the_list_and_not_the_stated_count(host, monkeypatch):
+    """The preparation writes one gradient per row entry.  Rows may lie anywhere in the list that they index,
+    whatever count a caller's AdjacencyList states."""
+    asked = []
+    monkeypatch.setattr(ops, "_gradient_buffer", lambda n, entries, d, device: asked.append(entries) or torch.empty(16 * (n + entries), dtype=torch.uint8))
+    solve(rows_of(nnz=3, length=32))
+    assert asked == [32]
+    (name, args), = host.calls
+    assert name == "sph_dfsph_solve_cached" and args[4] == 32

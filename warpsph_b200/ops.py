@@ -1033,9 +1033,10 @@ def jacobi_solve(params, mode: int, cfg, x, H, m, rho, v, dvdt, p_init, dt, adj:
     L = _capi.lib()
     with _timed("dfsph_div_solve" if mode == DIVERGENCE_FREE else "dfsph_density_solve"):
         rows = _lists(params, adj, True)      # a kept list is rewritten here, with the memory it needs, before the optional buffer
-        grads = _gradient_buffer(n, adj.nnz, d, m.device)
+        entries = adj.neighborList.numel()    # what bounds the rows (adj.nnz is the caller's word)
+        grads = _gradient_buffer(n, entries, d, m.device)
         if grads is not None:
-            check(L.sph_dfsph_solve_cached(mode, _p(params), _p(cfg), n, adj.nnz, fptr(x), fptr(H), fptr(m),
+            check(L.sph_dfsph_solve_cached(mode, _p(params), _p(cfg), n, entries, fptr(x), fptr(H), fptr(m),
                                            fptr(rho), fptr(v), fptr(dvdt), fptr(p_init), ptr(dt_tensor(dt, m.device)),
                                            *rows, ptr(ws), int(ws.numel()), ptr(grads), int(grads.numel()), ptr(pr),
                                            ptr(acc), ptr(hist), ptr(flags), ptr(flags[1:]), stream_ptr(m.device)), "jacobi solve")
