@@ -71,3 +71,32 @@ def test_the_buffer_covers_the_list_and_not_the_stated_count(host, monkeypatch):
     assert asked == [32]
     (name, args), = host.calls
     assert name == "sph_dfsph_solve_cached" and args[4] == 32
+
+
+def test_a_buffer_that_did_not_fit_is_not_tried_again_until_there_is_room(host, monkeypatch):
+    """Each failing allocation flushes the allocator's cache and synchronises, so it happens once."""
+    device = torch.device("cuda", 0)
+    monkeypatch.setattr(ops, "_gradient_refused", {})
+    free, tried = [1000], []
+
+    def empty(size, dtype=None, device=None):
+        tried.append(size)
+        if size > free[0]:
+            raise torch.cuda.OutOfMemoryError("out of memory")
+        return ("buffer", size)
+
+    monkeypatch.setattr(ops.torch, "empty", empty)
+    monkeypatch.setattr(ops.torch.cuda, "mem_get_info", lambda device: (free[0] - 300, 1 << 30))
+    monkeypatch.setattr(ops.torch.cuda, "memory_stats", lambda device: {
+        "reserved_bytes.all.current": 900, "active_bytes.all.current": 500, "inactive_split_bytes.all.current": 100})
+    big, small = 16 * (10 + 90), 16 * (10 + 20)
+    assert ops._gradient_buffer(10, 90, 3, device) is None and tried == [big]
+    for _ in range(3):
+        assert ops._gradient_buffer(10, 90, 3, device) is None
+    assert ops._gradient_buffer(10, 200, 3, device) is None
+    assert tried == [big]
+    # a smaller solve is unaffected, and the large one is served again once memory is back
+    assert ops._gradient_buffer(10, 20, 3, device) == ("buffer", small)
+    free[0] = 2000
+    assert ops._gradient_buffer(10, 90, 3, device) == ("buffer", big)
+    assert ops._gradient_refused == {}

@@ -1048,13 +1048,35 @@ def jacobi_solve(params, mode: int, cfg, x, H, m, rho, v, dvdt, p_init, dt, adj:
     return pr, acc, hist, flags[:1], flags[1:]
 
 
+_gradient_refused: dict = {}      # device index -> the smallest gradient buffer it had no room for
+
+
 def _gradient_buffer(n: int, entries: int, d: int, device) -> Optional[torch.Tensor]:
     """The cached pair gradients of one solve (16 bytes per row entry in 3D), or None when the
-    device has no room for them: the solve then forms each gradient in every iteration."""
-    try:
-        return torch.empty(int(_capi.lib().sph_dfsph_gradient_bytes(n, entries, d)), dtype=torch.uint8, device=device)
-    except torch.cuda.OutOfMemoryError:
+    device has no room for them: the solve then forms each gradient in every iteration.  A failing
+    allocation makes torch give back its cached blocks and synchronise, so after one the solves of
+    that size or larger ask for the room first and allocate only when it is there."""
+    want = int(_capi.lib().sph_dfsph_gradient_bytes(n, entries, d))
+    refused = _gradient_refused.get(device.index)
+    asked = refused is not None and want >= refused
+    if asked and want > _device_room(device):
         return None
+    try:
+        grads = torch.empty(want, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        _gradient_refused[device.index] = want if refused is None else min(want, refused)
+        return None
+    if asked:
+        _gradient_refused.pop(device.index, None)
+    return grads
+
+
+def _device_room(device) -> int:
+    """Bytes that one allocation can count on: the device's free memory and the cached blocks that
+    torch can give back whole."""
+    st = torch.cuda.memory_stats(device)
+    cached = st["reserved_bytes.all.current"] - st["active_bytes.all.current"] - st["inactive_split_bytes.all.current"]
+    return torch.cuda.mem_get_info(device)[0] + cached
 
 
 def _jacobi_workspace(n: int, d: int, device) -> torch.Tensor:
