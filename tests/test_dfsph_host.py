@@ -87,6 +87,7 @@ def test_a_buffer_that_did_not_fit_is_not_tried_again_until_there_is_room(host, 
 
     monkeypatch.setattr(ops.torch, "empty", empty)
     monkeypatch.setattr(ops.torch.cuda, "mem_get_info", lambda device: (free[0] - 300, 1 << 30))
+    monkeypatch.setattr(ops.torch.cuda, "get_per_process_memory_fraction", lambda device: 1.0)
     monkeypatch.setattr(ops.torch.cuda, "memory_stats", lambda device: {
         "reserved_bytes.all.current": 900, "active_bytes.all.current": 500, "inactive_split_bytes.all.current": 100})
     big, small = 16 * (10 + 90), 16 * (10 + 20)

@@ -1072,11 +1072,14 @@ def _gradient_buffer(n: int, entries: int, d: int, device) -> Optional[torch.Ten
 
 
 def _device_room(device) -> int:
-    """Bytes that one allocation can count on: the device's free memory and the cached blocks that
-    torch can give back whole."""
+    """Bytes that one allocation can count on: free memory within the process's share of the device,
+    and the cached blocks that torch can give back whole."""
     st = torch.cuda.memory_stats(device)
-    cached = st["reserved_bytes.all.current"] - st["active_bytes.all.current"] - st["inactive_split_bytes.all.current"]
-    return torch.cuda.mem_get_info(device)[0] + cached
+    reserved = st.get("reserved_bytes.all.current", 0)
+    free, total = torch.cuda.mem_get_info(device)
+    share = int(torch.cuda.get_per_process_memory_fraction(device) * total) - reserved
+    cached = reserved - st.get("active_bytes.all.current", 0) - st.get("inactive_split_bytes.all.current", 0)
+    return min(free, share) + cached
 
 
 def _jacobi_workspace(n: int, d: int, device) -> torch.Tensor:
