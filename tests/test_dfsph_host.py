@@ -1,8 +1,11 @@
 """Host side of the DFSPH pressure solves (no GPU): memory of the cached pair gradients."""
+import subprocess
+from pathlib import Path
+
 import pytest
 import torch
 
-from warpsph_b200 import _capi, ops
+from warpsph_b200 import _capi, build, ops
 from warpsph_b200.core import AdjacencyList
 
 
@@ -101,3 +104,18 @@ def test_a_buffer_that_did_not_fit_is_not_tried_again_until_there_is_room(host, 
     free[0] = 2000
     assert ops._gradient_buffer(10, 90, 3, device) == ("buffer", big)
     assert ops._gradient_refused == {}
+
+
+def test_blocks_of_a_persistent_launch(tmp_path):
+    """A kernel that keeps one particle per group for the whole solve is launched only when all particles fit
+    in one round of co-resident blocks, and no launch has more blocks than slots for their partial sums."""
+    root = Path(__file__).resolve().parent
+    exe = tmp_path / "persistent_grid_check"
+    subprocess.run([build.nvcc(), "-std=c++17", "-I", str(build.INCLUDE), "-I", str(build.CSRC), "-o", str(exe),
+                    str(root / "native" / "persistent_grid_check.cu")], check=True, capture_output=True)
+    cases = [((4736, 32, 296, 2048, 1), 148), ((4736, 32, 148, 2048, 1), 148), ((4736, 32, 147, 2048, 1), 0), ((4737, 32, 148, 2048, 1), 0),
+             ((18944, 64, 296, 2048, 1), 296), ((18944, 64, 148, 2048, 1), 0), ((18944, 64, 148, 2048, 0), 148), ((1, 64, 296, 2048, 1), 1),
+             ((1 << 29, 64, 592, 2048, 0), 592), ((1 << 29, 64, 4096, 2048, 0), 2048), ((1 << 29, 64, 4096, 1 << 62, 0), 4096),
+             ((200000, 64, 4096, 2048, 1), 0)]
+    out = subprocess.run([str(exe), *[str(v) for args, _ in cases for v in args]], check=True, capture_output=True, text=True).stdout.split()
+    assert [int(v) for v in out] == [want for _, want in cases]

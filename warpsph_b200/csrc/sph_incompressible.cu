@@ -25,7 +25,6 @@
 // Data written in one phase and read by other blocks in the next (p, a) is
 // loaded with ld.global.cg (L2), never through the non-coherent L1.
 #include <cuda_runtime.h>
-#include <algorithm>
 #include <mutex>
 #include "sph_pair_common.cuh"
 #include "sph_persistent.cuh"
@@ -655,11 +654,13 @@ static int device_sms() {
 }
 
 // One cooperative launch of a persistent solve kernel over n particles (KERN names the kernel, so
-// that each instantiation keeps its own occupancy).
-template <auto KERN, int BLOCK, int PPB, typename Args>
-static int launch_persistent(Args& a, cudaStream_t s) {
+// that each instantiation keeps its own occupancy), of at most LIMIT blocks.  ONE_ROUND: the kernel needs all
+// particles in one round; where they do not fit, nothing is launched and *launched stays false.
+template <auto KERN, int BLOCK, int PPB, bool ONE_ROUND, int64_t LIMIT, typename Args>
+static int launch_persistent(Args& a, cudaStream_t s, bool* launched) {
     static std::mutex mu;
     static int cached_dev = -1, blocks_per_sm = 0, num_sms = 0;
+    int64_t resident = 0;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return set_error(SPH_ERR_CUDA, "jacobi: cudaGetDevice: %s", cudaGetErrorString(e));
@@ -675,9 +676,11 @@ static int launch_persistent(Args& a, cudaStream_t s) {
             if (e != cudaSuccess || blocks_per_sm < 1) return set_error(SPH_ERR_CUDA, "jacobi: occupancy query failed");
             cached_dev = dev;
         }
+        resident = (int64_t)blocks_per_sm * num_sms;
     }
-    const int64_t need = (a.n + PPB - 1) / PPB;
-    const int grid = (int)std::min<int64_t>(need, (int64_t)blocks_per_sm * num_sms);
+    const int grid = persistent_grid(a.n, PPB, resident, LIMIT, ONE_ROUND);
+    if (grid == 0) return SPH_OK;
+    *launched = true;
     void* args[] = {&a};
     count_launch();
     e = cudaLaunchCooperativeKernel((const void*)KERN, dim3(grid), dim3(BLOCK), args, 0, s);
@@ -687,7 +690,8 @@ static int launch_persistent(Args& a, cudaStream_t s) {
 
 // Bytes per row entry and in all of the buffer of cached pair gradients: the particles' (p, 1 / rho^2)
 // and (a, 1 / rho), then one gradient per entry.
-constexpr size_t kSumsBytes = 2048 * sizeof(JacobiSums);     // of at most 2048 co-resident blocks
+constexpr int64_t kSumSlots = 2048;                          // one per block of a solve
+constexpr size_t kSumsBytes = kSumSlots * sizeof(JacobiSums);
 static int64_t dfsph_grad_bytes(int64_t n, int64_t entries, int dim) {
     return (int64_t)(kSumsBytes + align256((size_t)n * sizeof(float2)) + align256((size_t)n * sizeof(float4)) +
                      align256((size_t)entries * (dim == 3 ? 4 : dim) * sizeof(float)));
@@ -754,16 +758,16 @@ static int dfsph_solve(int mode, const SphParams* p, const SphJacobiConfig* cfg,
         a.offs = offs; a.cnt = cnt; a.list = list; a.pq = pq; a.a4 = a4; a.sums = static_cast<JacobiSums*>(gradients);
         a.p_out = p_out; a.acc = accel_out; a.hist = history; a.iters_out = iterations; a.status_out = status; a.ctl = ctl;
         a.barrier_ns = barrier_ns;
-        rc = SPH_ERR_UNSUPPORTED;
-        
 #define JACOBI_GRAD(G, U, MINB, HOLD) WSPH_DISPATCH_DIM(P.dim, \
-        (rc = launch_persistent<k_jacobi_grad<D, G, U, JAC_BLOCK, MINB, HOLD>, JAC_BLOCK, JAC_BLOCK / G>(a, s)))
+        (rc = launch_persistent<k_jacobi_grad<D, G, U, JAC_BLOCK, MINB, HOLD>, JAC_BLOCK, JAC_BLOCK / G, HOLD, kSumSlots>(a, s, &launched)))
         // The split by size (see k_jacobi_grad): one block of 8 lanes per particle on each SM, two
-        // blocks of 4 lanes, or a loop over particles.
+        // blocks of 4 lanes, or a loop over particles, which also takes what the first two cannot hold (fewer
+        // resident blocks than their launch bounds ask for).
         const int sms = device_sms();
+        bool launched = false;
         if (n <= (int64_t)sms * (JAC_BLOCK / 8)) { JACOBI_GRAD(8, 6, 2, true); }
         else if (n <= (int64_t)sms * 2 * (JAC_BLOCK / 4)) { JACOBI_GRAD(4, 10, 2, true); }
-        else { JACOBI_GRAD(4, 5, 4, false); }
+        if (rc == SPH_OK && !launched) { rc = SPH_ERR_UNSUPPORTED; JACOBI_GRAD(4, 5, 4, false); }
 #undef JACOBI_GRAD
         return rc;
     }
@@ -775,8 +779,9 @@ static int dfsph_solve(int mode, const SphParams* p, const SphJacobiConfig* cfg,
     a.praw = praw; a.p_out = p_out; a.acc = accel_out; a.hist = history;
     a.iters_out = iterations; a.status_out = status; a.ctl = ctl;
     a.barrier_ns = barrier_ns;
+    bool launched = false;
     rc = SPH_ERR_UNSUPPORTED;
-    WSPH_DISPATCH_KD(P.kernel, P.dim, (rc = launch_persistent<k_jacobi<KF, D>, JAC_BLOCK, JAC_PPB>(a, s)));
+    WSPH_DISPATCH_KD(P.kernel, P.dim, (rc = launch_persistent<k_jacobi<KF, D>, JAC_BLOCK, JAC_PPB, false, INT64_MAX>(a, s, &launched)));
     return rc;
 }
 

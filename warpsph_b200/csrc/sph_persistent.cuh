@@ -62,4 +62,13 @@ __device__ __forceinline__ bool grid_barrier(BarrierCtl* c, unsigned int& arrive
     return grid_wait(c, arrived, limit_ns);
 }
 
+// Blocks of a persistent launch over n particles with ppb of them per block and round: what n needs, at most
+// the co-resident blocks and `limit` (slots of per-block results).  With one_round, for a kernel whose groups keep
+// one particle each for the whole launch, 0 when that many blocks cannot hold the particles in one round.
+constexpr int persistent_grid(int64_t n, int ppb, int64_t resident, int64_t limit, bool one_round) {
+    const int64_t need = (n + ppb - 1) / ppb, cap = resident < limit ? resident : limit;
+    if (one_round && need > cap) return 0;
+    return (int)(need < cap ? need : cap);
+}
+
 }  // namespace wsph
