@@ -228,3 +228,18 @@ def test_mlp_forward_is_per_row(cuda, n):
     ref = torch.cat([ops.mlp_forward(th, x[a:a + step]) for a in range(0, n, step)])
     assert int(ops.mlp_status(cuda).item()) == 0
     assert torch.equal(y, ref)
+
+
+def test_gradient_reports_an_issuing_warp_that_gave_up(cuda, tmp_path):
+    """The kernel compiled with a stand-in for a wait that runs out before a block's last weight-gradient
+    product: each of 200 such launches returns the timeout status, and plain launches around them none and the same
+    gradient (1e-5 of its largest entry: its FP32 atomics add 148 partial sums in another order)."""
+    import subprocess
+    from pathlib import Path
+    from warpsph_b200 import build
+    src = Path(__file__).resolve().parent / "native" / "mlp_give_up_check.cu"
+    exe = tmp_path / "mlp_give_up_check"
+    subprocess.run([build.nvcc(), *build.ARCH_FLAGS, "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-I", str(build.INCLUDE), "-I",
+                    str(build.CSRC), str(src), "-o", str(exe)], check=True, capture_output=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=120).stdout.split()
+    assert out[:8] == ["plain", "0", "given_up", "200", "of", "200", "after", "0"] and float(out[9]) < 1e-5, out

@@ -641,6 +641,7 @@ k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restri
 // X alternates between two chunks because G_1 of a tile is issued after the next tile's X is
 // written.
 constexpr int GT_WGS = 3, GT_THREADS = (GT_WGS + 1) * TC_M, GT_TMEM_COLS = 512;
+constexpr int GT_SUMS_THREADS = GT_WGS * TC_M + 64;      // the warpgroups and the two issuing warps
 // registers per thread after the launch with 128: the w4 sums do not fit in 128
 constexpr int GT_REGS = 160, GT_REGS_MMA = 32;
 static_assert(TC_M * (GT_WGS * GT_REGS + GT_REGS_MMA) <= GT_THREADS * 128, "the shares add up to the launch's registers");
@@ -675,6 +676,10 @@ struct MlpGradTcSmem {
     int abort;
 };
 static_assert(sizeof(MlpGradTcSmem) + 128 <= 227 * 1024, "one CTA per SM");
+// A test's stand-in for a wait that runs out: the weight-gradient warp gives up before G_l of tile k.
+#ifndef GT_GIVE_UP
+#define GT_GIVE_UP(l, k) false
+#endif
 static_assert(sizeof(__nv_bfloat16) * MLP_H * (K1 + 2 * TC_K2) % 128 == 0, "128 B aligned operands");
 
 // 0xffff in the low and high half if bit j, j + 16 of m is set: prmt replicates the signs of bytes 1 and 3
@@ -797,6 +802,7 @@ k_mlp_grad_tc(const float* __restrict__ prm, int64_t n, const float* __restrict_
                     #pragma unroll 1
                     for (int w = 0; w < GT_WGS && k0 + w < ktiles; ++w) {
                         if (!wait_ready(aReady, w)) break;
+                        if (GT_GIVE_UP(l, k0 + w)) { ok = false; break; }
                         const uint32_t act = aAct + w * WG_BYTES;
                         const uint64_t dA = umma_desc_mnmajor(act + GT_DZ * GT_CHUNK, CORE, GT_CHUNK);
                         const uint64_t dB = umma_desc_mnmajor(act + (l == 3 ? GT_H2 : (l == 2 ? GT_H1 : x)) * GT_CHUNK, CORE, GT_CHUNK);
@@ -816,6 +822,8 @@ k_mlp_grad_tc(const float* __restrict__ prm, int64_t n, const float* __restrict_
             if (elect_one()) umma_commit(smem_u32(&s.done));
             // also after a timeout: nothing may be in flight when the TMEM columns are released
             if (!mbar_wait_bounded(smem_u32(&s.done), 0u, TC_WAIT_CYCLES) || !ok) s.abort = 1;
+            __syncwarp();
+            bar_sync_named(GT_WGS + 1, GT_SUMS_THREADS);
         }
     } else {
         setmaxnreg_inc<GT_REGS>();
@@ -1011,7 +1019,9 @@ k_mlp_grad_tc(const float* __restrict__ prm, int64_t n, const float* __restrict_
             gb += __shfl_xor_sync(0xffffffffu, gb, o);
         }
         if (lane == 0) { atomicAdd(&s.loss, lsum); atomicAdd(&s.gb4, gb); }
-        bar_sync_named(GT_WGS + 1, GT_WGS * TC_M);       // every warpgroup's sums and abort flag
+        // every warpgroup's sums, and the abort flag of both issuing warps: `done` alone says that nothing is in
+        // flight, also where a warp gave up before the last G_l
+        bar_sync_named(GT_WGS + 1, GT_SUMS_THREADS);
         if (s.abort) {
             if (tid == 0 && status) atomicOr(status, SPH_STATUS_TIMEOUT);
         } else {
