@@ -243,3 +243,17 @@ def test_gradient_reports_an_issuing_warp_that_gave_up(cuda, tmp_path):
                     str(build.CSRC), str(src), "-o", str(exe)], check=True, capture_output=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=120).stdout.split()
     assert out[:8] == ["plain", "0", "given_up", "200", "of", "200", "after", "0"] and float(out[9]) < 1e-5, out
+
+
+def test_inference_reports_a_single_thread_that_gave_up(cuda, tmp_path):
+    """One thread's stand-in for a wait that runs out on the last chain of its warpgroup: NaN in its row
+    and the timeout status, neither in the launches around it."""
+    import subprocess
+    from pathlib import Path
+    from warpsph_b200 import build
+    src = Path(__file__).resolve().parent / "native" / "mlp_forward_give_up_check.cu"
+    exe = tmp_path / "mlp_forward_give_up_check"
+    subprocess.run([build.nvcc(), *build.ARCH_FLAGS, "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-I", str(build.INCLUDE), "-I",
+                    str(build.CSRC), str(src), "-o", str(exe)], check=True, capture_output=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=120).stdout.split()
+    assert out == ["plain", "0", "0", "given_up", str(_capi.STATUS_TIMEOUT), "1", "after", "0", "0"], out

@@ -403,6 +403,11 @@ struct MlpTcSmem {
 static_assert((sizeof(__nv_bfloat16) * MLP_H * K1) % 128 == 0 && (sizeof(__nv_bfloat16) * MLP_H * TC_K2) % 128 == 0,
               "128 B aligned operands");
 
+// A test's stand-in for a wait that runs out: the thread gives up on the last chain of tile k.
+#ifndef FT_GIVE_UP
+#define FT_GIVE_UP(k) false
+#endif
+
 // relu of (lo, hi) rounded to BF16 and packed, lo in the low half
 __device__ __forceinline__ uint32_t relu_bf16x2(uint32_t lo, uint32_t hi) {
     uint32_t d;
@@ -549,6 +554,7 @@ k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restri
             }
             if (!ok) break;
             wait_chain();
+            ok = ok && !FT_GIVE_UP(k);
             // the next tile's first chain runs while the second half of the output layer is summed
             float y = 0.f;
             #pragma unroll
@@ -579,7 +585,9 @@ k_mlp_forward_tc(const float* __restrict__ prm, int64_t n, const float* __restri
             // are released; the status tells the host that the context is suspect, and the host stops
             // issuing work to this device's MLP after it.
             if (issuer) (void)mbar_wait_bounded(chain, phase ^ 1u, TC_WAIT_CYCLES);
-            if (r == 0 && status) atomicOr(status, SPH_STATUS_TIMEOUT);
+            // (every thread that gave up says so: behind the last chain of the last tile no barrier of the
+            // warpgroup follows that would tell the others)
+            if (status) atomicOr(status, SPH_STATUS_TIMEOUT);
             for (; k < ktiles; k += FT_WGS)
                 if (row_of(k) < n) out[row_of(k)] = __int_as_float(0x7fc00000);
         }
