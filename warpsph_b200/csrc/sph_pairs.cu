@@ -329,7 +329,7 @@ k_crk_factors(int n, DevParams P, const float* __restrict__ x, const float* __re
                 for (int c = u; c < D; ++c) {
                     const float gxx = gx * xij.v[c];
                     a.m2[a.at2(u, c)] += Wx * xij.v[c];
-                    a.g2[a.at2(u, c)] += gxx;
+                    a.g2[a.at2(u, c)] += u == c ? gxx + VW : gxx;
                     #pragma unroll
                     for (int w = c; w < D; ++w) a.g3[a.at3(u, c, w)] += gxx * xij.v[w];
                 }
@@ -343,9 +343,10 @@ k_crk_factors(int n, DevParams P, const float* __restrict__ x, const float* __re
     }
     if (!g.valid || g.lane != 0) return;
     const int i = g.i;
-    // The moments of the derivatives from the symmetric sums g1 = sum Vs x, g2 = sum Vs x x and
-    // g3 = sum Vs x x x (gradW = s x_ij): with m0 and m1,
-    //   dm0_w = g1_w,  dm1_uw = g2_uw + delta_uw m0,  dm2_ucw = g3_ucw + delta_uw m1_c + delta_cw m1_u
+    // The moments of the derivatives from the symmetric sums g1 = sum Vs x, g2 = sum (Vs x x + delta VW) and
+    // g3 = sum Vs x x x (gradW = s x_ij): with m1,
+    //   dm0_w = g1_w,  dm1 = g2,  dm2_ucw = g3_ucw + delta_uw m1_c + delta_cw m1_u
+    // The diagonal's two parts almost cancel: added up apart they cost gradB 12 % more error.
     double M2[D][D], Mi[D][D], G2[D][D], G3[D][D][D], tr = 0.0;
     #pragma unroll
     for (int u = 0; u < D; ++u) {
@@ -361,7 +362,6 @@ k_crk_factors(int n, DevParams P, const float* __restrict__ x, const float* __re
         }
         tr += (double)a.m2[a.at2(u, u)];
     }
-    auto dm1 = [&](int u, int w) { return G2[u][w] + (u == w ? (double)a.m0 : 0.0); };
     auto dm2 = [&](int u, int c, int w) { return G3[u][c][w] + (u == w ? (double)a.m1[c] : 0.0) + (c == w ? (double)a.m1[u] : 0.0); };
     double det = inv_sym<D>(M2, Mi);
     double sc = tr / D, sD = sc;
@@ -386,7 +386,7 @@ k_crk_factors(int n, DevParams P, const float* __restrict__ x, const float* __re
             double rhs[D];
             #pragma unroll
             for (int u = 0; u < D; ++u) {
-                double t = dm1(u, w);
+                double t = G2[u][w];
                 #pragma unroll
                 for (int c = 0; c < D; ++c) t += dm2(u, c, w) * Bv[c];
                 rhs[u] = t;
@@ -403,7 +403,7 @@ k_crk_factors(int n, DevParams P, const float* __restrict__ x, const float* __re
         for (int w = 0; w < D; ++w) {
             double t = (double)a.g1[w];
             #pragma unroll
-            for (int u = 0; u < D; ++u) t += dm1(u, w) * Bv[u] + (double)a.m1[u] * gB[u][w];
+            for (int u = 0; u < D; ++u) t += G2[u][w] * Bv[u] + (double)a.m1[u] * gB[u][w];
             gA[w] = -A * A * t;
         }
     } else {
