@@ -105,7 +105,6 @@ k_compsph_prep(int n, DevParams P, const float* __restrict__ x, const float* __r
                 scon += mj * sg;
             }
         }
-        sdh *= -(KernelTraits<KF, D>::C * ipow<D>(invHi)) * invHi;
     }
     if (want_om) sdh = gsum<G>(sdh);
     if (want_div) sdiv = gsum<G>(sdiv);
@@ -114,8 +113,8 @@ k_compsph_prep(int n, DevParams P, const float* __restrict__ x, const float* __r
     const int i = g.i;
     float om = 1.f;
     if (want_om) {
-        const float dh_drho = -H[i] / (rho[i] * (float)D);
-        om = 1.f - dh_drho * sdh;
+        // 1 - (-H / (rho d)) (-C / H^(d+1)) sum: the powers of H themselves, those of 1 / H would multiply its rounding
+        om = 1.f - KernelTraits<KF, D>::C * sdh / (ipow<D>(H[i]) * rho[i] * (float)D);
         omega[i] = om;
     }
     if (want_div) div[i] = sdiv;
