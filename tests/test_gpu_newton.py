@@ -41,3 +41,14 @@ def test_newton_bounds_hold_up_to_the_ends_of_the_range(cuda, tmp_path):
                     str(build.CSRC), str(src), "-o", str(exe)], check=True, capture_output=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
     assert out == ["sqrt", "0", "rcp", "0", "special", "0"], out
+
+
+def test_pair_image_equals_the_conditional_shift(cuda, tmp_path):
+    """The minimum image of the pair sums, bit for bit, around half the box above all."""
+    here = Path(__file__).resolve().parent / "native"
+    exe = tmp_path / "image_check"
+    subprocess.run([build.nvcc(), *build.ARCH_FLAGS, "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-I", str(build.INCLUDE), "-I",
+                    str(build.CSRC), str(here / "image_check.cu"), str(build.CSRC / "sph_neighbors.cu"), "-o", str(exe)], check=True,
+                   capture_output=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    assert out[:3] == ["differ", "0", "of"] and int(out[3]) > 900000, out

@@ -568,3 +568,20 @@ def test_gradient_of_the_correction_is_as_accurate_as_termwise_sums(cuda, dim, n
         for k, got in enumerate((crk.gradB.cpu().numpy().astype(np.float64), o32.crk_factors(p, x, H, m, V, nb)[3])):
             err[k] += np.linalg.norm(got - want) / np.linalg.norm(want)
     assert err[0] <= 1.05 * err[1], err / 4
+
+
+@pytest.mark.parametrize("dim,n_side", [(1, 8), (2, 6), (3, 4)])
+@pytest.mark.parametrize("L", [1.0, 3.0, 10.0])
+def test_supports_beyond_half_the_box(cuda, dim, n_side, L):
+    """Lattice pairs at exactly half the box inside each other's supports: the image of the oracle, not the one
+    on the other side (FP32 rounding, 2e-6 of scale; 1e-5 where the sum cancels)."""
+    cfg, sch, p = make_params(dim, L=L)
+    P = make_particles(dim, n_side, jitter=0.0, seed=7, L=L, h_spread=0.0)
+    P["supports"] = np.full_like(P["supports"], 0.8 * L)
+    G = to_gpu(P, cuda)
+    adj = ops.buildVerletList(G["positions"], G["supports"], p, p.verlet_scale)
+    rho = np.ones_like(P["masses"])
+    om, div, dr = ops.compsph_prep(p, G["positions"], G["supports"], G["masses"], torch.from_numpy(rho).to(cuda), G["velocities"], adj)
+    want = oracle.get("f32").compsph_prep(p, P["positions"], P["supports"], P["masses"], rho, P["velocities"], nb_numpy(adj))
+    for got, ref, tol, name in zip((om, div, dr), want, (2e-6, 1e-5, 1e-5), ("omega", "divergence", "drhodt")):
+        assert_close(got.cpu().numpy(), ref, tol, tol, name)

@@ -13,7 +13,7 @@ namespace wsph {
 // ---------------------------------------------------------------- params
 struct DomainF {
     float min[3], max[3], L[3], halfL[3];
-    float invL[3];          // 1 / L of a periodic axis, else 0
+    float turn[3];          // L / 2 of a periodic axis, else infinity
     int periodic[3];
 };
 
@@ -130,16 +130,17 @@ template <int D> __device__ __forceinline__ Vec<D> dist_vec(const Vec<D>& xi, co
     }
     return r;
 }
-// The same minimum image for the pair sums, with the image number k = rint(d / L) taken by adding
-// and subtracting 1.5 * 2^23: four multiply-add instructions per axis instead of three and four of
-// the half-rate comparison pipe.  d - k L is rounded once, as above, so the result is the same
-// float unless |d| is within a rounding of L / 2, where both images are equally far.
+// The same minimum image, bit for bit, for the pair sums: |d| > L / 2 as saturate((|d| - L / 2) 2^126), which is 1
+// or 0 (a difference of positions in a box longer than 1e-30 is 0 or above 2^-126), so that the half-rate comparison
+// pipe has one instruction per axis instead of four.  (Taking rint(d / L) by adding and subtracting 1.5 * 2^23
+// chooses another image than dist_vec where |d| is L / 2 and 1 / L is rounded up, which turns the pair's vector
+// round when a support exceeds half the box.)
 template <int D> __device__ __forceinline__ Vec<D> pair_vec(const Vec<D>& xi, const Vec<D>& xj, const DomainF& dom) {
     Vec<D> r;
     _Pragma("unroll") for (int a = 0; a < D; ++a) {
         const float d = __fsub_rn(xi.v[a], xj.v[a]);
-        const float k = __fsub_rn(__fmaf_rn(d, dom.invL[a], 12582912.f), 12582912.f);
-        r.v[a] = __fmaf_rn(-k, dom.L[a], d);
+        const float beyond = __saturatef(__fmul_rn(__fsub_rn(fabsf(d), dom.turn[a]), 8.5070592e37f));
+        r.v[a] = __fmaf_rn(-beyond, copysignf(dom.L[a], d), d);
     }
     return r;
 }

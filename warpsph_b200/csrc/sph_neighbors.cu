@@ -85,7 +85,7 @@ int params_to_dev(const SphParams* p, DevParams* o) {
         o->dom.L[a] = (float)(p->domain_max[a] - p->domain_min[a]);
         o->dom.halfL[a] = 0.5f * o->dom.L[a];
         o->dom.periodic[a] = p->periodic[a] ? 1 : 0;
-        o->dom.invL[a] = p->periodic[a] ? 1.f / o->dom.L[a] : 0.f;
+        o->dom.turn[a] = p->periodic[a] ? o->dom.halfL[a] : INFINITY;
         if (a < p->dim && !(o->dom.L[a] > 0.f)) return set_error(SPH_ERR_BAD_ARG, "domain extent along axis %d must be > 0", a);
     }
     o->verlet_scale = (float)p->verlet_scale;
