@@ -54,6 +54,17 @@ template <int D> __device__ __forceinline__ Vec<D> load_vec(const float* __restr
     }
     return r;
 }
+// The same past L1 (ld.global.cg), for arrays that other blocks rewrite inside one persistent launch.
+template <int D> __device__ __forceinline__ Vec<D> load_vec_cg(const float* p, int i) {
+    Vec<D> r;
+    if constexpr (D == 2) {
+        const float2 t = __ldcg(reinterpret_cast<const float2*>(p) + i);
+        r.v[0] = t.x; r.v[1] = t.y;
+    } else {
+        _Pragma("unroll") for (int a = 0; a < D; ++a) r.v[a] = __ldcg(p + (size_t)i * D + a);
+    }
+    return r;
+}
 template <int D> __device__ __forceinline__ void store_vec(float* __restrict__ p, size_t i, const Vec<D>& x) {
     if constexpr (D == 2) {
         reinterpret_cast<float2*>(p)[i] = make_float2(x.v[0], x.v[1]);

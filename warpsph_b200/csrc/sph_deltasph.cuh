@@ -46,21 +46,6 @@ static __global__ void k_wc_eos(int n, WcDev W, const float* __restrict__ rho, f
     if (i < n) out[i] = wc_eos(W, rho[i]);
 }
 
-// Loads of the pair passes.  CG: ld.global.cg (L2, coherent across blocks) for arrays
-// that other blocks rewrite inside one persistent launch; otherwise the read-only path.
-template <bool CG> __device__ __forceinline__ float ldf(const float* p) { return CG ? __ldcg(p) : __ldg(p); }
-template <int D, bool CG> __device__ __forceinline__ Vec<D> ldv(const float* p, int i) {
-    Vec<D> r;
-    if constexpr (D == 2) {
-        const float2 t = CG ? __ldcg(reinterpret_cast<const float2*>(p) + i) : __ldg(reinterpret_cast<const float2*>(p) + i);
-        r.v[0] = t.x; r.v[1] = t.y;
-    } else {
-        #pragma unroll
-        for (int a = 0; a < D; ++a) r.v[a] = ldf<CG>(p + (size_t)i * D + a);
-    }
-    return r;
-}
-
 // Renormalisation of pass A: L = M^-1 with M_ab = sum_j V_j gradW_a (x_j - x_i)_b; a
 // (near-)singular M (isolated particle) leaves the gradient unrenormalised.
 template <int D> __device__ __forceinline__ Vec<D> renormalise(const Mat<D>& M, const Vec<D>& g) {
@@ -93,22 +78,22 @@ template <int D> __device__ __forceinline__ Vec<D> renormalise(const Mat<D>& M, 
 }
 
 // Per-lane partial sums of pass A for particle i.
-template <int KF, int D, int G, bool CG = false>
+template <int KF, int D, int G>
 __device__ __forceinline__ void passA_partial(int i, int lane, const DevParams& P, const float* x,
                                               const float* __restrict__ H, const float* __restrict__ m,
                                               const float* rho, const int32_t* __restrict__ offs,
                                               const int32_t* __restrict__ cnt, const int32_t* __restrict__ list, Mat<D>& M,
                                               Vec<D>& g) {
-    const Vec<D> xi = ldv<D, CG>(x, i);
-    const float Hi = H[i], rhoi = ldf<CG>(rho + i);
+    const Vec<D> xi = load_vec<D>(x, i);
+    const float Hi = H[i], rhoi = __ldg(rho + i);
     const int b = offs[i], e = b + cnt[i];
     for (int q = b + lane; q < e; q += G) {
         int j, k; entry(list, q, j, k);
-        const Vec<D> xij = dist_vec<D>(xi, ldv<D, CG>(x, j), P.dom);
+        const Vec<D> xij = dist_vec<D>(xi, load_vec<D>(x, j), P.dom);
         const float r = safe_sqrt(dot<D>(xij, xij));
         float W; Vec<D> gW;
         kernelWG<KF, D>(xij, r, wmax(Hi, __ldg(H + j)), W, gW);
-        const float rj = ldf<CG>(rho + j);
+        const float rj = __ldg(rho + j);
         const float Vj = __ldg(m + j) / rj;
         const float dr = rj - rhoi;
         #pragma unroll
@@ -135,29 +120,29 @@ template <int D, int G> __device__ __forceinline__ void passA_reduce(Mat<D>& M, 
 // and continuity of the DFSPH step.  smask (nullable) is the free-surface indicator of
 // each particle; the Antuono pressure term takes P_j + P_i when P_i >= 0, P_j >= 0 or
 // particle i lies on the free surface (wp_surfaceAware.py:89-92).
-template <int KF, int D, int G, bool CG = false, bool FULL = true>
+template <int KF, int D, int G, bool FULL = true>
 __device__ __forceinline__ void passB_partial(int i, int lane, const DevParams& P, const WcDev& W, const float* x,
                                               const float* __restrict__ H, const float* __restrict__ m, const float* rho,
                                               const float* v, const float* gL, const float* Pr, const int32_t* __restrict__ smask,
                                               const int32_t* __restrict__ offs, const int32_t* __restrict__ cnt,
                                               const int32_t* __restrict__ list, float& cont, float& dd, Vec<D>& pf, Vec<D>& visc) {
-    const Vec<D> xi = ldv<D, CG>(x, i), vi = ldv<D, CG>(v, i);
-    const Vec<D> gLi = FULL ? ldv<D, CG>(gL, i) : vzero<D>();
-    const float Hi = H[i], rhoi = ldf<CG>(rho + i), Pi = FULL ? ldf<CG>(Pr + i) : 0.f;
+    const Vec<D> xi = load_vec<D>(x, i), vi = load_vec<D>(v, i);
+    const Vec<D> gLi = FULL ? load_vec<D>(gL, i) : vzero<D>();
+    const float Hi = H[i], rhoi = __ldg(rho + i), Pi = FULL ? __ldg(Pr + i) : 0.f;
     const bool surf_i = FULL && smask != nullptr && smask[i] == 1;
     const float eps = 1.0e-14f * Hi;
     const float factor = W.inviscid ? W.alpha * W.c0 * Hi / W.xi : W.visc_nu;
     const int b = offs[i], e = b + cnt[i];
     for (int q = b + lane; q < e; q += G) {
         int j, k; entry(list, q, j, k);
-        const Vec<D> xij = dist_vec<D>(xi, ldv<D, CG>(x, j), P.dom);
+        const Vec<D> xij = dist_vec<D>(xi, load_vec<D>(x, j), P.dom);
         const float r2 = dot<D>(xij, xij);
         const float r = safe_sqrt(r2);
         float Wv; Vec<D> gW;
         kernelWG<KF, D>(xij, r, wmax(Hi, __ldg(H + j)), Wv, gW);
-        const float rj = ldf<CG>(rho + j);
+        const float rj = __ldg(rho + j);
         const float Vj = __ldg(m + j) / rj;
-        const Vec<D> vj = ldv<D, CG>(v, j);
+        const Vec<D> vj = load_vec<D>(v, j);
         // continuity (inconsistent.py:19-31): V_j (v_j - v_i).gW
         float t = 0.f;
         #pragma unroll
@@ -165,7 +150,7 @@ __device__ __forceinline__ void passB_partial(int i, int lane, const DevParams& 
         cont += Vj * t;
         // density diffusion (wp_densityDelta.py:88-117)
         if constexpr (FULL) {
-            const Vec<D> gLj = ldv<D, CG>(gL, j);
+            const Vec<D> gLj = load_vec<D>(gL, j);
             const float inv = 1.f / (r + eps);
             const float s = 2.f * (rj - rhoi) * inv * inv;      // 2 (rho_j - rho_i) n_ij / (r + eps), n_ij = x_ij / (r + eps)
             float pd = 0.f;
@@ -181,7 +166,7 @@ __device__ __forceinline__ void passB_partial(int i, int lane, const DevParams& 
         }
         // pressure (wp_surfaceAware.py:48-102)
         if constexpr (FULL) {
-            const float Pj = ldf<CG>(Pr + j);
+            const float Pj = __ldg(Pr + j);
             float pij;
             switch (W.pressure_term) {
                 case SPH_PRESSURE_CONSERVATIVE: pij = Pj - Pi; break;
@@ -264,7 +249,7 @@ k_visc_cont(int n, DevParams P, WcDev W, const float* __restrict__ x, const floa
     Grp<G> g(n);
     float cont = 0.f, dd = 0.f;
     Vec<D> pf = vzero<D>(), visc = vzero<D>();
-    if (g.valid) passB_partial<KF, D, G, false, false>(g.i, g.lane, P, W, x, H, m, rho, v, nullptr, nullptr, nullptr, offs, cnt, list, cont, dd, pf,
+    if (g.valid) passB_partial<KF, D, G, false>(g.i, g.lane, P, W, x, H, m, rho, v, nullptr, nullptr, nullptr, offs, cnt, list, cont, dd, pf,
                                                        visc);
     cont = gsum<G>(cont);
     #pragma unroll

@@ -531,7 +531,7 @@ k_ens_step(const __grid_constant__ EnsArgs a) {
                     store_vec<D>(a.dv1, i, dv);
                     a.drho1[i] = dr;
                 } else {
-                    const Vec<D> v1 = get_v<D>(st, i, get_x_word<D>(st, i)), k1 = ldv<D, true>(a.dv1, i);
+                    const Vec<D> v1 = get_v<D>(st, i, get_x_word<D>(st, i)), k1 = load_vec_cg<D>(a.dv1, i);
                     const float h = 0.5f * dt;
                     Vec<D> xn, vn;
                     #pragma unroll

@@ -49,13 +49,6 @@ __device__ __forceinline__ float o2f(unsigned int o) {
     return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
 }
 
-template <int D> __device__ __forceinline__ Vec<D> load_vec_cg(const float* p, int i) {
-    Vec<D> r;
-    #pragma unroll
-    for (int a = 0; a < D; ++a) r.v[a] = __ldcg(p + (size_t)i * D + a);
-    return r;
-}
-
 // ---------------------------------------------------------------- per-lane partial sums
 // Pressure acceleration, modules/pressure/iisph.py:7-24 with the symmetric gradient
 // rho_i sum_j m_j (q_i/rho_i^2 + q_j/rho_j^2) gradW(x_ij, H_j).  p_j = praw_j - mu.
