@@ -446,11 +446,11 @@ int sph_crk_accel_dudt(const SphParams* p, int64_t n, const float* x, const floa
                        const int32_t* offs, const int32_t* cnt, const int32_t* list,
                        const int32_t* verlet_cnt, float* dvdt_out, float* dudt_out,
                        float* dEdt_out, float* ap_ij, float* av_ij, void* stream);
-/* The same pass over packed particle records: a first launch copies the fields the pass
- * reads into records [n, R] (R = sph_crk_record_floats(dim) floats per particle: 12, 24
- * and 36 in 1D, 2D and 3D; 16-byte aligned, caller-owned scratch), and the pair launch
- * gathers each neighbour as R/4 128-bit loads from that one record.  Outputs and
- * arguments otherwise as sph_crk_accel_dudt. */
+/* The same pass over packed particle records: a first launch forms what the pass reads of a
+ * particle in records (n * R floats, R = sph_crk_record_floats(dim): 12, 24 and 36 in 1D, 2D and 3D;
+ * 16-byte aligned, caller-owned scratch whose content and layout are the library's own), and the
+ * pair launch gathers each neighbour as R/4 128-bit loads from them.  Outputs and arguments
+ * otherwise as sph_crk_accel_dudt. */
 int sph_crk_record_floats(int32_t dim);
 int sph_crk_accel_dudt_packed(const SphParams* p, int64_t n, const float* x, const float* H,
                               const float* m, const float* rho, const float* V,

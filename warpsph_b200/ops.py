@@ -553,7 +553,8 @@ def crk_factors(params, x, H, m, V, adj: AdjacencyList):
 
 def crk_factors_eos(params, x, H, m, V, adj: AdjacencyList, u):
     """crk_factors with the ideal-gas EOS of the CRK density in the same pass
-    (sph_crk_factors_eos): (crk, rho, entropy, P, c)."""
+    (sph_crk_factors_eos): (crk, rho, entropy, P, c).  For callers that keep separate arrays; the
+    CRK step takes crk_rhs_fields."""
     n, d = H.shape[0], int(params.dim)
     A, B, gA, gB, rho = _empty(n, H), _empty((n, d), H), _empty((n, d), H), _empty((n, d, d), H), _empty(n, H)
     Ae, P, c = _empty(n, H), _empty(n, H), _empty(n, H)
@@ -611,8 +612,9 @@ def eos_ideal_gas(params, u, rho):
 
 
 def grad_v(params, x, H, m, rho, V, crk: CRKState, v, c, adj: AdjacencyList, cullen: bool, want_vsig: bool = False):
-    """CRK velocity gradient (+ the Cullen divergence when `cullen`).  v_sig needs the
-    Verlet set; the step computes it in the Cullen pass, tests may ask for it here."""
+    """CRK velocity gradient (+ the Cullen divergence when `cullen`) from separate arrays; the CRK
+    step takes crk_rhs_fields.  v_sig needs the Verlet set; the step computes it in the Cullen
+    pass, other callers may ask for it here."""
     n, d = H.shape[0], int(params.dim)
     G, drho = _empty((n, d, d), H), _empty(n, H)
     div = _empty(n, H) if cullen else None
