@@ -36,3 +36,19 @@ def test_scratch_sizes_are_asked_once_per_dimension(monkeypatch):
 def test_empty_keeps_shape_type_and_device(shape):
     t = ops._empty(shape, torch.zeros(2), torch.int32)
     assert tuple(t.shape) == (shape if isinstance(shape, tuple) else (shape,)) and t.dtype == torch.int32 and t.is_contiguous()
+
+
+def test_untimed_calls_share_one_context(monkeypatch):
+    monkeypatch.setattr(ops, "TIMER", None)
+    assert ops._timed("a") is ops._timed("b")
+    monkeypatch.setattr(ops, "TIMER", ops.KernelTimer(names={"a"}))
+    assert ops._timed("b") is ops._UNTIMED and ops._timed("a") is not ops._UNTIMED
+
+
+@pytest.mark.parametrize("fn,good", [(_capi.fptr, torch.float32), (_capi.iptr, torch.int32)])
+def test_pointer_checks_refuse_what_they_refused(fn, good):
+    assert fn(None) is None
+    with pytest.raises(RuntimeError, match="expected"):
+        fn(torch.zeros(4, dtype=torch.float64))
+    with pytest.raises(RuntimeError, match="CUDA"):
+        fn(torch.zeros(4, dtype=good))

@@ -256,14 +256,23 @@ def ptr(t) -> int | None:
     raise RuntimeError("warpsph_b200 requires contiguous tensors")
 
 
-def fptr(t) -> int | None:
-    if t is not None and t.dtype != torch.float32:
+def fptr(t, _dtype=torch.float32) -> int | None:
+    # the usual tensor first, in one expression: a step makes some 250 of these calls
+    if t is None:
+        return None
+    if t.dtype is _dtype and t.is_cuda and t.is_contiguous():
+        return t.data_ptr()
+    if t.dtype != torch.float32:
         raise RuntimeError(f"expected float32 tensor, got {t.dtype}")
     return ptr(t)
 
 
-def iptr(t) -> int | None:
-    if t is not None and t.dtype != torch.int32:
+def iptr(t, _dtype=torch.int32) -> int | None:
+    if t is None:
+        return None
+    if t.dtype is _dtype and t.is_cuda and t.is_contiguous():
+        return t.data_ptr()
+    if t.dtype != torch.int32:
         raise RuntimeError(f"expected int32 tensor, got {t.dtype}")
     return ptr(t)
 

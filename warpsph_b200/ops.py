@@ -43,23 +43,27 @@ class KernelTimer:
 TIMER: Optional[KernelTimer] = None
 
 
-class _timed:
+class _Timed:
     def __init__(self, name: str):
         self.name = name
 
     def __enter__(self):
-        t = TIMER
-        self.ev = None
-        if t is not None and t.wants(self.name):
-            self.ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
-            self.ev[0].record()
+        self.ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
+        self.ev[0].record()
         return self
 
     def __exit__(self, *exc):
-        if self.ev is not None:
-            self.ev[1].record()
-            TIMER.events.append((self.name, self.ev[0], self.ev[1]))
+        self.ev[1].record()
+        TIMER.events.append((self.name, self.ev[0], self.ev[1]))
         return False
+
+
+_UNTIMED = contextlib.nullcontext()
+
+
+def _timed(name: str):
+    """Times the block when TIMER wants `name`; otherwise one shared context that does nothing."""
+    return _UNTIMED if TIMER is None or not TIMER.wants(name) else _Timed(name)
 
 
 _SUPPORT = {SupportScheme.Gather: 0, SupportScheme.Scatter: 1, SupportScheme.Symmetric: 2,
