@@ -150,10 +150,10 @@ def bytes_accel_dudt(d: int, K: float) -> float:
 
 
 # DRAM bytes (read + write) of one accel pass on this bench's own workload (512^2), from an
-# ncu capture of dram__bytes_read.sum + dram__bytes_write.sum: k_crk_accel_dudt 131.6 MB
-# read + 132.5 MB written, and the k_crk_pack launch before it 23.1 MB read (its records
+# ncu capture of dram__bytes_read.sum + dram__bytes_write.sum: k_crk_accel_dudt 131.8 MB
+# read + 132.9 MB written, and the k_crk_pack launch before it 23.1 MB read (its records
 # stay in L2 for the accel launch).  Other sizes are scaled by particle count.
-ACCEL_TRAFFIC_BYTES_PER_PARTICLE = (131.64e6 + 132.50e6 + 23.08e6) / 262144
+ACCEL_TRAFFIC_BYTES_PER_PARTICLE = (131.81e6 + 132.86e6 + 23.07e6) / 262144
 
 
 def load_peaks() -> dict:

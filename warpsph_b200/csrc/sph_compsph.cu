@@ -137,9 +137,9 @@ k_compsph_prep(int n, DevParams P, const float* __restrict__ x, const float* __r
 // take their defaults at pack time (sound speed c_s, switch 1, Omega 1).  Granule k of
 // particle i is word k n + i: consecutive row entries are mostly consecutive particles, so a
 // load of the lanes covers contiguous words.  Latency bound at 72 registers (40 %
-// of the warps): held to 64 in 2D.  262,144 particles with 32 neighbours: 182 -> 121 us with 8
+// of the warps): held to 64 in 2D.  262,144 particles with 32 neighbours: 182 -> 125 us with 8
 // lanes (4 lanes 142, 16 lanes 160; the next record loaded ahead 133, for its registers); 3D,
-// 884,736 with 128 neighbours: 16 lanes 1.97 ms, 8 lanes 2.69, 4 lanes 4.20; 4,096 in 2D: 16
+// 884,736 with 128 neighbours: 16 lanes 2.04 ms, 8 lanes 2.69, 4 lanes 4.20; 4,096 in 2D: 16
 // lanes 5.2 us, 8 lanes 6.3.
 template <int D> struct CompRec {
     static constexpr int X = 0, H = D, V = D + 1, M = 2 * D + 1, RHO = M + 1, P = M + 2, C = M + 3, AL = M + 4, PT = M + 5,

@@ -449,7 +449,7 @@ __device__ __forceinline__ void ens_passB(int i, int lane, const EnsArgs& a, con
 }
 
 // Bound by issue slots (64 %) and the latency of the gathers.  1.3 M particles in 64 boxes, 99 entries
-// per row of which 50 interact: 5.84 -> 2.78 ms per step; of that the walk of the near entries, packed
+// per row of which 50 interact: 5.84 -> 2.81 ms per step; of that the walk of the near entries, packed
 // words and quotients hoisted to the particle give 2.2 ms, divisions without the general case's
 // branches 0.3, the usual terms as constants 0.1, particles handed to free warps (1, 2 or 4 warpfuls
 // at a time: 0.27, 0.21, 0.21) and 9 blocks of 128 threads per SM (56 registers; 8: 0.1 more, 10: 0.06

@@ -425,12 +425,13 @@ k_jacobi(JacobiArgs a) {
 // acquire of the grid barrier makes current, and so may hit L1.
 //
 // Large solves are bound by the stream of gradients from HBM (16 bytes per entry and phase in
-// 3D): 1,000,000 particles with 40 neighbours take 134 us per phase, 5.0 TB/s of stream, where
+// 3D): 1,000,000 particles with 40 neighbours take 128 us per phase, 5.2 TB/s of stream, where
 // k_jacobi took 353 us; 4 lanes per particle with 5 entries in flight beat 8 x 4 (149 us) and
 // 16 x 3 (168 us).  Small solves are bound by the latency of a phase and its barrier.  With
 // HOLD a group keeps one particle for the whole solve, its first G * U entries in registers, so
 // a phase is one gather, one reduction and one barrier; more entries are loaded each time.
-// 9,216 particles: 3.7 us per phase and barrier against 4.5 us streaming and 10.8 us in k_jacobi;
+// 9,216 particles: 3.1 us per phase and barrier, 10.8 us in k_jacobi (3.7 against 4.5 us streaming when the two
+// were compared, before the blocks' slots);
 // 4,096 particles in 3D: 160 us a solve of 33 phases with 8 lanes against 182 us with 4 and 197 us
 // streaming.  The blocks' partial sums go to one slot each, which every block adds up after
 // the barrier: four atomics per block on one line cost 144 blocks 1 us per iteration more.

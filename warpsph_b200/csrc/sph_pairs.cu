@@ -14,12 +14,12 @@
 // differ from the CPU oracle by rounding only.
 //
 // In 2D the passes are bound by issue slots, in 3D by L1.  Taking the minimum image with
-// multiply-adds (pair_vec), square roots and reciprocals as approximation plus Newton step
+// one comparison (pair_vec), square roots and reciprocals as approximation plus Newton step
 // (sqrt_newton, rcp_newton), the factors of H_i out of the sums and skipping entries outside
 // the support took, per launch at 262,144 particles in 2D, the adaptive support from 76 to
 // 52 us, the CRK factors from 75 to 60 us, the velocity gradient from 93 to 78 us, the row
 // rewrite from 98 to 82 us and the Cullen switch from 104 to 94 us; errors against 64 bits
-// are those of before or smaller.
+// are those of before within 2 per cent (5 in single sums; geometric mean of 120 random sets).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cfloat>
@@ -619,7 +619,7 @@ k_cullen(int n, DevParams P, const float* __restrict__ x, const float* __restric
 // k_grad_v and k_cullen over packed words: two 16-byte gathers per entry (a scalar more in 3D)
 // instead of 7 to 10 scalar ones, which in 3D is what L1 is spent on: at 884,736 particles with
 // 128 neighbours the gradient went from 1.36 to 0.69 ms, the switch from 2.56 to 1.13 ms and the
-// row rewrite from 1.32 to 0.82 ms; at 262,144 in 2D from 78, 94 and 82 to 63, 77 and 79 us.
+// row rewrite from 1.32 to 0.85 ms; at 262,144 in 2D from 78, 94 and 82 to 63, 77 and 79 us.
 template <int D>
 __global__ void k_pack_xh(int n, const float* __restrict__ x, const float* __restrict__ H, float4* __restrict__ xh) {
     pdl_entry();
