@@ -256,7 +256,7 @@ int sph_neighbors_rewrite(const SphParams* p, int64_t n, const float* x, const f
                           float* V_out, int32_t* status, void* stream);
 
 /* The two rewrites above with their gathers from packed words (sph_pack_xh of the same x and
- * H; null: from x and H). */
+ * H, 16-byte aligned; null: from x and H). */
 int sph_neighbors_refresh_volume_packed(const SphParams* p, int64_t n, const float* x, const float* H,
                                         const float* xh, const float* x0, const float* H0,
                                         const int32_t* neighbor_offsets, const int32_t* num_neighbors,

@@ -138,3 +138,13 @@ def test_python_call_sites_pass_every_argument():
                 assert n == len(protos[node.func.attr]), f"{path.name}:{node.lineno} {node.func.attr}: {n} != {len(protos[node.func.attr])}"
                 checked += 1
     assert checked > 30
+
+
+def test_packed_rewrites_refuse_misaligned_words():
+    """Their 16-byte loads would fault: refused on the host, before anything is enqueued."""
+    p = _params()
+    pp, lib, d = C.byref(p), _capi.lib(), 256      # d: never dereferenced
+    rc = lib.sph_neighbors_refresh_volume_packed(pp, 10, d, d, d + 8, d, d, d, d, d, 2 * d, d, d, d, d, d, None)
+    assert rc == -1 and "16-byte" in _capi.last_error()
+    rc = lib.sph_neighbors_rewrite_packed(pp, 10, d, d, d + 4, d, d, d, 2 * d, d, d, d, d, d, d, None)
+    assert rc == -1 and "16-byte" in _capi.last_error()

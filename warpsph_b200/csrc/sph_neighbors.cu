@@ -1463,6 +1463,7 @@ int sph_neighbors_refresh_volume_packed(const SphParams* p, int64_t n, const flo
     int rc = params_to_dev(p, &P);
     if (rc) return rc;
     if (n < 0 || n > 0x7fffffff) return set_error(SPH_ERR_BAD_ARG, "sph_neighbors_refresh_volume: n out of range");
+    if (reinterpret_cast<uintptr_t>(xh) & 15) return set_error(SPH_ERR_BAD_ARG, "sph_neighbors_refresh_volume_packed: xh must be 16-byte aligned");
     WSPH_CHECK_PTR(scratch); WSPH_CHECK_PTR(status); WSPH_CHECK_PTR(inter_nnz_out);
     cudaStream_t s = WSPH_STREAM(stream);
     cudaMemsetAsync(inter_nnz_out, 0, sizeof(int64_t), s);
@@ -1550,6 +1551,7 @@ int sph_neighbors_rewrite_packed(const SphParams* p, int64_t n, const float* x, 
     int rc = params_to_dev(p, &P);
     if (rc) return rc;
     if (n < 0 || n > 0x7fffffff) return set_error(SPH_ERR_BAD_ARG, "sph_neighbors_rewrite: n out of range");
+    if (reinterpret_cast<uintptr_t>(xh) & 15) return set_error(SPH_ERR_BAD_ARG, "sph_neighbors_rewrite_packed: xh must be 16-byte aligned");
     WSPH_CHECK_PTR(inter_nnz_out); WSPH_CHECK_PTR(status);
     cudaStream_t s = WSPH_STREAM(stream);
     cudaMemsetAsync(inter_nnz_out, 0, sizeof(int64_t), s);
